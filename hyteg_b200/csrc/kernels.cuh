@@ -1147,13 +1147,11 @@ __device__ __forceinline__ T p2GatherNode(const P2Tables& tb, const T* Kc, const
   return s;
 }
 
-// colour, sel: when sel >= 0 only nodes whose colour (low 7 bits of the per-slot colour byte)
-// is sel are computed (one pass of the multicolour SOR); bit 7 of the byte marks owned slots.
+// The diagonal of the operator (MODE_DIAG) on every node of the closed macro-cells.
 template <class T, int MODE>
 __global__ void __launch_bounds__(kBlock) p2CellKernel(LevelDev lv, P2Tables tb, const T* __restrict__ K,
                                                        T* __restrict__ dst, const T* __restrict__ src,
-                                                       const T* __restrict__ rhs, unsigned mask,
-                                                       const unsigned char* __restrict__ colour, int sel) {
+                                                       const T* __restrict__ rhs, unsigned mask) {
   const int M = lv.N, N = M / 2, nPl = M + 1, w = lv.w;
   const int c = blockIdx.x / nPl, Z = blockIdx.x % nPl;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -1172,7 +1170,6 @@ __global__ void __launch_bounds__(kBlock) p2CellKernel(LevelDev lv, P2Tables tb,
     const int r0 = pb + rowStart(w - Z, Y);
     for (int X = lane; X <= M - Z - Y; X += 32) {
       const int64_t i = base + r0 + X;
-      if (sel >= 0 && (colour[i] & 0x7f) != sel) continue;
       const T s = p2GatherNode<T, MODE == MODE_DIAG>(tb, Kc, src + base, pbz, w, N, X, Y, Z);
       const bool interior = X >= 1 && Y >= 1 && Z >= 1 && X + Y + Z <= M - 1;
       if (!interior) dst[i] = s;
@@ -1207,10 +1204,9 @@ __device__ __forceinline__ T p2StencilDot(p2s::List<p2s::O<DX, DY, DZ>...>, std:
   return (s[0] + s[1]) + (s[2] + s[3]);
 }
 
-// One row (Y, Z) of class PC: MODE_REPLACE dst = A src, MODE_RESIDUAL dst = rhs - A src,
-// MODE_SOR dst (== src) += omega (rhs - A dst) / a_ii. With sel >= 0 only the nodes of colour sel
-// are computed: the vertex class is split into four colours, read from the colour bytes; a whole
-// edge class is one colour in a cell's frame.
+// One row (Y, Z) of class PC, only the nodes of colour sel: MODE_REPLACE dst = A src, MODE_SOR
+// dst (== src) += omega (rhs - A dst) / a_ii. The vertex class is split into four colours, read from
+// the colour bytes; a whole edge class is one colour in a cell's frame.
 template <class T, int MODE, int PC>
 __device__ __forceinline__ void p2StencilRow(const T* wts, T* dst, const T* src, const T* rhs, int64_t base,
                                              const int (&pbz)[5], int w, int M, int Y, int Z, int lane,
@@ -1220,7 +1216,7 @@ __device__ __forceinline__ void p2StencilRow(const T* wts, T* dst, const T* src,
   const T* wt = wts + kFirst;
   const int r0 = pbz[2] + rowStart(w - Z, Y);
   int X0 = ((PC & 1) ? 1 : 2) + 2 * lane, dX = 64;
-  if (PC == 0 && sel >= 0) {
+  if (PC == 0) {
     // vertex colour sel along the row: the colour of the vertex node 2 + 2t is c(2) + vstep t mod 4,
     // so the lanes take every fourth (vstep odd) or every second (vstep 2) vertex node from the first
     if (M - 1 - Y - Z < 2) return;
@@ -1240,12 +1236,10 @@ __device__ __forceinline__ void p2StencilRow(const T* wts, T* dst, const T* src,
 #pragma unroll 1
   for (int X = X0; X <= M - 1 - Y - Z; X += dX) {
     const int64_t i = base + r0 + X;
-    if (PC == 0 && sel >= 0 && (colour[i] & 0x7f) != sel) continue;
+    if (PC == 0 && (colour[i] & 0x7f) != sel) continue;
     const T s = p2StencilDot<T>(S{}, std::make_integer_sequence<int, kLen>{}, src + base, wt, pbz, w, X, Y, Z);
     if (MODE == MODE_REPLACE)
       dst[i] = s;
-    else if (MODE == MODE_RESIDUAL)
-      dst[i] = rhs[i] - s;
     else
       dst[i] += omega * (rhs[i] - s) / wt[kCentre];
   }
@@ -1269,12 +1263,11 @@ __device__ __forceinline__ void p2StencilRowAny(int pc, const T* wts, T* dst, co
 }
 
 // Grid: nCells * (M - 3) blocks, block b on cell b / (M - 3), plane Z = 1 + b % (M - 3) (the
-// planes holding interior nodes; needs M >= 4). Only cells of a flagged DoF type are written.
-// sel >= 0 (one colour pass of the SOR, MODE_SOR or MODE_REPLACE): classOfColour[cell * 12 + sel]
-// is the class of colour sel in the cell's frame (0 for the four vertex colours, -1 when no
-// interior node has the colour), classOfColour[cell * 12 + 11] the change of the vertex colour
-// from one vertex node of a row to the next (1, 2 or 3). MODE_SOR updates in place: dst == src,
-// rhs = b.
+// planes holding interior nodes; needs M >= 4). Only cells of a flagged DoF type are written. One
+// colour pass of the SOR (MODE_SOR or MODE_REPLACE): classOfColour[cell * 12 + sel] is the class
+// of colour sel in the cell's frame (0 for the four vertex colours, -1 when no interior node has
+// the colour), classOfColour[cell * 12 + 11] the change of the vertex colour from one vertex node
+// of a row to the next (1, 2 or 3). MODE_SOR updates in place: dst == src, rhs = b.
 template <class T, int MODE>
 __global__ void __launch_bounds__(kBlock, 2) p2StencilKernel(LevelDev lv, const T* __restrict__ W, T* dst, const T* src,
                                                           const T* __restrict__ rhs, unsigned mask,
@@ -1284,12 +1277,8 @@ __global__ void __launch_bounds__(kBlock, 2) p2StencilKernel(LevelDev lv, const 
   const int M = lv.N, w = lv.w, nPl = M - 3;
   const int c = blockIdx.x / nPl, Z = 1 + blockIdx.x % nPl;
   if (!(lv.cellType[c] & mask)) return;
-  int pcSel = 0, vstep = 1;
-  if (sel >= 0) {
-    pcSel = classOfColour[c * 12 + sel];
-    vstep = classOfColour[c * 12 + 11];
-    if (pcSel < 0 || ((pcSel >> 2) & 1) != (Z & 1)) return;
-  }
+  const int pcSel = classOfColour[c * 12 + sel], vstep = classOfColour[c * 12 + 11];
+  if (pcSel < 0 || ((pcSel >> 2) & 1) != (Z & 1)) return;
   __shared__ T wts[p2s::kTotal];
   for (int k = threadIdx.x; k < p2s::kTotal; k += blockDim.x) wts[k] = W[(int64_t)c * p2s::kTotal + k];
   __syncthreads();
@@ -1301,32 +1290,14 @@ __global__ void __launch_bounds__(kBlock, 2) p2StencilKernel(LevelDev lv, const 
   }
   const int64_t base = lv.cellOff[c];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (sel >= 0) {
 #pragma unroll 1
-    for (int Y = (((pcSel >> 1) & 1) ? 1 : 2) + 2 * warp; Y <= M - 2 - Z; Y += 2 * (kBlock / 32))
-      p2StencilRowAny<T, MODE>(pcSel, wts, dst, src, rhs, base, pbz, w, M, Y, Z, lane, colour, sel, omega, vstep);
-  } else {
-#pragma unroll 1
-    for (int Y = 1 + warp; Y <= M - 2 - Z; Y += kBlock / 32) {
-#pragma unroll 1
-      for (int px = 0; px < 2; ++px)
-        p2StencilRowAny<T, MODE>(px | ((Y & 1) << 1) | ((Z & 1) << 2), wts, dst, src, rhs, base, pbz, w, M, Y, Z, lane,
-                                 colour, sel, omega, vstep);
-    }
-  }
+  for (int Y = (((pcSel >> 1) & 1) ? 1 : 2) + 2 * warp; Y <= M - 2 - Z; Y += 2 * (kBlock / 32))
+    p2StencilRowAny<T, MODE>(pcSel, wts, dst, src, rhs, base, pbz, w, M, Y, Z, lane, colour, sel, omega, vstep);
 }
 
-// The closure nodes of every macro-cell (its faces, edges and vertices): this cell's share of
-// row j of A, written into the cell's closure slot (p2AddKernel sums the shares into the owner).
-// A node inside one face of the cell sees the same micro-cells at every node of its (face, class):
-// its share is a constant stencil (p2s::FaceList, weights FW[cell][p2s::kFaceTotal]). Nodes on the
-// cell's edges and vertices take the element gather. Grid: nCells * (M + p2FaceChunks(M)) blocks.
-// Per cell, M blocks take the planes Z = 1 .. M: on each, warps 0-5 walk the lines of faces
-// Y = 0, X = 0 and X + Y + Z = M (one warp per line and parity, so a warp runs one class), warp 6
-// the three edge nodes of the plane. p2FaceChunks(M) blocks take the face Z = 0 in chunks of eight
-// rows (a warp per row).
-__host__ __device__ __forceinline__ int p2FaceChunks(int M) { return (M + 1 + 7) / 8; }
-
+// A node inside one face of a macro-cell sees the same micro-cells of that cell at every node of
+// its (face, class): the cell's share of its row is a constant stencil (p2s::FaceList, weights
+// FW[cell][p2s::kFaceTotal]). Nodes on the cell's edges and vertices take the element gather.
 template <class T, int K>
 __device__ __forceinline__ T p2FaceDot(const T* u, const T* fw, const int (&pbz)[5], int w, int X, int Y, int Z) {
   using S = typename p2s::FaceList<K>::type;
@@ -1357,84 +1328,7 @@ __device__ __forceinline__ T p2FaceDotAny(int k, const T* u, const T* fw, const 
   }
 }
 
-// Entry of (face f, class pc) in the face tables; the classes of a face are listed ascending:
-// Z = 0: {0, 1, 2, 3}; Y = 0: {0, 1, 4, 5}; X = 0: {0, 2, 4, 6}; X + Y + Z = M: {0, 3, 5, 6}.
-__device__ __forceinline__ int p2FaceEntry(int f, int pc) {
-  switch (f) {
-    case 0: return pc;
-    case 1: return 4 + ((pc & 1) | ((pc >> 1) & 2));
-    case 2: return 8 + (((pc >> 1) & 1) | ((pc >> 1) & 2));
-    default: return 12 + (pc == 0 ? 0 : pc == 3 ? 1 : pc == 5 ? 2 : 3);
-  }
-}
-
-template <class T>
-__global__ void __launch_bounds__(kBlock) p2ClosureKernel(LevelDev lv, P2Tables tb, const T* __restrict__ K,
-                                                          const T* __restrict__ FW, T* __restrict__ dst,
-                                                          const T* __restrict__ src,
-                                                          const unsigned char* __restrict__ colour, int sel) {
-  const int M = lv.N, N = M / 2, w = lv.w, perCell = M + p2FaceChunks(M);
-  const int c = blockIdx.x / perCell, q = blockIdx.x % perCell;
-  const int Z = q < M ? q + 1 : 0;
-  const int64_t base = lv.cellOff[c];
-  const T* Kc = K + (int64_t)c * 600;
-  __shared__ T fw[p2s::kFaceTotal];
-  for (int k = threadIdx.x; k < p2s::kFaceTotal; k += blockDim.x) fw[k] = FW[(int64_t)c * p2s::kFaceTotal + k];
-  __syncthreads();
-  int pbz[5];
-#pragma unroll
-  for (int d = 0; d < 5; ++d) {
-    const int z = Z - 2 + d;
-    pbz[d] = (z >= 0 && z <= M) ? int(tetSize(w) - tetSize(w - z)) : 0;
-  }
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  auto gatherNode = [&](int X, int Y) {
-    const int64_t i = base + pbz[2] + rowStart(w - Z, Y) + X;
-    if (sel < 0 || (colour[i] & 0x7f) == sel) dst[i] = p2GatherNode<T, false>(tb, Kc, src + base, pbz, w, N, X, Y, Z);
-  };
-  auto faceNode = [&](int k, int X, int Y) {
-    const int64_t i = base + pbz[2] + rowStart(w - Z, Y) + X;
-    if (sel < 0 || (colour[i] & 0x7f) == sel) dst[i] = p2FaceDotAny<T>(k, src + base, fw, pbz, w, X, Y, Z);
-  };
-  const int n = M - Z;
-  if (Z == 0) {
-    const int Y = (q - M) * 8 + warp;
-    if (Y > n) return;
-    if (Y == 0) {
-      for (int X = lane; X <= n; X += 32) gatherNode(X, 0);
-      return;
-    }
-    if (lane == 0) gatherNode(0, Y);
-    if (lane == 1 && n - Y > 0) gatherNode(n - Y, Y);
-#pragma unroll 1
-    for (int px = 0; px < 2; ++px) {
-      const int k = p2FaceEntry(0, px | ((Y & 1) << 1));
-      for (int X = (px ? 1 : 2) + 2 * lane; X <= n - 1 - Y; X += 64) faceNode(k, X, Y);
-    }
-  } else if (n == 0) {
-    if (threadIdx.x == 0) gatherNode(0, 0);
-  } else if (warp < 6) {
-    const int line = warp >> 1, par = warp & 1, zb = (Z & 1) << 2;
-    for (int t = (par ? 1 : 2) + 2 * lane; t <= n - 1; t += 64) {
-      if (line == 0)  // face Y = 0: X = t
-        faceNode(p2FaceEntry(1, par | zb), t, 0);
-      else if (line == 1)  // face X = 0: Y = t
-        faceNode(p2FaceEntry(2, (par << 1) | zb), 0, t);
-      else  // face X + Y + Z = M: Y = t, X = n - t
-        faceNode(p2FaceEntry(3, ((n - t) & 1) | (par << 1) | zb), n - t, t);
-    }
-  } else if (warp == 6 && lane < 3) {
-    if (lane == 0)
-      gatherNode(0, 0);
-    else if (lane == 1)
-      gatherNode(n, 0);
-    else
-      gatherNode(0, n);
-  }
-}
-
-// The closure nodes of one SOR colour from a per-colour list (one thread per node): the same
-// shares as p2ClosureKernel, without visiting the nodes of the other colours. k = face-stencil
+// The closure nodes of one SOR colour from a per-colour list (one thread per node). k = face-stencil
 // entry of a face-interior node, -1 for a node on a cell edge or vertex (element gather).
 struct P2ClosureNode {
   int cell;
@@ -1829,11 +1723,9 @@ template <class T, int MODE>
 __global__ void __launch_bounds__(kBlock) p2AddKernel(const int64_t* __restrict__ owner, const int* __restrict__ ptr,
                                                       const int64_t* __restrict__ copies,
                                                       const unsigned char* __restrict__ type, int n, T* dst,
-                                                      const T* __restrict__ rhs, unsigned mask,
-                                                      const unsigned char* __restrict__ colour, int sel) {
+                                                      const T* __restrict__ rhs, unsigned mask) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n || !(type[i] & mask)) return;
-  if (sel >= 0 && (colour[owner[i]] & 0x7f) != sel) return;
   T v = T(0);
   for (int k = ptr[i]; k < ptr[i + 1]; ++k) v += dst[copies[k]];
   const int64_t o = owner[i];

@@ -14,6 +14,7 @@
 #include "../../include/hyteg_b200.h"
 #include "discretization.hpp"
 #include "kernels.cuh"
+#include "p2_apply.cuh"
 #include "solvers.hpp"
 #include "storage.hpp"
 
@@ -65,6 +66,11 @@ static unsigned char dofType(int meshFlag) {
   }
 }
 
+template <class F>
+static void allowSmem(F kernel, size_t bytes) {
+  cudaCheck(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes), "kernel shared memory");
+}
+
 Storage::Storage(const Topology& topo, int maxLevel) : disc(topo, maxLevel) {
   cudaCheck(cudaGetDevice(&device), "cudaGetDevice");
   cudaCheck(cudaStreamCreateWithFlags(&ownStream, cudaStreamNonBlocking), "cudaStreamCreate");
@@ -80,6 +86,10 @@ Storage::Storage(const Topology& topo, int maxLevel) : disc(topo, maxLevel) {
   cudaCheck(cudaFuncSetAttribute(dev::cellSorWaveKernel<float, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)dev::waveSmemBytes<float, 1>(dev::kWaveMaxN)),
             "wave kernel shared memory");
+  allowSmem(dev::p2ApplyKernel<double, dev::MODE_REPLACE>, dev::p2TileSmem<double>());
+  allowSmem(dev::p2ApplyKernel<double, dev::MODE_RESIDUAL>, dev::p2TileSmem<double>());
+  allowSmem(dev::p2ApplyKernel<float, dev::MODE_REPLACE>, dev::p2TileSmem<float>());
+  allowSmem(dev::p2ApplyKernel<float, dev::MODE_RESIDUAL>, dev::p2TileSmem<float>());
   stream = ownStream;
   levels.resize(maxLevel + 1);
   for (int L = 0; L <= maxLevel; ++L) buildLevel(L);
@@ -947,6 +957,19 @@ static dev::P2Tables p2Tables() {
   return tb;
 }
 
+// The work list of p2ApplyKernel for one lattice level of size M, the same for every macro-cell.
+static std::vector<dev::P2Item> p2Items(int M) {
+  std::vector<dev::P2Item> items;
+  for (int e = 0; e < 6 * (M - 1) + 4; e += dev::kBlock) items.push_back({dev::P2_EDGES, e, 0, 0});
+  for (int z = 0; z + 3 <= M - 1; z += dev::kP2Tile)
+    for (int y = 0; y + z + 3 <= M - 1; y += dev::kP2Tile)
+      for (int x = 0; x + y + z + 3 <= M - 1; x += dev::kP2Tile) items.push_back({dev::P2_TILE, x, y, z});
+  for (int f = 0; f < 4; ++f)
+    for (int t = 0; t + 2 <= M - 1; t += dev::kP2FaceTile)
+      for (int s = 0; s + t + 2 <= M - 1; s += dev::kP2FaceTile) items.push_back({dev::P2_FACE, f, s, t});
+  return items;
+}
+
 P2Additive& Storage::p2Additive(int Lf) {
   if ((int)p2add.size() <= Lf) p2add.resize(maxLevel() + 1);
   P2Additive& ad = p2add[Lf];
@@ -1130,6 +1153,11 @@ P2Additive& Storage::p2Additive(int Lf) {
     for (int k = ptr[i]; k < ptr[i + 1]; ++k) mult[(size_t)cp[k]] = (unsigned char)(ptr[i + 1] - ptr[i]);
   ad.mult.alloc(mult.size());
   cudaCheck(cudaMemcpyAsync(ad.mult.p, mult.data(), mult.size(), cudaMemcpyHostToDevice, stream), "p2 mult");
+  const std::vector<dev::P2Item> items = p2Items(ld.lv.N);
+  ad.nItems = (int)items.size();
+  ad.items.alloc(items.size() * sizeof(dev::P2Item));
+  cudaCheck(cudaMemcpyAsync(ad.items.p, items.data(), items.size() * sizeof(dev::P2Item), cudaMemcpyHostToDevice, stream),
+            "p2 items");
   cudaCheck(cudaStreamSynchronize(stream), "p2 add");
   ad.built = true;
   return ad;
@@ -1189,37 +1217,29 @@ static std::vector<double> p2FaceStencils(const std::vector<double>& K, int nCel
   return S;
 }
 
-// Cell gather + additive owner sums for one P2 level: dst = A src, rhs - A src or diag(A), on the
-// flagged DoFs of colour `sel` (all when sel < 0). The copies of dst are not refreshed here.
+// Cell sweep + additive owner sums for one P2 level: dst = A src, rhs - A src or diag(A) on the
+// flagged DoFs. The copies of dst are not refreshed here.
 template <class T, int MODE>
-void Storage::p2Launch(P2Operator& o, int L, T* dst, const T* src, const T* rhs, unsigned mask, int sel) {
+void Storage::p2Launch(P2Operator& o, int L, T* dst, const T* src, const T* rhs, unsigned mask) {
   const int Lf = L + 1;
   const LevelData& ld = levels[Lf];
   P2Additive& ad = p2Additive(Lf);
   const T* K = (const T*)(sizeof(T) == 8 ? o.kd[L - o.minL]->p : o.kf[L - o.minL]->p);
-  const int nb = ld.lv.nCells * (ld.lv.N + 1);
-  const unsigned char* col = (const unsigned char*)ad.colour.p;
   if constexpr (MODE == dev::MODE_DIAG) {
-    dev::p2CellKernel<T, MODE><<<nb, dev::kBlock, 0, stream>>>(ld.lv, p2TablesOnce(), K, dst, src, rhs, mask, col, sel);
-    ++launches;
+    const int nb = ld.lv.nCells * (ld.lv.N + 1);
+    dev::p2CellKernel<T, MODE><<<nb, dev::kBlock, 0, stream>>>(ld.lv, p2TablesOnce(), K, dst, src, rhs, mask);
   } else {
-    // interior nodes by their constant stencils, closure nodes by the element gather
-    if (ld.lv.N >= 4) {
-      const T* W = (const T*)(sizeof(T) == 8 ? o.sd[L - o.minL]->p : o.sf[L - o.minL]->p);
-      dev::p2StencilKernel<T, MODE><<<ld.lv.nCells * (ld.lv.N - 3), dev::kBlock, 0, stream>>>(
-          ld.lv, W, dst, src, rhs, mask, col, (const signed char*)ad.classOfColour.p, sel, T(0));
-      ++launches;
-    }
+    const T* W = (const T*)(sizeof(T) == 8 ? o.sd[L - o.minL]->p : o.sf[L - o.minL]->p);
     const T* FW = (const T*)(sizeof(T) == 8 ? o.fd[L - o.minL]->p : o.ff[L - o.minL]->p);
-    dev::p2ClosureKernel<T><<<ld.lv.nCells * (ld.lv.N + dev::p2FaceChunks(ld.lv.N)), dev::kBlock, 0, stream>>>(
-        ld.lv, p2TablesOnce(), K, FW, dst, src, col, sel);
-    ++launches;
+    dev::p2ApplyKernel<T, MODE><<<ld.lv.nCells * ad.nItems, dev::kBlock, dev::p2TileSmem<T>(), stream>>>(
+        ld.lv, p2TablesOnce(), (const dev::P2Item*)ad.items.p, W, FW, K, dst, src, rhs, mask);
   }
+  ++launches;
   if (ad.n) {
     constexpr int AM = MODE == dev::MODE_RESIDUAL ? dev::MODE_RESIDUAL : dev::MODE_REPLACE;
     dev::p2AddKernel<T, AM><<<(ad.n + dev::kBlock - 1) / dev::kBlock, dev::kBlock, 0, stream>>>(
         (const int64_t*)ad.owner.p, (const int*)ad.ptr.p, (const int64_t*)ad.copies.p, (const unsigned char*)ad.type.p,
-        ad.n, dst, rhs, mask, col, sel);
+        ad.n, dst, rhs, mask);
     ++launches;
   }
   cudaCheck(cudaGetLastError(), "P2 kernels");
@@ -1242,15 +1262,15 @@ void Storage::p2Apply(int opId, int src, int dst, int rhs, int L, unsigned mask,
   if (fs.prec == 8) {
     const double* r = mode ? (const double*)data(rhs, Lf) : nullptr;
     if (mode == 0)
-      p2Launch<double, dev::MODE_REPLACE>(o, L, (double*)data(dst, Lf), (const double*)data(src, Lf), r, mask, -1);
+      p2Launch<double, dev::MODE_REPLACE>(o, L, (double*)data(dst, Lf), (const double*)data(src, Lf), r, mask);
     else
-      p2Launch<double, dev::MODE_RESIDUAL>(o, L, (double*)data(dst, Lf), (const double*)data(src, Lf), r, mask, -1);
+      p2Launch<double, dev::MODE_RESIDUAL>(o, L, (double*)data(dst, Lf), (const double*)data(src, Lf), r, mask);
   } else {
     const float* r = mode ? (const float*)data(rhs, Lf) : nullptr;
     if (mode == 0)
-      p2Launch<float, dev::MODE_REPLACE>(o, L, (float*)data(dst, Lf), (const float*)data(src, Lf), r, mask, -1);
+      p2Launch<float, dev::MODE_REPLACE>(o, L, (float*)data(dst, Lf), (const float*)data(src, Lf), r, mask);
     else
-      p2Launch<float, dev::MODE_RESIDUAL>(o, L, (float*)data(dst, Lf), (const float*)data(src, Lf), r, mask, -1);
+      p2Launch<float, dev::MODE_RESIDUAL>(o, L, (float*)data(dst, Lf), (const float*)data(src, Lf), r, mask);
   }
   communicate(dst, Lf, kAllGroups);
 }
@@ -1264,9 +1284,9 @@ int Storage::p2Diagonal(int opId, int L, int prec) {
   const int Lf = L + 1;
   const int d = createFunction(Lf, Lf, prec);
   if (prec == 8)
-    p2Launch<double, dev::MODE_DIAG>(o, L, (double*)data(d, Lf), nullptr, nullptr, HG_ALL, -1);
+    p2Launch<double, dev::MODE_DIAG>(o, L, (double*)data(d, Lf), nullptr, nullptr, HG_ALL);
   else
-    p2Launch<float, dev::MODE_DIAG>(o, L, (float*)data(d, Lf), nullptr, nullptr, HG_ALL, -1);
+    p2Launch<float, dev::MODE_DIAG>(o, L, (float*)data(d, Lf), nullptr, nullptr, HG_ALL);
   communicate(d, Lf, kAllGroups);
   o.diag[key] = d;
   return d;
@@ -1534,7 +1554,7 @@ void Storage::p2Restrict(int id, int Lf, unsigned mask) {
     if (adc.n)
       dev::p2AddKernel<double, dev::MODE_REPLACE><<<na, dev::kBlock, 0, stream>>>(
           (const int64_t*)adc.owner.p, (const int*)adc.ptr.p, (const int64_t*)adc.copies.p,
-          (const unsigned char*)adc.type.p, adc.n, (double*)data(id, Lcf), nullptr, mask, nullptr, -1);
+          (const unsigned char*)adc.type.p, adc.n, (double*)data(id, Lcf), nullptr, mask);
   } else {
     dev::p2RestrictGatherKernel<float><<<nb, dev::kBlock, 0, stream>>>(
         lc.lv, lf.lv, (const int*)gt.ptr.p, (const int*)gt.idx.p, (const float*)gt.wf.p, gt.nCoarse, bpc,
@@ -1543,7 +1563,7 @@ void Storage::p2Restrict(int id, int Lf, unsigned mask) {
     if (adc.n)
       dev::p2AddKernel<float, dev::MODE_REPLACE><<<na, dev::kBlock, 0, stream>>>(
           (const int64_t*)adc.owner.p, (const int*)adc.ptr.p, (const int64_t*)adc.copies.p,
-          (const unsigned char*)adc.type.p, adc.n, (float*)data(id, Lcf), nullptr, mask, nullptr, -1);
+          (const unsigned char*)adc.type.p, adc.n, (float*)data(id, Lcf), nullptr, mask);
   }
   launches += adc.n ? 2 : 1;
   cudaCheck(cudaGetLastError(), "P2 restriction");
@@ -1669,7 +1689,7 @@ static void stokesDivTImpl(Storage& st, P2Operator& o, int p, const int v[3], in
     if (adv.n)
       dev::p2AddKernel<T, dev::MODE_REPLACE><<<(adv.n + dev::kBlock - 1) / dev::kBlock, dev::kBlock, 0, st.stream>>>(
           (const int64_t*)adv.owner.p, (const int*)adv.ptr.p, (const int64_t*)adv.copies.p,
-          (const unsigned char*)adv.type.p, adv.n, (T*)st.data(sc[k], Lv), nullptr, maskV, nullptr, -1);
+          (const unsigned char*)adv.type.p, adv.n, (T*)st.data(sc[k], Lv), nullptr, maskV);
     const double one = 1.0;
     st.lincomb(v[k], Lv, maskV, 1, &one, &sc[k], add, 0.0);
     st.communicate(v[k], Lv, (1 << G_COUNT) - 1);
@@ -1709,7 +1729,7 @@ static void stokesDivImpl(Storage& st, P2Operator& o, const int u[3], int q, int
   if (adp.n) {
     dev::p2AddKernel<T, dev::MODE_REPLACE><<<(adp.n + dev::kBlock - 1) / dev::kBlock, dev::kBlock, 0, st.stream>>>(
         (const int64_t*)adp.owner.p, (const int*)adp.ptr.p, (const int64_t*)adp.copies.p,
-        (const unsigned char*)adp.type.p, adp.n, (T*)st.data(q, Lp), nullptr, maskP, nullptr, -1);
+        (const unsigned char*)adp.type.p, adp.n, (T*)st.data(q, Lp), nullptr, maskP);
     ++st.launches;
   }
   cudaCheck(cudaGetLastError(), "Stokes div");

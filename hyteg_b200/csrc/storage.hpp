@@ -135,6 +135,8 @@ struct P2Additive {
   int updInnerBegin[12] = {0};
   DevBuf closureList;                       // closure nodes of the cells (dev::P2ClosureNode) by colour
   int closureBegin[12] = {0};               // first entry of colour k; closureBegin[11] = total
+  DevBuf items;                             // work list of the apply (dev::P2Item), per macro-cell
+  int nItems = 0;
   std::vector<int64_t> hostOwner;           // the owner slot of every DoF (levels up to 2^20 slots)
   std::vector<unsigned char> hostOwnerType;  // and its DoF type
 };
@@ -279,7 +281,7 @@ struct Storage {
   int p1Diagonal(int op, int L);
   int p2Scratch(int Lf, int prec);
   template <class T, int MODE>
-  void p2Launch(P2Operator& o, int L, T* dst, const T* src, const T* rhs, unsigned mask, int sel);
+  void p2Launch(P2Operator& o, int L, T* dst, const T* src, const T* rhs, unsigned mask);
   template <class T>
   void p2SorT(P2Operator& o, int opId, int x, int b, int L, unsigned mask, T omega, bool backwards);
   // Re-assemble an operator's stencils from the current cell coefficients into its device

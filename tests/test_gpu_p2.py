@@ -84,6 +84,17 @@ def test_p2_apply_fp32(cube2, L):
     assert rel(got, ref, inner) < 2e-5
 
 
+@pytest.mark.parametrize("L", [4, 5])
+@pytest.mark.parametrize("residual", [False, True])
+@pytest.mark.parametrize("dtype,tol", [(np.float64, 1e-13), (np.float32, 2e-5)])
+def test_p2_apply_across_tiles(L, residual, dtype, tol):
+    # lattices 32 and 64: several 16^3 interior tiles and 32 x 32 face pieces per macro-cell, whole
+    # ones and ones cut by the sloped face
+    got, ref, inner, d0 = run_apply(setup(1, L), L, dtype, residual, 40 + L)
+    assert rel(got, ref, inner) < tol
+    assert np.array_equal(got[~inner], d0[~inner])
+
+
 @pytest.mark.parametrize("L", [0, 1])
 def test_p2_apply_inner_vertices_and_edges(cube3, L):
     # the 3x3x3 cube has inner macro-vertices and inner macro-edges: sums over up to 24 cells
