@@ -515,6 +515,122 @@ __global__ void __launch_bounds__(kBlock) cellSorSplitKernel(LevelDev lv, const 
 }
 
 // ---------------------------------------------------------------------------------------
+// The whole cell phase of a sweep with the macro-cell resident in shared memory, for levels whose
+// closed cell and right-hand side fit there (residentLevel). A block owns a macro-cell: it refreshes
+// the cell's closure copies (its entries range[c] of the halo table; nullptr: they are up to
+// date), reads u and rhs once into the colour-split order (perm: natural index -> position), runs
+// the four colour passes of cellSorSplitKernel with a block barrier between them, and writes u
+// back in place. No tile halo is recomputed and no second buffer is written; the price is one
+// block per macro-cell, which is right for the small levels only. The tables do not depend on the
+// data: the record of a thread's next point is read one point ahead, across the barrier.
+// ---------------------------------------------------------------------------------------
+constexpr int kResidentMaxN = 32;
+inline bool residentLevel(int N) { return N >= 4 && N <= kResidentMaxN; }
+inline int residentThreads(int N) { return N <= 8 ? 64 : N <= 16 ? 128 : 576; }  // about half a colour's points at N = 32
+template <class T>
+inline size_t residentSmem(int N) {
+  const size_t w = size_t(N) + 1;
+  return 2 * (w * (w + 1) * (w + 2) / 6) * sizeof(T);
+}
+
+struct ResidentTables {
+  const uint16_t* perm;       // [tet(w)]
+  const SplitRow* rows[4];    // per colour
+  const unsigned* points[4];
+  int n[4];
+  const uint2* comm;          // the level's halo table
+  const int2* range;          // per cell (nullptr: no refresh)
+};
+
+template <class T>
+__global__ void __launch_bounds__(576, sizeof(T) == 4 ? 2 : 1) cellSorResidentKernel(LevelDev lv, const T* __restrict__ cellW, T* u,
+                                                                const T* __restrict__ rhs, unsigned mask,
+                                                                ResidentTables tb, T omega, int backwards) {
+  extern __shared__ __align__(16) unsigned char residentSmemRaw[];
+  __shared__ const SplitRow* rows[4];
+  __shared__ const unsigned* points[4];
+  __shared__ int count[4];
+  const int c = blockIdx.x, tid = threadIdx.x, nt = blockDim.x;
+  if (tid == 0) {  // in the order of the passes
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      rows[k] = backwards ? tb.rows[3 - k] : tb.rows[k];
+      points[k] = backwards ? tb.points[3 - k] : tb.points[k];
+      count[k] = backwards ? tb.n[3 - k] : tb.n[k];
+    }
+  }
+  if (tb.range) {
+    const int2 r = tb.range[c];
+    for (int i = r.x + tid; i < r.y; i += nt) {
+      const uint2 t = tb.comm[i];
+      u[t.x] = u[t.y];
+    }
+  }
+  if (!(lv.cellType[c] & mask)) return;
+  __syncthreads();
+  const int w = lv.w, size = int(tetSize(w));
+  T* su = reinterpret_cast<T*>(residentSmemRaw);
+  T* sf = su + size;
+  T* uc = u + lv.cellOff[c];
+  const T* __restrict__ f = rhs + lv.cellOff[c];
+  for (int i = tid; i < size; i += nt) {
+    const int p = tb.perm[i];
+    su[p] = uc[i];
+    sf[p] = f[i];
+  }
+  T wt[15];
+#pragma unroll
+  for (int k = 0; k < 15; ++k) wt[k] = __ldg(cellW + 16 * c + k);
+  const T om1 = T(1) - omega, dinv = omega / wt[0];
+  int4 r0, r1, r2, r3;
+  int j = 0;
+  auto fetch = [&](int pass, int t) {  // record of point t of a pass's colour
+    if (t < count[pass]) {
+      const unsigned e = __ldg(points[pass] + t);
+      const int4* rp = reinterpret_cast<const int4*>(rows[pass] + (e >> kSplitJBits));
+      j = int(e & ((1u << kSplitJBits) - 1));
+      r0 = __ldg(rp);
+      r1 = __ldg(rp + 1);
+      r2 = __ldg(rp + 2);
+      r3 = __ldg(rp + 3);
+    }
+  };
+  fetch(0, tid);
+  __syncthreads();
+#pragma unroll 1
+  for (int pass = 0; pass < 4; ++pass) {
+    const int n = count[pass];
+#pragma unroll 1
+    for (int t = tid; t < n; t += nt) {
+      const T* s = su + j;
+      const int centre = r0.x;
+      T a = wt[1] * s[r0.y];
+      T b = wt[7] * s[r1.w];
+      T d = wt[11] * s[r2.w];
+      a += wt[2] * s[r0.z];
+      b += wt[8] * s[r2.x];
+      d += wt[12] * s[r3.x];
+      a += wt[3] * s[r0.w];
+      b += wt[9] * s[r2.y];
+      d += wt[13] * s[r3.y];
+      a += wt[4] * s[r1.x];
+      b += wt[10] * s[r2.z];
+      d += wt[14] * s[r3.z];
+      a += wt[5] * s[r1.y];
+      a += wt[6] * s[r1.z];
+      T* x = su + j + centre;
+      const T v = om1 * *x + (sf[j + centre] - (a + (b + d))) * dinv;
+      // the next record before the store: this colour's next point, or the next colour's first one
+      if (t + nt < n) fetch(pass, t + nt);
+      *x = v;
+    }
+    if (pass < 3) fetch(pass + 1, tid);
+    __syncthreads();
+  }
+  for (int i = tid; i < size; i += nt) uc[i] = su[tb.perm[i]];
+}
+
+// ---------------------------------------------------------------------------------------
 // Register-blocked 2.5-D cell sweep (the kernel behind apply and residual on cell interiors).
 // A warp owns a strip of 30 x-columns (lanes 1..30; lanes 0 and 31 only carry the x-halo) by
 // R rows (StripCfg) and marches up z through a range of planes. Each lane keeps the rows

@@ -90,6 +90,8 @@ Storage::Storage(const Topology& topo, int maxLevel) : disc(topo, maxLevel) {
   allowSmem(dev::p2ApplyKernel<double, dev::MODE_RESIDUAL>, dev::p2TileSmem<double>());
   allowSmem(dev::p2ApplyKernel<float, dev::MODE_REPLACE>, dev::p2TileSmem<float>());
   allowSmem(dev::p2ApplyKernel<float, dev::MODE_RESIDUAL>, dev::p2TileSmem<float>());
+  allowSmem(dev::cellSorResidentKernel<double>, dev::residentSmem<double>(dev::kResidentMaxN));
+  allowSmem(dev::cellSorResidentKernel<float>, dev::residentSmem<float>(dev::kResidentMaxN));
   stream = ownStream;
   levels.resize(maxLevel + 1);
   for (int L = 0; L <= maxLevel; ++L) buildLevel(L);
@@ -226,6 +228,7 @@ void Storage::buildLevel(int L) {
     std::vector<int2> fr = ranges(G_FACE_BOUNDARY, KF, lv.nFaces);
     if (!low.empty()) ld.lowRange = (const int2*)upload(ld.keep, low, stream);
     if (!fr.empty()) ld.faceRange = (const int2*)upload(ld.keep, fr, stream);
+    if (dev::residentLevel((int)N)) ld.cellRange = (const int2*)upload(ld.keep, ranges(G_CELL, KC, lv.nCells), stream);
   }
 
   auto& keep = ld.keep;
@@ -485,6 +488,10 @@ void Storage::buildSplit(int L) {
     ld.splitRows[col] = (const dev::SplitRow*)upload(ld.keep, rows, stream);
     ld.splitPoints[col] = (const unsigned*)upload(ld.keep, points, stream);
     ld.nSplitPoints[col] = (int)points.size();
+  }
+  if (dev::residentLevel((int)N)) {
+    const std::vector<uint16_t> perm16(perm.begin(), perm.end());
+    ld.splitPerm = (const uint16_t*)upload(ld.keep, perm16, stream);
   }
   cudaCheck(cudaStreamSynchronize(stream), "colour-split tables");  // the host vectors go out of scope
   ld.commSplit = commSplit;
@@ -2040,6 +2047,24 @@ void Storage::sorT(Operator& o, int dstId, int L, T* u, const T* rhs, unsigned m
       return;
     }
     const int schedule = sorScheduleFor(L, (int)sizeof(T));
+    // Schedule 0 keeps a small macro-cell resident in shared memory (in place, closure refresh
+    // folded in) and sweeps larger ones in the wavefront pass.
+    if (schedule == 0 && dev::residentLevel(lv.N)) {
+      buildSplit(L);
+      dev::ResidentTables tb{};
+      tb.perm = ld.splitPerm;
+      for (int k = 0; k < 4; ++k) {
+        tb.rows[k] = ld.splitRows[k];
+        tb.points[k] = ld.splitPoints[k];
+        tb.n[k] = ld.nSplitPoints[k];
+      }
+      tb.comm = ld.comm;
+      tb.range = refresh ? ld.cellRange : nullptr;
+      dev::cellSorResidentKernel<T><<<lv.nCells, dev::residentThreads(lv.N), dev::residentSmem<T>(lv.N), stream>>>(
+          lv, st.cellW, u, rhs, mask, tb, omega, rev ? 1 : 0);
+      ++launches;
+      return;
+    }
     const int pi = sizeof(T) == 4 ? 1 : 0, gv = schedule == 2 ? 1 : 0;
     if ((schedule == 0 || schedule == 2) && ld.nWaveTiles[pi][gv]) {
       // one pass into the spare buffer of this level, which then becomes the function's buffer
@@ -2081,6 +2106,8 @@ void Storage::sorT(Operator& o, int dstId, int L, T* u, const T* rhs, unsigned m
   // rows (owned by edges and vertices) before the faces, vertex ghosts (owned by edges, faces and
   // cells) before the vertices of a backward sweep. Edge ghost layers end on the neighbouring
   // edges and face ghost layers on other faces, so those refreshes stay launches of their own.
+  const bool resident =  // the cell phase refreshes the closure copies itself
+      !cellU && (kinds & (1 << KC)) && sorScheduleFor(L, (int)sizeof(T)) == 0 && dev::residentLevel(lv.N);
   if (fusedSorPhases) {
     const uint2* table = cellU ? ld.commSplit : ld.comm;
     const int64_t cellEnd = ld.nonCellBegin;
@@ -2104,13 +2131,16 @@ void Storage::sorT(Operator& o, int dstId, int L, T* u, const T* rhs, unsigned m
       comm(1 << G_EDGE);              // Vertex -> Edge
       lowPhase(true, false, false);   // edges
       facePhase(true, false);         // Edge -> Face, faces
-      comm(1 << G_CELL);              // Face -> Cell
+      if (!resident) comm(1 << G_CELL);  // Face -> Cell
       cellPhase(false);
     } else {
-      comm((1 << G_CELL) | (1 << G_FACE_BOUNDARY));
+      // the face phase refreshes its boundary rows itself: their owners (edges and vertices) have not
+      // changed by then
+      const bool faces = lv.nFaceBlocks > 0 && (kinds & (1 << KF));
+      comm((resident ? 0 : 1 << G_CELL) | (faces ? 0 : 1 << G_FACE_BOUNDARY));
       cellPhase(true);
       comm(1 << G_FACE_GHOST);        // Cell -> Face
-      facePhase(false, true);
+      facePhase(true, true);
       comm(1 << G_EDGE);              // Face -> Edge
       lowPhase(true, false, true);    // edges
       lowPhase(false, true, true);    // Edge -> Vertex, vertices
@@ -2132,7 +2162,7 @@ void Storage::sorT(Operator& o, int dstId, int L, T* u, const T* rhs, unsigned m
     edges(1);
     comm(1 << G_FACE_BOUNDARY);  // Edge -> Face
     for (int c = 0; c < 3; ++c) faces(c);
-    comm(1 << G_CELL);           // Face -> Cell
+    if (!resident) comm(1 << G_CELL);  // Face -> Cell
     cellPhase(false);
   } else {
     cellPhase(true);

@@ -60,6 +60,10 @@ struct LevelData {
   const dev::SplitRow* splitRows[4] = {nullptr, nullptr, nullptr, nullptr};
   const unsigned* splitPoints[4] = {nullptr, nullptr, nullptr, nullptr};
   int nSplitPoints[4] = {0, 0, 0, 0};
+  // resident cell phase (dev::residentLevel): positions in the colour-split order, and per cell its
+  // entries (begin, end) in comm of the cell-closure group
+  const uint16_t* splitPerm = nullptr;
+  const int2* cellRange = nullptr;
   std::vector<unsigned char> hostCellType, hostFaceType, hostLowType;
   std::vector<std::unique_ptr<DevBuf>> keep;
 };

@@ -118,7 +118,8 @@ int hg_storage_set_cell_coefficients(hg_storage* s, const double* k, int ncells)
  * (32 x 12 instead of 32 x 24 / 28), 3 = four colour passes on copies of the cell arrays in the
  * colour-split order (each row ordered by x mod 4; the copies are made once per group of sweeps
  * of a multigrid smoothing step and the result is copied back). All give the same multicolour
- * sweep. */
+ * sweep. Under schedule 0, levels with at most 2^5 micro-edges per macro-edge keep each macro-cell
+ * in shared memory for the whole cell phase and update the level buffer in place. */
 int hg_storage_set_sor_schedule(hg_storage* s, int schedule);
 /* Launch structure of the face, edge and vertex phases of the multicolour SOR (no counterpart in
  * the reference; the same sweep either way, bit for bit): on = 1 (default) runs each phase as one
@@ -205,7 +206,7 @@ int hg_mesh_low_stencil(const hg_mesh* m, int level, int form, int kind, int pri
 int hg_function_create(hg_storage* s, int min_level, int max_level, int precision, int* fn);
 int hg_function_destroy(hg_storage* s, int fn);
 /* The address of a level buffer is stable except across multicolour SOR on that level under
- * schedule 0 (hg_storage_set_sor_schedule): the sweep writes the second buffer of the level and
+ * schedule 0 or 2 (hg_storage_set_sor_schedule): the sweep writes the second buffer of the level and
  * the two are exchanged, so re-query the address after smoothing (an even number of sweeps
  * per level, as in a V(3,3) cycle, returns every buffer to its original address). */
 int hg_function_device_ptr(hg_storage* s, int fn, int level, void** ptr);

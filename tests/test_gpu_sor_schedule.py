@@ -63,6 +63,14 @@ def test_single_pass_equals_colour_passes(cube6, L, backwards, dtype, tol, sched
     assert np.abs(got[used] - ref[used]).max() / np.abs(ref[used]).max() < tol
 
 
+@pytest.mark.parametrize("L", [2, 3, 4])
+@pytest.mark.parametrize("backwards", [False, True])
+@pytest.mark.parametrize("dtype,tol", [(np.float64, 1e-13), (np.float32, 1e-5)])
+def test_resident_cells_equal_colour_passes(cube6, L, backwards, dtype, tol):
+    # levels below 5 under schedule 0: fewer points per colour than threads, down to one interior point
+    test_single_pass_equals_colour_passes(cube6, L, backwards, dtype, tol, 0)
+
+
 @pytest.mark.parametrize("schedule", [0, 3])
 def test_single_pass_matches_oracle_level5(schedule):
     if hg.device_count() == 0:
