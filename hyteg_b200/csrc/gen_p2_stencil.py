@@ -101,6 +101,36 @@ def face_stencils(M=16):
     return out
 
 
+def rim_node(e, odd, M=16):
+    """A node of edge e of a macro-cell of lattice M with an even or odd distance from the edge's
+    first vertex; e = 6 .. 9: the macro-vertices."""
+    t = 4 + odd
+    return [(t, 0, 0), (0, t, 0), (0, 0, t), (M - t, t, 0), (M - t, 0, t), (0, M - t, t),
+            (0, 0, 0), (M, 0, 0), (0, M, 0), (0, 0, M)][e]
+
+
+def rim_stencils(M=16):
+    """Per edge of a macro-cell and parity along it (even, odd), then per vertex: class, micro-cells
+    and offsets as in face_stencils."""
+    off = node_offsets()
+    N = M // 2
+    out = []
+    for e, odd in [(e, odd) for e in range(6) for odd in (0, 1)] + [(e, 0) for e in range(6, 10)]:
+        q = rim_node(e, odd, M)
+        pc = (q[0] & 1) | ((q[1] & 1) << 1) | ((q[2] & 1) << 2)
+        cand = []
+        for t in range(6):
+            for j in range(10):
+                if tuple(c & 1 for c in off[t][j]) != tuple(c & 1 for c in q):
+                    continue
+                a = [(c - o) >> 1 for c, o in zip(q, off[t][j])]
+                if min(a) >= 0 and sum(a) < N - WIDTH_REDUCTION[t]:
+                    cand.append((t, j))
+        s = {tuple(off[t][m][d] - off[t][j][d] for d in range(3)) for t, j in cand for m in range(10)}
+        out.append((e, pc, cand, sorted(s, key=lambda o: (o[2], o[1], o[0]))))
+    return out
+
+
 def divt_stencils():
     """Per velocity class: the pressure-lattice offsets (relative to (X >> 1, Y >> 1, Z >> 1)) of
     the vertices of the micro-cells around an interior velocity node, with the (type, local node j,
@@ -157,15 +187,18 @@ def render():
     ]
     for pc, s in enumerate(st):
         lines.append("using S%d = List<%s>;" % (pc, ", ".join("O<%d, %d, %d>" % o for o in s)))
-    fs = face_stencils()
+    fs = face_stencils() + rim_stencils()
     fmax = max(len(f[3]) for f in fs)
     cmax = max(len(f[2]) for f in fs)
     lines += [
         "",
         "// Face-interior nodes (a node on exactly one face of the macro-cell) couple to the nodes of",
         "// the micro-cells inside the cell that hold them, the same ones at every node of a (face, class):",
-        "// faces 0: Z = 0, 1: Y = 0, 2: X = 0, 3: X + Y + Z = M; four classes per face. Entry k of the",
-        "// tables below is face k / 4, class kFaceClass[k]; kFaceCand lists its micro-cells (type, local node).",
+        "// faces 0: Z = 0, 1: Y = 0, 2: X = 0, 3: X + Y + Z = M; four classes per face. Entry k < 16 of",
+        "// the tables below is face k / 4, class kFaceClass[k]; kFaceCand lists its micro-cells (type, local",
+        "// node). The same holds along the macro-cell's edges (0: X axis, 1: Y axis, 2: Z axis, 3: (M - t, t, 0),",
+        "// 4: (M - t, 0, t), 5: (0, M - t, t)): entry 16 + 2 e + (t & 1) is edge e at distance t from its first",
+        "// vertex, and entry 28 + v is macro-vertex v.",
         "constexpr int kFaceStencils = %d;" % len(fs),
         "constexpr int kFaceMaxLen = %d;" % fmax,
         "constexpr int kFaceClass[%d] = {%s};" % (len(fs), ", ".join(str(f[1]) for f in fs)),
@@ -182,8 +215,9 @@ def render():
         lines.append("    {" + ", ".join("{%d, %d, %d}" % o for o in f[3]) + "},")
     lines.append("};")
     for k, f in enumerate(fs):
-        lines.append("using F%d = List<%s>;  // face %d (%s), class %d" % (k, ", ".join("O<%d, %d, %d>" % o for o in f[3]),
-                                                                        f[0], FACES[f[0]], f[1]))
+        what = "face %d (%s), class %d" % (f[0], FACES[f[0]], f[1]) if k < 16 else (
+            "edge %d, class %d" % (f[0], f[1]) if k < 28 else "vertex %d" % (k - 28))
+        lines.append("using F%d = List<%s>;  // %s" % (k, ", ".join("O<%d, %d, %d>" % o for o in f[3]), what))
     dt = divt_stencils()
     lines += [
         "",

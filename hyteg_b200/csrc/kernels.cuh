@@ -1221,11 +1221,10 @@ static __global__ void __launch_bounds__(kBlock) coarseCgKernel(StencilDev<doubl
 // P2 operator of level L on the vertex-DoF lattice of level L + 1 (size M = 2N per edge).
 // Node (X, Y, Z) of a macro-cell is local node j of the level-L micro-cell (t, a) exactly when
 // (X, Y, Z) = 2a + off[t][j]; its parity class (X, Y, Z mod 2) fixes the candidates (t, j).
-// A thread owns one node of the closed macro-cell and sums, over the candidate micro-cells that
-// lie inside the cell, row j of that micro-cell's 10 x 10 element matrix times the ten nodal
-// values (gather form of the element-by-element product; deterministic). Interior nodes get
-// their final value; nodes on the cell's faces, edges and vertices get this cell's share in the
-// cell's closure slots, which p2AddKernel sums into the owning primitive.
+// Within one macro-cell the candidates inside the cell are the same at every interior node of a
+// class, at every node inside a face of a class, along an edge and at a vertex, so every row is a
+// constant stencil. Interior nodes get their final value; nodes on the cell's faces, edges and
+// vertices get this cell's share in the cell's closure slots, which are summed into the owner.
 // ---------------------------------------------------------------------------------------
 struct P2Tables {
   signed char off[6][10][3];   // lattice offset of local node j of micro-cell type t from 2a
@@ -1234,83 +1233,41 @@ struct P2Tables {
   unsigned char widthRed[6];   // micro-cells of type t: a_x + a_y + a_z < N - widthRed[t]
 };
 
-constexpr int MODE_DIAG = 3;  // P2: sum of the element diagonals (the matrix diagonal)
-constexpr int MODE_SOR = 4;   // P2 interior: x += omega (b - A x) / a_ii in place, one colour
-
-// Row j of A at node (X, Y, Z) of a macro-cell restricted to that cell: the sum over the level-L
-// micro-cells inside the cell holding the node as local node j (DIAG: of their diagonals only).
-// u is the cell's array, pbz the first index of the planes Z-2 .. Z+2.
-template <class T, bool DIAG>
-__device__ __forceinline__ T p2GatherNode(const P2Tables& tb, const T* Kc, const T* __restrict__ u, const int (&pbz)[5],
-                                          int w, int N, int X, int Y, int Z) {
-  const int pc = (X & 1) | ((Y & 1) << 1) | ((Z & 1) << 2);
-  T s = T(0);
-  for (int k = 0; k < tb.nCand[pc]; ++k) {
-    const int t = tb.cand[pc][k][0], j = tb.cand[pc][k][1];
-    const int ax = (X - tb.off[t][j][0]) >> 1, ay = (Y - tb.off[t][j][1]) >> 1, az = (Z - tb.off[t][j][2]) >> 1;
-    if (ax < 0 || ay < 0 || az < 0 || ax + ay + az >= N - tb.widthRed[t]) continue;
-    const T* Kr = Kc + t * 100 + j * 10;
-    if (DIAG) {
-      s += Kr[j];
-      continue;
-    }
-#pragma unroll
-    for (int m = 0; m < 10; ++m) {
-      const int qx = 2 * ax + tb.off[t][m][0], qy = 2 * ay + tb.off[t][m][1], qz = 2 * az + tb.off[t][m][2];
-      s += Kr[m] * __ldg(u + pbz[qz - Z + 2] + rowStart(w - qz, qy) + qx);
-    }
-  }
-  return s;
-}
-
-// The diagonal of the operator (MODE_DIAG) on every node of the closed macro-cells.
-template <class T, int MODE>
-__global__ void __launch_bounds__(kBlock) p2CellKernel(LevelDev lv, P2Tables tb, const T* __restrict__ K,
-                                                       T* __restrict__ dst, const T* __restrict__ src,
-                                                       const T* __restrict__ rhs, unsigned mask) {
+// The diagonal of the operator on every node of the closed macro-cells: per node the sum of the
+// element diagonals of the level-L micro-cells inside the cell that hold it.
+template <class T>
+__global__ void __launch_bounds__(kBlock) p2DiagonalKernel(LevelDev lv, P2Tables tb, const T* __restrict__ K,
+                                                           T* __restrict__ dst) {
   const int M = lv.N, N = M / 2, nPl = M + 1, w = lv.w;
   const int c = blockIdx.x / nPl, Z = blockIdx.x % nPl;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t base = lv.cellOff[c];
-  const bool cellOn = (lv.cellType[c] & mask) != 0;
   const T* Kc = K + (int64_t)c * 600;
-  // first index of the planes Z-2 .. Z+2 (the ones a micro-cell around a node of plane Z reaches)
-  int pbz[5];
-#pragma unroll
-  for (int d = 0; d < 5; ++d) {
-    const int z = Z - 2 + d;
-    pbz[d] = (z >= 0 && z <= M) ? int(tetSize(w) - tetSize(w - z)) : 0;
-  }
-  const int pb = pbz[2];
-  for (int Y = warp; Y <= M - Z; Y += kBlock / 32) {
-    const int r0 = pb + rowStart(w - Z, Y);
+  const int pb = int(tetSize(w) - tetSize(w - Z));
+  for (int Y = warp; Y <= M - Z; Y += kBlock / 32)
     for (int X = lane; X <= M - Z - Y; X += 32) {
-      const int64_t i = base + r0 + X;
-      const T s = p2GatherNode<T, MODE == MODE_DIAG>(tb, Kc, src + base, pbz, w, N, X, Y, Z);
-      const bool interior = X >= 1 && Y >= 1 && Z >= 1 && X + Y + Z <= M - 1;
-      if (!interior) dst[i] = s;
-      else if (cellOn) dst[i] = MODE == MODE_RESIDUAL ? rhs[i] - s : s;
+      const int pc = (X & 1) | ((Y & 1) << 1) | ((Z & 1) << 2);
+      T s = T(0);
+      for (int k = 0; k < tb.nCand[pc]; ++k) {
+        const int t = tb.cand[pc][k][0], j = tb.cand[pc][k][1];
+        const int ax = (X - tb.off[t][j][0]) >> 1, ay = (Y - tb.off[t][j][1]) >> 1, az = (Z - tb.off[t][j][2]) >> 1;
+        if (ax < 0 || ay < 0 || az < 0 || ax + ay + az >= N - tb.widthRed[t]) continue;
+        s += Kc[t * 100 + j * 11];
+      }
+      dst[base + pb + rowStart(w - Z, Y) + X] = s;
     }
-  }
 }
 
 // ---------------------------------------------------------------------------------------
-// P2 interior nodes by constant stencils. An interior node of a macro-cell (X, Y, Z >= 1,
-// X + Y + Z <= M - 1 on lattice M = 2^(L+1)) couples only to nodes of the micro-cells inside the
-// cell, in the same pattern for every node of its parity class, so its row of A is a constant
-// stencil per (cell, class): the offsets are compile-time lists (p2_stencil.h), the weights a
-// per-cell table W[cell][p2s::kTotal] assembled on the host from the element matrices. A block
-// works on one (cell, plane Z); each warp takes whole rows, its lanes every second node of the
-// row, so all lanes of a warp run the same class.
+// P2 rows by constant stencils: the offsets are compile-time lists (p2_stencil.h), the weights
+// per-cell tables assembled on the host from the element matrices (W[cell][p2s::kTotal] for the
+// interior classes, FW[cell][p2s::kFaceTotal] for the closure).
 // ---------------------------------------------------------------------------------------
 template <int DY, int DZ>
 __device__ __forceinline__ int p2RowBase(const int (&pbz)[5], int w, int Y, int Z) {
   return pbz[DZ + 2] + rowStart(w - Z - DZ, Y + DY);
 }
 
-// The loads go through the read-only path also in the in-place SOR pass: no thread reads a value
-// that another thread writes during the launch (a colour class couples to no node of its own
-// colour), and each thread reads its own node before writing it.
 // Four partial sums (entry I into sum I mod 4) keep the FMA dependency chains short.
 template <class T, int... DX, int... DY, int... DZ, int... I>
 __device__ __forceinline__ T p2StencilDot(p2s::List<p2s::O<DX, DY, DZ>...>, std::integer_sequence<int, I...>,
@@ -1320,100 +1277,8 @@ __device__ __forceinline__ T p2StencilDot(p2s::List<p2s::O<DX, DY, DZ>...>, std:
   return (s[0] + s[1]) + (s[2] + s[3]);
 }
 
-// One row (Y, Z) of class PC, only the nodes of colour sel: MODE_REPLACE dst = A src, MODE_SOR
-// dst (== src) += omega (rhs - A dst) / a_ii. The vertex class is split into four colours, read from
-// the colour bytes; a whole edge class is one colour in a cell's frame.
-template <class T, int MODE, int PC>
-__device__ __forceinline__ void p2StencilRow(const T* wts, T* dst, const T* src, const T* rhs, int64_t base,
-                                             const int (&pbz)[5], int w, int M, int Y, int Z, int lane,
-                                             const unsigned char* __restrict__ colour, int sel, T omega, int vstep) {
-  using S = typename p2s::Class<PC>::type;
-  constexpr int kFirst = p2s::kFirst[PC], kCentre = p2s::kCentre[PC], kLen = p2s::kLen[PC];
-  const T* wt = wts + kFirst;
-  const int r0 = pbz[2] + rowStart(w - Z, Y);
-  int X0 = ((PC & 1) ? 1 : 2) + 2 * lane, dX = 64;
-  if (PC == 0) {
-    // vertex colour sel along the row: the colour of the vertex node 2 + 2t is c(2) + vstep t mod 4,
-    // so the lanes take every fourth (vstep odd) or every second (vstep 2) vertex node from the first
-    if (M - 1 - Y - Z < 2) return;
-    const int diff = (sel - (colour[base + r0 + 2] & 0x7f)) & 3;
-    int t0, ts;
-    if (vstep & 1) {
-      t0 = (diff * vstep) & 3;
-      ts = 4;
-    } else {
-      if (diff & 1) return;
-      t0 = (diff >> 1) & 1;
-      ts = 2;
-    }
-    X0 = 2 + 2 * t0 + 2 * ts * lane;
-    dX = 64 * ts;
-  }
-#pragma unroll 1
-  for (int X = X0; X <= M - 1 - Y - Z; X += dX) {
-    const int64_t i = base + r0 + X;
-    if (PC == 0 && (colour[i] & 0x7f) != sel) continue;
-    const T s = p2StencilDot<T>(S{}, std::make_integer_sequence<int, kLen>{}, src + base, wt, pbz, w, X, Y, Z);
-    if (MODE == MODE_REPLACE)
-      dst[i] = s;
-    else
-      dst[i] += omega * (rhs[i] - s) / wt[kCentre];
-  }
-}
-
-template <class T, int MODE>
-__device__ __forceinline__ void p2StencilRowAny(int pc, const T* wts, T* dst, const T* src, const T* rhs, int64_t base,
-                                                const int (&pbz)[5], int w, int M, int Y, int Z, int lane,
-                                                const unsigned char* __restrict__ colour, int sel, T omega,
-                                                int vstep) {
-  switch (pc) {
-    case 0: p2StencilRow<T, MODE, 0>(wts, dst, src, rhs, base, pbz, w, M, Y, Z, lane, colour, sel, omega, vstep); break;
-    case 1: p2StencilRow<T, MODE, 1>(wts, dst, src, rhs, base, pbz, w, M, Y, Z, lane, colour, sel, omega, vstep); break;
-    case 2: p2StencilRow<T, MODE, 2>(wts, dst, src, rhs, base, pbz, w, M, Y, Z, lane, colour, sel, omega, vstep); break;
-    case 3: p2StencilRow<T, MODE, 3>(wts, dst, src, rhs, base, pbz, w, M, Y, Z, lane, colour, sel, omega, vstep); break;
-    case 4: p2StencilRow<T, MODE, 4>(wts, dst, src, rhs, base, pbz, w, M, Y, Z, lane, colour, sel, omega, vstep); break;
-    case 5: p2StencilRow<T, MODE, 5>(wts, dst, src, rhs, base, pbz, w, M, Y, Z, lane, colour, sel, omega, vstep); break;
-    case 6: p2StencilRow<T, MODE, 6>(wts, dst, src, rhs, base, pbz, w, M, Y, Z, lane, colour, sel, omega, vstep); break;
-    default: p2StencilRow<T, MODE, 7>(wts, dst, src, rhs, base, pbz, w, M, Y, Z, lane, colour, sel, omega, vstep); break;
-  }
-}
-
-// Grid: nCells * (M - 3) blocks, block b on cell b / (M - 3), plane Z = 1 + b % (M - 3) (the
-// planes holding interior nodes; needs M >= 4). Only cells of a flagged DoF type are written. One
-// colour pass of the SOR (MODE_SOR or MODE_REPLACE): classOfColour[cell * 12 + sel] is the class
-// of colour sel in the cell's frame (0 for the four vertex colours, -1 when no interior node has
-// the colour), classOfColour[cell * 12 + 11] the change of the vertex colour from one vertex node
-// of a row to the next (1, 2 or 3). MODE_SOR updates in place: dst == src, rhs = b.
-template <class T, int MODE>
-__global__ void __launch_bounds__(kBlock, 2) p2StencilKernel(LevelDev lv, const T* __restrict__ W, T* dst, const T* src,
-                                                          const T* __restrict__ rhs, unsigned mask,
-                                                          const unsigned char* __restrict__ colour,
-                                                          const signed char* __restrict__ classOfColour, int sel,
-                                                          T omega) {
-  const int M = lv.N, w = lv.w, nPl = M - 3;
-  const int c = blockIdx.x / nPl, Z = 1 + blockIdx.x % nPl;
-  if (!(lv.cellType[c] & mask)) return;
-  const int pcSel = classOfColour[c * 12 + sel], vstep = classOfColour[c * 12 + 11];
-  if (pcSel < 0 || ((pcSel >> 2) & 1) != (Z & 1)) return;
-  __shared__ T wts[p2s::kTotal];
-  for (int k = threadIdx.x; k < p2s::kTotal; k += blockDim.x) wts[k] = W[(int64_t)c * p2s::kTotal + k];
-  __syncthreads();
-  int pbz[5];
-#pragma unroll
-  for (int d = 0; d < 5; ++d) {
-    const int z = Z - 2 + d;
-    pbz[d] = (z >= 0 && z <= M) ? int(tetSize(w) - tetSize(w - z)) : 0;
-  }
-  const int64_t base = lv.cellOff[c];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-#pragma unroll 1
-  for (int Y = (((pcSel >> 1) & 1) ? 1 : 2) + 2 * warp; Y <= M - 2 - Z; Y += 2 * (kBlock / 32))
-    p2StencilRowAny<T, MODE>(pcSel, wts, dst, src, rhs, base, pbz, w, M, Y, Z, lane, colour, sel, omega, vstep);
-}
-
-// A node inside one face of a macro-cell sees the same micro-cells of that cell at every node of
-// its (face, class): the cell's share of its row is a constant stencil (p2s::FaceList, weights
-// FW[cell][p2s::kFaceTotal]). Nodes on the cell's edges and vertices take the element gather.
+// This cell's share of a closure node's row, by the node's entry (face and class, edge and
+// parity, or vertex; p2_stencil.h).
 template <class T, int K>
 __device__ __forceinline__ T p2FaceDot(const T* u, const T* fw, const int (&pbz)[5], int w, int X, int Y, int Z) {
   using S = typename p2s::FaceList<K>::type;
@@ -1440,39 +1305,33 @@ __device__ __forceinline__ T p2FaceDotAny(int k, const T* u, const T* fw, const 
     case 12: return p2FaceDot<T, 12>(u, fw, pbz, w, X, Y, Z);
     case 13: return p2FaceDot<T, 13>(u, fw, pbz, w, X, Y, Z);
     case 14: return p2FaceDot<T, 14>(u, fw, pbz, w, X, Y, Z);
-    default: return p2FaceDot<T, 15>(u, fw, pbz, w, X, Y, Z);
+    case 15: return p2FaceDot<T, 15>(u, fw, pbz, w, X, Y, Z);
+    case 16: return p2FaceDot<T, 16>(u, fw, pbz, w, X, Y, Z);
+    case 17: return p2FaceDot<T, 17>(u, fw, pbz, w, X, Y, Z);
+    case 18: return p2FaceDot<T, 18>(u, fw, pbz, w, X, Y, Z);
+    case 19: return p2FaceDot<T, 19>(u, fw, pbz, w, X, Y, Z);
+    case 20: return p2FaceDot<T, 20>(u, fw, pbz, w, X, Y, Z);
+    case 21: return p2FaceDot<T, 21>(u, fw, pbz, w, X, Y, Z);
+    case 22: return p2FaceDot<T, 22>(u, fw, pbz, w, X, Y, Z);
+    case 23: return p2FaceDot<T, 23>(u, fw, pbz, w, X, Y, Z);
+    case 24: return p2FaceDot<T, 24>(u, fw, pbz, w, X, Y, Z);
+    case 25: return p2FaceDot<T, 25>(u, fw, pbz, w, X, Y, Z);
+    case 26: return p2FaceDot<T, 26>(u, fw, pbz, w, X, Y, Z);
+    case 27: return p2FaceDot<T, 27>(u, fw, pbz, w, X, Y, Z);
+    case 28: return p2FaceDot<T, 28>(u, fw, pbz, w, X, Y, Z);
+    case 29: return p2FaceDot<T, 29>(u, fw, pbz, w, X, Y, Z);
+    case 30: return p2FaceDot<T, 30>(u, fw, pbz, w, X, Y, Z);
+    default: return p2FaceDot<T, 31>(u, fw, pbz, w, X, Y, Z);
   }
 }
 
-// The closure nodes of one SOR colour from a per-colour list (one thread per node). k = face-stencil
-// entry of a face-interior node, -1 for a node on a cell edge or vertex (element gather).
+// A closure node of a macro-cell and its entry in the closure stencils.
 struct P2ClosureNode {
   int cell;
   unsigned short x, y, z;
   signed char k;
   unsigned char pad;
 };
-
-template <class T>
-__global__ void __launch_bounds__(kBlock) p2ClosureListKernel(LevelDev lv, P2Tables tb, const T* __restrict__ K,
-                                                              const T* __restrict__ FW, T* __restrict__ dst,
-                                                              const T* __restrict__ src,
-                                                              const P2ClosureNode* __restrict__ list, int n) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const P2ClosureNode nd = list[i];
-  const int M = lv.N, N = M / 2, w = lv.w, X = nd.x, Y = nd.y, Z = nd.z;
-  int pbz[5];
-#pragma unroll
-  for (int d = 0; d < 5; ++d) {
-    const int z = Z - 2 + d;
-    pbz[d] = (z >= 0 && z <= M) ? int(tetSize(w) - tetSize(w - z)) : 0;
-  }
-  const int64_t base = lv.cellOff[nd.cell];
-  const T s = nd.k >= 0 ? p2FaceDotAny<T>(nd.k, src + base, FW + (int64_t)nd.cell * p2s::kFaceTotal, pbz, w, X, Y, Z)
-                        : p2GatherNode<T, false>(tb, K + (int64_t)nd.cell * 600, src + base, pbz, w, N, X, Y, Z);
-  dst[base + pbz[2] + rowStart(w - Z, Y) + X] = s;
-}
 
 // ---------------------------------------------------------------------------------------
 // P2 quadratic transfers between P2 levels L and L + 1 (vertex lattices L + 1 and L + 2).
@@ -2137,40 +1996,6 @@ static __global__ void __launch_bounds__(kBlock) blockDenseCorrectKernel(const i
   double t = 0.0;
   for (int k = 0; k < n; ++k) t += Kinv[(int64_t)k * n + i] * rs[k];
   bp.x[comp[i]][idx[i]] += t;
-}
-
-// The owner update of one P2 SOR colour from per-colour lists: entries t < nAdd are indices into
-// the owner table (a face, edge or vertex DoF: its cells' shares are summed here), the others are
-// interior slots whose A x is in ax (the vertex colours). x += omega (b - A x) / diag.
-template <class T>
-__global__ void __launch_bounds__(kBlock) p2SorOwnersKernel(const int64_t* __restrict__ owner,
-                                                            const int* __restrict__ ptr,
-                                                            const int64_t* __restrict__ copies,
-                                                            const unsigned char* __restrict__ type,
-                                                            const int* __restrict__ addIdx, int nAdd,
-                                                            const int64_t* __restrict__ inner,
-                                                            const unsigned char* __restrict__ innerType, int nInner,
-                                                            unsigned mask, T* x, const T* __restrict__ b,
-                                                            const T* __restrict__ ax, const T* __restrict__ diag,
-                                                            T omega) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t < nAdd) {
-    const int j = addIdx[t];
-    if (!(type[j] & mask)) return;
-    T s = T(0);
-    for (int k = ptr[j]; k < ptr[j + 1]; ++k) s += ax[copies[k]];
-    const int64_t o = owner[j];
-    const T v = x[o] + omega * (b[o] - s) / diag[o];
-    x[o] = v;
-    // the owner's copies in the cell closures of x take the new value at once (the refresh of this
-    // colour's copies before the next colour pass)
-    for (int k = ptr[j]; k < ptr[j + 1]; ++k) x[copies[k]] = v;
-  } else if (t < nAdd + nInner) {
-    const int q = t - nAdd;
-    if (!(innerType[q] & mask)) return;
-    const int64_t o = inner[q];
-    x[o] += omega * (b[o] - ax[o]) / diag[o];
-  }
 }
 
 // Seeded uniform values in [lo, hi) at every slot of the flagged primitives' arrays; the value

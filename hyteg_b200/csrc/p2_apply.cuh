@@ -3,8 +3,7 @@
 // A level's work list (P2Item, the same for every macro-cell) holds three kinds of blocks:
 //   interior tiles of 16 x 16 x 16 lattice nodes, staged in shared memory;
 //   32 x 32 pieces of the cell's four faces;
-//   the nodes on the cell's edges and vertices (element gather), first in the list because a
-//   node there is a chain of up to 24 micro-cells.
+//   the nodes on the cell's edges and vertices.
 // Interior and face threads own a block of 2 x 2 x 2 (2 x 2) nodes, one of each parity class, and
 // walk over the distinct lattice positions the block's stencils read: a position is loaded once
 // and enters every row that uses it, so 89 loads serve the 230 products of eight nodes. The rows
@@ -86,7 +85,7 @@ struct P2FaceEntry {
   bool first;
   short weight;  // index into the cell's face weights p2s::kFaceTotal
 };
-constexpr int kP2FaceEntries = 92;
+constexpr int kP2FaceEntries = 92;  // of each face: its four classes
 struct P2FaceTable {
   P2FaceEntry e[4][kP2FaceEntries];
 };
@@ -212,12 +211,34 @@ __device__ __forceinline__ void p2FaceBlock(std::integer_sequence<int, E...>, co
   }
 }
 
+// An edge or vertex node's share (entries 16 .. 31 of the closure stencils).
+template <class T>
+__device__ __forceinline__ T p2RimDot(int k, const T* u, const T* fw, const int (&pbz)[5], int w, int X, int Y, int Z) {
+  switch (k) {
+    case 16: return p2FaceDot<T, 16>(u, fw, pbz, w, X, Y, Z);
+    case 17: return p2FaceDot<T, 17>(u, fw, pbz, w, X, Y, Z);
+    case 18: return p2FaceDot<T, 18>(u, fw, pbz, w, X, Y, Z);
+    case 19: return p2FaceDot<T, 19>(u, fw, pbz, w, X, Y, Z);
+    case 20: return p2FaceDot<T, 20>(u, fw, pbz, w, X, Y, Z);
+    case 21: return p2FaceDot<T, 21>(u, fw, pbz, w, X, Y, Z);
+    case 22: return p2FaceDot<T, 22>(u, fw, pbz, w, X, Y, Z);
+    case 23: return p2FaceDot<T, 23>(u, fw, pbz, w, X, Y, Z);
+    case 24: return p2FaceDot<T, 24>(u, fw, pbz, w, X, Y, Z);
+    case 25: return p2FaceDot<T, 25>(u, fw, pbz, w, X, Y, Z);
+    case 26: return p2FaceDot<T, 26>(u, fw, pbz, w, X, Y, Z);
+    case 27: return p2FaceDot<T, 27>(u, fw, pbz, w, X, Y, Z);
+    case 28: return p2FaceDot<T, 28>(u, fw, pbz, w, X, Y, Z);
+    case 29: return p2FaceDot<T, 29>(u, fw, pbz, w, X, Y, Z);
+    case 30: return p2FaceDot<T, 30>(u, fw, pbz, w, X, Y, Z);
+    default: return p2FaceDot<T, 31>(u, fw, pbz, w, X, Y, Z);
+  }
+}
+
 template <class T, int MODE>
-__global__ void __launch_bounds__(kBlock, 2) p2ApplyKernel(LevelDev lv, P2Tables tb, const P2Item* __restrict__ items,
+__global__ void __launch_bounds__(kBlock, 2) p2ApplyKernel(LevelDev lv, const P2Item* __restrict__ items,
                                                            const T* __restrict__ W, const T* __restrict__ FW,
-                                                           const T* __restrict__ K, T* __restrict__ dst,
-                                                           const T* __restrict__ src, const T* __restrict__ rhs,
-                                                           unsigned mask) {
+                                                           T* __restrict__ dst, const T* __restrict__ src,
+                                                           const T* __restrict__ rhs, unsigned mask) {
   extern __shared__ __align__(16) unsigned char p2Smem[];
   const int c = blockIdx.x % lv.nCells;
   const P2Item it = items[blockIdx.x / lv.nCells];
@@ -290,19 +311,22 @@ __global__ void __launch_bounds__(kBlock, 2) p2ApplyKernel(LevelDev lv, P2Tables
       default: p2FaceBlock<T, 3>(S{}, u, fw, d, w, M, s, t); break;
     }
   } else {
+    // per edge its odd nodes, then its even ones, so that the lanes of a warp mostly run one entry
     const int e = it.a + tid;
     if (e >= 6 * (M - 1) + 4) return;
-    int X = 0, Y = 0, Z = 0;
+    int X = 0, Y = 0, Z = 0, entry;
     if (e >= 6 * (M - 1)) {
       const int v = e - 6 * (M - 1);
       X = v == 1 ? M : 0;
       Y = v == 2 ? M : 0;
       Z = v == 3 ? M : 0;
+      entry = 28 + v;
     } else {
-      const int k = e / (M - 1), t = 1 + e - k * (M - 1);
+      const int k = e / (M - 1), r = e - k * (M - 1), t = r < M / 2 ? 2 * r + 1 : 2 * (r - M / 2) + 2;
       X = k == 0 ? t : k == 3 || k == 4 ? M - t : 0;
       Y = k == 1 || k == 3 ? t : k == 5 ? M - t : 0;
       Z = k == 2 || k == 4 || k == 5 ? t : 0;
+      entry = 16 + 2 * k + (t & 1);
     }
     int pbz[5];
 #pragma unroll
@@ -310,7 +334,7 @@ __global__ void __launch_bounds__(kBlock, 2) p2ApplyKernel(LevelDev lv, P2Tables
       const int z = Z - 2 + k;
       pbz[k] = z >= 0 && z <= M ? int(tetSize(w) - tetSize(w - z)) : 0;
     }
-    d[pbz[2] + rowStart(w - Z, Y) + X] = p2GatherNode<T, false>(tb, K + (int64_t)c * 600, u, pbz, w, M / 2, X, Y, Z);
+    d[pbz[2] + rowStart(w - Z, Y) + X] = p2RimDot<T>(entry, u, FW + (int64_t)c * p2s::kFaceTotal, pbz, w, X, Y, Z);
   }
 }
 

@@ -15,6 +15,7 @@
 #include "discretization.hpp"
 #include "kernels.cuh"
 #include "p2_apply.cuh"
+#include "p2_sor.cuh"
 #include "solvers.hpp"
 #include "storage.hpp"
 
@@ -977,195 +978,190 @@ static std::vector<dev::P2Item> p2Items(int M) {
   return items;
 }
 
+// Entry of a closure node of a macro-cell of lattice M in the closure stencils (p2_stencil.h).
+static int p2ClosureEntry(int64_t X, int64_t Y, int64_t Z, int64_t M) {
+  const bool on[4] = {Z == 0, Y == 0, X == 0, X + Y + Z == M};
+  const int n = on[0] + on[1] + on[2] + on[3];
+  if (n == 3) return 28 + (X == M ? 1 : Y == M ? 2 : Z == M ? 3 : 0);
+  if (n == 2) {  // edges: X axis, Y axis, Z axis, then opposite the origin in the faces Z, Y, X = 0
+    const int e = on[0] && on[1] ? 0 : on[0] && on[2] ? 1 : on[1] && on[2] ? 2 : on[0] ? 3 : on[1] ? 4 : 5;
+    const int64_t t = e == 0 ? X : e == 1 || e == 3 ? Y : Z;
+    return 16 + 2 * e + int(t & 1);
+  }
+  const int pc = int((X & 1) | ((Y & 1) << 1) | ((Z & 1) << 2));
+  for (int k = on[0] ? 0 : on[1] ? 4 : on[2] ? 8 : 12;; ++k)
+    if (p2s::kFaceClass[k] == pc) return k;
+}
+
 P2Additive& Storage::p2Additive(int Lf) {
   if ((int)p2add.size() <= Lf) p2add.resize(maxLevel() + 1);
   P2Additive& ad = p2add[Lf];
   if (ad.built) return ad;
   const LevelData& ld = levels[Lf];
-  // owner <- its copies in the closure slots of its cells (the cell-closure halo group)
-  std::map<int64_t, std::vector<int64_t>> byOwner;
-  const auto& cd = ld.lay->commDst[G_CELL];
-  const auto& cs = ld.lay->commSrc[G_CELL];
-  for (size_t i = 0; i < cd.size(); ++i) byOwner[cs[i]].push_back(cd[i]);
-  std::vector<int64_t> own, cp;
-  std::vector<int> ptr{0};
-  std::vector<unsigned char> ty;
-  auto typeOf = [&](int64_t slot) {  // DoF type of the primitive whose array holds the slot
-    for (int k : {KF, KE, KV})
-      for (size_t pr = 0; pr < ld.lay->off[k].size(); ++pr)
-        if (slot >= ld.lay->off[k][pr] && slot < ld.lay->off[k][pr] + ld.lay->size[k][pr])
-          return k == KF ? ld.hostFaceType[pr] : k == KE ? ld.hostLowType[pr] : ld.hostLowType[ld.lv.nEdges + pr];
-    throw Error(HG_ERR_INTERNAL, "owner slot outside the face, edge and vertex arrays");
+  const LevelLayout& lay = *ld.lay;
+  const Topology& topo = disc.topo();
+  const int64_t M = ld.lv.N;
+  auto put = [&](DevBuf& buf, const void* h, size_t bytes) {
+    buf.alloc(std::max<size_t>(bytes, 16));
+    if (bytes) cudaCheck(cudaMemcpyAsync(buf.p, h, bytes, cudaMemcpyHostToDevice, stream), "p2 tables");
   };
-  for (auto& kv : byOwner) {
-    own.push_back(kv.first);
-    for (int64_t c : kv.second) cp.push_back(c);
-    ptr.push_back((int)cp.size());
-    ty.push_back(typeOf(kv.first));
-  }
-  ad.n = (int)own.size();
-  ad.owner.alloc(std::max<size_t>(1, own.size()) * sizeof(int64_t));
-  ad.ptr.alloc(ptr.size() * sizeof(int));
-  ad.copies.alloc(std::max<size_t>(1, cp.size()) * sizeof(int64_t));
-  ad.type.alloc(std::max<size_t>(1, ty.size()));
-  if (!own.empty()) {
-    cudaCheck(cudaMemcpyAsync(ad.owner.p, own.data(), own.size() * sizeof(int64_t), cudaMemcpyHostToDevice, stream), "p2 add");
-    cudaCheck(cudaMemcpyAsync(ad.copies.p, cp.data(), cp.size() * sizeof(int64_t), cudaMemcpyHostToDevice, stream), "p2 add");
-    cudaCheck(cudaMemcpyAsync(ad.type.p, ty.data(), ty.size(), cudaMemcpyHostToDevice, stream), "p2 add");
-  }
-  cudaCheck(cudaMemcpyAsync(ad.ptr.p, ptr.data(), ptr.size() * sizeof(int), cudaMemcpyHostToDevice, stream), "p2 add");
-  // colour of every slot (the colour of the DoF it holds; bit 7 set on the owner slot): from the
-  // DoF's barycentric weights in ascending vertex-ID order (b0, b1, b2, b3), parity class
-  // p = (b1 & 1) | (b2 & 1) << 1 | (b3 & 1) << 2; p = 0 (micro-vertices of the coarse level) is
-  // split into ((b1 >> 1) + 2 (b2 >> 1) + 3 (b3 >> 1)) mod 4, the others are colours 3 + p
-  std::vector<unsigned char> col((size_t)ld.lay->total, 0x7f);
-  const bool keepOwners = ld.lay->total <= (int64_t(1) << 20);  // small (coarse) levels only
-  for (int k = 0; k < 4; ++k)
-    for (size_t pr = 0; pr < ld.lay->off[k].size(); ++pr)
-      for (int64_t loc = 0; loc < ld.lay->size[k][pr]; ++loc) {
-        const Bary b = disc.slotBary(Lf, k, (int)pr, loc);
-        int64_t w[4] = {0, 0, 0, 0};
-        for (int i = 0; i < b.n; ++i) w[i] = b.b[i];
-        const int par = int(w[1] & 1) | (int(w[2] & 1) << 1) | (int(w[3] & 1) << 2);
-        int c = par ? 3 + par : int(((w[1] >> 1) + 2 * (w[2] >> 1) + 3 * (w[3] >> 1)) % 4);
-        const Slot o = disc.owner(Lf, b);
-        if (o.kind == k && o.prim == (int)pr && o.local == loc) {
-          c |= 0x80;
-          if (!keepOwners) {
-            col[(size_t)(ld.lay->off[k][pr] + loc)] = (unsigned char)c;
+  // SOR colour of a DoF from its barycentric weights in ascending vertex-ID order (b0, b1, b2, b3),
+  // parity class p = (b1 & 1) | (b2 & 1) << 1 | (b3 & 1) << 2: p = 0 (micro-vertices of the coarse
+  // level) is split into ((b1 >> 1) + 2 (b2 >> 1) + 3 (b3 >> 1)) mod 4, the others are colours 3 + p
+  auto colourOf = [](const Bary& b) {
+    int64_t w[4] = {0, 0, 0, 0};
+    for (int i = 0; i < b.n; ++i) w[i] = b.b[i];
+    const int par = int(w[1] & 1) | (int(w[2] & 1) << 1) | (int(w[3] & 1) << 2);
+    return par ? 3 + par : int(((w[1] >> 1) + 2 * (w[2] >> 1) + 3 * (w[3] >> 1)) % 4);
+  };
+  // The closure nodes of every cell in the order of the cell-closure halo group (cell, Z, Y, X),
+  // which gives each its owner.
+  const auto& cd = lay.commDst[G_CELL];
+  const auto& cs = lay.commSrc[G_CELL];
+  std::vector<dev::P2ClosureNode> nodes;
+  std::vector<unsigned char> nodeColour;
+  nodes.reserve(cd.size());
+  nodeColour.reserve(cd.size());
+  for (int c = 0; c < ld.lv.nCells; ++c)
+    for (int64_t Z = 0; Z <= M; ++Z)
+      for (int64_t Y = 0; Y + Z <= M; ++Y)
+        for (int64_t X = 0; X + Y + Z <= M; ++X) {
+          if (X != 0 && Y != 0 && Z != 0 && X + Y + Z != M) {
+            X = M - Y - Z - 1;  // on to the last node of the row
             continue;
           }
-          ad.hostOwner.push_back(ld.lay->off[k][pr] + loc);
-          ad.hostOwnerType.push_back(k == KC   ? ld.hostCellType[pr]
-                                     : k == KF ? ld.hostFaceType[pr]
-                                     : k == KE ? ld.hostLowType[pr]
-                                               : ld.hostLowType[ld.lv.nEdges + pr]);
+          const size_t i = nodes.size();
+          argCheck(i < cd.size() && cd[i] == lay.off[KC][c] + cellIdx(lay.w, X, Y, Z), "closure order");
+          const int64_t wts[4] = {M - X - Y - Z, X, Y, Z};
+          nodeColour.push_back((unsigned char)colourOf(makeBary(topo.cells[c].v, wts, 4)));
+          nodes.push_back({c, (unsigned short)X, (unsigned short)Y, (unsigned short)Z,
+                           (signed char)p2ClosureEntry(X, Y, Z, M), 0});
         }
-        col[(size_t)(ld.lay->off[k][pr] + loc)] = (unsigned char)c;
-      }
-  ad.colour.alloc(col.size());
-  cudaCheck(cudaMemcpyAsync(ad.colour.p, col.data(), col.size(), cudaMemcpyHostToDevice, stream), "p2 colour");
-  // the parity class of each colour's interior nodes per cell: an edge class is one colour in a
-  // cell's frame (read at its interior node nearest the origin), the vertex class holds colours 0-3
-  {
-    const int64_t M = ld.lv.N, w = M + 1;
-    auto tet = [](int64_t n) { return n * (n + 1) * (n + 2) / 6; };
-    std::vector<signed char> cls((size_t)ld.lv.nCells * 12, -1);
-    auto colourAt = [&](int c, int64_t X, int64_t Y, int64_t Z) {
-      const int64_t loc = tet(w) - tet(w - Z) + Y * (w - Z + 1) - Y * (Y + 1) / 2 + X;
-      return col[(size_t)(ld.lay->off[KC][c] + loc)] & 0x7f;
-    };
-    for (int c = 0; c < ld.lv.nCells; ++c) {
-      for (int k = 0; k < 4 && M >= 8; ++k) cls[(size_t)c * 12 + k] = 0;
-      // step of the vertex colour along a row (1 when a row holds at most one interior vertex node)
-      cls[(size_t)c * 12 + 11] = (signed char)(M >= 16 ? (colourAt(c, 4, 2, 2) - colourAt(c, 2, 2, 2)) & 3 : 1);
-      argCheck(cls[(size_t)c * 12 + 11] != 0, "P2 vertex colours do not change along a row");
-      for (int pc = 1; pc < 8; ++pc) {
-        const int64_t X = (pc & 1) ? 1 : 2, Y = (pc & 2) ? 1 : 2, Z = (pc & 4) ? 1 : 2;
-        if (X + Y + Z > M - 1) continue;
-        const int colr = colourAt(c, X, Y, Z);
-        argCheck(colr >= 4 && colr < 11 && cls[(size_t)c * 12 + colr] < 0, "P2 colour classes are inconsistent");
-        cls[(size_t)c * 12 + colr] = (signed char)pc;
-      }
-    }
-    ad.classOfColour.alloc(cls.size());
-    cudaCheck(cudaMemcpyAsync(ad.classOfColour.p, cls.data(), cls.size(), cudaMemcpyHostToDevice, stream), "p2 colour");
-    // closure nodes of every cell grouped by colour (then by face-stencil entry, so that the warps
-    // of the list kernel mostly run one stencil)
-    auto faceEntry = [](int f, int pc) {
-      switch (f) {
-        case 0: return pc;
-        case 1: return 4 + ((pc & 1) | ((pc >> 1) & 2));
-        case 2: return 8 + (((pc >> 1) & 1) | ((pc >> 1) & 2));
-        default: return 12 + (pc == 0 ? 0 : pc == 3 ? 1 : pc == 5 ? 2 : 3);
-      }
-    };
-    std::vector<std::pair<int, dev::P2ClosureNode>> nodes;
-    for (int c = 0; c < ld.lv.nCells; ++c)
-      for (int64_t Z = 0; Z <= M; ++Z)
-        for (int64_t Y = 0; Y <= M - Z; ++Y)
-          for (int64_t X = 0; X <= M - Z - Y; ++X) {
-            const bool on[4] = {Z == 0, Y == 0, X == 0, X + Y + Z == M};
-            const int nOn = on[0] + on[1] + on[2] + on[3];
-            if (nOn == 0) continue;
-            int k = -1;
-            if (nOn == 1) {
-              const int f = on[0] ? 0 : on[1] ? 1 : on[2] ? 2 : 3;
-              k = faceEntry(f, int((X & 1) | ((Y & 1) << 1) | ((Z & 1) << 2)));
-            }
-            dev::P2ClosureNode nd{c, (unsigned short)X, (unsigned short)Y, (unsigned short)Z, (signed char)k, 0};
-            nodes.push_back({colourAt(c, X, Y, Z) * 32 + (k + 1), nd});
-          }
-    std::stable_sort(nodes.begin(), nodes.end(), [](const auto& a, const auto& b) { return a.first < b.first; });
-    std::vector<dev::P2ClosureNode> list(nodes.size());
-    for (int k = 0; k < 12; ++k) ad.closureBegin[k] = 0;
-    int cur = 0;
-    for (size_t i = 0; i < nodes.size(); ++i) {
-      list[i] = nodes[i].second;
-      const int colr = nodes[i].first / 32;
-      argCheck(colr < 11, "closure node without an SOR colour");
-      while (cur < colr) ad.closureBegin[++cur] = (int)i;
-    }
-    while (cur < 11) ad.closureBegin[++cur] = (int)nodes.size();
-    // the owner updates by colour: face, edge and vertex owners (indices into the owner table)
-    // and, for the vertex colours, the interior vertex nodes of the cells
-    std::vector<std::vector<int>> addBy(11);
-    for (size_t i = 0; i < own.size(); ++i) addBy[col[(size_t)own[i]] & 0x7f].push_back((int)i);
-    std::vector<std::vector<int64_t>> innerBy(4);
-    std::vector<std::vector<unsigned char>> innerTy(4);
-    for (int c = 0; c < ld.lv.nCells; ++c)
-      for (int64_t Z = 2; Z <= M - 1; Z += 2)
-        for (int64_t Y = 2; Y + Z <= M - 1; Y += 2)
-          for (int64_t X = 2; X + Y + Z <= M - 1; X += 2) {
-            const int colr = colourAt(c, X, Y, Z);
-            const int64_t loc = tet(w) - tet(w - Z) + Y * (w - Z + 1) - Y * (Y + 1) / 2 + X;
-            innerBy[colr].push_back(ld.lay->off[KC][c] + loc);
-            innerTy[colr].push_back(ld.hostCellType[c]);
-          }
-    std::vector<int> addFlat;
-    std::vector<int64_t> innerFlat;
-    std::vector<unsigned char> innerTyFlat;
-    for (int k = 0; k < 11; ++k) {
-      ad.updAddBegin[k] = (int)addFlat.size();
-      addFlat.insert(addFlat.end(), addBy[k].begin(), addBy[k].end());
-      ad.updInnerBegin[k] = (int)innerFlat.size();
-      if (k < 4) {
-        innerFlat.insert(innerFlat.end(), innerBy[k].begin(), innerBy[k].end());
-        innerTyFlat.insert(innerTyFlat.end(), innerTy[k].begin(), innerTy[k].end());
-      }
-    }
-    ad.updAddBegin[11] = (int)addFlat.size();
-    ad.updInnerBegin[11] = (int)innerFlat.size();
-    ad.updAdd.alloc(std::max<size_t>(1, addFlat.size()) * sizeof(int));
-    ad.updInner.alloc(std::max<size_t>(1, innerFlat.size()) * sizeof(int64_t));
-    ad.updInnerType.alloc(std::max<size_t>(1, innerTyFlat.size()));
-    if (!addFlat.empty())
-      cudaCheck(cudaMemcpyAsync(ad.updAdd.p, addFlat.data(), addFlat.size() * sizeof(int), cudaMemcpyHostToDevice, stream),
-                "p2 update lists");
-    if (!innerFlat.empty()) {
-      cudaCheck(cudaMemcpyAsync(ad.updInner.p, innerFlat.data(), innerFlat.size() * sizeof(int64_t),
-                                cudaMemcpyHostToDevice, stream),
-                "p2 update lists");
-      cudaCheck(cudaMemcpyAsync(ad.updInnerType.p, innerTyFlat.data(), innerTyFlat.size(), cudaMemcpyHostToDevice, stream),
-                "p2 update lists");
-    }
-    ad.closureList.alloc(std::max<size_t>(1, list.size()) * sizeof(dev::P2ClosureNode));
-    if (!list.empty())
-      cudaCheck(cudaMemcpyAsync(ad.closureList.p, list.data(), list.size() * sizeof(dev::P2ClosureNode),
-                                cudaMemcpyHostToDevice, stream),
-                "p2 closure list");
+  argCheck(nodes.size() == cd.size(), "closure order");
+  // owner <- its copies, owners ascending, copies in table order (a counting sort on the owners,
+  // which lie behind the cell arrays)
+  const int64_t first = ld.nonCellBegin, nSlots = lay.total - first;
+  std::vector<int> copyCount((size_t)nSlots, 0);
+  std::vector<unsigned char> slotType((size_t)nSlots, 0), slotColour((size_t)nSlots, 0);
+  auto setType = [&](int kind, size_t pr, unsigned char t) {
+    std::fill_n(slotType.begin() + (lay.off[kind][pr] - first), lay.size[kind][pr], t);
+  };
+  for (size_t f = 0; f < topo.faces.size(); ++f) setType(KF, f, ld.hostFaceType[f]);
+  for (size_t e = 0; e < topo.edges.size(); ++e) setType(KE, e, ld.hostLowType[e]);
+  for (size_t v = 0; v < topo.verts.size(); ++v) setType(KV, v, ld.hostLowType[ld.lv.nEdges + v]);
+  for (size_t i = 0; i < cs.size(); ++i) {
+    argCheck(cs[i] >= first, "owner slot outside the face, edge and vertex arrays");
+    ++copyCount[(size_t)(cs[i] - first)];
+    slotColour[(size_t)(cs[i] - first)] = nodeColour[i];
   }
-  std::vector<unsigned char> mult((size_t)ld.lay->total, 1);
+  std::vector<int64_t> own;
+  std::vector<int> ptr{0}, next((size_t)nSlots, 0);
+  std::vector<unsigned char> ty;
+  for (int64_t q = 0; q < nSlots; ++q)
+    if (copyCount[(size_t)q]) {
+      next[(size_t)q] = ptr.back();
+      own.push_back(first + q);
+      ty.push_back(slotType[(size_t)q]);
+      ptr.push_back(ptr.back() + copyCount[(size_t)q]);
+    }
+  std::vector<int64_t> cp(cd.size());
+  for (size_t i = 0; i < cd.size(); ++i) cp[(size_t)next[(size_t)(cs[i] - first)]++] = cd[i];
+  ad.n = (int)own.size();
+  put(ad.owner, own.data(), own.size() * sizeof(int64_t));
+  put(ad.ptr, ptr.data(), ptr.size() * sizeof(int));
+  put(ad.copies, cp.data(), cp.size() * sizeof(int64_t));
+  put(ad.type, ty.data(), ty.size());
+  // the owner slot and DoF type of every DoF, in slot order per kind (coarse levels only)
+  if (lay.total <= (int64_t(1) << 20)) {
+    auto add = [&](int64_t slot, unsigned char t) {
+      ad.hostOwner.push_back(slot);
+      ad.hostOwnerType.push_back(t);
+    };
+    for (size_t v = 0; v < topo.verts.size(); ++v) add(lay.off[KV][v], ld.hostLowType[ld.lv.nEdges + v]);
+    for (size_t e = 0; e < topo.edges.size(); ++e)
+      for (int64_t x = 1; x < M; ++x) add(lay.off[KE][e] + x, ld.hostLowType[e]);
+    for (size_t f = 0; f < topo.faces.size(); ++f)
+      for (int64_t y = 1; y < M; ++y)
+        for (int64_t x = 1; x + y < M; ++x) add(lay.off[KF][f] + faceIdx(lay.w, x, y), ld.hostFaceType[f]);
+    for (size_t c = 0; c < topo.cells.size(); ++c)
+      for (int64_t z = 1; z < M; ++z)
+        for (int64_t y = 1; y + z < M; ++y)
+          for (int64_t x = 1; x + y + z < M; ++x) add(lay.off[KC][c] + cellIdx(lay.w, x, y, z), ld.hostCellType[c]);
+  }
+  // SOR: closure nodes by colour, then by entry, so that the warps mostly run one stencil
+  {
+    std::vector<size_t> bucket(11 * 32 + 1, 0);
+    auto key = [&](size_t i) { return (size_t)nodeColour[i] * 32 + (size_t)nodes[i].k; };
+    for (size_t i = 0; i < nodes.size(); ++i) ++bucket[key(i) + 1];
+    for (size_t k = 0; k + 1 < bucket.size(); ++k) bucket[k + 1] += bucket[k];
+    for (int k = 0; k <= 11; ++k) ad.closureBegin[k] = (int)bucket[(size_t)k * 32];
+    std::vector<dev::P2ClosureNode> list(nodes.size());
+    for (size_t i = 0; i < nodes.size(); ++i) list[bucket[key(i)]++] = nodes[i];
+    put(ad.closureList, list.data(), list.size() * sizeof(dev::P2ClosureNode));
+    // owners by colour
+    std::vector<dev::P2Owner> owners;
+    owners.reserve(own.size());
+    for (int k = 0; k < 11; ++k) {
+      ad.sorOwnerBegin[k] = (int)owners.size();
+      for (size_t i = 0; i < own.size(); ++i)
+        if (slotColour[(size_t)(own[i] - first)] == k)
+          owners.push_back({(unsigned)own[i], ptr[i], (unsigned short)(ptr[i + 1] - ptr[i]), ty[i]});
+    }
+    ad.sorOwnerBegin[11] = (int)owners.size();
+    argCheck(owners.size() == own.size(), "owner without an SOR colour");
+    const std::vector<unsigned> cp32(cp.begin(), cp.end());
+    put(ad.sorOwners, owners.data(), owners.size() * sizeof(dev::P2Owner));
+    put(ad.sorCopies, cp32.data(), cp32.size() * sizeof(unsigned));
+    // interior nodes by class
+    argCheck(M <= 1024, "P2 smoother: lattice too large");
+    std::vector<unsigned> inner(dev::kP2NodeHead);
+    for (int pc = 0; pc < 8; ++pc) {
+      inner[(size_t)pc] = (unsigned)inner.size();
+      for (int64_t Z = pc & 4 ? 1 : 2; Z <= M - 1; Z += 2)
+        for (int64_t Y = pc & 2 ? 1 : 2; Y + Z <= M - 1; Y += 2)
+          for (int64_t X = pc & 1 ? 1 : 2; X + Y + Z <= M - 1; X += pc ? 2 : 8)
+            inner.push_back((unsigned)(X | Y << 10 | Z << 20));
+    }
+    inner[8] = (unsigned)inner.size();
+    put(ad.sorInner, inner.data(), inner.size() * sizeof(unsigned));
+    ad.sorVertexNodes = (int)(inner[1] - inner[0]);
+    ad.sorEdgeNodes = 0;
+    for (int pc = 1; pc < 8; ++pc) ad.sorEdgeNodes = std::max(ad.sorEdgeNodes, (int)(inner[pc + 1] - inner[pc]));
+    // colours in the cells' frames: rank of a cell's vertex i among its vertex IDs
+    std::vector<dev::P2CellColour> cc((size_t)ld.lv.nCells);
+    for (int c = 0; c < ld.lv.nCells; ++c) {
+      const int* v = topo.cells[c].v;
+      int rank[4];
+      for (int i = 0; i < 4; ++i) {
+        rank[i] = 0;
+        for (int j = 0; j < 4; ++j) rank[i] += v[j] < v[i];
+      }
+      dev::P2CellColour& q = cc[(size_t)c];
+      for (int k = 0; k < 11; ++k) q.cls[k] = k < 4 ? 0 : -1;
+      q.c0 = (unsigned char)((rank[0] * (M / 2)) & 3);
+      q.cx = (unsigned char)((rank[1] - rank[0]) & 3);
+      q.cy = (unsigned char)((rank[2] - rank[0]) & 3);
+      q.cz = (unsigned char)((rank[3] - rank[0]) & 3);
+      for (int pc = 1; pc < 8; ++pc) {
+        const int odd[4] = {(pc ^ (pc >> 1) ^ (pc >> 2)) & 1, pc & 1, (pc >> 1) & 1, (pc >> 2) & 1};
+        int par = 0;
+        for (int i = 0; i < 4; ++i)
+          if (odd[i] && rank[i] > 0) par |= 1 << (rank[i] - 1);
+        argCheck(par != 0 && q.cls[3 + par] < 0, "P2 colour classes are inconsistent");
+        q.cls[3 + par] = (signed char)pc;
+      }
+    }
+    put(ad.sorCells, cc.data(), cc.size() * sizeof(dev::P2CellColour));
+    cudaCheck(cudaStreamSynchronize(stream), "p2 tables");  // the host lists go out of scope
+  }
+  std::vector<unsigned char> mult((size_t)lay.total, 1);
   for (size_t i = 0; i + 1 < ptr.size(); ++i)
     for (int k = ptr[i]; k < ptr[i + 1]; ++k) mult[(size_t)cp[k]] = (unsigned char)(ptr[i + 1] - ptr[i]);
-  ad.mult.alloc(mult.size());
-  cudaCheck(cudaMemcpyAsync(ad.mult.p, mult.data(), mult.size(), cudaMemcpyHostToDevice, stream), "p2 mult");
-  const std::vector<dev::P2Item> items = p2Items(ld.lv.N);
+  put(ad.mult, mult.data(), mult.size());
+  const std::vector<dev::P2Item> items = p2Items((int)M);
   ad.nItems = (int)items.size();
-  ad.items.alloc(items.size() * sizeof(dev::P2Item));
-  cudaCheck(cudaMemcpyAsync(ad.items.p, items.data(), items.size() * sizeof(dev::P2Item), cudaMemcpyHostToDevice, stream),
-            "p2 items");
-  cudaCheck(cudaStreamSynchronize(stream), "p2 add");
+  put(ad.items, items.data(), items.size() * sizeof(dev::P2Item));
+  cudaCheck(cudaStreamSynchronize(stream), "p2 tables");
   ad.built = true;
   return ad;
 }
@@ -1224,31 +1220,29 @@ static std::vector<double> p2FaceStencils(const std::vector<double>& K, int nCel
   return S;
 }
 
-// Cell sweep + additive owner sums for one P2 level: dst = A src, rhs - A src or diag(A) on the
-// flagged DoFs. The copies of dst are not refreshed here.
+// Sums of the cells' shares into the owners: dst = sum, or rhs - sum for a residual.
+template <class T, int MODE>
+void Storage::p2AddOwners(const P2Additive& ad, T* dst, const T* rhs, unsigned mask) {
+  if (!ad.n) return;
+  dev::p2AddKernel<T, MODE><<<(ad.n + dev::kBlock - 1) / dev::kBlock, dev::kBlock, 0, stream>>>(
+      (const int64_t*)ad.owner.p, (const int*)ad.ptr.p, (const int64_t*)ad.copies.p, (const unsigned char*)ad.type.p,
+      ad.n, dst, rhs, mask);
+  ++launches;
+}
+
+// Cell sweep + additive owner sums for one P2 level: dst = A src or rhs - A src on the flagged
+// DoFs. The copies of dst are not refreshed here.
 template <class T, int MODE>
 void Storage::p2Launch(P2Operator& o, int L, T* dst, const T* src, const T* rhs, unsigned mask) {
   const int Lf = L + 1;
   const LevelData& ld = levels[Lf];
   P2Additive& ad = p2Additive(Lf);
-  const T* K = (const T*)(sizeof(T) == 8 ? o.kd[L - o.minL]->p : o.kf[L - o.minL]->p);
-  if constexpr (MODE == dev::MODE_DIAG) {
-    const int nb = ld.lv.nCells * (ld.lv.N + 1);
-    dev::p2CellKernel<T, MODE><<<nb, dev::kBlock, 0, stream>>>(ld.lv, p2TablesOnce(), K, dst, src, rhs, mask);
-  } else {
-    const T* W = (const T*)(sizeof(T) == 8 ? o.sd[L - o.minL]->p : o.sf[L - o.minL]->p);
-    const T* FW = (const T*)(sizeof(T) == 8 ? o.fd[L - o.minL]->p : o.ff[L - o.minL]->p);
-    dev::p2ApplyKernel<T, MODE><<<ld.lv.nCells * ad.nItems, dev::kBlock, dev::p2TileSmem<T>(), stream>>>(
-        ld.lv, p2TablesOnce(), (const dev::P2Item*)ad.items.p, W, FW, K, dst, src, rhs, mask);
-  }
+  const T* W = (const T*)(sizeof(T) == 8 ? o.sd[L - o.minL]->p : o.sf[L - o.minL]->p);
+  const T* FW = (const T*)(sizeof(T) == 8 ? o.fd[L - o.minL]->p : o.ff[L - o.minL]->p);
+  dev::p2ApplyKernel<T, MODE><<<ld.lv.nCells * ad.nItems, dev::kBlock, dev::p2TileSmem<T>(), stream>>>(
+      ld.lv, (const dev::P2Item*)ad.items.p, W, FW, dst, src, rhs, mask);
   ++launches;
-  if (ad.n) {
-    constexpr int AM = MODE == dev::MODE_RESIDUAL ? dev::MODE_RESIDUAL : dev::MODE_REPLACE;
-    dev::p2AddKernel<T, AM><<<(ad.n + dev::kBlock - 1) / dev::kBlock, dev::kBlock, 0, stream>>>(
-        (const int64_t*)ad.owner.p, (const int*)ad.ptr.p, (const int64_t*)ad.copies.p, (const unsigned char*)ad.type.p,
-        ad.n, dst, rhs, mask);
-    ++launches;
-  }
+  p2AddOwners<T, MODE>(ad, dst, rhs, mask);
   cudaCheck(cudaGetLastError(), "P2 kernels");
 }
 
@@ -1290,10 +1284,19 @@ int Storage::p2Diagonal(int opId, int L, int prec) {
   if (it != o.diag.end()) return it->second;
   const int Lf = L + 1;
   const int d = createFunction(Lf, Lf, prec);
-  if (prec == 8)
-    p2Launch<double, dev::MODE_DIAG>(o, L, (double*)data(d, Lf), nullptr, nullptr, HG_ALL);
-  else
-    p2Launch<float, dev::MODE_DIAG>(o, L, (float*)data(d, Lf), nullptr, nullptr, HG_ALL);
+  const LevelData& ld = levels[Lf];
+  const P2Additive& ad = p2Additive(Lf);
+  auto run = [&](auto zero) {
+    using T = decltype(zero);
+    const T* K = (const T*)(sizeof(T) == 8 ? o.kd[L - o.minL]->p : o.kf[L - o.minL]->p);
+    dev::p2DiagonalKernel<T><<<ld.lv.nCells * (ld.lv.N + 1), dev::kBlock, 0, stream>>>(ld.lv, p2TablesOnce(), K,
+                                                                                     (T*)data(d, Lf));
+    ++launches;
+    p2AddOwners<T, dev::MODE_REPLACE>(ad, (T*)data(d, Lf), nullptr, HG_ALL);
+  };
+  if (prec == 8) run(0.0);
+  else run(0.0f);
+  cudaCheck(cudaGetLastError(), "P2 diagonal");
   communicate(d, Lf, kAllGroups);
   o.diag[key] = d;
   return d;
@@ -1304,60 +1307,34 @@ void Storage::p2SorT(P2Operator& o, int opId, int x, int b, int L, unsigned mask
   const int Lf = L + 1;
   const int prec = (int)sizeof(T);
   const int dg = p2Diagonal(opId, L, prec);
-  const auto key = p2ScratchKey(Lf, prec);
-  if (!p2scratch.count(key)) p2scratch[key] = createFunction(Lf, Lf, prec);
-  const int ax = p2scratch[key];
+  const int ax = p2Scratch(Lf, prec);
   const LevelData& ld = levels[Lf];
   P2Additive& ad = p2Additive(Lf);
-  const T* K = (const T*)(sizeof(T) == 8 ? o.kd[L - o.minL]->p : o.kf[L - o.minL]->p);
   const T* W = (const T*)(sizeof(T) == 8 ? o.sd[L - o.minL]->p : o.sf[L - o.minL]->p);
   const T* FW = (const T*)(sizeof(T) == 8 ? o.fd[L - o.minL]->p : o.ff[L - o.minL]->p);
-  const unsigned char* col = (const unsigned char*)ad.colour.p;
+  const dev::P2CellColour* cells = (const dev::P2CellColour*)ad.sorCells.p;
+  T* xd = (T*)data(x, Lf);
+  const T* bd = (const T*)data(b, Lf);
+  T* axd = (T*)data(ax, Lf);
+  auto blocks = [](int n) { return (n + dev::kBlock - 1) / dev::kBlock; };
+  communicate(x, Lf, 1 << G_CELL);
   for (int k = 0; k < 11; ++k) {
     const int c = backwards ? 10 - k : k;
-    // the cell-closure copies: all at the first colour; after that the owners kernel of each colour
-    // writes its owners' new values into their copies
-    if (k == 0) communicate(x, Lf, 1 << G_CELL);
-    T* xd = (T*)data(x, Lf);
-    const T* bd = (const T*)data(b, Lf);
-    T* axd = (T*)data(ax, Lf);
-    // face, edge and vertex DoFs of colour c: each cell's share of A x from the pass's start values
-    // (the colours of DoFs on different primitives are defined in different vertex frames, so a
-    // closure DoF may couple to an interior DoF of the same colour: its share is taken first)
-    const int nList = ad.closureBegin[c + 1] - ad.closureBegin[c];
-    if (nList > 0) {
-      dev::p2ClosureListKernel<T><<<(nList + dev::kBlock - 1) / dev::kBlock, dev::kBlock, 0, stream>>>(
-          ld.lv, p2TablesOnce(), K, FW, axd, xd, (const dev::P2ClosureNode*)ad.closureList.p + ad.closureBegin[c],
-          nList);
+    const int chunks = blocks(c < 4 ? ad.sorVertexNodes : ad.sorEdgeNodes);
+    const int nList = ad.closureBegin[c + 1] - ad.closureBegin[c], listBlocks = blocks(nList);
+    const int nOwn = ad.sorOwnerBegin[c + 1] - ad.sorOwnerBegin[c], ownBlocks = blocks(nOwn);
+    const int inner = ld.lv.nCells * chunks;
+    if (listBlocks + inner > 0) {
+      dev::p2SorGatherKernel<T><<<listBlocks + inner, dev::kBlock, 0, stream>>>(
+          ld.lv, W, FW, (const dev::P2ClosureNode*)ad.closureList.p + ad.closureBegin[c], nList, listBlocks,
+          (const unsigned*)ad.sorInner.p, cells, c, std::max(chunks, 1), xd, bd, axd, mask, omega);
       ++launches;
     }
-    // interior nodes of colour c. An edge colour is one parity class in a cell's frame and couples
-    // to no other node of its class, so those are updated in place (the closure copies keep their
-    // start values until the next refresh). The four vertex colours ((b1 + 2 b2 + 3 b3) / 2 mod 4
-    // in ascending vertex-ID order) separate the micro-edges along the macro-edges but not every
-    // diagonal micro-edge (barycentric step (1, -1, 1, -1)), so a vertex colour takes A x into the
-    // scratch first and is updated with the other owners.
-    const bool vertexColour = c < 4;
-    if (ld.lv.N >= 4) {
-      const signed char* cls = (const signed char*)ad.classOfColour.p;
-      if (vertexColour)
-        dev::p2StencilKernel<T, dev::MODE_REPLACE><<<ld.lv.nCells * (ld.lv.N - 3), dev::kBlock, 0, stream>>>(
-            ld.lv, W, axd, xd, nullptr, mask, col, cls, c, T(0));
-      else
-        dev::p2StencilKernel<T, dev::MODE_SOR><<<ld.lv.nCells * (ld.lv.N - 3), dev::kBlock, 0, stream>>>(
-            ld.lv, W, xd, xd, bd, mask, col, cls, c, omega);
-      ++launches;
-    }
-    // owner sums of the shares and the update of the face, edge and vertex DoFs (of the cell
-    // interiors too for a vertex colour)
-    const int nAdd = ad.updAddBegin[c + 1] - ad.updAddBegin[c];
-    const int nInner = ad.updInnerBegin[c + 1] - ad.updInnerBegin[c];
-    if (nAdd + nInner > 0) {
-      dev::p2SorOwnersKernel<T><<<(nAdd + nInner + dev::kBlock - 1) / dev::kBlock, dev::kBlock, 0, stream>>>(
-          (const int64_t*)ad.owner.p, (const int*)ad.ptr.p, (const int64_t*)ad.copies.p, (const unsigned char*)ad.type.p,
-          (const int*)ad.updAdd.p + ad.updAddBegin[c], nAdd, (const int64_t*)ad.updInner.p + ad.updInnerBegin[c],
-          (const unsigned char*)ad.updInnerType.p + ad.updInnerBegin[c], nInner, mask, xd, bd, axd,
-          (const T*)data(dg, Lf), omega);
+    if (ownBlocks + inner > 0) {
+      dev::p2SorUpdateKernel<T><<<ownBlocks + inner, dev::kBlock, 0, stream>>>(
+          ld.lv, (const dev::P2Owner*)ad.sorOwners.p + ad.sorOwnerBegin[c], nOwn, ownBlocks,
+          (const unsigned*)ad.sorCopies.p, (const unsigned*)ad.sorInner.p, cells, c, std::max(chunks, 1), xd, bd, axd,
+          (const T*)data(dg, Lf), mask, omega);
       ++launches;
     }
   }

@@ -12,6 +12,7 @@
 
 #include "discretization.hpp"
 #include "kernels.cuh"
+#include "p2_sor.cuh"
 
 namespace hg {
 
@@ -130,15 +131,13 @@ struct P2Additive {
   bool built = false;
   int n = 0;
   DevBuf owner, ptr, copies, type;
-  DevBuf colour;  // per slot: SOR colour of the DoF (0..10), bit 7 on its owner slot
   DevBuf mult;    // per slot: number of macro-cells holding the DoF (1 for cell-owned)
-  DevBuf classOfColour;  // per cell: [0..10] parity class of colour k's interior nodes (or -1), [11] vertex colour step
-  DevBuf updAdd;                            // owner-table indices of the face/edge/vertex DoFs by colour
-  int updAddBegin[12] = {0};
-  DevBuf updInner, updInnerType;            // interior vertex slots (and their cell's type) by colour
-  int updInnerBegin[12] = {0};
-  DevBuf closureList;                       // closure nodes of the cells (dev::P2ClosureNode) by colour
+  DevBuf closureList;                       // closure nodes of the cells (dev::P2ClosureNode) by SOR colour
   int closureBegin[12] = {0};               // first entry of colour k; closureBegin[11] = total
+  DevBuf sorOwners, sorCopies;              // the owners (dev::P2Owner) by colour and their copies
+  int sorOwnerBegin[12] = {0};
+  DevBuf sorInner, sorCells;                // interior nodes by class; the cells' colours (dev::P2CellColour)
+  int sorVertexNodes = 0, sorEdgeNodes = 0;  // entries of the vertex class, of the longest edge class
   DevBuf items;                             // work list of the apply (dev::P2Item), per macro-cell
   int nItems = 0;
   std::vector<int64_t> hostOwner;           // the owner slot of every DoF (levels up to 2^20 slots)
@@ -286,6 +285,8 @@ struct Storage {
   int p2Scratch(int Lf, int prec);
   template <class T, int MODE>
   void p2Launch(P2Operator& o, int L, T* dst, const T* src, const T* rhs, unsigned mask);
+  template <class T, int MODE>
+  void p2AddOwners(const P2Additive& ad, T* dst, const T* rhs, unsigned mask);
   template <class T>
   void p2SorT(P2Operator& o, int opId, int x, int b, int L, unsigned mask, T omega, bool backwards);
   // Re-assemble an operator's stencils from the current cell coefficients into its device

@@ -102,6 +102,28 @@ def test_p2_apply_inner_vertices_and_edges(cube3, L):
     assert rel(got, ref, inner) < 1e-13
 
 
+@pytest.mark.parametrize("backwards", [False, True])
+@pytest.mark.parametrize("dtype,tol", [(np.float64, 1e-13), (np.float32, 2e-5)])
+def test_p2_multicolour_sor_many_blocks(backwards, dtype, tol):
+    # lattice 32: several blocks of nodes per macro-cell and colour, groups of four vertex nodes cut
+    # by the sloped face
+    L = 4
+    st, orc, maps = setup(1, L)
+    node, owned = maps[L]
+    n = orc.n(L + 1)
+    rng = np.random.default_rng(90 + backwards)
+    u0, f0 = (rng.uniform(-1, 1, n).astype(dtype).astype(np.float64) for _ in range(2))
+    A = hg.P2ConstantLaplaceOperator(st, L, L)
+    x, b = hg.P2Function("x", st, L, L, dtype=dtype), hg.P2Function("b", st, L, L, dtype=dtype)
+    x.from_numpy(L, H.scatter(node, u0).astype(dtype))
+    b.from_numpy(L, H.scatter(node, f0).astype(dtype))
+    (A.smooth_sor_backwards if backwards else A.smooth_sor)(x, b, 0.8, L)
+    got = H.gather_owned(x.to_numpy(L).astype(np.float64), node, owned, n)
+    ref = orc.p2_sor(L, u0, f0, 0.8, sweeps=1, backwards=backwards)
+    inner = ~orc.dirichlet(L + 1)
+    assert rel(got, ref, inner) < tol
+
+
 @pytest.mark.parametrize("L", [0, 1, 2, 3])
 @pytest.mark.parametrize("backwards", [False, True])
 def test_p2_multicolour_sor(cube2, L, backwards):

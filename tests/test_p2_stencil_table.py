@@ -69,3 +69,31 @@ def test_face_stencils_are_constant_per_face_and_class():
                         assert valid == cand
                         assert all(X + dx >= 0 and Y + dy >= 0 and Z + dz >= 0 and X + Y + Z + dx + dy + dz <= M
                                    for dx, dy, dz in offs)
+
+
+def test_rim_stencils_are_constant_per_edge_and_vertex():
+    # at every node of an edge of a macro-cell (lattices 2..16) and at its vertices, the micro-cells
+    # inside the cell that hold the node are the generated candidates of the kernels' entry, and the
+    # stencil reads stay in the cell
+    gen = load_generator()
+    off = gen.node_offsets()
+    rs = gen.rim_stencils()
+    assert len(rs) == 16
+    for M in (2, 4, 8, 16):
+        N = M // 2
+        nodes = [(2 * e + (t & 1), [(t, 0, 0), (0, t, 0), (0, 0, t), (M - t, t, 0), (M - t, 0, t), (0, M - t, t)][e])
+                 for e in range(6) for t in range(1, M)]
+        nodes += [(12 + v, [(0, 0, 0), (M, 0, 0), (0, M, 0), (0, 0, M)][v]) for v in range(4)]
+        for k, q in nodes:
+            _, pc, cand, offs = rs[k]
+            assert (q[0] & 1) | ((q[1] & 1) << 1) | ((q[2] & 1) << 2) == pc
+            valid = []
+            for t in range(6):
+                for j in range(10):
+                    if tuple(c & 1 for c in off[t][j]) != tuple(c & 1 for c in q):
+                        continue
+                    a = [(c - o) >> 1 for c, o in zip(q, off[t][j])]
+                    if min(a) >= 0 and sum(a) < N - gen.WIDTH_REDUCTION[t]:
+                        valid.append((t, j))
+            assert valid == cand
+            assert all(min(c + d for c, d in zip(q, o)) >= 0 and sum(q) + sum(o) <= M for o in offs)
