@@ -152,6 +152,18 @@ def divt_stencils():
     return out
 
 
+def divt_closure_stencils():
+    """Per closure entry (faces by class, then the rim): the pressure-lattice offsets, relative to
+    (X >> 1, Y >> 1, Z >> 1), of the vertices of its micro-cells."""
+    off = node_offsets()
+    out = []
+    for _, pc, cand, _ in face_stencils() + rim_stencils():
+        par = (pc & 1, (pc >> 1) & 1, (pc >> 2) & 1)
+        s = {tuple((off[t][i][d] - off[t][j][d] + par[d]) // 2 for d in range(3)) for t, j in cand for i in range(4)}
+        out.append(sorted(s, key=lambda o: (o[2], o[1], o[0])))
+    return out
+
+
 def render():
     st = stencils()
     n = max(len(s) for s in st)
@@ -235,6 +247,26 @@ def render():
     lines.append("};")
     for pc, d in enumerate(dt):
         lines.append("using T%d = List<%s>;" % (pc, ", ".join("O<%d, %d, %d>" % o for o in d)))
+    dc = divt_closure_stencils()
+    n = len(dc)
+    lines += [
+        "",
+        "// The same at the closure nodes, by closure entry. The divergence at a closure pressure node reads",
+        "// the velocity nodes of the vertex-class entry of its face, edge or vertex.",
+        "constexpr int kDivTFaceMaxLen = %d;" % max(len(d) for d in dc),
+        "constexpr int kDivTFaceLen[%d] = {%s};" % (n, ", ".join(str(len(d)) for d in dc)),
+        "constexpr int kDivTFaceTotal = %d;" % sum(len(d) for d in dc),
+        "constexpr int kDivTFaceFirst[%d] = {%s};" % (n, ", ".join(str(sum(len(x) for x in dc[:k])) for k in range(n))),
+        "constexpr signed char kDivTFaceOff[%d][kDivTFaceMaxLen][3] = {" % n,
+    ]
+    for d in dc:
+        lines.append("    {" + ", ".join("{%d, %d, %d}" % o for o in d) + "},")
+    lines.append("};")
+    for k, d in enumerate(dc):
+        lines.append("using TF%d = List<%s>;" % (k, ", ".join("O<%d, %d, %d>" % o for o in d)))
+    lines += ["", "template <int K>", "struct DivTFaceList;"]
+    for k in range(n):
+        lines += ["template <>", "struct DivTFaceList<%d> {" % k, "  using type = TF%d;" % k, "};"]
     lines += ["", "template <int PC>", "struct DivTList;"]
     for pc in range(8):
         lines += ["template <>", "struct DivTList<%d> {" % pc, "  using type = T%d;" % pc, "};"]

@@ -849,7 +849,7 @@ static std::vector<double> symmetricPinv(std::vector<double>& A, int n) {
 StokesGmg::StokesGmg(Storage& st, int op_, int minL_, int maxL_, int pre_, int post_, double omega_, int sweeps)
     : s(st), op(op_), minL(minL_), maxL(maxL_), pre(pre_), post(post_), omega(omega_), velocitySweeps(sweeps) {
   P2Operator& o = s.p2op(op);
-  argCheck(!o.dd.empty(), "Stokes multigrid: not a Stokes operator");
+  argCheck(!o.wdivd.empty(), "Stokes multigrid: not a Stokes operator");
   argCheck(minL >= o.minL && maxL <= o.maxL && minL <= maxL, "Stokes multigrid: levels outside the operator's range");
   argCheck(pre >= 0 && post >= 0 && sweeps >= 1, "Stokes multigrid: invalid smoothing steps");
   for (int k = 0; k < 3; ++k) {
@@ -890,7 +890,7 @@ void StokesGmg::smooth(const int u[3], int p, const int f[3], int g, int L) {
   const unsigned fv = HG_INNER | HG_NEUMANN, fp = HG_ALL;
   const int Lv = L + 1;
   const double a[2] = {1.0, -1.0};
-  s.stokesDivT(op, p, ru, L, fv, false);
+  s.stokesDivT(op, p, ru, L, fv);
   for (int k = 0; k < 3; ++k) {
     const int src[2] = {f[k], ru[k]};
     s.lincomb(ru[k], Lv, fv, 2, a, src, false, 0.0);
@@ -965,7 +965,7 @@ double StokesGmg::estimateOmega(int L, int iters, uint64_t seed) {
   s.fillRandom(itv, L, all, seed, 0.0, 1.0);
   auto E = [&](int src, int dst) {
     for (int k = 0; k < 3; ++k) s.lincomb(ru[k], Lv, all, 0, nullptr, nullptr, false, 0.0);
-    s.stokesDivT(op, src, tu, L, all, false);
+    s.stokesDivT(op, src, tu, L, all);
     for (int i = 0; i < velocitySweeps; ++i)
       for (int k = 0; k < 3; ++k) s.p2Sor(op, ru[k], tu[k], 1.0, L, fv, false);
     s.stokesDiv(op, ru, dst, L, all);

@@ -16,6 +16,7 @@
 #include "kernels.cuh"
 #include "p2_apply.cuh"
 #include "p2_sor.cuh"
+#include "p2_stokes.cuh"
 #include "solvers.hpp"
 #include "storage.hpp"
 
@@ -1230,10 +1231,10 @@ void Storage::p2AddOwners(const P2Additive& ad, T* dst, const T* rhs, unsigned m
   ++launches;
 }
 
-// Cell sweep + additive owner sums for one P2 level: dst = A src or rhs - A src on the flagged
-// DoFs. The copies of dst are not refreshed here.
+// The cells' part of dst = A src or rhs - A src on one P2 level: final values at the interior nodes
+// of the flagged cells, shares of A src in the closure slots.
 template <class T, int MODE>
-void Storage::p2Launch(P2Operator& o, int L, T* dst, const T* src, const T* rhs, unsigned mask) {
+void Storage::p2Sweep(P2Operator& o, int L, T* dst, const T* src, const T* rhs, unsigned mask) {
   const int Lf = L + 1;
   const LevelData& ld = levels[Lf];
   P2Additive& ad = p2Additive(Lf);
@@ -1242,7 +1243,14 @@ void Storage::p2Launch(P2Operator& o, int L, T* dst, const T* src, const T* rhs,
   dev::p2ApplyKernel<T, MODE><<<ld.lv.nCells * ad.nItems, dev::kBlock, dev::p2TileSmem<T>(), stream>>>(
       ld.lv, (const dev::P2Item*)ad.items.p, W, FW, dst, src, rhs, mask);
   ++launches;
-  p2AddOwners<T, MODE>(ad, dst, rhs, mask);
+  cudaCheck(cudaGetLastError(), "P2 kernels");
+}
+
+// dst = A src or rhs - A src on the flagged DoFs. The copies of dst are not refreshed here.
+template <class T, int MODE>
+void Storage::p2Launch(P2Operator& o, int L, T* dst, const T* src, const T* rhs, unsigned mask) {
+  p2Sweep<T, MODE>(o, L, dst, src, rhs, mask);
+  p2AddOwners<T, MODE>(p2Additive(L + 1), dst, rhs, mask);
   cudaCheck(cudaGetLastError(), "P2 kernels");
 }
 
@@ -1554,170 +1562,149 @@ void Storage::p2Restrict(int id, int Lf, unsigned mask) {
   communicate(id, Lcf, kAllGroups);
 }
 
-// Interior coupling stencils of every cell from the divergence elements D[cell][t][k][i][j]:
-// div weights on p2s::kOff[0] (a pressure vertex i of micro-cell t sees node j at off_j - off_i),
-// divT weights on p2s::kDivTOff (velocity node j of class pc sees vertex i at (off_i - off_j + pc)/2).
-static void p2DivStencils(const std::vector<double>& D, int nCells, std::vector<double>& WD, std::vector<double>& WT) {
+// Coupling stencils of every cell from the divergence elements D[cell][t][k][i][j]. Interior: div
+// weights on p2s::kOff[0] (a pressure vertex i of micro-cell t sees node j at off_j - off_i), divT
+// weights on p2s::kDivTOff (velocity node j of class pc sees vertex i at (off_i - off_j + pc) / 2).
+// Closure: the same over the micro-cells of each closure entry, div on the vertex-class entries.
+struct DivStencils {
+  std::vector<double> div, divT, divClosure, divTClosure;
+};
+
+static DivStencils p2DivStencils(const std::vector<double>& D, int nCells) {
   const dev::P2Tables& tb = p2TablesOnce();
-  WD.assign((size_t)nCells * 195, 0.0);
-  WT.assign((size_t)nCells * 195, 0.0);
+  DivStencils S;
+  S.div.assign((size_t)nCells * 195, 0.0);
+  S.divT.assign((size_t)nCells * 195, 0.0);
+  S.divClosure.assign((size_t)nCells * 3 * p2s::kFaceTotal, 0.0);
+  S.divTClosure.assign((size_t)nCells * 3 * p2s::kDivTFaceTotal, 0.0);
   auto find = [](const signed char (*tab)[3], int len, int dx, int dy, int dz) {
     for (int e = 0; e < len; ++e)
       if (tab[e][0] == dx && tab[e][1] == dy && tab[e][2] == dz) return e;
     throw Error(HG_ERR_INTERNAL, "Taylor-Hood stencil table does not match the micro-cells");
+  };
+  auto velocity = [&](const signed char (*tab)[3], int len, int t, int i, int j) {
+    return find(tab, len, tb.off[t][j][0] - tb.off[t][i][0], tb.off[t][j][1] - tb.off[t][i][1],
+                tb.off[t][j][2] - tb.off[t][i][2]);
+  };
+  auto pressure = [&](const signed char (*tab)[3], int len, int pc, int t, int i, int j) {
+    return find(tab, len, (tb.off[t][i][0] - tb.off[t][j][0] + (pc & 1)) / 2,
+                (tb.off[t][i][1] - tb.off[t][j][1] + ((pc >> 1) & 1)) / 2,
+                (tb.off[t][i][2] - tb.off[t][j][2] + ((pc >> 2) & 1)) / 2);
   };
   for (int c = 0; c < nCells; ++c) {
     const double* Dc = D.data() + (size_t)c * 720;
     for (int t = 0; t < 6; ++t)
       for (int i = 0; i < 4; ++i)
         for (int j = 0; j < 10; ++j) {
-          const int e = find(p2s::kOff[0], p2s::kLen[0], tb.off[t][j][0] - tb.off[t][i][0],
-                             tb.off[t][j][1] - tb.off[t][i][1], tb.off[t][j][2] - tb.off[t][i][2]);
-          for (int k = 0; k < 3; ++k) WD[(size_t)c * 195 + k * 65 + e] += Dc[t * 120 + k * 40 + i * 10 + j];
+          const int e = velocity(p2s::kOff[0], p2s::kLen[0], t, i, j);
+          for (int k = 0; k < 3; ++k) S.div[(size_t)c * 195 + k * 65 + e] += Dc[t * 120 + k * 40 + i * 10 + j];
         }
-    for (int pc = 0; pc < 8; ++pc) {
-      const int par[3] = {pc & 1, (pc >> 1) & 1, (pc >> 2) & 1};
+    for (int pc = 0; pc < 8; ++pc)
       for (int q = 0; q < tb.nCand[pc]; ++q) {
         const int t = tb.cand[pc][q][0], j = tb.cand[pc][q][1];
         for (int i = 0; i < 4; ++i) {
-          const int e = find(p2s::kDivTOff[pc], p2s::kDivTLen[pc], (tb.off[t][i][0] - tb.off[t][j][0] + par[0]) / 2,
-                             (tb.off[t][i][1] - tb.off[t][j][1] + par[1]) / 2,
-                             (tb.off[t][i][2] - tb.off[t][j][2] + par[2]) / 2);
+          const int e = pressure(p2s::kDivTOff[pc], p2s::kDivTLen[pc], pc, t, i, j);
           for (int k = 0; k < 3; ++k)
-            WT[(size_t)c * 195 + k * 65 + p2s::kDivTFirst[pc] + e] += Dc[t * 120 + k * 40 + i * 10 + j];
+            S.divT[(size_t)c * 195 + k * 65 + p2s::kDivTFirst[pc] + e] += Dc[t * 120 + k * 40 + i * 10 + j];
+        }
+      }
+    for (int n = 0; n < p2s::kFaceStencils; ++n) {
+      const int pc = p2s::kFaceClass[n];
+      for (int q = 0; q < p2s::kFaceNCand[n]; ++q) {
+        const int t = p2s::kFaceCand[n][q][0], j = p2s::kFaceCand[n][q][1];
+        for (int i = 0; i < 4; ++i) {
+          const int e = pressure(p2s::kDivTFaceOff[n], p2s::kDivTFaceLen[n], pc, t, i, j);
+          for (int k = 0; k < 3; ++k)
+            S.divTClosure[((size_t)c * 3 + k) * p2s::kDivTFaceTotal + p2s::kDivTFaceFirst[n] + e] +=
+                Dc[t * 120 + k * 40 + i * 10 + j];
+        }
+        if (pc != 0) continue;
+        for (int m = 0; m < 10; ++m) {  // local node j of a vertex-class entry is pressure vertex j
+          const int e = velocity(p2s::kFaceOff[n], p2s::kFaceLen[n], t, j, m);
+          for (int k = 0; k < 3; ++k)
+            S.divClosure[((size_t)c * 3 + k) * p2s::kFaceTotal + p2s::kFaceFirst[n] + e] +=
+                Dc[t * 120 + k * 40 + j * 10 + m];
         }
       }
     }
   }
+  return S;
 }
 
 int Storage::createStokesOperator(int minL, int maxL) {
   const int id = createP2Operator(FORM_LAPLACE, minL, maxL);
   P2Operator& o = p2op(id);
+  auto up = [&](std::vector<std::unique_ptr<DevBuf>>& d64, std::vector<std::unique_ptr<DevBuf>>& d32,
+                const std::vector<double>& v) {
+    const std::vector<float> f(v.begin(), v.end());
+    d64.emplace_back(new DevBuf());
+    d64.back()->alloc(v.size() * sizeof(double));
+    cudaCheck(cudaMemcpyAsync(d64.back()->p, v.data(), v.size() * sizeof(double), cudaMemcpyHostToDevice, stream),
+              "div stencils");
+    d32.emplace_back(new DevBuf());
+    d32.back()->alloc(f.size() * sizeof(float));
+    cudaCheck(cudaMemcpyAsync(d32.back()->p, f.data(), f.size() * sizeof(float), cudaMemcpyHostToDevice, stream),
+              "div stencils");
+    cudaCheck(cudaStreamSynchronize(stream), "div stencils");
+  };
   for (int L = minL; L <= maxL; ++L) {
-    const std::vector<double> D = p2p1CellDiv(disc.topo(), L);
-    {
-      std::vector<double> WD, WT;
-      p2DivStencils(D, (int)disc.topo().cells.size(), WD, WT);
-      auto up = [&](std::vector<std::unique_ptr<DevBuf>>& dst, const std::vector<double>& v, bool fp32) {
-        dst.emplace_back(new DevBuf());
-        if (fp32) {
-          std::vector<float> f(v.begin(), v.end());
-          dst.back()->alloc(f.size() * sizeof(float));
-          cudaCheck(cudaMemcpyAsync(dst.back()->p, f.data(), f.size() * sizeof(float), cudaMemcpyHostToDevice, stream),
-                    "div stencils");
-          cudaCheck(cudaStreamSynchronize(stream), "div stencils");
-        } else {
-          dst.back()->alloc(v.size() * sizeof(double));
-          cudaCheck(cudaMemcpyAsync(dst.back()->p, v.data(), v.size() * sizeof(double), cudaMemcpyHostToDevice, stream),
-                    "div stencils");
-          cudaCheck(cudaStreamSynchronize(stream), "div stencils");
-        }
-      };
-      up(o.wdivd, WD, false);
-      up(o.wdivf, WD, true);
-      up(o.wdivtd, WT, false);
-      up(o.wdivtf, WT, true);
-    }
-    std::vector<float> Df(D.begin(), D.end());
-    o.dd.emplace_back(new DevBuf());
-    o.dd.back()->alloc(D.size() * sizeof(double));
-    cudaCheck(cudaMemcpyAsync(o.dd.back()->p, D.data(), D.size() * sizeof(double), cudaMemcpyHostToDevice, stream),
-              "div upload");
-    o.df.emplace_back(new DevBuf());
-    o.df.back()->alloc(Df.size() * sizeof(float));
-    cudaCheck(cudaMemcpyAsync(o.df.back()->p, Df.data(), Df.size() * sizeof(float), cudaMemcpyHostToDevice, stream),
-              "div upload");
-    cudaCheck(cudaStreamSynchronize(stream), "div upload");
+    const DivStencils S = p2DivStencils(p2p1CellDiv(disc.topo(), L), (int)disc.topo().cells.size());
+    up(o.wdivd, o.wdivf, S.div);
+    up(o.wdivtd, o.wdivtf, S.divT);
+    up(o.wdivcd, o.wdivcf, S.divClosure);
+    up(o.wdivtcd, o.wdivtcf, S.divTClosure);
   }
   return id;
 }
 
-// v_k = D_k^T p (or += with add) at the velocity DoFs flagged by maskV: shares into three scratch
-// functions, owner sums, then written where flagged.
-template <class T>
-static void stokesDivTImpl(Storage& st, P2Operator& o, int p, const int v[3], int L, unsigned maskV, bool add) {
+// D_k^T p into v_k: final at the interior nodes of the flagged cells, shares in the closure slots;
+// with ADD both are added to what is there.
+template <class T, bool ADD>
+static void launchDivT(Storage& st, P2Operator& o, int p, const int v[3], int L, unsigned maskV) {
   const int Lv = L + 1, Lp = L;
   const LevelData& lvv = st.levels[Lv];
   const LevelData& lvp = st.levels[Lp];
-  const T* D = (const T*)(sizeof(T) == 8 ? o.dd[L - o.minL]->p : o.df[L - o.minL]->p);
-  const int prec = (int)sizeof(T);
-  int sc[3];
-  for (int k = 0; k < 3; ++k) {
-    auto key = std::make_pair(Lv, 16 + 8 * k + prec);  // three distinct scratch buffers per level
-    if (!st.p2scratch.count(key)) st.p2scratch[key] = st.createFunction(Lv, Lv, prec);
-    sc[k] = st.p2scratch[key];
-  }
-  st.communicate(p, Lp, 1 << G_CELL);
   P2Additive& adv = st.p2Additive(Lv);
-  const bool interior = lvv.lv.N >= 4;
-  if (interior) {
-    const T* WT = (const T*)(sizeof(T) == 8 ? o.wdivtd[L - o.minL]->p : o.wdivtf[L - o.minL]->p);
-    dev::p2DivTStencilKernel<T><<<lvv.lv.nCells * (lvv.lv.N - 3), dev::kBlock, 0, st.stream>>>(
-        lvv.lv, lvp.lv, WT, (T*)st.data(sc[0], Lv), (T*)st.data(sc[1], Lv), (T*)st.data(sc[2], Lv),
-        (const T*)st.data(p, Lp), maskV);
-    ++st.launches;
-  }
-  const int nClosure = adv.closureBegin[11];
-  if (interior && nClosure > 0) {  // the closure nodes from the list, one thread each
-    dev::p2DivTClosureListKernel<T><<<(nClosure + dev::kBlock - 1) / dev::kBlock, dev::kBlock, 0, st.stream>>>(
-        lvv.lv, lvp.lv, p2TablesOnce(), D, (T*)st.data(sc[0], Lv), (T*)st.data(sc[1], Lv), (T*)st.data(sc[2], Lv),
-        (const T*)st.data(p, Lp), (const dev::P2ClosureNode*)adv.closureList.p, nClosure);
-  } else {
-    dev::p2DivTKernel<T><<<lvv.lv.nCells * (lvv.lv.N + 1), dev::kBlock, 0, st.stream>>>(
-        lvv.lv, lvp.lv, p2TablesOnce(), D, (T*)st.data(sc[0], Lv), (T*)st.data(sc[1], Lv), (T*)st.data(sc[2], Lv),
-        (const T*)st.data(p, Lp), maskV, interior);
-  }
+  const T* WT = (const T*)(sizeof(T) == 8 ? o.wdivtd[L - o.minL]->p : o.wdivtf[L - o.minL]->p);
+  const T* WC = (const T*)(sizeof(T) == 8 ? o.wdivtcd[L - o.minL]->p : o.wdivtcf[L - o.minL]->p);
+  const int nList = adv.closureBegin[11], listBlocks = (nList + dev::kBlock - 1) / dev::kBlock;
+  const int inner = lvv.lv.N >= 4 ? lvv.lv.nCells * (lvv.lv.N - 3) : 0;
+  dev::p2DivTKernel<T, ADD><<<listBlocks + inner, dev::kBlock, 0, st.stream>>>(
+      lvv.lv, lvp.lv, WT, WC, (const dev::P2ClosureNode*)adv.closureList.p, nList, listBlocks, (T*)st.data(v[0], Lv),
+      (T*)st.data(v[1], Lv), (T*)st.data(v[2], Lv), (const T*)st.data(p, Lp), maskV);
   ++st.launches;
-  for (int k = 0; k < 3; ++k) {
-    if (adv.n)
-      dev::p2AddKernel<T, dev::MODE_REPLACE><<<(adv.n + dev::kBlock - 1) / dev::kBlock, dev::kBlock, 0, st.stream>>>(
-          (const int64_t*)adv.owner.p, (const int*)adv.ptr.p, (const int64_t*)adv.copies.p,
-          (const unsigned char*)adv.type.p, adv.n, (T*)st.data(sc[k], Lv), nullptr, maskV);
-    const double one = 1.0;
-    st.lincomb(v[k], Lv, maskV, 1, &one, &sc[k], add, 0.0);
-    st.communicate(v[k], Lv, (1 << G_COUNT) - 1);
-    st.launches += adv.n ? 1 : 0;
-  }
-  cudaCheck(cudaGetLastError(), "Stokes divT");
 }
 
-// q = sum_k D_k u_k at the pressure DoFs flagged by maskP.
+// q = sum_k D_k u_k: final at the interior nodes of the flagged cells, shares in the closure slots,
+// then the owners' sums. The closure copies of u hold their owners' values.
 template <class T>
-static void stokesDivImpl(Storage& st, P2Operator& o, const int u[3], int q, int L, unsigned maskP) {
+static void launchDiv(Storage& st, P2Operator& o, const int u[3], int q, int L, unsigned maskP) {
   const int Lv = L + 1, Lp = L;
   const LevelData& lvv = st.levels[Lv];
   const LevelData& lvp = st.levels[Lp];
-  const T* D = (const T*)(sizeof(T) == 8 ? o.dd[L - o.minL]->p : o.df[L - o.minL]->p);
-  for (int k = 0; k < 3; ++k) st.communicate(u[k], Lv, 1 << G_CELL);
   P2Additive& adp = st.p2Additive(Lp);
-  const bool interior = lvp.lv.N >= 4;
-  if (interior) {
-    const T* WD = (const T*)(sizeof(T) == 8 ? o.wdivd[L - o.minL]->p : o.wdivf[L - o.minL]->p);
-    dev::p2DivStencilKernel<T><<<lvp.lv.nCells * (lvp.lv.N - 3), dev::kBlock, 0, st.stream>>>(
-        lvp.lv, lvv.lv, WD, (T*)st.data(q, Lp), (const T*)st.data(u[0], Lv), (const T*)st.data(u[1], Lv),
-        (const T*)st.data(u[2], Lv), maskP);
-    ++st.launches;
-  }
-  const int nClosure = adp.closureBegin[11];
-  if (interior && nClosure > 0) {
-    dev::p2DivClosureListKernel<T><<<(nClosure + dev::kBlock - 1) / dev::kBlock, dev::kBlock, 0, st.stream>>>(
-        lvp.lv, lvv.lv, p2TablesOnce(), D, (T*)st.data(q, Lp), (const T*)st.data(u[0], Lv), (const T*)st.data(u[1], Lv),
-        (const T*)st.data(u[2], Lv), (const dev::P2ClosureNode*)adp.closureList.p, nClosure);
-  } else {
-    dev::p2DivKernel<T><<<lvp.lv.nCells * (lvp.lv.N + 1), dev::kBlock, 0, st.stream>>>(
-        lvp.lv, lvv.lv, p2TablesOnce(), D, (T*)st.data(q, Lp), (const T*)st.data(u[0], Lv), (const T*)st.data(u[1], Lv),
-        (const T*)st.data(u[2], Lv), maskP, interior);
-  }
+  const T* WD = (const T*)(sizeof(T) == 8 ? o.wdivd[L - o.minL]->p : o.wdivf[L - o.minL]->p);
+  const T* WC = (const T*)(sizeof(T) == 8 ? o.wdivcd[L - o.minL]->p : o.wdivcf[L - o.minL]->p);
+  const int nList = adp.closureBegin[11], listBlocks = (nList + dev::kBlock - 1) / dev::kBlock;
+  const int inner = lvp.lv.N >= 4 ? lvp.lv.nCells * (lvp.lv.N - 3) : 0;
+  dev::p2DivKernel<T><<<listBlocks + inner, dev::kBlock, 0, st.stream>>>(
+      lvp.lv, lvv.lv, WD, WC, (const dev::P2ClosureNode*)adp.closureList.p, nList, listBlocks, (T*)st.data(q, Lp),
+      (const T*)st.data(u[0], Lv), (const T*)st.data(u[1], Lv), (const T*)st.data(u[2], Lv), maskP);
   ++st.launches;
-  if (adp.n) {
-    dev::p2AddKernel<T, dev::MODE_REPLACE><<<(adp.n + dev::kBlock - 1) / dev::kBlock, dev::kBlock, 0, st.stream>>>(
-        (const int64_t*)adp.owner.p, (const int*)adp.ptr.p, (const int64_t*)adp.copies.p,
-        (const unsigned char*)adp.type.p, adp.n, (T*)st.data(q, Lp), nullptr, maskP);
-    ++st.launches;
-  }
+  st.p2AddOwners<T, dev::MODE_REPLACE>(adp, (T*)st.data(q, Lp), nullptr, maskP);
   cudaCheck(cudaGetLastError(), "Stokes div");
-  st.communicate(q, Lp, (1 << G_COUNT) - 1);
+}
+
+// v_k = D_k^T p at the velocity DoFs flagged by maskV.
+template <class T>
+static void stokesDivTImpl(Storage& st, P2Operator& o, int p, const int v[3], int L, unsigned maskV) {
+  const int Lv = L + 1;
+  st.communicate(p, L, 1 << G_CELL);
+  launchDivT<T, false>(st, o, p, v, L, maskV);
+  P2Additive& adv = st.p2Additive(Lv);
+  for (int k = 0; k < 3; ++k) st.p2AddOwners<T, dev::MODE_REPLACE>(adv, (T*)st.data(v[k], Lv), nullptr, maskV);
+  cudaCheck(cudaGetLastError(), "Stokes divT");
+  for (int k = 0; k < 3; ++k) st.communicate(v[k], Lv, kAllGroups);
 }
 
 int Storage::p1Diagonal(int opId, int L) {
@@ -1752,37 +1739,59 @@ int Storage::p1Diagonal(int opId, int L) {
   return d;
 }
 
-void Storage::stokesDivT(int opId, int p, const int v[3], int L, unsigned maskV, bool add) {
+void Storage::stokesDivT(int opId, int p, const int v[3], int L, unsigned maskV) {
   P2Operator& o = p2op(opId);
-  argCheck(!o.dd.empty(), "not a Stokes operator");
+  argCheck(!o.wdivd.empty(), "not a Stokes operator");
   argCheck(L >= o.minL && L <= o.maxL, "level outside the Stokes operator's level range");
   if (fn(p).prec == 8)
-    stokesDivTImpl<double>(*this, o, p, v, L, maskV, add);
+    stokesDivTImpl<double>(*this, o, p, v, L, maskV);
   else
-    stokesDivTImpl<float>(*this, o, p, v, L, maskV, add);
+    stokesDivTImpl<float>(*this, o, p, v, L, maskV);
 }
 
 void Storage::stokesDiv(int opId, const int u[3], int q, int L, unsigned maskP) {
   P2Operator& o = p2op(opId);
-  argCheck(!o.dd.empty(), "not a Stokes operator");
+  argCheck(!o.wdivd.empty(), "not a Stokes operator");
   argCheck(L >= o.minL && L <= o.maxL, "level outside the Stokes operator's level range");
+  for (int k = 0; k < 3; ++k) communicate(u[k], L + 1, 1 << G_CELL);
   if (fn(q).prec == 8)
-    stokesDivImpl<double>(*this, o, u, q, L, maskP);
+    launchDiv<double>(*this, o, u, q, L, maskP);
   else
-    stokesDivImpl<float>(*this, o, u, q, L, maskP);
+    launchDiv<float>(*this, o, u, q, L, maskP);
+  communicate(q, L, kAllGroups);
+}
+
+// The velocity block and the gradient leave their shares in the same closure slots of v, so one sum
+// and one refresh per component serve both.
+template <class T>
+void Storage::stokesApplyT(P2Operator& o, const int u[3], int p, const int v[3], int q, int L, unsigned maskV,
+                           unsigned maskP) {
+  const int Lv = L + 1;
+  const P2Additive& ad = p2Additive(Lv);
+  for (int k = 0; k < 3; ++k) communicate(u[k], Lv, 1 << G_CELL);
+  communicate(p, L, 1 << G_CELL);
+  for (int k = 0; k < 3; ++k)
+    p2Sweep<T, dev::MODE_REPLACE>(o, L, (T*)data(v[k], Lv), (const T*)data(u[k], Lv), nullptr, maskV);
+  launchDivT<T, true>(*this, o, p, v, L, maskV);
+  for (int k = 0; k < 3; ++k) p2AddOwners<T, dev::MODE_REPLACE>(ad, (T*)data(v[k], Lv), nullptr, maskV);
+  launchDiv<T>(*this, o, u, q, L, maskP);
+  for (int k = 0; k < 3; ++k) communicate(v[k], Lv, kAllGroups);
+  communicate(q, L, kAllGroups);
 }
 
 void Storage::stokesApply(int opId, const int u[3], int p, const int v[3], int q, int L, unsigned maskV,
                           unsigned maskP) {
   P2Operator& o = p2op(opId);
-  argCheck(!o.dd.empty(), "not a Stokes operator");
+  argCheck(!o.wdivd.empty(), "not a Stokes operator");
   argCheck(L >= o.minL && L <= o.maxL, "level outside the Stokes operator's level range");
   const int prec = fn(p).prec;
   for (int k = 0; k < 3; ++k) argCheck(fn(u[k]).prec == prec && fn(v[k]).prec == prec, "Stokes: precision mismatch");
   argCheck(fn(q).prec == prec, "Stokes: precision mismatch");
-  for (int k = 0; k < 3; ++k) p2Apply(opId, u[k], v[k], -1, L, maskV, 0);
-  stokesDivT(opId, p, v, L, maskV, true);
-  stokesDiv(opId, u, q, L, maskP);
+  for (int k = 0; k < 3; ++k) argCheck(u[k] != v[k], "P2 apply: distinct functions required");
+  if (prec == 8)
+    stokesApplyT<double>(o, u, p, v, q, L, maskV, maskP);
+  else
+    stokesApplyT<float>(o, u, p, v, q, L, maskV, maskP);
 }
 
 void Storage::autotuneSor(int minL, int maxL, int prec, int reps, double* ms) {

@@ -118,12 +118,13 @@ struct P2Operator {
   int form = 0, minL = 0, maxL = 0;
   std::vector<std::unique_ptr<DevBuf>> kd, kf;  // per level: [cell][type][10][10] in FP64 / FP32
   std::map<std::pair<int, int>, int> diag;      // (level, precision) -> diagonal function
-  std::vector<std::unique_ptr<DevBuf>> dd, df;  // Taylor-Hood divergence per level: [cell][type][3][4][10]
   std::vector<std::unique_ptr<DevBuf>> sd, sf;  // interior stencils per level: [cell][p2s::kTotal]
   std::vector<std::unique_ptr<DevBuf>> fd, ff;  // face-interior stencils per level: [cell][p2s::kFaceTotal]
   // Taylor-Hood coupling at interior nodes per level, [cell][component][65]: div (offsets p2s::S0 on
   // the velocity lattice) and divT (offsets p2s::DivTList per velocity class on the pressure lattice)
   std::vector<std::unique_ptr<DevBuf>> wdivd, wdivf, wdivtd, wdivtf;
+  // and at the closure nodes, [cell][component][p2s::kFaceTotal / p2s::kDivTFaceTotal]
+  std::vector<std::unique_ptr<DevBuf>> wdivcd, wdivcf, wdivtcd, wdivtcf;
 };
 
 // Cell-closure copies of every DoF owned by a face, edge or vertex of one lattice level.
@@ -276,13 +277,17 @@ struct Storage {
   //   q   = sum_k D_k u_k     (pressure DoFs flagged by maskP)
   int createStokesOperator(int minL, int maxL);
   void stokesApply(int op, const int u[3], int p, const int v[3], int q, int L, unsigned maskV, unsigned maskP);
-  // the coupling blocks alone: v_k = D_k^T p (v_k += with add), q = sum_k D_k u_k
-  void stokesDivT(int op, int p, const int v[3], int L, unsigned maskV, bool add);
+  template <class T>
+  void stokesApplyT(P2Operator& o, const int u[3], int p, const int v[3], int q, int L, unsigned maskV, unsigned maskP);
+  // the coupling blocks alone: v_k = D_k^T p, q = sum_k D_k u_k
+  void stokesDivT(int op, int p, const int v[3], int L, unsigned maskV);
   void stokesDiv(int op, const int u[3], int q, int L, unsigned maskP);
   // Diagonal of a P1 operator on level L (the stencil centre of each primitive's DoFs) as a new
   // FP64 function of that level, owned by the caller.
   int p1Diagonal(int op, int L);
   int p2Scratch(int Lf, int prec);
+  template <class T, int MODE>
+  void p2Sweep(P2Operator& o, int L, T* dst, const T* src, const T* rhs, unsigned mask);
   template <class T, int MODE>
   void p2Launch(P2Operator& o, int L, T* dst, const T* src, const T* rhs, unsigned mask);
   template <class T, int MODE>
