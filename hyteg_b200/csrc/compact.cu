@@ -34,39 +34,46 @@ __device__ __forceinline__ const T* compactStencil(const StencilDev<T>& st, int 
   return st.lowEntW + st.lowEntOff[prim + (kind == 2 ? sh.z : sh.w)];
 }
 
-// Values of a row's entries [e, min(e + 16, e1)), all loads issued before any is used: from snap
-// where bit 31 of the entry is set (SNAP), else from x.
-template <class T, bool SNAP>
-__device__ __forceinline__ void compactValues(const int* __restrict__ cols, int e, int e1, const T* x, const T* snap,
-                                              T (&v)[16]) {
-  int c[16];
+// A row and its first 16 entries, read independently of the row's values: the entries of 32
+// consecutive rows are coalesced (read row by row, 56 bytes apart, they cost 14 L1 wavefronts per
+// load), and a thread holds its next row while it waits for the current one. With x in shared
+// memory the V(3,3) cycle of one sub-cube (levels 0-4, FP64, one block) takes 305 us instead of 369.
+struct CompactItem {
+  CompactRow row;
+  int4 c[4];
+};
+__device__ __forceinline__ void compactFetch(CompactItem& it, const CompactRow* __restrict__ rows,
+                                             const int4* __restrict__ ell, int pitch, int r) {
+  const int4 q = __ldg(reinterpret_cast<const int4*>(rows) + r);
+  it.row = {q.x, q.y, q.z, q.w};
 #pragma unroll
-  for (int j = 0; j < 16; ++j) c[j] = e + j < e1 ? __ldg(cols + e + j) : 0;
-#pragma unroll
-  for (int j = 0; j < 16; ++j) {
-    const int cj = c[j];
-    v[j] = e + j < e1 ? ((SNAP && cj < 0) ? snap[cj & 0x7fffffff] : x[cj & 0x7fffffff]) : T(0);
-  }
+  for (int k = 0; k < 4; ++k) it.c[k] = __ldg(ell + (int64_t)k * pitch + r);
+}
+__device__ __forceinline__ int compactEntry(const CompactItem& it, int j) {
+  const int4 q = it.c[j >> 2];
+  return (j & 3) == 0 ? q.x : (j & 3) == 1 ? q.y : (j & 3) == 2 ? q.z : q.w;
 }
 
-// s - sum_k w_k v_k (SUB) or s + sum_k w_k v_k over a row's off-diagonal entries, in entry order.
-template <class T, bool SNAP, bool SUB>
-__device__ __forceinline__ T compactRowSum(T s, const T* w, int stride, const int* __restrict__ cols, int e0, int e1,
+// sum_k w_k v_k over a row's off-diagonal entries (values from snap where bit 31 of the entry is
+// set, SNAP, else from x), in four partial sums; entries beyond 16 from cols.
+template <class T, bool SNAP>
+__device__ __forceinline__ T compactRowSum(const CompactItem& it, const T* w, int stride, const int* __restrict__ cols,
                                            const T* x, const T* snap) {
-  for (int e = e0; e < e1; e += 16) {
-    T v[16];
-    compactValues<T, SNAP>(cols, e, e1, x, snap, v);
-    const T* wk = w + (1 + e - e0) * stride;
+  const int n = it.row.e1 - it.row.e0;
+  T v[16], s[4] = {T(0), T(0), T(0), T(0)};
 #pragma unroll
-    for (int j = 0; j < 16; ++j)
-      if (e + j < e1) {
-        if (SUB)
-          s -= wk[j * stride] * v[j];
-        else
-          s += wk[j * stride] * v[j];
-      }
+  for (int j = 0; j < 16; ++j) {
+    const int c = compactEntry(it, j);
+    v[j] = j < n ? ((SNAP && c < 0) ? snap[c & 0x7fffffff] : x[c & 0x7fffffff]) : T(0);
   }
-  return s;
+#pragma unroll
+  for (int j = 0; j < 16; ++j)
+    if (j < n) s[j & 3] += w[(1 + j) * stride] * v[j];
+  for (int j = 16; j < n; ++j) {
+    const int c = __ldg(cols + it.row.e0 + j);
+    s[j & 3] += w[(1 + j) * stride] * ((SNAP && c < 0) ? snap[c & 0x7fffffff] : x[c & 0x7fffffff]);
+  }
+  return (s[0] + s[1]) + (s[2] + s[3]);
 }
 
 // Grid: groups * CL blocks of kCompactThreads, clusters of CL consecutive blocks; cluster g works
@@ -78,6 +85,7 @@ __global__ void __launch_bounds__(kCompactThreads, 1) compactCycleKernel(const _
                                                                       double* cgScratch, int xZero, int pre, int post,
                                                                       T omega, int cgMaxIter, double cgTol) {
   namespace cgrp = cooperative_groups;
+  extern __shared__ __align__(16) unsigned char compactSmem[];
   __shared__ double red[33];
   __shared__ double part[2];
   int rank = 0;
@@ -91,7 +99,11 @@ __global__ void __launch_bounds__(kCompactThreads, 1) compactCycleKernel(const _
       cgrp::this_cluster().sync();
   };
   T* sc = scratch + grp * cd.groupStride;
-  T* snap = sc + cd.snap;
+  // x of every level and the snapshot: in shared memory where one block owns the group and they fit
+  T* sm = reinterpret_cast<T*>(compactSmem);
+  const bool inSmem = CL == 1 && cd.smemSnap >= 0;
+  T* snap = inSmem ? sm + cd.smemSnap : sc + cd.snap;
+  auto xOf = [&](const CompactLevel<T>& L) { return inSmem ? sm + L.sx : sc + L.x; };
   const int4 sh = make_int4(grp * cd.primsPerGroup[0], grp * cd.primsPerGroup[1], grp * cd.primsPerGroup[2],
                             grp * cd.primsPerGroup[3]);
   const T om1 = T(1) - omega;
@@ -101,44 +113,54 @@ __global__ void __launch_bounds__(kCompactThreads, 1) compactCycleKernel(const _
   {
     const CompactLevel<T>& L = cd.lv[K];
     const int64_t* g = cd.gather + (int64_t)grp * L.n;
+    T* x = xOf(L);
     for (int i = t0; i < L.n; i += nt) {
-      sc[L.x + i] = xZero ? T(0) : xs[g[i]];
+      x[i] = xZero ? T(0) : xs[g[i]];
       sc[L.b + i] = bs[g[i]];
     }
   }
   sync();
 
-  // x_i <- (1 - omega) x_i + omega (b_i - sum_j a_ij x_j) / a_ii, the lowSorPhaseKernel update
-  auto sorRow = [&](const CompactLevel<T>& L, const CompactRow row, T* x, const T* b) {
-    int stride;
-    const T* w = compactStencil(L.st, row.wsel, sh, stride);
-    const T s = compactRowSum<T, true, true>(b[row.idx], w, stride, L.cols, row.e0, row.e1, x, snap);
-    x[row.idx] = om1 * x[row.idx] + (s * omega) / w[0];
+  CompactItem next;  // the thread's next row
+  auto fetch = [&](const CompactLevel<T>& L, int r, int r1) {
+    if (r < r1) compactFetch(next, L.rows, L.ell, L.pitch, r);
+  };
+  // x_i <- (1 - omega) x_i + omega (b_i - sum_j a_ij x_j) / a_ii on rows [r0, r1), the
+  // lowSorPhaseKernel update; the first row is already in next.
+  auto sorRows = [&](const CompactLevel<T>& L, int r0, int r1, T* x, const T* b, const T* saved) {
+    for (int r = r0 + t0; r < r1; r += nt) {
+      const CompactItem it = next;
+      fetch(L, r + nt, r1);
+      int stride;
+      const T bi = b[it.row.idx];
+      const T* w = compactStencil(L.st, it.row.wsel, sh, stride);
+      const T s = bi - compactRowSum<T, true>(it, w, stride, L.cols, x, saved);
+      x[it.row.idx] = om1 * x[it.row.idx] + (s * omega) / w[0];
+    }
   };
   // Sweeps. The vertex rows update while the edge and face values are saved: they write only
   // vertex values, and they read edge and face values from x, which this sweep has not changed
-  // yet; only edge and face rows read the saved values. Then one barrier per colour group.
+  // yet; only edge and face rows read the saved values. Then one barrier per colour group; a
+  // group's first rows are read before the barrier ahead of it.
   auto sweeps = [&](const CompactLevel<T>& L, int count) {
-    T* x = sc + L.x;
+    T* x = xOf(L);
+    T* saved = snap - (inSmem ? L.snapBegin : 0);
     const T* b = sc + L.b;
+    fetch(L, t0, L.nVertexRows);
     for (int it = 0; it < count; ++it) {
-      for (int i = L.snapBegin + t0; i < L.snapEnd; i += nt) snap[i] = x[i];
-      for (int r = t0; r < L.nVertexRows; r += nt) sorRow(L, L.rows[r], x, b);
-      sync();
+      for (int i = L.snapBegin + t0; i < L.snapEnd; i += nt) saved[i] = x[i];
+      sorRows(L, 0, L.nVertexRows, x, b, saved);
       int r0 = L.nVertexRows;
       for (int gi = 0; gi < L.nGroups; ++gi) {
         const int r1 = L.groupEnd[gi];
-        for (int r = r0 + t0; r < r1; r += nt) sorRow(L, L.rows[r], x, b);
-        r0 = r1;
+        fetch(L, r0 + t0, r1);
         sync();
+        sorRows(L, r0, r1, x, b, saved);
+        r0 = r1;
       }
+      fetch(L, t0, L.nVertexRows);
+      sync();
     }
-  };
-  // (A u)_row with every value current
-  auto applyRow = [&](const StencilDev<T>& st, const int* cols, const CompactRow row, const T* u) {
-    int stride;
-    const T* w = compactStencil(st, row.wsel, sh, stride);
-    return compactRowSum<T, false, false>(w[0] * u[row.idx], w, stride, cols, row.e0, row.e1, u, u);
   };
 
   // descent: pre-smoothing, residual, restriction into the coarser right-hand side
@@ -146,24 +168,38 @@ __global__ void __launch_bounds__(kCompactThreads, 1) compactCycleKernel(const _
     const CompactLevel<T>& F = cd.lv[k];
     const CompactLevel<T>& C = cd.lv[k - 1];
     sweeps(F, pre);
-    T* xf = sc + F.x;
+    T* xf = xOf(F);
     const T* bf = sc + F.b;
     T* rf = sc + F.r;
-    for (int r = t0; r < F.nRows; r += nt) {
-      const CompactRow row = F.rows[r];
-      rf[row.idx] = bf[row.idx] - applyRow(F.st, F.cols, row, xf);
+    fetch(F, t0, F.nRows);
+    for (int r = t0; r < F.nRows; r += nt) {  // every value current
+      const CompactItem it = next;
+      fetch(F, r + nt, F.nRows);
+      int stride;
+      const T* w = compactStencil(F.st, it.row.wsel, sh, stride);
+      const int i = it.row.idx;
+      rf[i] = bf[i] - (w[0] * xf[i] + compactRowSum<T, false>(it, w, stride, F.cols, xf, xf));
     }
     sync();
-    T* xc = sc + C.x;
+    T* xc = xOf(C);
     T* bc = sc + C.b;
     for (int r = t0; r < C.nRows; r += nt) {
-      T s = T(0);
-      for (int e = C.rPtr[r]; e < C.rPtr[r + 1]; ++e) {
-        const int c = C.rIdx[e];
-        const T v = rf[c & 0x7fffffff];
-        s += c < 0 ? T(0.5) * v : v;
+      compactFetch(next, C.rows, C.rEll, C.pitch, r);
+      const int e0 = C.rPtr[r], n = C.rPtr[r + 1] - e0;
+      T v[16], s = T(0);
+#pragma unroll
+      for (int j = 0; j < 16; ++j) {
+        const int c = compactEntry(next, j);
+        v[j] = j < n ? (c < 0 ? T(0.5) : T(1)) * rf[c & 0x7fffffff] : T(0);
       }
-      bc[C.rows[r].idx] = s;
+#pragma unroll
+      for (int j = 0; j < 16; ++j) s += v[j];
+      for (int j = 16; j < n; ++j) {
+        const int c = C.rIdx[e0 + j];
+        const T q = rf[c & 0x7fffffff];
+        s += c < 0 ? T(0.5) * q : q;
+      }
+      bc[next.row.idx] = s;
     }
     for (int i = t0; i < C.n; i += nt) xc[i] = T(0);
     sync();
@@ -177,7 +213,7 @@ __global__ void __launch_bounds__(kCompactThreads, 1) compactCycleKernel(const _
     double* cr = cb + C.n;
     double* cp = cr + C.n;
     double* cap = cp + C.n;
-    T* x0 = sc + C.x;
+    T* x0 = xOf(C);
     const T* b0 = sc + C.b;
     int par = 0;
     auto dot = [&](const double* u, const double* v) {
@@ -203,7 +239,9 @@ __global__ void __launch_bounds__(kCompactThreads, 1) compactCycleKernel(const _
     auto applyCg = [&](const CompactRow row, const double* u) {
       int stride;
       const double* w = compactStencil(cd.cgSt, row.wsel, sh, stride);
-      return compactRowSum<double, false, false>(w[0] * u[row.idx], w, stride, C.cols, row.e0, row.e1, u, u);
+      double s = w[0] * u[row.idx];
+      for (int e = row.e0; e < row.e1; ++e) s += w[(1 + e - row.e0) * stride] * u[__ldg(C.cols + e)];
+      return s;
     };
     for (int i = t0; i < C.n; i += nt) {
       cx[i] = double(x0[i]);
@@ -250,8 +288,8 @@ __global__ void __launch_bounds__(kCompactThreads, 1) compactCycleKernel(const _
   // ascent: prolongation added to the flagged unknowns, post-smoothing
   for (int k = 1; k <= K; ++k) {
     const CompactLevel<T>& F = cd.lv[k];
-    const T* xc = sc + cd.lv[k - 1].x;
-    T* xf = sc + F.x;
+    const T* xc = xOf(cd.lv[k - 1]);
+    T* xf = xOf(F);
     for (int r = t0; r < F.nRows; r += nt) {
       const int2 p = F.pro[r];
       const T v = p.y < 0 ? xc[p.x] : T(0.5) * (xc[p.x] + xc[p.y]);
@@ -263,7 +301,7 @@ __global__ void __launch_bounds__(kCompactThreads, 1) compactCycleKernel(const _
 
   // x back to every slot of the top level that holds a DoF
   {
-    const T* xt = sc + cd.lv[K].x;
+    const T* xt = xOf(cd.lv[K]);
     for (int e = cd.scatterOff[grp] + t0; e < cd.scatterOff[grp + 1]; e += nt) xs[cd.scatterSlot[e]] = xt[cd.scatterIdx[e]];
   }
   if constexpr (CL > 1) sync();  // no block leaves while another may still read its shared memory
@@ -272,6 +310,8 @@ __global__ void __launch_bounds__(kCompactThreads, 1) compactCycleKernel(const _
 }  // namespace dev
 
 namespace {
+
+constexpr size_t kCompactSmem = 200 << 10;  // shared memory the vectors may take
 
 int batchKind(int kind) { return kind == KC ? 0 : kind == KF ? 1 : kind == KE ? 2 : 3; }
 
@@ -525,7 +565,8 @@ void fillDev(CompactCycle& cc, dev::CompactCycleDev<T>& d, Storage& s, const Ope
              const std::vector<int>& scIdx, const std::vector<int>& scOff) {
   d = dev::CompactCycleDev<T>{};
   d.nLevels = (int)lbs.size();
-  int64_t off = 0, maxN = 0;
+  int64_t off = 0, maxN = 0, smem = 0;  // shared memory in elements
+  int maxSnap = 0;
   auto vec = [&](int64_t n) {
     const int64_t at = off;
     off += (n + 31) / 32 * 32;
@@ -548,6 +589,19 @@ void fillDev(CompactCycle& cc, dev::CompactCycleDev<T>& d, Storage& s, const Ope
     L.pro = put(cc, lb.pro, s.stream);
     L.rPtr = put(cc, lb.rPtr, s.stream);
     L.rIdx = put(cc, lb.rIdx, s.stream);
+    L.pitch = ((int)lb.rows.size() + 31) / 32 * 32;
+    std::vector<int4> ell((size_t)L.pitch * 4, make_int4(0, 0, 0, 0)), rEll(ell);
+    for (size_t r = 0; r < lb.rows.size(); ++r)
+      for (int j = 0; j < 16; ++j) {
+        const size_t at = (size_t)(j >> 2) * L.pitch + r;
+        if (lb.rows[r].e0 + j < lb.rows[r].e1) (&ell[at].x)[j & 3] = lb.cols[(size_t)(lb.rows[r].e0 + j)];
+        if (!lb.rIdx.empty() && lb.rPtr[r] + j < lb.rPtr[r + 1]) (&rEll[at].x)[j & 3] = lb.rIdx[(size_t)(lb.rPtr[r] + j)];
+      }
+    L.ell = put(cc, ell, s.stream);
+    L.rEll = put(cc, rEll, s.stream);
+    L.sx = (int)smem;
+    smem += (L.n + 1) / 2 * 2;
+    maxSnap = std::max(maxSnap, L.snapEnd - L.snapBegin);
     const int oi = lb.L - o.minL;
     if constexpr (sizeof(T) == 8)
       L.st = o.d[(size_t)oi];
@@ -559,6 +613,16 @@ void fillDev(CompactCycle& cc, dev::CompactCycleDev<T>& d, Storage& s, const Ope
     maxN = std::max<int64_t>(maxN, L.n);
   }
   d.snap = vec(maxN);
+  cc.smem = (size_t)(smem + maxSnap) * sizeof(T);
+  d.smemSnap = (int)smem;
+  if (cc.cluster > 1 || cc.smem > kCompactSmem) {
+    d.smemSnap = -1;
+    cc.smem = 0;
+  } else {
+    cudaCheck(cudaFuncSetAttribute(dev::compactCycleKernel<T, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)kCompactSmem),
+              "compact cycle");
+  }
   d.groupStride = off;
   d.cgStride = 5 * (int64_t)lbs[0].dofs.size();
   d.cgSt = o.d[(size_t)(lbs[0].L - o.minL)];
@@ -578,7 +642,7 @@ void launchT(CompactCycle& c, const dev::CompactCycleDev<T>& d, Storage& s, void
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(c.groups * CL));
   cfg.blockDim = dim3(dev::kCompactThreads);
-  cfg.dynamicSmemBytes = 0;
+  cfg.dynamicSmemBytes = c.smem;
   cfg.stream = s.stream;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;

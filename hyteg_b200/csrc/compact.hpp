@@ -47,11 +47,15 @@ struct CompactLevel {
   const CompactRow* rows;
   const CompactRow* cgRows;
   const int* cols;   // entry -> unknown index; bit 31: the value of the sweep's start
+  const int4* ell;   // the first 16 entries of row r: ell[q * pitch + r], q = 0 .. 3 (the same values)
+  const int4* rEll;  // the first 16 of the restriction into row r, same layout; rPtr holds the counts
+  int pitch;
   const int2* pro;   // [nRows] coarse unknowns of the prolongation into this row (y < 0: coincident)
   const int* rPtr;   // [nRows + 1] restriction into this level's rows from the level above
   const int* rIdx;   // fine unknown index; bit 31: weight 1/2 (else 1)
   StencilDev<T> st;
   int64_t x, b, r;   // offsets of the level's vectors in a group's scratch
+  int sx;            // offset of x in shared memory (CompactCycleDev::smemSnap >= 0)
 };
 
 template <class T>
@@ -60,6 +64,7 @@ struct CompactCycleDev {
   int nLevels;
   int64_t groupStride;  // scratch elements per group
   int64_t snap;         // offset of the snapshot vector in a group's scratch
+  int smemSnap;         // x of every level in shared memory, then from here the snapshot (-1: in scratch)
   int64_t cgStride;     // FP64 coarse-CG scratch per group (five vectors)
   const int64_t* gather;       // [groups][n(top)] owner slot of each top-level unknown
   const int64_t* scatterSlot;  // per group, every slot of the top level holding a DoF ...
@@ -73,6 +78,7 @@ struct CompactCycleDev {
 
 struct CompactCycle {
   int minL = 0, top = -1, groups = 1, cluster = 1, prec = 8;
+  size_t smem = 0;  // dynamic shared memory of the launch
   dev::CompactCycleDev<double> d64{};
   dev::CompactCycleDev<float> d32{};
   std::vector<std::unique_ptr<DevBuf>> keep;
