@@ -525,18 +525,9 @@ int hg_cg_solve(hg_storage* h, int op, int x, int b, int level, int max_iter, do
                 double* final_residual) {
   HG_TRY
   hg::Storage& s = S(h);
-  const int prec = s.fn(x).prec;
-  const int p = s.createFunction(level, level, prec), z = s.createFunction(level, level, prec),
-            ap = s.createFunction(level, level, prec), r = s.createFunction(level, level, prec);
-  int it = 0;
+  const std::array<int, 3> w = s.cgWork(level, s.fn(x).prec);
   double res = 0;
-  try {
-    it = hg::cgSolve(s, op, x, b, level, max_iter, tol, p, z, ap, r, &res);
-  } catch (...) {
-    for (int id : {p, z, ap, r}) s.fns.erase(id);
-    throw;
-  }
-  for (int id : {p, z, ap, r}) s.fns.erase(id);
+  const int it = hg::cgSolve(s, op, x, b, level, max_iter, tol, w[0], w[1], w[2], &res);
   if (iterations) *iterations = it;
   if (final_residual) *final_residual = res;
   HG_CATCH

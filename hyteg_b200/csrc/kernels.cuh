@@ -50,6 +50,8 @@ struct LevelDev {
   int nCellBlocks;  // nCells * (N - 3) blocks (one per macro-cell and z-plane), 0 below level 2
   const FaceBlock* faceBlocks;
   int nFaceBlocks;
+  const FaceBlock* faceBands;  // the same rows in bands of kFaceBand
+  int nFaceBands;
   const LowBlock* lowBlocks;
   int nLowBlocks;  // edges' blocks first (nLowEdgeBlocks of them), then vertices
   int nLowEdgeBlocks;
@@ -118,47 +120,6 @@ __device__ __forceinline__ T cellOffDiag(const T* wt, const CellRow& r, int x, L
   s += wt[13] * ld(r.rBN + x);
   s += wt[14] * ld(r.rBN + x - 1);
   return s;
-}
-
-// dst = A src | dst += A src | dst = rhs - A src on cell interiors. The weights live in shared
-// memory (broadcast reads) and every lane handles two points per iteration, so up to 30
-// independent loads per thread are in flight.
-template <class T, int MODE>
-__global__ void __launch_bounds__(kBlock, 4) cellStencilKernel(LevelDev lv, const T* __restrict__ cellW,
-                                                               T* __restrict__ dst, const T* __restrict__ src,
-                                                               const T* __restrict__ rhs, unsigned mask) {
-  const int nPl = lv.N - 3;
-  const int c = blockIdx.x / nPl, z = 1 + blockIdx.x % nPl;
-  if (!(lv.cellType[c] & mask)) return;
-  __shared__ T wt[16];
-  if (threadIdx.x < 15) wt[threadIdx.x] = cellW[16 * c + threadIdx.x];
-  __syncthreads();
-  const int64_t base = lv.cellOff[c];
-  const T* __restrict__ u = src + base;
-  T* __restrict__ d = dst + base;
-  const T* __restrict__ f = rhs + base;
-  const int W = lv.w - z;
-  auto ld = [u](int i) { return __ldg(u + i); };
-  for (int y = 1 + (int)(threadIdx.x >> 5); y <= W - 3; y += kBlock / 32) {
-    const CellRow r = cellRow(lv.w, z, y);
-    const int len = W - 2 - y;
-    for (int x = 1 + (int)(threadIdx.x & 31); x <= len; x += 64) {
-      const int x2 = x + 32;
-      const bool two = x2 <= len;
-      const T s1 = wt[0] * ld(r.r0 + x) + cellOffDiag(wt, r, x, ld);
-      const T s2 = two ? wt[0] * ld(r.r0 + x2) + cellOffDiag(wt, r, x2, ld) : T(0);
-      if (MODE == MODE_REPLACE) {
-        d[r.r0 + x] = s1;
-        if (two) d[r.r0 + x2] = s2;
-      } else if (MODE == MODE_ADD) {
-        d[r.r0 + x] += s1;
-        if (two) d[r.r0 + x2] += s2;
-      } else {
-        d[r.r0 + x] = f[r.r0 + x] - s1;
-        if (two) d[r.r0 + x2] = f[r.r0 + x2] - s2;
-      }
-    }
-  }
 }
 
 // Multicolour SOR on cell interiors, colour = (x + 2y + 3z) mod 4: the lanes of a warp step
@@ -642,7 +603,10 @@ __global__ void __launch_bounds__(576, sizeof(T) == 4 ? 2 : 1) cellSorResidentKe
 // rows, L1 hits). No shared memory, no block synchronisation.
 // ---------------------------------------------------------------------------------------
 constexpr int kStripX = 30;                         // computed columns per warp
-constexpr int kStripZ = 32;                         // planes per work item
+// Planes per work item. Each item reads two planes more than it computes, so long items read less;
+// short ones give the small levels enough blocks (N = 64, 48 cells: 240 items of 32 planes on 444
+// block slots, 768 of 8).
+inline int stripPlanes(int N) { return N <= 64 ? 8 : N <= 128 ? 16 : 32; }
 constexpr int kStripRows = 32;                      // rows per block (strips stacked in y)
 // Rows per strip and blocks per SM by precision. Eight rows per warp keep ten rows of the next
 // plane in flight per lane and re-read a quarter of the rows (the neighbouring strips' halo
@@ -679,12 +643,11 @@ __device__ __forceinline__ T shDown(T v) {  // value of lane + 1 (x + 1)
 }
 
 template <class T, int OP>
-__global__ void __launch_bounds__(stripThreads<T>(), StripCfg<T>::MIN_BLOCKS)
-    cellStripKernel(LevelDev lv, const StripItem* __restrict__ items, const T* __restrict__ cellW, T* __restrict__ dst,
-                    const T* __restrict__ src, const T* __restrict__ rhs, unsigned mask) {
+__device__ __forceinline__ void cellStrip(const LevelDev& lv, const StripItem it, const T* __restrict__ cellW,
+                                          T* __restrict__ dst, const T* __restrict__ src, const T* __restrict__ rhs,
+                                          unsigned mask) {
   constexpr int kStripR = StripCfg<T>::R;       // rows per strip
   constexpr int kStripH = kStripR + 2;          // rows held per plane (with y-halo)
-  const StripItem it = items[blockIdx.x];
   if (!(lv.cellType[it.cell] & mask)) return;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int N = lv.N, w = lv.w;
@@ -785,14 +748,17 @@ __global__ void __launch_bounds__(stripThreads<T>(), StripCfg<T>::MIN_BLOCKS)
   }
 }
 
+__device__ __forceinline__ int cellIndexDev(int w, int x, int y, int z) {
+  const int W = w - z;
+  return int(tetSize(w) - tetSize(W)) + rowStart(W, y) + x;
+}
+
 // Full-weighting restriction at coarse cell-interior points: coarse = fine[2p] + 1/2 sum fine[2p+d]
-// (restrict_3D_macrocell_P1_pull_additive.cpp; on interior points every weight is 1 or 1/2).
+// (restrict_3D_macrocell_P1_pull_additive.cpp; on interior points every weight is 1 or 1/2). Plane z
+// of macro-cell c.
 template <class T>
-__global__ void __launch_bounds__(kBlock) cellRestrictKernel(LevelDev lc, LevelDev lf, T* __restrict__ coarse,
-                                                             const T* __restrict__ fine, unsigned mask) {
-  const int nPl = lc.N - 3;
-  const int c = blockIdx.x / nPl, z = 1 + blockIdx.x % nPl;
-  if (!(lc.cellType[c] & mask)) return;
+__device__ __forceinline__ void cellRestrictPlane(const LevelDev& lc, const LevelDev& lf, int c, int z, T* __restrict__ coarse,
+                                                  const T* __restrict__ fine) {
   const T* __restrict__ uf = fine + lf.cellOff[c];
   T* __restrict__ uc = coarse + lc.cellOff[c];
   const T one[15] = {T(1), T(1), T(1), T(1), T(1), T(1), T(1), T(1), T(1), T(1), T(1), T(1), T(1), T(1), T(1)};
@@ -807,50 +773,54 @@ __global__ void __launch_bounds__(kBlock) cellRestrictKernel(LevelDev lc, LevelD
   }
 }
 
-__device__ __forceinline__ int cellIndexDev(int w, int x, int y, int z) {
-  const int W = w - z;
-  return int(tetSize(w) - tetSize(W)) + rowStart(W, y) + x;
+// Linear prolongation (prolongate_3D_macrocell_P1_push_additive.cpp): even points copy the coarse
+// value, every other point is the mean of the two coarse end points of the coarse micro-edge it
+// bisects. With yl = y >> 1, yh = (y + 1) >> 1 and the same for x and z, that edge runs from
+// (xh, P) to (xl, Q) whatever the parity of x, where the rows P and Q depend on the parities of y
+// and z only:
+//   (even, even) (yl, zl), (yl, zl)   (odd, even) (yl, zl), (yh, zl)
+//   (even, odd)  (yl, zl), (yl, zh)   (odd, odd)  (yl, zh), (yh, zl)
+// One row of points from rows p and q of the coarse array.
+template <class T>
+__device__ __forceinline__ T prolongPoint(const T* __restrict__ uc, int p, int q, int x) {
+  const T a = __ldg(uc + p + ((x + 1) >> 1)), b = __ldg(uc + q + (x >> 1));
+  return p == q && !(x & 1) ? a : T(0.5) * (a + b);
 }
 
-// Linear prolongation at fine cell-interior points (prolongate_3D_macrocell_P1_push_additive.cpp):
-// even points copy the coarse value, every other point is the mean of the two coarse end
-// points of the coarse micro-edge it bisects. The bisected direction depends on the parity of
-// (x, y, z); for one fine row only the x parity varies, so two row pairs are set up per row.
+// Plane z of macro-cell c, kProlongRows rows per warp at a time with all their loads in flight: the
+// kernel streams the fine array twice (read and write, 17 B per point in FP64).
+constexpr int kProlongRows = 4;
 template <class T, bool ADD>
-__global__ void __launch_bounds__(kBlock) cellProlongKernel(LevelDev lf, LevelDev lc, T* __restrict__ fine,
-                                                            const T* __restrict__ coarse, unsigned mask) {
-  const int nPl = lf.N - 3;
-  const int c = blockIdx.x / nPl, z = 1 + blockIdx.x % nPl;
-  if (!(lf.cellType[c] & mask)) return;
-  T* __restrict__ uf = fine + lf.cellOff[c];
+__device__ __forceinline__ void cellProlongPlane(const LevelDev& lf, const LevelDev& lc, int c, int z, T* __restrict__ fine,
+                                                 const T* __restrict__ coarse) {
+  const int W = lf.w - z, zl = z >> 1, zh = (z + 1) >> 1;
+  T* __restrict__ uf = fine + lf.cellOff[c] + (tetSize(lf.w) - tetSize(W));
   const T* __restrict__ uc = coarse + lc.cellOff[c];
-  const int W = lf.w - z;
-  // directions of the bisected coarse micro-edge by parity code (x | y << 1 | z << 2)
-  const int DX[8] = {0, 1, 0, -1, 0, -1, 0, -1};
-  const int DY[8] = {0, 0, 1, 1, 0, 0, -1, 1};
-  const int DZ[8] = {0, 0, 0, 0, 1, 1, 1, -1};
-  for (int y = 1 + (int)(threadIdx.x >> 5); y <= W - 3; y += kBlock / 32) {
-    const int rf = int(tetSize(lf.w) - tetSize(W)) + rowStart(W, y);
-    const int len = W - 2 - y;
-    // for x parity p: coarse row base of end point a (x offset (x - dx) / 2) and of b = a + d
-    int ra[2], rb[2], dxp[2];
-    bool single[2];
-    for (int p = 0; p < 2; ++p) {
-      const int code = p | ((y & 1) << 1) | ((z & 1) << 2);
-      const int dx = DX[code], dy = DY[code], dz = DZ[code];
-      const int ay = (y - dy) >> 1, az = (z - dz) >> 1;
-      ra[p] = cellIndexDev(lc.w, 0, ay, az);
-      rb[p] = cellIndexDev(lc.w, 0, ay + dy, az + dz);
-      dxp[p] = dx;
-      single[p] = code == 0;
+  const int Wl = lc.w - zl, Wh = lc.w - zh;
+  const int bl = int(tetSize(lc.w) - tetSize(Wl)), bh = int(tetSize(lc.w) - tetSize(Wh));
+  constexpr int kWarps = kBlock / 32;
+  for (int y0 = 1 + (int)(threadIdx.x >> 5); y0 <= W - 3; y0 += kProlongRows * kWarps) {
+    int r[kProlongRows], p[kProlongRows], q[kProlongRows], len[kProlongRows];
+#pragma unroll
+    for (int k = 0; k < kProlongRows; ++k) {
+      const int y = y0 + k * kWarps, yl = y >> 1, yh = (y + 1) >> 1;
+      const bool oy = y & 1, oz = z & 1;
+      r[k] = rowStart(W, y);
+      len[k] = y <= W - 3 ? W - 2 - y : 0;
+      p[k] = oy && oz ? bh + rowStart(Wh, yl) : bl + rowStart(Wl, yl);
+      q[k] = oy ? bl + rowStart(Wl, yh) : bh + rowStart(Wh, yl);
     }
-    for (int x = 1 + (int)(threadIdx.x & 31); x <= len; x += 32) {
-      const int p = x & 1;
-      const int ax = (x - dxp[p]) >> 1;
-      const T v = single[p] ? __ldg(uc + ra[p] + ax)
-                            : T(0.5) * (__ldg(uc + ra[p] + ax) + __ldg(uc + rb[p] + ax + dxp[p]));
-      if (ADD) uf[rf + x] += v;
-      else uf[rf + x] = v;
+    for (int x = 1 + (int)(threadIdx.x & 31); x <= len[0]; x += 32) {  // the first row is the longest
+      T v[kProlongRows], f[kProlongRows];
+#pragma unroll
+      for (int k = 0; k < kProlongRows; ++k)
+        if (x <= len[k]) {
+          v[k] = prolongPoint(uc, p[k], q[k], x);
+          if (ADD) f[k] = uf[r[k] + x];
+        }
+#pragma unroll
+      for (int k = 0; k < kProlongRows; ++k)
+        if (x <= len[k]) uf[r[k] + x] = ADD ? f[k] + v[k] : v[k];
     }
   }
 }
@@ -863,6 +833,7 @@ __global__ void __launch_bounds__(kBlock) cellProlongKernel(LevelDev lf, LevelDe
 // slot offsets once (shared memory), then every lane adds x.
 // ---------------------------------------------------------------------------------------
 constexpr int kFaceRows = 32;
+constexpr int kFaceBand = 8;  // rows per block of the apply: short, so that the rows of a face spread over many blocks
 
 __device__ __forceinline__ int faceSlot(int w, int layer, int x, int y) {
   if (layer == 0) return rowStart(w, y) + x;
@@ -881,34 +852,6 @@ __device__ __forceinline__ int loadFaceEntries(FaceShared<T>& sh, const StencilD
   if (threadIdx.x < ne) sh.ent[threadIdx.x] = st.faceEnt[16 * face + threadIdx.x];
   __syncthreads();
   return ne;
-}
-
-template <class T, int MODE>
-__global__ void __launch_bounds__(kBlock) faceStencilKernel(LevelDev lv, StencilDev<T> st, T* __restrict__ dst,
-                                                            const T* __restrict__ src, const T* __restrict__ rhs,
-                                                            unsigned mask) {
-  const FaceBlock b = lv.faceBlocks[blockIdx.x];
-  if (!(lv.faceType[b.face] & mask)) return;
-  __shared__ FaceShared<T> sh;
-  const int ne = loadFaceEntries(sh, st, b.face);
-  const int w = lv.w, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int64_t base = lv.faceOff[b.face];
-  const T* __restrict__ u = src + base;
-  const int yEnd = min(b.start + kFaceRows, w - 2);
-  for (int y = b.start + warp; y < yEnd; y += kBlock / 32) {
-    if (lane < ne) sh.off[warp][lane] = faceSlot(w, sh.ent[lane].layer, sh.ent[lane].dx, y + sh.ent[lane].dy);
-    __syncwarp();
-    const int len = w - 2 - y, r0 = rowStart(w, y);
-    for (int x = 1 + lane; x <= len; x += 32) {
-      T s = T(0);
-      for (int k = 0; k < ne; ++k) s += sh.ent[k].w * __ldg(u + sh.off[warp][k] + x);
-      const int64_t i = base + r0 + x;
-      if (MODE == MODE_REPLACE) dst[i] = s;
-      else if (MODE == MODE_ADD) dst[i] += s;
-      else dst[i] = rhs[i] - s;
-    }
-    __syncwarp();
-  }
 }
 
 // Face SOR, colour = (x + 2y) mod 3; entry 0 is the diagonal.
@@ -1037,62 +980,44 @@ __global__ void __launch_bounds__(kFacePhaseThreads) faceSorPhaseKernel(LevelDev
 }
 
 // Restriction at coarse face-interior points from the fine face and its ghost layers: the fine
-// stencil structure of the face with weight 1 at the centre and 1/2 at every neighbour.
+// stencil structure of the face with weight 1 at the centre and 1/2 at every neighbour. One row per
+// warp.
 template <class T>
-__global__ void __launch_bounds__(kBlock) faceRestrictKernel(LevelDev lc, LevelDev lf, StencilDev<T> stf,
-                                                             T* __restrict__ coarse, const T* __restrict__ fine,
-                                                             unsigned mask) {
-  const FaceBlock b = lc.faceBlocks[blockIdx.x];
-  if (!(lc.faceType[b.face] & mask)) return;
+__device__ __forceinline__ void faceRestrictBand(const LevelDev& lc, const LevelDev& lf, const StencilDev<T>& stf,
+                                                 const FaceBlock b, T* __restrict__ coarse, const T* __restrict__ fine) {
   __shared__ FaceShared<T> sh;
   const int ne = loadFaceEntries(sh, stf, b.face);
   const int w = lc.w, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const T* __restrict__ uf = fine + lf.faceOff[b.face];
   T* __restrict__ uc = coarse + lc.faceOff[b.face];
-  const int yEnd = min(b.start + kFaceRows, w - 2);
-  for (int y = b.start + warp; y < yEnd; y += kBlock / 32) {
-    if (lane < ne) sh.off[warp][lane] = faceSlot(lf.w, sh.ent[lane].layer, sh.ent[lane].dx, 2 * y + sh.ent[lane].dy);
-    __syncwarp();
-    const int len = w - 2 - y, r0 = rowStart(w, y);
-    for (int x = 1 + lane; x <= len; x += 32) {
-      T s = T(0);
-      for (int k = 1; k < ne; ++k) s += __ldg(uf + sh.off[warp][k] + 2 * x);
-      uc[r0 + x] = __ldg(uf + sh.off[warp][0] + 2 * x) + T(0.5) * s;
-    }
-    __syncwarp();
+  const int y = b.start + warp;
+  if (y >= min(b.start + kFaceBand, w - 2)) return;
+  if (lane < 16)
+    sh.off[warp][lane] = lane < ne ? faceSlot(lf.w, sh.ent[lane].layer, sh.ent[lane].dx, 2 * y + sh.ent[lane].dy) : 0;
+  __syncwarp();
+  const int len = w - 2 - y, r0 = rowStart(w, y);
+  for (int x = 1 + lane; x <= len; x += 32) {
+    T v[16], s = T(0);
+#pragma unroll
+    for (int k = 0; k < 16; ++k) v[k] = k < ne ? __ldg(uf + sh.off[warp][k] + 2 * x) : T(0);
+#pragma unroll
+    for (int k = 1; k < 16; ++k) s += v[k];
+    uc[r0 + x] = v[0] + T(0.5) * s;
   }
 }
 
+// One row per warp; the rows P and Q of an odd row are (yl) and (yh) as in a cell's even plane.
 template <class T, bool ADD>
-__global__ void __launch_bounds__(kBlock) faceProlongKernel(LevelDev lf, LevelDev lc, T* __restrict__ fine,
-                                                            const T* __restrict__ coarse, unsigned mask) {
-  const FaceBlock b = lf.faceBlocks[blockIdx.x];
-  if (!(lf.faceType[b.face] & mask)) return;
-  const int w = lf.w, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  T* __restrict__ uf = fine + lf.faceOff[b.face];
+__device__ __forceinline__ void faceProlongBand(const LevelDev& lf, const LevelDev& lc, const FaceBlock b, T* __restrict__ fine,
+                                                const T* __restrict__ coarse) {
+  const int w = lf.w, y = b.start + (int)(threadIdx.x >> 5);
+  if (y >= min(b.start + kFaceBand, w - 2)) return;
+  T* __restrict__ uf = fine + lf.faceOff[b.face] + rowStart(w, y);
   const T* __restrict__ uc = coarse + lc.faceOff[b.face];
-  const int yEnd = min(b.start + kFaceRows, w - 2);
-  for (int y = b.start + warp; y < yEnd; y += kBlock / 32) {
-    const int len = w - 2 - y, r0 = rowStart(w, y);
-    // bisected coarse micro-edge by parity (x | y << 1): (1,0), (0,1) or (-1,1)
-    int ra[2], rb[2], dxp[2];
-    for (int p = 0; p < 2; ++p) {
-      const int code = p | ((y & 1) << 1);
-      const int dx = code == 1 ? 1 : (code == 3 ? -1 : 0), dy = (code >= 2) ? 1 : 0;
-      const int ay = (y - dy) >> 1;
-      ra[p] = rowStart(lc.w, ay);
-      rb[p] = rowStart(lc.w, ay + dy);
-      dxp[p] = dx;
-    }
-    const bool evenRow = (y & 1) == 0;
-    for (int x = 1 + lane; x <= len; x += 32) {
-      const int p = x & 1;
-      const int ax = (x - dxp[p]) >> 1;
-      const T v = (evenRow && p == 0) ? __ldg(uc + ra[0] + ax)
-                                      : T(0.5) * (__ldg(uc + ra[p] + ax) + __ldg(uc + rb[p] + ax + dxp[p]));
-      if (ADD) uf[r0 + x] += v;
-      else uf[r0 + x] = v;
-    }
+  const int p = rowStart(lc.w, y >> 1), q = rowStart(lc.w, (y + 1) >> 1);
+  for (int x = 1 + (int)(threadIdx.x & 31); x <= w - 2 - y; x += 32) {
+    const T v = prolongPoint(uc, p, q, x);
+    uf[x] = ADD ? uf[x] + v : v;
   }
 }
 
@@ -1100,20 +1025,78 @@ __global__ void __launch_bounds__(kBlock) faceProlongKernel(LevelDev lf, LevelDe
 // Edges and vertices (apply_edge P1Operator.hpp:1040-1104, macrovertex::apply
 // VertexDoFMacroVertex.hpp:160-184): per primitive a list of (relative slot, weight).
 // ---------------------------------------------------------------------------------------
+// Face, edge and vertex rows of levelStencilKernel.
+constexpr int kLevelThreads = 128;
+static_assert(stripThreads<double>() == kLevelThreads && stripThreads<float>() == kLevelThreads, "strip block size");
+
 template <class T, int MODE>
-__global__ void __launch_bounds__(kBlock) lowStencilKernel(LevelDev lv, StencilDev<T> st, T* __restrict__ dst,
-                                                           const T* __restrict__ src, const T* __restrict__ rhs,
-                                                           unsigned mask, int blockBegin) {
-  const LowBlock b = lv.lowBlocks[blockBegin + blockIdx.x];
-  if (!(lv.lowType[b.prim] & mask)) return;
-  const int x = b.start + threadIdx.x;
-  if (x >= lv.lowFirst[b.prim] + lv.lowCount[b.prim]) return;
-  const int64_t c = lv.lowOff[b.prim] + x;
+__device__ __forceinline__ void faceBand(const LevelDev& lv, const StencilDev<T>& st, const FaceBlock b, T* __restrict__ dst,
+                                         const T* __restrict__ src, const T* __restrict__ rhs, unsigned mask) {
+  if (!(lv.faceType[b.face] & mask)) return;
+  __shared__ FaceEnt<T> ent[16];
+  __shared__ int off[kLevelThreads / 32][16];
+  const int ne = st.faceEntCount[b.face];
+  if (threadIdx.x < 16)
+    ent[threadIdx.x] = (int)threadIdx.x < ne ? st.faceEnt[16 * b.face + threadIdx.x] : FaceEnt<T>{T(0), 0, 0, 0};
+  __syncthreads();
+  const int w = lv.w, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int64_t base = lv.faceOff[b.face];
+  const T* __restrict__ u = src + base;
+  const int yEnd = min(b.start + kFaceBand, w - 2);
+  for (int y = b.start + warp; y < yEnd; y += kLevelThreads / 32) {
+    // missing entries read the centre with weight zero
+    if (lane < 16)
+      off[warp][lane] = lane < ne ? faceSlot(w, ent[lane].layer, ent[lane].dx, y + ent[lane].dy) : rowStart(w, y);
+    __syncwarp();
+    const int len = w - 2 - y, r0 = rowStart(w, y);
+    for (int x = 1 + lane; x <= len; x += 32) {
+      T v[16], s = T(0);
+#pragma unroll
+      for (int k = 0; k < 16; ++k) v[k] = k < ne ? __ldg(u + off[warp][k] + x) : T(0);
+#pragma unroll
+      for (int k = 0; k < 16; ++k)
+        if (k < ne) s += ent[k].w * v[k];
+      const int64_t i = base + r0 + x;
+      if (MODE == MODE_REPLACE) dst[i] = s;
+      else if (MODE == MODE_ADD) dst[i] += s;
+      else dst[i] = rhs[i] - s;
+    }
+    __syncwarp();
+  }
+}
+
+template <class T, int MODE>
+__device__ __forceinline__ void lowRow(const LevelDev& lv, const StencilDev<T>& st, int prim, int x, T* __restrict__ dst,
+                                       const T* __restrict__ src, const T* __restrict__ rhs) {
+  const int64_t c = lv.lowOff[prim] + x;
   T s = T(0);
-  for (int k = st.lowEntOff[b.prim]; k < st.lowEntOff[b.prim + 1]; ++k) s += st.lowEntW[k] * __ldg(src + c + st.lowEntRel[k]);
+#pragma unroll 8
+  for (int k = st.lowEntOff[prim]; k < st.lowEntOff[prim + 1]; ++k) s += st.lowEntW[k] * __ldg(src + c + st.lowEntRel[k]);
   if (MODE == MODE_REPLACE) dst[c] = s;
   else if (MODE == MODE_ADD) dst[c] += s;
   else dst[c] = rhs[c] - s;
+}
+
+// dst = A src | dst += A src | dst = rhs - A src on a level, one launch: blocks [0, nLow) take edges
+// and vertices (the level's low blocks from lowBegin), the next nFace bands of face rows, the
+// others cell strips. The small ones go first and run beside the strips. Measured, FP64, 48 cells:
+// level 8 710 us instead of 638 + 84 + 8 in three launches, level 6 37 instead of 43 + 22 + 8.
+template <class T, int MODE>
+__global__ void __launch_bounds__(kLevelThreads, StripCfg<T>::MIN_BLOCKS)
+    levelStencilKernel(LevelDev lv, StencilDev<T> st, const StripItem* __restrict__ items, int nLow, int lowBegin, int nFace,
+                       T* __restrict__ dst, const T* __restrict__ src, const T* __restrict__ rhs, unsigned mask) {
+  const int blk = blockIdx.x;
+  if (blk < nLow) {
+    const LowBlock b = lv.lowBlocks[lowBegin + blk];
+    if (!(lv.lowType[b.prim] & mask)) return;
+    const int end = min(b.start + kBlock, lv.lowFirst[b.prim] + lv.lowCount[b.prim]);
+    for (int x = b.start + (int)threadIdx.x; x < end; x += kLevelThreads) lowRow<T, MODE>(lv, st, b.prim, x, dst, src, rhs);
+  } else if (blk < nLow + nFace) {
+    faceBand<T, MODE>(lv, st, lv.faceBands[blk - nLow], dst, src, rhs, mask);
+  } else {
+    cellStrip<T, MODE == MODE_REPLACE ? STRIP_REPLACE : MODE == MODE_ADD ? STRIP_ADD : STRIP_RESIDUAL>(
+        lv, items[blk - nLow - nFace], st.cellW, dst, src, rhs, mask);
+  }
 }
 
 // ---------------------------------------------------------------------------------------
@@ -1458,34 +1441,55 @@ __global__ void __launch_bounds__(kBlock) lowSorKernel(LevelDev lv, StencilDev<T
   u[c] = (T(1) - omega) * u[c] + (s * omega) / st.lowEntW[e0];
 }
 
+// The transfers of a level, one launch each: edge and vertex blocks, face bands, then one block per
+// macro-cell and plane. The small ones run beside the cells instead of after them.
+static_assert(kFaceBand == kBlock / 32, "a band has one row per warp");
+
 template <class T>
-__global__ void __launch_bounds__(kBlock) lowRestrictKernel(LevelDev lc, LevelDev lf, StencilDev<T> stf,
-                                                            T* __restrict__ coarse, const T* __restrict__ fine,
-                                                            unsigned mask) {
-  const LowBlock b = lc.lowBlocks[blockIdx.x];
-  if (!(lc.lowType[b.prim] & mask)) return;
-  const int x = b.start + threadIdx.x;
-  if (x >= lc.lowFirst[b.prim] + lc.lowCount[b.prim]) return;
-  const int64_t cf = lf.lowOff[b.prim] + 2 * x;
-  const int e0 = stf.lowEntOff[b.prim];
-  T s = T(0);
-  for (int k = e0 + 1; k < stf.lowEntOff[b.prim + 1]; ++k) s += __ldg(fine + cf + stf.lowEntRel[k]);
-  coarse[lc.lowOff[b.prim] + x] = __ldg(fine + cf) + T(0.5) * s;
+__global__ void __launch_bounds__(kBlock) levelRestrictKernel(LevelDev lc, LevelDev lf, StencilDev<T> stf,
+                                                              T* __restrict__ coarse, const T* __restrict__ fine,
+                                                              unsigned mask) {
+  int blk = blockIdx.x;
+  if (blk < lc.nLowBlocks) {
+    const LowBlock b = lc.lowBlocks[blk];
+    const int x = b.start + threadIdx.x;
+    if (!(lc.lowType[b.prim] & mask) || x >= lc.lowFirst[b.prim] + lc.lowCount[b.prim]) return;
+    const int64_t cf = lf.lowOff[b.prim] + 2 * x;
+    const int e0 = stf.lowEntOff[b.prim];
+    T s = T(0);
+#pragma unroll 8
+    for (int k = e0 + 1; k < stf.lowEntOff[b.prim + 1]; ++k) s += __ldg(fine + cf + stf.lowEntRel[k]);
+    coarse[lc.lowOff[b.prim] + x] = __ldg(fine + cf) + T(0.5) * s;
+  } else if ((blk -= lc.nLowBlocks) < lc.nFaceBands) {
+    const FaceBlock b = lc.faceBands[blk];
+    if (lc.faceType[b.face] & mask) faceRestrictBand<T>(lc, lf, stf, b, coarse, fine);
+  } else {
+    blk -= lc.nFaceBands;
+    const int nPl = lc.N - 3, c = blk / nPl;
+    if (lc.cellType[c] & mask) cellRestrictPlane<T>(lc, lf, c, 1 + blk - c * nPl, coarse, fine);
+  }
 }
 
 template <class T, bool ADD>
-__global__ void __launch_bounds__(kBlock) lowProlongKernel(LevelDev lf, LevelDev lc, T* __restrict__ fine,
-                                                           const T* __restrict__ coarse, unsigned mask) {
-  const LowBlock b = lf.lowBlocks[blockIdx.x];
-  if (!(lf.lowType[b.prim] & mask)) return;
-  const int x = b.start + threadIdx.x;
-  if (x >= lf.lowFirst[b.prim] + lf.lowCount[b.prim]) return;
-  const int64_t cb = lc.lowOff[b.prim];
-  const T v = (x & 1) ? T(0.5) * (__ldg(coarse + cb + (x >> 1)) + __ldg(coarse + cb + (x >> 1) + 1))
-                      : __ldg(coarse + cb + (x >> 1));
-  const int64_t c = lf.lowOff[b.prim] + x;
-  if (ADD) fine[c] += v;
-  else fine[c] = v;
+__global__ void __launch_bounds__(kBlock) levelProlongKernel(LevelDev lf, LevelDev lc, T* __restrict__ fine,
+                                                             const T* __restrict__ coarse, unsigned mask) {
+  int blk = blockIdx.x;
+  if (blk < lf.nLowBlocks) {
+    const LowBlock b = lf.lowBlocks[blk];
+    const int x = b.start + threadIdx.x;
+    if (!(lf.lowType[b.prim] & mask) || x >= lf.lowFirst[b.prim] + lf.lowCount[b.prim]) return;
+    const T* uc = coarse + lc.lowOff[b.prim];
+    const T v = (x & 1) ? T(0.5) * (__ldg(uc + (x >> 1)) + __ldg(uc + (x >> 1) + 1)) : __ldg(uc + (x >> 1));
+    T* u = fine + lf.lowOff[b.prim] + x;
+    *u = ADD ? *u + v : v;
+  } else if ((blk -= lf.nLowBlocks) < lf.nFaceBands) {
+    const FaceBlock b = lf.faceBands[blk];
+    if (lf.faceType[b.face] & mask) faceProlongBand<T, ADD>(lf, lc, b, fine, coarse);
+  } else {
+    blk -= lf.nFaceBands;
+    const int nPl = lf.N - 3, c = blk / nPl;
+    if (lf.cellType[c] & mask) cellProlongPlane<T, ADD>(lf, lc, c, 1 + blk - c * nPl, fine, coarse);
+  }
 }
 
 // ---------------------------------------------------------------------------------------
@@ -1650,19 +1654,78 @@ struct Chunk {
   int type;
 };
 
-template <class T>
-__global__ void __launch_bounds__(kBlock) lincombKernel(const Chunk* __restrict__ chunks, unsigned mask, T* dst, int nsrc,
-                                                        const T* s0, const T* s1, const T* s2, double a0, double a1,
-                                                        double a2, int addToDst, double constant) {
+// dst = constant + sum a_i s_i, or dst += with ADD. Bound by bandwidth: eight elements per thread
+// and round, all their loads before the first store. A copy of a level-6 vector (18 MB) takes 8.6 us,
+// 21 us with one element at a time.
+constexpr int kLincombUnroll = 8;
+template <class T, int NSRC, bool ADD>
+__global__ void __launch_bounds__(kBlock) lincombKernel(const Chunk* __restrict__ chunks, unsigned mask, T* dst,
+                                                        const T* s0, const T* s1, const T* s2, T a0, T a1, T a2,
+                                                        T constant) {
   const Chunk ch = chunks[blockIdx.x];
   if (!(ch.type & mask)) return;
-  for (int i = threadIdx.x; i < ch.len; i += blockDim.x) {
-    const int64_t j = ch.start + i;
-    T v = addToDst ? dst[j] : T(constant);
-    if (nsrc > 0) v += T(a0) * s0[j];
-    if (nsrc > 1) v += T(a1) * s1[j];
-    if (nsrc > 2) v += T(a2) * s2[j];
-    dst[j] = v;
+  T* d = dst + ch.start;
+  for (int i0 = threadIdx.x; i0 < ch.len; i0 += kBlock * kLincombUnroll) {
+    T v[kLincombUnroll], u[3][kLincombUnroll];
+#pragma unroll
+    for (int k = 0; k < kLincombUnroll; ++k) {
+      const int i = i0 + k * kBlock;
+      if (i >= ch.len) continue;
+      v[k] = ADD ? d[i] : constant;
+      if (NSRC > 0) u[0][k] = s0[ch.start + i];
+      if (NSRC > 1) u[1][k] = s1[ch.start + i];
+      if (NSRC > 2) u[2][k] = s2[ch.start + i];
+    }
+#pragma unroll
+    for (int k = 0; k < kLincombUnroll; ++k) {
+      const int i = i0 + k * kBlock;
+      if (i >= ch.len) continue;
+      if (NSRC > 0) v[k] += a0 * u[0][k];
+      if (NSRC > 1) v[k] += a1 * u[1][k];
+      if (NSRC > 2) v[k] += a2 * u[2][k];
+      d[i] = v[k];
+    }
+  }
+}
+
+// The vector updates of one CG iteration with their coefficients from the device scalars, so that
+// the host waits once per iteration (for the new residual norm) instead of three times. Ten
+// iterations on level 6, 48 cells, FP64: 1.39 ms, 5.30 ms with host coefficients, single updates
+// and work vectors allocated per solve. x += alpha p, r -= alpha ap with
+// alpha = num / den, and p = r + beta p with beta = num / den.
+template <class T, bool DIRECTION>
+__global__ void __launch_bounds__(kBlock) cgUpdateKernel(const Chunk* __restrict__ chunks, unsigned mask,
+                                                         const double* __restrict__ num, const double* __restrict__ den,
+                                                         T* x, T* r, T* p, const T* ap) {
+  const Chunk ch = chunks[blockIdx.x];
+  if (!(ch.type & mask)) return;
+  constexpr int kU = 4;
+  const double q = *num / *den;
+  const T c = T(q), mc = T(-q);
+  for (int i0 = threadIdx.x; i0 < ch.len; i0 += kBlock * kU) {
+    T xv[kU], rv[kU], pv[kU], av[kU];
+#pragma unroll
+    for (int k = 0; k < kU; ++k) {
+      const int64_t j = ch.start + i0 + k * kBlock;
+      if (i0 + k * kBlock >= ch.len) continue;
+      rv[k] = r[j];
+      pv[k] = p[j];
+      if (!DIRECTION) {
+        xv[k] = x[j];
+        av[k] = ap[j];
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < kU; ++k) {
+      const int64_t j = ch.start + i0 + k * kBlock;
+      if (i0 + k * kBlock >= ch.len) continue;
+      if (DIRECTION) {
+        p[j] = rv[k] + c * pv[k];
+      } else {
+        x[j] = xv[k] + c * pv[k];
+        r[j] = rv[k] + mc * av[k];
+      }
+    }
   }
 }
 
@@ -1773,35 +1836,61 @@ __device__ __forceinline__ double blockReduce(double v) {
   return r;
 }
 
+// The rows of one thread block's band: kDotRows rows per warp at a time, so that their loads overlap
+// (rows are short: 21 points on average at N = 64).
+constexpr int kDotRows = 4;
+template <class T, class ROW>
+__device__ __forceinline__ double dotRows(const T* __restrict__ pa, const T* __restrict__ pb, int y0, int yEnd, ROW row) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  double v = 0.0;
+  for (int y = y0 + warp; y < yEnd; y += kDotRows * (kBlock / 32)) {
+    int r0[kDotRows], len[kDotRows];
+#pragma unroll
+    for (int k = 0; k < kDotRows; ++k) {
+      const int yk = y + k * (kBlock / 32);
+      len[k] = 0;
+      r0[k] = 0;
+      if (yk < yEnd) row(yk, r0[k], len[k]);
+    }
+    for (int x = 1 + lane; x <= len[0]; x += 32) {  // the first row is the longest
+      T a[kDotRows], b[kDotRows];
+#pragma unroll
+      for (int k = 0; k < kDotRows; ++k) {
+        a[k] = x <= len[k] ? pa[r0[k] + x] : T(0);
+        b[k] = x <= len[k] ? pb[r0[k] + x] : T(0);
+      }
+#pragma unroll
+      for (int k = 0; k < kDotRows; ++k) v += double(a[k]) * double(b[k]);
+    }
+  }
+  return v;
+}
+
 template <class T>
-__global__ void __launch_bounds__(kBlock) dotKernel(LevelDev lv, const T* __restrict__ a, const T* __restrict__ b,
-                                                    unsigned mask, double* partial) {
+__device__ __forceinline__ double dotBlock(const LevelDev& lv, const T* __restrict__ a, const T* __restrict__ b, unsigned mask) {
   double v = 0.0;
   int blk = blockIdx.x;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nCellGrid = lv.N >= 4 ? lv.nCells * (lv.N - 3) : 0;
   if (blk < nCellGrid) {
     const int nPl = lv.N - 3;
     const int c = blk / nPl, z = 1 + blk % nPl;
     if (lv.cellType[c] & mask) {
-      const T* __restrict__ pa = a + lv.cellOff[c];
-      const T* __restrict__ pb = b + lv.cellOff[c];
       const int W = lv.w - z;
-      for (int y = 1 + warp; y <= W - 3; y += kBlock / 32) {
-        const int r0 = int(tetSize(lv.w) - tetSize(W)) + rowStart(W, y);
-        for (int x = 1 + lane; x <= W - 2 - y; x += 32) v += double(pa[r0 + x]) * double(pb[r0 + x]);
-      }
+      const int64_t base = lv.cellOff[c] + (tetSize(lv.w) - tetSize(W));
+      v = dotRows<T>(a + base, b + base, 1, W - 2, [W](int y, int& r0, int& len) {
+        r0 = rowStart(W, y);
+        len = W - 2 - y;
+      });
     }
   } else if ((blk -= nCellGrid) < lv.nFaceBlocks) {
     const FaceBlock fb = lv.faceBlocks[blk];
     if (lv.faceType[fb.face] & mask) {
-      const T* __restrict__ pa = a + lv.faceOff[fb.face];
-      const T* __restrict__ pb = b + lv.faceOff[fb.face];
-      const int yEnd = min(fb.start + kFaceRows, lv.w - 2);
-      for (int y = fb.start + warp; y < yEnd; y += kBlock / 32) {
-        const int r0 = rowStart(lv.w, y);
-        for (int x = 1 + lane; x <= lv.w - 2 - y; x += 32) v += double(pa[r0 + x]) * double(pb[r0 + x]);
-      }
+      const int w = lv.w;
+      v = dotRows<T>(a + lv.faceOff[fb.face], b + lv.faceOff[fb.face], fb.start, min(fb.start + kFaceRows, w - 2),
+                     [w](int y, int& r0, int& len) {
+                       r0 = rowStart(w, y);
+                       len = w - 2 - y;
+                     });
     }
   } else {
     blk -= lv.nFaceBlocks;
@@ -1814,7 +1903,13 @@ __global__ void __launch_bounds__(kBlock) dotKernel(LevelDev lv, const T* __rest
       }
     }
   }
-  const double r = blockReduce<T>(v);
+  return blockReduce<T>(v);
+}
+
+template <class T>
+__global__ void __launch_bounds__(kBlock) dotKernel(LevelDev lv, const T* __restrict__ a, const T* __restrict__ b,
+                                                    unsigned mask, double* partial) {
+  const double r = dotBlock<T>(lv, a, b, mask);
   if (threadIdx.x == 0) partial[blockIdx.x] = r;
 }
 
@@ -1823,6 +1918,30 @@ static __global__ void __launch_bounds__(kBlock) reduceKernel(const double* __re
   for (int i = threadIdx.x; i < n; i += blockDim.x) v += partial[i];
   const double r = blockReduce<double>(v);
   if (threadIdx.x == 0) *out = r;
+}
+
+// dotKernel with reduceKernel's sum (same order, same value) taken by the block that finishes last:
+// one launch per dot product instead of two. arrived is zero before and after.
+template <class T>
+__global__ void __launch_bounds__(kBlock) dotReduceKernel(LevelDev lv, const T* __restrict__ a, const T* __restrict__ b,
+                                                          unsigned mask, double* partial, unsigned* arrived, double* out) {
+  const double r = dotBlock<T>(lv, a, b, mask);
+  __shared__ bool last;
+  if (threadIdx.x == 0) {
+    partial[blockIdx.x] = r;
+    __threadfence();
+    last = atomicAdd(arrived, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  double v = 0.0;
+  for (unsigned i = threadIdx.x; i < gridDim.x; i += kBlock) v += __ldcg(partial + i);
+  const double s = blockReduce<double>(v);
+  if (threadIdx.x == 0) {
+    *out = s;
+    *arrived = 0;
+  }
 }
 
 // ---------------------------------------------------------------------------------------

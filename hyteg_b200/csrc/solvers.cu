@@ -12,45 +12,43 @@
 namespace hg {
 
 // CGSolver::solve (src/hyteg/solvers/CGSolver.hpp:69-150) with the identity preconditioner
-// (solvers/preconditioners/IdentityPreconditioner.hpp:39-45): z = r.
-int cgSolve(Storage& s, int op, int x, int b, int L, int maxIter, double tol, int p, int z, int ap, int r,
-            double* finalRes) {
+// (solvers/preconditioners/IdentityPreconditioner.hpp:39-45): z = r, so <r, z> is <r, r> and z is
+// not stored. The coefficients stay on the device; the host waits for the residual norm only.
+int cgSolve(Storage& s, int op, int x, int b, int L, int maxIter, double tol, int p, int ap, int r, double* finalRes) {
   const unsigned flag = HG_INNER | HG_NEUMANN | HG_FREESLIP;
   const double one = 1.0;
   if (finalRes) *finalRes = 0.0;
   if (maxIter == 0) return 0;
+  double* rr = (double*)s.scalars.p;  // <r, r> of this iteration and of the next, taken in turn
+  double* pap = rr + 2;
+  auto residual = [&](double* d) {
+    s.dotAsync(r, r, L, flag, d);
+    double h = 0;
+    cudaCheck(cudaMemcpyAsync(&h, d, sizeof(double), cudaMemcpyDeviceToHost, s.stream), "dot readback");
+    cudaCheck(cudaStreamSynchronize(s.stream), "dot sync");
+    return std::sqrt(h);
+  };
   s.apply(op, x, p, L, flag, 0);
   {
     const double sc[2] = {1.0, -1.0};
     const int src[2] = {b, p};
     s.lincomb(r, L, flag, 2, sc, src, false, 0.0);
   }
-  s.lincomb(z, L, flag, 1, &one, &r, false, 0.0);
-  s.lincomb(p, L, flag, 1, &one, &z, false, 0.0);
-  double prsold = s.dot(r, z, L, flag);
-  const double resStart = std::sqrt(s.dot(r, r, L, flag));
+  s.lincomb(p, L, flag, 1, &one, &r, false, 0.0);
+  const double resStart = residual(rr);
   if (finalRes) *finalRes = resStart;
   if (resStart < tol) return 0;
   int it = 0;
   for (int i = 0; i < maxIter; ++i) {
     it = i + 1;
+    double *now = rr + (i & 1), *next = rr + 1 - (i & 1);
     s.apply(op, p, ap, L, flag, 0);
-    const double pAp = s.dot(p, ap, L, flag);
-    const double alpha = prsold / pAp;
-    s.lincomb(x, L, flag, 1, &alpha, &p, true, 0.0);
-    const double malpha = -alpha;
-    s.lincomb(r, L, flag, 1, &malpha, &ap, true, 0.0);
-    const double rsnew = s.dot(r, r, L, flag);
-    const double sq = std::sqrt(rsnew);
+    s.dotAsync(p, ap, L, flag, pap);
+    s.cgUpdate(L, flag, false, now, pap, x, r, p, ap);
+    const double sq = residual(next);
     if (finalRes) *finalRes = sq;
     if (sq < tol) break;
-    s.lincomb(z, L, flag, 1, &one, &r, false, 0.0);
-    const double prsnew = s.dot(r, z, L, flag);
-    const double beta = prsnew / prsold;
-    const double sc[2] = {1.0, beta};
-    const int src[2] = {z, p};
-    s.lincomb(p, L, flag, 2, sc, src, false, 0.0);
-    prsold = prsnew;
+    s.cgUpdate(L, flag, true, next, now, -1, r, p, -1);
   }
   return it;
 }
@@ -62,7 +60,6 @@ Gmg::Gmg(Storage& st, int op_, int minL_, int maxL_, int pre_, int post_, double
   tmp = s.createFunction(minL, maxL, prec);
   // the coarse-grid CG always runs in FP64
   cp = s.createFunction(minL, minL, 8);
-  cz = s.createFunction(minL, minL, 8);
   cap = s.createFunction(minL, minL, 8);
   cr = s.createFunction(minL, minL, 8);
   if (prec == 4) {
@@ -176,7 +173,7 @@ void Gmg::buildCompact(bool strict) {
 
 Gmg::~Gmg() {
   cache.clear();
-  for (int id : {tmp, cp, cz, cap, cr, cx64, cb64, x32, b32, r64})
+  for (int id : {tmp, cp, cap, cr, cx64, cb64, x32, b32, r64})
     if (id >= 0) s.fns.erase(id);
 }
 
@@ -405,7 +402,7 @@ void Gmg::coarseSolve(int x, int b, int L) {
     ++s.launches;
     cudaCheck(cudaGetLastError(), "coarse CG");
   } else {
-    cgSolve(s, op, xs, bs, L, coarseMaxIter, coarseTol, cp, cz, cap, cr, nullptr);
+    cgSolve(s, op, xs, bs, L, coarseMaxIter, coarseTol, cp, cap, cr, nullptr);
   }
   if (timing) timing->stop(s.stream, "CG Solver");
   if (prec == 4) s.copyCast(x, cx64, L, HG_ALL, false);
@@ -428,7 +425,7 @@ std::vector<uintptr_t> Gmg::signature(int x, int b, int L) {
     sig.push_back((uintptr_t)s.levels[l].commSplit);
     sig.push_back((uintptr_t)o.d[l - o.minL].cellW);
   }
-  for (int id : {cp, cz, cap, cr, cx64, cb64})
+  for (int id : {cp, cap, cr, cx64, cb64})
     if (id >= 0) sig.push_back((uintptr_t)s.data(id, minL));
   sig.push_back(cgDofs ? (uintptr_t)cgDofs->p : 0);
   sig.push_back((uintptr_t)coarseGroups);
@@ -613,7 +610,6 @@ P2Gmg::P2Gmg(Storage& st, int op_, int minL_, int maxL_, int pre_, int post_, do
   argCheck(prec == 8 || prec == 4, "P2 multigrid: precision must be 8 or 4");
   tmp = s.createFunction(minL + 1, maxL + 1, prec);
   cp = s.createFunction(minL + 1, minL + 1, 8);
-  cz = s.createFunction(minL + 1, minL + 1, 8);
   cap = s.createFunction(minL + 1, minL + 1, 8);
   cr = s.createFunction(minL + 1, minL + 1, 8);
   if (prec == 4) {
@@ -624,7 +620,7 @@ P2Gmg::P2Gmg(Storage& st, int op_, int minL_, int maxL_, int pre_, int post_, do
 
 P2Gmg::~P2Gmg() {
   cache.clear();
-  for (int id : {tmp, cp, cz, cap, cr, cx64, cb64})
+  for (int id : {tmp, cp, cap, cr, cx64, cb64})
     if (id >= 0) s.fns.erase(id);
 }
 

@@ -70,8 +70,7 @@ struct GraphCache {
 };
 
 // Returns the number of iterations taken; workspace functions must cover level L.
-int cgSolve(Storage& s, int op, int x, int b, int L, int maxIter, double tol, int p, int z, int ap, int r,
-            double* finalRes);
+int cgSolve(Storage& s, int op, int x, int b, int L, int maxIter, double tol, int p, int ap, int r, double* finalRes);
 
 struct Gmg {
   Gmg(Storage& s, int op, int minL, int maxL, int pre, int post, double omega, int cycle, int coarseMaxIter,
@@ -111,7 +110,7 @@ struct Gmg {
   int cycle, coarseMaxIter;
   double coarseTol;
   int prec;
-  int tmp, cp, cz, cap, cr;
+  int tmp, cp, cap, cr;
   // FP32 solvers: FP64 coarse-grid workspace and the FP32 correction / defect hierarchy
   int cx64 = -1, cb64 = -1, x32 = -1, b32 = -1, r64 = -1;
   // Device coarse CG: one block per group of unknowns, the whole mesh (1) or each copy of a
@@ -156,7 +155,7 @@ struct P2Gmg {
   double omega;
   int coarseMaxIter;
   double coarseTol;
-  int tmp, cp, cz, cap, cr;
+  int tmp, cp, cap, cr;
   int prec = 8;                      // precision of the cycle (4: FP32 hierarchy, coarse CG in FP64)
   int cx64 = -1, cb64 = -1;          // FP64 coarse-level copies for an FP32 cycle
   bool symmetric = false;  // post-smoothing with backward sweeps (a symmetric cycle)

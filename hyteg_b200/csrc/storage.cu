@@ -2,6 +2,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <array>
 #include <cmath>
 #include <cstdint>
 #include <cstring>
@@ -9,6 +10,7 @@
 #include <memory>
 #include <stdexcept>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "../../include/hyteg_b200.h"
@@ -176,6 +178,10 @@ void Storage::buildLevel(int L) {
   if (N >= 3)
     for (int f = 0; f < lv.nFaces; ++f)
       for (int y = 1; y < (int)w - 2; y += dev::kFaceRows) fb.push_back({f, y});
+  std::vector<dev::FaceBlock> bands;
+  if (N >= 3)
+    for (int f = 0; f < lv.nFaces; ++f)
+      for (int y = 1; y < (int)w - 2; y += dev::kFaceBand) bands.push_back({f, y});
   std::vector<dev::LowBlock> lb;
   for (int p = 0; p < lv.nLow; ++p) {
     if (p == lv.nEdges) lv.nLowEdgeBlocks = (int)lb.size();
@@ -244,6 +250,8 @@ void Storage::buildLevel(int L) {
   lv.lowType = (const unsigned char*)upload(keep, lowType, stream);
   lv.faceBlocks = (const dev::FaceBlock*)upload(keep, fb, stream);
   lv.nFaceBlocks = (int)fb.size();
+  lv.faceBands = (const dev::FaceBlock*)upload(keep, bands, stream);
+  lv.nFaceBands = (int)bands.size();
   lv.lowBlocks = (const dev::LowBlock*)upload(keep, lb, stream);
   lv.nLowBlocks = (int)lb.size();
   ld.comm = (uint2*)upload(keep, comm, stream);
@@ -275,11 +283,14 @@ void Storage::buildLevel(int L) {
     ld.nonCellBegin = first;
   }
   ld.nChunks = (int)chunks.size();
-  ld.partial.alloc(sizeof(double) * std::max(1, lv.nCellBlocks + lv.nFaceBlocks + lv.nLowBlocks));
+  const int nPartial = std::max(1, lv.nCellBlocks + lv.nFaceBlocks + lv.nLowBlocks);
+  ld.partial.alloc(sizeof(double) * (size_t)(nPartial + 1));
+  ld.arrived = (unsigned*)((double*)ld.partial.p + nPartial);
+  cudaCheck(cudaMemsetAsync(ld.arrived, 0, sizeof(double), stream), "dot counter");
   cudaCheck(cudaStreamSynchronize(stream), "level upload");
 }
 
-// Cell-sweep work items: (cell, 30-column x 32-row block of strips, <= kStripZ planes), the
+// Cell-sweep work items: (cell, 30-column x 32-row block of strips, a few planes), the
 // longest first inside groups of macro-cells whose two FP64 vectors fit into the L2 budget;
 // the SOR colours of a group run back to back so that their re-reads hit L2.
 void Storage::buildTiles(int L) {
@@ -297,8 +308,9 @@ void Storage::buildTiles(int L) {
         for (int x0 = 1; x0 <= N - 3; x0 += dev::kStripX) {
           const int zmax = (int)N - 1 - x0 - y0;  // last plane with an interior point in the block
           if (zmax < 1) continue;
-          for (int z0 = 1; z0 <= zmax; z0 += dev::kStripZ)
-            grp.push_back({c, x0, y0, z0, std::min(zmax + 1, z0 + dev::kStripZ), 0, 0, 0});
+          const int planes = dev::stripPlanes((int)N);
+          for (int z0 = 1; z0 <= zmax; z0 += planes)
+            grp.push_back({c, x0, y0, z0, std::min(zmax + 1, z0 + planes), 0, 0, 0});
         }
     std::stable_sort(grp.begin(), grp.end(),
                      [](const dev::StripItem& a, const dev::StripItem& b) { return (a.z1 - a.z0) > (b.z1 - b.z0); });
@@ -325,6 +337,45 @@ void Storage::setL2Budget(int64_t bytes) {
 // ------------------------------------------------------------------------------------------
 // functions
 // ------------------------------------------------------------------------------------------
+const std::array<int, 3>& Storage::cgWork(int L, int prec) {
+  auto it = cgWorks.find({L, prec});
+  if (it != cgWorks.end()) return it->second;
+  std::array<int, 3> w{-1, -1, -1};
+  try {
+    for (int& id : w) id = createFunction(L, L, prec);
+  } catch (...) {
+    for (int id : w) fns.erase(id);
+    throw;
+  }
+  return cgWorks[{L, prec}] = w;
+}
+
+void Storage::releaseCgWork() {
+  for (auto& w : cgWorks)
+    for (int id : w.second) fns.erase(id);
+  cgWorks.clear();
+}
+
+void Storage::cgUpdate(int L, unsigned mask, bool direction, const double* num, const double* den, int x, int r, int p,
+                       int ap) {
+  const LevelData& ld = levels[L];
+  if (!ld.nChunks) return;
+  auto run = [&](auto zero) {
+    using T = decltype(zero);
+    T *xd = direction ? nullptr : (T*)data(x, L), *ad = direction ? nullptr : (T*)data(ap, L);
+    if (direction)
+      dev::cgUpdateKernel<T, true><<<ld.nChunks, dev::kBlock, 0, stream>>>(ld.chunks, mask, num, den, xd, (T*)data(r, L),
+                                                                           (T*)data(p, L), ad);
+    else
+      dev::cgUpdateKernel<T, false><<<ld.nChunks, dev::kBlock, 0, stream>>>(ld.chunks, mask, num, den, xd, (T*)data(r, L),
+                                                                            (T*)data(p, L), ad);
+  };
+  if (fn(r).prec == 8) run(0.0);
+  else run(0.0f);
+  ++launches;
+  cudaCheck(cudaGetLastError(), "CG update");
+}
+
 Function& Storage::fn(int id) {
   auto it = fns.find(id);
   argCheck(it != fns.end(), "unknown function handle");
@@ -345,7 +396,13 @@ int Storage::createFunction(int minL, int maxL, int prec) {
   for (int L = minL; L <= maxL; ++L) {
     f->levels.emplace_back(new DevBuf());
     const size_t bytes = (size_t)levels[L].lay->total * prec;
-    f->levels.back()->alloc(bytes);
+    try {
+      f->levels.back()->alloc(bytes);
+    } catch (const Error& e) {  // kept workspace goes first
+      if (e.code != HG_ERR_OOM || cgWorks.empty()) throw;
+      releaseCgWork();
+      f->levels.back()->alloc(bytes);
+    }
     cudaCheck(cudaMemsetAsync(f->levels.back()->p, 0, bytes, stream), "memset");
   }
   const int id = nextId++;
@@ -529,14 +586,24 @@ void Storage::lincomb(int dst, int L, unsigned mask, int n, const double* a, con
   }
   const LevelData& ld = levels[L];
   if (ld.nChunks == 0) return;
-  if (fd.prec == 8)
-    dev::lincombKernel<double><<<ld.nChunks, dev::kBlock, 0, stream>>>(
-        ld.chunks, mask, (double*)pd, n, (const double*)ps[0], (const double*)ps[1], (const double*)ps[2], sc[0], sc[1],
-        sc[2], add ? 1 : 0, constant);
-  else
-    dev::lincombKernel<float><<<ld.nChunks, dev::kBlock, 0, stream>>>(
-        ld.chunks, mask, (float*)pd, n, (const float*)ps[0], (const float*)ps[1], (const float*)ps[2], sc[0], sc[1],
-        sc[2], add ? 1 : 0, constant);
+  auto run = [&](auto zero) {
+    using T = decltype(zero);
+    auto go = [&](auto nsrc, auto addTo) {
+      dev::lincombKernel<T, decltype(nsrc)::value, decltype(addTo)::value><<<ld.nChunks, dev::kBlock, 0, stream>>>(
+          ld.chunks, mask, (T*)pd, (const T*)ps[0], (const T*)ps[1], (const T*)ps[2], T(sc[0]), T(sc[1]), T(sc[2]),
+          T(constant));
+    };
+    auto pick = [&](auto nsrc) {
+      if (add) go(nsrc, std::true_type{});
+      else go(nsrc, std::false_type{});
+    };
+    if (n == 0) pick(std::integral_constant<int, 0>{});
+    else if (n == 1) pick(std::integral_constant<int, 1>{});
+    else if (n == 2) pick(std::integral_constant<int, 2>{});
+    else pick(std::integral_constant<int, 3>{});
+  };
+  if (fd.prec == 8) run(0.0);
+  else run(0.0f);
   ++launches;
   cudaCheck(cudaGetLastError(), "lincomb");
 }
@@ -576,14 +643,14 @@ void Storage::dotAsync(int a, int b, int L, unsigned mask, double* dOut) {
   argCheck(fa.prec == fn(b).prec, "dot requires functions of equal precision");
   const LevelData& ld = levels[L];
   const int nb = ld.lv.nCellBlocks + ld.lv.nFaceBlocks + ld.lv.nLowBlocks;
+  double* partial = (double*)ld.partial.p;
   if (fa.prec == 8)
-    dev::dotKernel<double><<<nb, dev::kBlock, 0, stream>>>(ld.lv, (const double*)data(a, L), (const double*)data(b, L), mask,
-                                                           (double*)ld.partial.p);
+    dev::dotReduceKernel<double><<<nb, dev::kBlock, 0, stream>>>(ld.lv, (const double*)data(a, L),
+                                                                 (const double*)data(b, L), mask, partial, ld.arrived, dOut);
   else
-    dev::dotKernel<float><<<nb, dev::kBlock, 0, stream>>>(ld.lv, (const float*)data(a, L), (const float*)data(b, L), mask,
-                                                          (double*)ld.partial.p);
-  dev::reduceKernel<<<1, dev::kBlock, 0, stream>>>((const double*)ld.partial.p, nb, dOut);
-  launches += 2;
+    dev::dotReduceKernel<float><<<nb, dev::kBlock, 0, stream>>>(ld.lv, (const float*)data(a, L), (const float*)data(b, L),
+                                                                mask, partial, ld.arrived, dOut);
+  ++launches;
   cudaCheck(cudaGetLastError(), "dot");
 }
 
@@ -1928,29 +1995,14 @@ template <class T, int MODE>
 void Storage::stencilOp(Operator& o, int L, T* dst, const T* src, const T* rhs, unsigned mask, int kinds) {
   const LevelData& ld = levels[L];
   const dev::StencilDev<T>& st = stencilOf<T>(o, L);
-  if (ld.nTiles && (kinds & (1 << KC))) {
-    constexpr int op =
-        MODE == dev::MODE_REPLACE ? dev::STRIP_REPLACE : MODE == dev::MODE_ADD ? dev::STRIP_ADD : dev::STRIP_RESIDUAL;
-    dev::cellStripKernel<T, op><<<ld.nTiles, dev::stripThreads<T>(), 0, stream>>>(ld.lv, ld.tiles, st.cellW, dst, src,
-                                                                                  rhs, mask);
-    ++launches;
-  }
-  if (ld.lv.nFaceBlocks && (kinds & (1 << KF))) {
-    dev::faceStencilKernel<T, MODE><<<ld.lv.nFaceBlocks, dev::kBlock, 0, stream>>>(ld.lv, st, dst, src, rhs, mask);
-    ++launches;
-  }
   const int nVertBlocks = ld.lv.nLowBlocks - ld.lv.nLowEdgeBlocks;
-  if ((kinds & (1 << KE)) && (kinds & (1 << KV)) && ld.lv.nLowBlocks) {
-    dev::lowStencilKernel<T, MODE><<<ld.lv.nLowBlocks, dev::kBlock, 0, stream>>>(ld.lv, st, dst, src, rhs, mask, 0);
-    ++launches;
-  } else if ((kinds & (1 << KE)) && ld.lv.nLowEdgeBlocks) {
-    dev::lowStencilKernel<T, MODE><<<ld.lv.nLowEdgeBlocks, dev::kBlock, 0, stream>>>(ld.lv, st, dst, src, rhs, mask, 0);
-    ++launches;
-  } else if ((kinds & (1 << KV)) && nVertBlocks) {
-    dev::lowStencilKernel<T, MODE><<<nVertBlocks, dev::kBlock, 0, stream>>>(ld.lv, st, dst, src, rhs, mask,
-                                                                              ld.lv.nLowEdgeBlocks);
-    ++launches;
-  }
+  const bool edges = kinds & (1 << KE), verts = kinds & (1 << KV);
+  const int nCell = kinds & (1 << KC) ? ld.nTiles : 0, nFace = kinds & (1 << KF) ? ld.lv.nFaceBands : 0;
+  const int nLow = (edges ? ld.lv.nLowEdgeBlocks : 0) + (verts ? nVertBlocks : 0);
+  if (nCell + nFace + nLow == 0) return;
+  dev::levelStencilKernel<T, MODE><<<nLow + nFace + nCell, dev::kLevelThreads, 0, stream>>>(
+      ld.lv, st, ld.tiles, nLow, edges ? 0 : ld.lv.nLowEdgeBlocks, nFace, dst, src, rhs, mask);
+  ++launches;
   cudaCheck(cudaGetLastError(), "stencil kernel");
 }
 
@@ -2237,18 +2289,10 @@ void Storage::restrictT(int id, int Lf, unsigned mask, int coarseDst) {
   Operator& so = const_cast<Operator&>(structure());
   const dev::StencilDev<T>& stf = stencilOf<T>(so, Lf);
   communicate(id, Lf, kAllGroups);
-  if (lc.lv.nCellBlocks) {
-    dev::cellRestrictKernel<T><<<lc.lv.nCellBlocks, dev::kBlock, 0, stream>>>(lc.lv, lf.lv, coarse, fine, mask);
-    ++launches;
-  }
-  if (lc.lv.nFaceBlocks) {
-    dev::faceRestrictKernel<T><<<lc.lv.nFaceBlocks, dev::kBlock, 0, stream>>>(lc.lv, lf.lv, stf, coarse, fine, mask);
-    ++launches;
-  }
-  if (lc.lv.nLowBlocks) {
-    dev::lowRestrictKernel<T><<<lc.lv.nLowBlocks, dev::kBlock, 0, stream>>>(lc.lv, lf.lv, stf, coarse, fine, mask);
-    ++launches;
-  }
+  const int nb = lc.lv.nLowBlocks + lc.lv.nFaceBands + lc.lv.nCellBlocks;
+  if (nb == 0) return;
+  dev::levelRestrictKernel<T><<<nb, dev::kBlock, 0, stream>>>(lc.lv, lf.lv, stf, coarse, fine, mask);
+  ++launches;
   cudaCheck(cudaGetLastError(), "restrict");
 }
 
@@ -2271,21 +2315,13 @@ void Storage::prolongT(int id, int Lc, unsigned mask, bool add) {
   T* fine = (T*)data(id, Lf);
   const T* coarse = (const T*)data(id, Lc);
   communicate(id, Lc, kAllGroups);
-  if (lf.lv.nCellBlocks) {
-    if (add) dev::cellProlongKernel<T, true><<<lf.lv.nCellBlocks, dev::kBlock, 0, stream>>>(lf.lv, lc.lv, fine, coarse, mask);
-    else dev::cellProlongKernel<T, false><<<lf.lv.nCellBlocks, dev::kBlock, 0, stream>>>(lf.lv, lc.lv, fine, coarse, mask);
-    ++launches;
-  }
-  if (lf.lv.nFaceBlocks) {
-    if (add) dev::faceProlongKernel<T, true><<<lf.lv.nFaceBlocks, dev::kBlock, 0, stream>>>(lf.lv, lc.lv, fine, coarse, mask);
-    else dev::faceProlongKernel<T, false><<<lf.lv.nFaceBlocks, dev::kBlock, 0, stream>>>(lf.lv, lc.lv, fine, coarse, mask);
-    ++launches;
-  }
-  if (lf.lv.nLowBlocks) {
-    if (add) dev::lowProlongKernel<T, true><<<lf.lv.nLowBlocks, dev::kBlock, 0, stream>>>(lf.lv, lc.lv, fine, coarse, mask);
-    else dev::lowProlongKernel<T, false><<<lf.lv.nLowBlocks, dev::kBlock, 0, stream>>>(lf.lv, lc.lv, fine, coarse, mask);
-    ++launches;
-  }
+  const int nb = lf.lv.nLowBlocks + lf.lv.nFaceBands + lf.lv.nCellBlocks;
+  if (nb == 0) return;
+  if (add)
+    dev::levelProlongKernel<T, true><<<nb, dev::kBlock, 0, stream>>>(lf.lv, lc.lv, fine, coarse, mask);
+  else
+    dev::levelProlongKernel<T, false><<<nb, dev::kBlock, 0, stream>>>(lf.lv, lc.lv, fine, coarse, mask);
+  ++launches;
   cudaCheck(cudaGetLastError(), "prolongate");
 }
 

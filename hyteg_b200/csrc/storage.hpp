@@ -3,6 +3,7 @@
 
 #include <cuda_runtime.h>
 
+#include <array>
 #include <deque>
 #include <map>
 #include <memory>
@@ -45,7 +46,8 @@ struct LevelData {
   std::vector<int> tileGroupBegin;  // group g: items [tileGroupBegin[g], tileGroupBegin[g + 1])
   int cellsPerGroup = 0;
   std::unique_ptr<DevBuf> tileBuf;
-  DevBuf partial;
+  DevBuf partial;               // the dot product's block sums, then the count of finished blocks
+  unsigned* arrived = nullptr;
   // single-pass SOR: one 32 x 32 (x, y) tile of a macro-cell per block, the tallest first
   // single-pass SOR tiles per [precision: 0 FP64, 1 FP32][tile geometry: 0, 1]
   dev::WaveTile* waveTiles[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};
@@ -229,6 +231,13 @@ struct Storage {
   // dst = a / b elementwise on the flagged primitives' slots (FP64)
   void divideBy(int dst, int a, int b, int L, unsigned mask);
   void dotAsync(int a, int b, int L, unsigned mask, double* dOut);
+  // Work vectors (p, ap, r) of CG solves on one level, kept from solve to solve with the storage and
+  // given up when a function cannot be allocated otherwise.
+  std::map<std::pair<int, int>, std::array<int, 3>> cgWorks;  // (level, precision)
+  const std::array<int, 3>& cgWork(int L, int prec);
+  void releaseCgWork();
+  // x += alpha p, r -= alpha ap with alpha = num / den, or (direction) p = r + beta p with beta = num / den
+  void cgUpdate(int L, unsigned mask, bool direction, const double* num, const double* den, int x, int r, int p, int ap);
   // Batched solves on a storage of `copies` disjoint copies of one macro-mesh (meshCuboidCopies):
   // the map of level L (checked against the layout), the right-hand sides of the first `active`
   // copies from their seeds (device array; the others 0), the dot product of every copy
