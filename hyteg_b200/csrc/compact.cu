@@ -88,6 +88,7 @@ __global__ void __launch_bounds__(kCompactThreads, 1) compactCycleKernel(const _
   extern __shared__ __align__(16) unsigned char compactSmem[];
   __shared__ double red[33];
   __shared__ double part[2];
+  waitForPredecessor(xs, bs, scratch, cgScratch);
   int rank = 0;
   if constexpr (CL > 1) rank = (int)cgrp::this_cluster().block_rank();
   const int grp = blockIdx.x / CL;
@@ -644,13 +645,15 @@ void launchT(CompactCycle& c, const dev::CompactCycleDev<T>& d, Storage& s, void
   cfg.blockDim = dim3(dev::kCompactThreads);
   cfg.dynamicSmemBytes = c.smem;
   cfg.stream = s.stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = CL;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = CL;
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = CL > 1 ? 1 : 0;
+  cfg.numAttrs = CL > 1 ? 2 : 1;
   cudaCheck(cudaLaunchKernelEx(&cfg, dev::compactCycleKernel<T, CL>, d, (T*)x, (const T*)b, (T*)c.scratch.p,
                                (double*)c.cg.p, (int)xZero, pre, post, (T)omega, cgMaxIter, cgTol),
             "compact cycle");

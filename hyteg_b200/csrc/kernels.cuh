@@ -22,6 +22,22 @@ namespace dev {
 
 constexpr int kBlock = 256;
 
+// Start of a kernel that is launched while its predecessor on the stream may still run (launchNext):
+// lets its own successor be set up, then waits until every predecessor has finished and its writes
+// are visible. The pointers are those to data that earlier kernels write; passing them through here
+// keeps the compiler from moving loads of read-only data in front of the wait.
+template <class P>
+__device__ __forceinline__ void heldBack(P& p) {
+  asm volatile("" : "+l"(p)::"memory");
+  __builtin_assume(__isGlobal(p));
+}
+template <class... P>
+__device__ __forceinline__ void waitForPredecessor(P&... p) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  (heldBack(p), ...);
+}
+
 struct FaceBlock {
   int face, start;  // rows [start, start + kFaceRows) of the face interior
 };
@@ -401,6 +417,7 @@ __device__ __forceinline__ int splitOfPlanePoint(int W, int p) {
 constexpr int kSplitUnroll = 4;
 template <class T, bool TO_SPLIT>
 __global__ void __launch_bounds__(kBlock) cellSplitKernel(LevelDev lv, T* __restrict__ dst, const T* __restrict__ src) {
+  waitForPredecessor(dst, src);
   const int nPl = lv.N + 1;
   const int c = blockIdx.x / nPl, z = blockIdx.x - (blockIdx.x / nPl) * nPl;
   const int W = lv.w - z;  // points on an edge of plane z
@@ -444,6 +461,7 @@ __global__ void __launch_bounds__(kBlock) cellSorSplitKernel(LevelDev lv, const 
                                                              const SplitRow* __restrict__ rows,
                                                              const unsigned* __restrict__ points, int nPoints,
                                                              int blocksPerCell, T omega) {
+  waitForPredecessor(u, rhs);
   const int c = blockIdx.x / blocksPerCell;
   if (!(lv.cellType[c] & mask)) return;
   __shared__ T wt[16];
@@ -507,6 +525,7 @@ template <class T>
 __global__ void __launch_bounds__(576, sizeof(T) == 4 ? 2 : 1) cellSorResidentKernel(LevelDev lv, const T* __restrict__ cellW, T* u,
                                                                 const T* __restrict__ rhs, unsigned mask,
                                                                 ResidentTables tb, T omega, int backwards) {
+  waitForPredecessor(u, rhs);
   extern __shared__ __align__(16) unsigned char residentSmemRaw[];
   __shared__ const SplitRow* rows[4];
   __shared__ const unsigned* points[4];
@@ -912,14 +931,16 @@ __global__ void __launch_bounds__(kBlock) lowSorPhaseKernel(LevelDev lv, Stencil
                                                             const uint2* __restrict__ table, const int2* __restrict__ range,
                                                             T* cells, int64_t cellEnd) {
   const int p = firstPrim + blockIdx.x;
+  const int first = lv.lowFirst[p], count = lv.lowCount[p];
+  const int64_t o = lv.lowOff[p];
+  const int e0 = st.lowEntOff[p], e1 = st.lowEntOff[p + 1];
+  const bool on = lv.lowType[p] & mask;
+  waitForPredecessor(u, rhs);
   if (range) {
     gatherRange(u, cells, table, range[p].x, range[p].y, cellEnd);
     __syncthreads();
   }
-  if (!(lv.lowType[p] & mask)) return;
-  const int first = lv.lowFirst[p], count = lv.lowCount[p];
-  const int64_t o = lv.lowOff[p];
-  const int e0 = st.lowEntOff[p], e1 = st.lowEntOff[p + 1];
+  if (!on) return;
   const int passes = p < lv.nEdges ? 2 : 1;
   const T om1 = T(1) - omega;
   for (int pass = 0; pass < passes; ++pass) {
@@ -946,16 +967,15 @@ __global__ void __launch_bounds__(kFacePhaseThreads) faceSorPhaseKernel(LevelDev
                                                                         int64_t cellEnd) {
   constexpr int kWarps = kFacePhaseThreads / 32;
   const int face = blockIdx.x;
-  if (range) {
-    gatherRange(u, cells, table, range[face].x, range[face].y, cellEnd);
-    __syncthreads();
-  }
-  if (!(lv.faceType[face] & mask)) return;
   __shared__ FaceEnt<T> ent[16];
   __shared__ int off[kWarps][16];
   const int ne = st.faceEntCount[face];
+  const bool on = lv.faceType[face] & mask;
   if (threadIdx.x < ne) ent[threadIdx.x] = st.faceEnt[16 * face + threadIdx.x];
+  waitForPredecessor(u, rhs);
+  if (range) gatherRange(u, cells, table, range[face].x, range[face].y, cellEnd);
   __syncthreads();
+  if (!on) return;
   const int w = lv.w, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t base = lv.faceOff[face];
   T* uf = u + base;
@@ -1085,6 +1105,7 @@ template <class T, int MODE>
 __global__ void __launch_bounds__(kLevelThreads, StripCfg<T>::MIN_BLOCKS)
     levelStencilKernel(LevelDev lv, StencilDev<T> st, const StripItem* __restrict__ items, int nLow, int lowBegin, int nFace,
                        T* __restrict__ dst, const T* __restrict__ src, const T* __restrict__ rhs, unsigned mask) {
+  waitForPredecessor(dst, src, rhs);
   const int blk = blockIdx.x;
   if (blk < nLow) {
     const LowBlock b = lv.lowBlocks[lowBegin + blk];
@@ -1348,6 +1369,7 @@ template <class T>
 __global__ void __launch_bounds__(kBlock) p2ProlongKernel(LevelDev lvc, LevelDev lvf, P2Tables tb, P2TransferDev tr,
                                                           const T* __restrict__ wts, const T* __restrict__ coarse,
                                                           T* __restrict__ fine) {
+  waitForPredecessor(coarse, fine);
   const int Mf = lvf.N, Mc = lvc.N, N = Mc / 2, nPl = Mf + 1, wf = lvf.w, wc = lvc.w;
   const int c = blockIdx.x / nPl, Z = blockIdx.x % nPl;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -1387,6 +1409,7 @@ __global__ void __launch_bounds__(kBlock) p2RestrictGatherKernel(LevelDev lvc, L
                                                                  const int* __restrict__ idx, const T* __restrict__ w,
                                                                  int nCoarse, int blocksPerCell, const T* __restrict__ fine,
                                                                  const unsigned char* __restrict__ mult, T* coarse) {
+  waitForPredecessor(fine, coarse);
   const int c = blockIdx.x / blocksPerCell;
   const int node = (blockIdx.x - c * blocksPerCell) * kBlock + threadIdx.x;
   if (node >= nCoarse) return;
@@ -1405,6 +1428,7 @@ __global__ void __launch_bounds__(kBlock) p2PickKernel(const int64_t* __restrict
                                                        const int64_t* __restrict__ copies,
                                                        const unsigned char* __restrict__ type, int n, T* dst,
                                                        unsigned mask) {
+  waitForPredecessor(dst);
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n || !(type[i] & mask)) return;
   dst[owner[i]] = dst[copies[ptr[i]]];
@@ -1418,10 +1442,19 @@ __global__ void __launch_bounds__(kBlock) p2AddKernel(const int64_t* __restrict_
                                                       const unsigned char* __restrict__ type, int n, T* dst,
                                                       const T* __restrict__ rhs, unsigned mask) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n || !(type[i] & mask)) return;
+  const bool on = i < n && (type[i] & mask);
+  const int k0 = on ? ptr[i] : 0, k1 = on ? ptr[i + 1] : 0;
+  const int64_t o = on ? owner[i] : 0;
+  int64_t c[2];  // most owners lie on faces: two copies
+#pragma unroll
+  for (int k = 0; k < 2; ++k) c[k] = k0 + k < k1 ? copies[k0 + k] : 0;
+  waitForPredecessor(dst, rhs);
+  if (!on) return;
   T v = T(0);
-  for (int k = ptr[i]; k < ptr[i + 1]; ++k) v += dst[copies[k]];
-  const int64_t o = owner[i];
+#pragma unroll
+  for (int k = 0; k < 2; ++k)
+    if (k0 + k < k1) v += dst[c[k]];
+  for (int k = k0 + 2; k < k1; ++k) v += dst[copies[k]];
   dst[o] = MODE == MODE_RESIDUAL ? rhs[o] - v : v;
 }
 
@@ -1449,6 +1482,7 @@ template <class T>
 __global__ void __launch_bounds__(kBlock) levelRestrictKernel(LevelDev lc, LevelDev lf, StencilDev<T> stf,
                                                               T* __restrict__ coarse, const T* __restrict__ fine,
                                                               unsigned mask) {
+  waitForPredecessor(coarse, fine);
   int blk = blockIdx.x;
   if (blk < lc.nLowBlocks) {
     const LowBlock b = lc.lowBlocks[blk];
@@ -1473,6 +1507,7 @@ __global__ void __launch_bounds__(kBlock) levelRestrictKernel(LevelDev lc, Level
 template <class T, bool ADD>
 __global__ void __launch_bounds__(kBlock) levelProlongKernel(LevelDev lf, LevelDev lc, T* __restrict__ fine,
                                                              const T* __restrict__ coarse, unsigned mask) {
+  waitForPredecessor(fine, coarse);
   int blk = blockIdx.x;
   if (blk < lf.nLowBlocks) {
     const LowBlock b = lf.lowBlocks[blk];
@@ -1615,13 +1650,18 @@ static __global__ void __launch_bounds__(kBlock)
 constexpr int kCommUnroll = 4;
 template <class T>
 __global__ void commGatherKernel(T* buf, const uint2* __restrict__ table, int64_t n) {
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t i0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i0 < n; i0 += kCommUnroll * stride) {
-    uint2 t[kCommUnroll];
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x, first = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  uint2 t[kCommUnroll];
+#pragma unroll
+  for (int k = 0; k < kCommUnroll; ++k)
+    if (first + k * stride < n) t[k] = __ldg(table + first + k * stride);
+  waitForPredecessor(buf);
+  for (int64_t i0 = first; i0 < n; i0 += kCommUnroll * stride) {
     T v[kCommUnroll];
 #pragma unroll
-    for (int k = 0; k < kCommUnroll; ++k)
-      if (i0 + k * stride < n) t[k] = table[i0 + k * stride];
+    for (int k = 0; k < kCommUnroll; ++k) {
+      if (i0 != first && i0 + k * stride < n) t[k] = __ldg(table + i0 + k * stride);
+    }
 #pragma unroll
     for (int k = 0; k < kCommUnroll; ++k)
       if (i0 + k * stride < n) v[k] = buf[t[k].y];
@@ -1636,6 +1676,7 @@ __global__ void commGatherKernel(T* buf, const uint2* __restrict__ table, int64_
 // cells, the others in buf.
 template <class T>
 __global__ void commGatherSplitKernel(T* buf, T* cells, const uint2* __restrict__ table, int64_t n, int64_t cellEnd) {
+  waitForPredecessor(buf, cells);
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     const uint2 t = table[i];
     const T v = t.y < cellEnd ? cells[t.y] : buf[t.y];
@@ -1663,6 +1704,7 @@ __global__ void __launch_bounds__(kBlock) lincombKernel(const Chunk* __restrict_
                                                         const T* s0, const T* s1, const T* s2, T a0, T a1, T a2,
                                                         T constant) {
   const Chunk ch = chunks[blockIdx.x];
+  waitForPredecessor(dst, s0, s1, s2);
   if (!(ch.type & mask)) return;
   T* d = dst + ch.start;
   for (int i0 = threadIdx.x; i0 < ch.len; i0 += kBlock * kLincombUnroll) {
@@ -1698,6 +1740,7 @@ __global__ void __launch_bounds__(kBlock) cgUpdateKernel(const Chunk* __restrict
                                                          const double* __restrict__ num, const double* __restrict__ den,
                                                          T* x, T* r, T* p, const T* ap) {
   const Chunk ch = chunks[blockIdx.x];
+  waitForPredecessor(num, den, x, r, p, ap);
   if (!(ch.type & mask)) return;
   constexpr int kU = 4;
   const double q = *num / *den;
@@ -1743,6 +1786,7 @@ static __global__ void __launch_bounds__(kBlock) divideKernel(const Chunk* __res
 template <class TD, class TS>
 __global__ void __launch_bounds__(kBlock) castKernel(const Chunk* __restrict__ chunks, unsigned mask, TD* dst,
                                                      const TS* src, int add) {
+  waitForPredecessor(dst, src);
   const Chunk ch = chunks[blockIdx.x];
   if (!(ch.type & mask)) return;
   for (int i = threadIdx.x; i < ch.len; i += blockDim.x) {
@@ -1758,6 +1802,7 @@ __global__ void __launch_bounds__(kBlock) castKernel(const Chunk* __restrict__ c
 static __global__ void __launch_bounds__(kBlock) denseCorrectKernel(const int64_t* __restrict__ idx, int n,
                                                                     const double* __restrict__ Ainv,
                                                                     const double* __restrict__ r, double* x) {
+  waitForPredecessor(r, x);
   extern __shared__ double rs[];
   for (int k = threadIdx.x; k < n; k += blockDim.x) rs[k] = r[idx[k]];
   __syncthreads();
@@ -1925,6 +1970,7 @@ static __global__ void __launch_bounds__(kBlock) reduceKernel(const double* __re
 template <class T>
 __global__ void __launch_bounds__(kBlock) dotReduceKernel(LevelDev lv, const T* __restrict__ a, const T* __restrict__ b,
                                                           unsigned mask, double* partial, unsigned* arrived, double* out) {
+  waitForPredecessor(a, b, partial, arrived, out);
   const double r = dotBlock<T>(lv, a, b, mask);
   __shared__ bool last;
   if (threadIdx.x == 0) {

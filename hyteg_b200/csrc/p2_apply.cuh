@@ -239,6 +239,7 @@ __global__ void __launch_bounds__(kBlock, 2) p2ApplyKernel(LevelDev lv, const P2
                                                            const T* __restrict__ W, const T* __restrict__ FW,
                                                            T* __restrict__ dst, const T* __restrict__ src,
                                                            const T* __restrict__ rhs, unsigned mask) {
+  waitForPredecessor(dst, src, rhs);
   extern __shared__ __align__(16) unsigned char p2Smem[];
   const int c = blockIdx.x % lv.nCells;
   const P2Item it = items[blockIdx.x / lv.nCells];

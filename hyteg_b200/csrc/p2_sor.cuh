@@ -93,8 +93,10 @@ __global__ void __launch_bounds__(kBlock, 3) p2SorGatherKernel(LevelDev lv, cons
   const int M = lv.N, w = lv.w;
   if ((int)blockIdx.x < listBlocks) {
     const int i = blockIdx.x * kBlock + threadIdx.x;
+    const P2ClosureNode nd = list[min(i, nList - 1)];
+    const int64_t base = lv.cellOff[nd.cell];
+    waitForPredecessor(x, b, ax);
     if (i >= nList) return;
-    const P2ClosureNode nd = list[i];
     const int X = nd.x, Y = nd.y, Z = nd.z;
     int pbz[5];
 #pragma unroll
@@ -102,20 +104,20 @@ __global__ void __launch_bounds__(kBlock, 3) p2SorGatherKernel(LevelDev lv, cons
       const int z = Z - 2 + d;
       pbz[d] = (z >= 0 && z <= M) ? int(tetSize(w) - tetSize(w - z)) : 0;
     }
-    const int64_t base = lv.cellOff[nd.cell];
     ax[base + pbz[2] + rowStart(w - Z, Y) + X] =
         p2FaceDotAny<T>(nd.k, x + base, FW + (int64_t)nd.cell * p2s::kFaceTotal, pbz, w, X, Y, Z);
     return;
   }
+  // the list entry is read before the wait, whether or not the cell has the colour
   const int q = blockIdx.x - listBlocks, c = q / chunks;
-  if (!(lv.cellType[c] & mask)) return;
+  const bool on = lv.cellType[c] & mask;
   const P2CellColour cc = cells[c];
   const int pc = cells[c].cls[sel];
-  if (pc < 0) return;
-  const unsigned t = nodes[pc] + (q - c * chunks) * kBlock + threadIdx.x;
-  if (t >= nodes[pc + 1]) return;
-  const unsigned e = __ldg(nodes + t);
+  const unsigned end = nodes[max(pc, 0) + 1], t = nodes[max(pc, 0)] + (q - c * chunks) * kBlock + threadIdx.x;
+  const unsigned e = t < end ? __ldg(nodes + t) : 0;
   const int64_t base = lv.cellOff[c];
+  waitForPredecessor(x, b, ax);
+  if (!on || pc < 0 || t >= end) return;
   const T* wc = W + (int64_t)c * p2s::kTotal;
   switch (pc) {
     case 0: p2SorNodes<T, 0>(e, cc, sel, x + base, b + base, ax + base, wc, w, M, omega); break;
@@ -139,9 +141,9 @@ __global__ void __launch_bounds__(kBlock) p2SorUpdateKernel(LevelDev lv, const P
                                                             unsigned mask, T omega) {
   if ((int)blockIdx.x < ownerBlocks) {
     const int t = blockIdx.x * kBlock + threadIdx.x;
-    if (t >= nOwners) return;
-    const P2Owner o = owners[t];
-    if (!(o.type & mask)) return;
+    const P2Owner o = owners[min(t, nOwners - 1)];
+    waitForPredecessor(x, b, ax, diag);
+    if (t >= nOwners || !(o.type & mask)) return;
     const T x0 = x[o.slot], b0 = __ldg(b + o.slot), d0 = __ldg(diag + o.slot);
     T s = T(0);
     for (int k = o.first; k < o.first + o.count; ++k) s += __ldg(ax + copies[k]);
@@ -152,14 +154,14 @@ __global__ void __launch_bounds__(kBlock) p2SorUpdateKernel(LevelDev lv, const P
     return;
   }
   const int M = lv.N, w = lv.w, q = blockIdx.x - ownerBlocks, c = q / chunks;
-  if (!(lv.cellType[c] & mask)) return;
+  const bool on = lv.cellType[c] & mask;
   const P2CellColour cc = cells[c];
   const int pc = cells[c].cls[sel];
-  if (pc < 0) return;
-  const unsigned t = nodes[pc] + (q - c * chunks) * kBlock + threadIdx.x;
-  if (t >= nodes[pc + 1]) return;
-  const unsigned e = __ldg(nodes + t);
+  const unsigned end = nodes[max(pc, 0) + 1], t = nodes[max(pc, 0)] + (q - c * chunks) * kBlock + threadIdx.x;
+  const unsigned e = t < end ? __ldg(nodes + t) : 0;
   const int64_t base = lv.cellOff[c];
+  waitForPredecessor(x, b, ax, diag);
+  if (!on || pc < 0 || t >= end) return;
   auto take = [&](int X, int Y, int Z) {
     const int64_t i = base + int(tetSize(w) - tetSize(w - Z)) + rowStart(w - Z, Y) + X;
     x[i] = __ldg(ax + i);

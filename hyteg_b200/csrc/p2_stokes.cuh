@@ -85,6 +85,7 @@ __global__ void __launch_bounds__(kBlock) p2DivKernel(LevelDev lvp, LevelDev lvv
                                                       int nList, int listBlocks, T* __restrict__ q,
                                                       const T* __restrict__ u0, const T* __restrict__ u1,
                                                       const T* __restrict__ u2, unsigned mask) {
+  waitForPredecessor(q, u0, u1, u2);
   const int N = lvp.N, wp = lvp.w, wv = lvv.w, M = lvv.N;
   int pbz[5];
   if ((int)blockIdx.x < listBlocks) {
@@ -178,6 +179,7 @@ __global__ void __launch_bounds__(kBlock) p2DivTKernel(LevelDev lvv, LevelDev lv
                                                        const T* __restrict__ WC, const P2ClosureNode* __restrict__ list,
                                                        int nList, int listBlocks, T* __restrict__ v0, T* __restrict__ v1,
                                                        T* __restrict__ v2, const T* __restrict__ p, unsigned mask) {
+  waitForPredecessor(v0, v1, v2, p);
   const int M = lvv.N, wv = lvv.w, wp = lvp.w, Np = lvp.N;
   int pbz[5];
   if ((int)blockIdx.x < listBlocks) {

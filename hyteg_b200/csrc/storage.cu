@@ -364,10 +364,10 @@ void Storage::cgUpdate(int L, unsigned mask, bool direction, const double* num, 
     using T = decltype(zero);
     T *xd = direction ? nullptr : (T*)data(x, L), *ad = direction ? nullptr : (T*)data(ap, L);
     if (direction)
-      dev::cgUpdateKernel<T, true><<<ld.nChunks, dev::kBlock, 0, stream>>>(ld.chunks, mask, num, den, xd, (T*)data(r, L),
+      launchNext(stream, dev::cgUpdateKernel<T, true>, ld.nChunks, dev::kBlock, 0, ld.chunks, mask, num, den, xd, (T*)data(r, L),
                                                                            (T*)data(p, L), ad);
     else
-      dev::cgUpdateKernel<T, false><<<ld.nChunks, dev::kBlock, 0, stream>>>(ld.chunks, mask, num, den, xd, (T*)data(r, L),
+      launchNext(stream, dev::cgUpdateKernel<T, false>, ld.nChunks, dev::kBlock, 0, ld.chunks, mask, num, den, xd, (T*)data(r, L),
                                                                             (T*)data(p, L), ad);
   };
   if (fn(r).prec == 8) run(0.0);
@@ -428,9 +428,9 @@ void Storage::communicate(int id, int L, int groupMask) {
     while (k < G_COUNT && (groupMask & (1 << kCommOrder[k]))) n += ld.commCount[kCommOrder[k++]];
     if (n == 0) continue;
     if (f.prec == 8)
-      dev::commGatherKernel<double><<<grid1d(n), 256, 0, stream>>>((double*)d, ld.comm + begin, n);
+      launchNext(stream, dev::commGatherKernel<double>, grid1d(n), 256, 0, (double*)d, ld.comm + begin, n);
     else
-      dev::commGatherKernel<float><<<grid1d(n), 256, 0, stream>>>((float*)d, ld.comm + begin, n);
+      launchNext(stream, dev::commGatherKernel<float>, grid1d(n), 256, 0, (float*)d, ld.comm + begin, n);
     ++launches;
   }
   cudaCheck(cudaGetLastError(), "communicate");
@@ -451,7 +451,7 @@ void Storage::communicateSplit(T* buf, T* cells, int L, int groupMask) {
     int64_t n = 0;
     while (k < G_COUNT && (groupMask & (1 << kCommOrder[k]))) n += ld.commCount[kCommOrder[k++]];
     if (n == 0) continue;
-    dev::commGatherSplitKernel<T><<<grid1d(n), 256, 0, stream>>>(buf, cells, table + begin, n, ld.nonCellBegin);
+    launchNext(stream, dev::commGatherSplitKernel<T>, grid1d(n), 256, 0, buf, cells, table + begin, n, ld.nonCellBegin);
     ++launches;
   }
   cudaCheck(cudaGetLastError(), "communicate (split)");
@@ -589,8 +589,7 @@ void Storage::lincomb(int dst, int L, unsigned mask, int n, const double* a, con
   auto run = [&](auto zero) {
     using T = decltype(zero);
     auto go = [&](auto nsrc, auto addTo) {
-      dev::lincombKernel<T, decltype(nsrc)::value, decltype(addTo)::value><<<ld.nChunks, dev::kBlock, 0, stream>>>(
-          ld.chunks, mask, (T*)pd, (const T*)ps[0], (const T*)ps[1], (const T*)ps[2], T(sc[0]), T(sc[1]), T(sc[2]),
+      launchNext(stream, dev::lincombKernel<T, decltype(nsrc)::value, decltype(addTo)::value>, ld.nChunks, dev::kBlock, 0, ld.chunks, mask, (T*)pd, (const T*)ps[0], (const T*)ps[1], (const T*)ps[2], T(sc[0]), T(sc[1]), T(sc[2]),
           T(constant));
     };
     auto pick = [&](auto nsrc) {
@@ -627,13 +626,13 @@ void Storage::copyCast(int dst, int src, int L, unsigned mask, bool add) {
   if (ld.nChunks == 0) return;
   const int a = add ? 1 : 0;
   if (fd.prec == 8 && fs.prec == 8)
-    dev::castKernel<double, double><<<ld.nChunks, dev::kBlock, 0, stream>>>(ld.chunks, mask, (double*)pd, (const double*)ps, a);
+    launchNext(stream, dev::castKernel<double, double>, ld.nChunks, dev::kBlock, 0, ld.chunks, mask, (double*)pd, (const double*)ps, a);
   else if (fd.prec == 8)
-    dev::castKernel<double, float><<<ld.nChunks, dev::kBlock, 0, stream>>>(ld.chunks, mask, (double*)pd, (const float*)ps, a);
+    launchNext(stream, dev::castKernel<double, float>, ld.nChunks, dev::kBlock, 0, ld.chunks, mask, (double*)pd, (const float*)ps, a);
   else if (fs.prec == 8)
-    dev::castKernel<float, double><<<ld.nChunks, dev::kBlock, 0, stream>>>(ld.chunks, mask, (float*)pd, (const double*)ps, a);
+    launchNext(stream, dev::castKernel<float, double>, ld.nChunks, dev::kBlock, 0, ld.chunks, mask, (float*)pd, (const double*)ps, a);
   else
-    dev::castKernel<float, float><<<ld.nChunks, dev::kBlock, 0, stream>>>(ld.chunks, mask, (float*)pd, (const float*)ps, a);
+    launchNext(stream, dev::castKernel<float, float>, ld.nChunks, dev::kBlock, 0, ld.chunks, mask, (float*)pd, (const float*)ps, a);
   ++launches;
   cudaCheck(cudaGetLastError(), "copyCast");
 }
@@ -645,10 +644,10 @@ void Storage::dotAsync(int a, int b, int L, unsigned mask, double* dOut) {
   const int nb = ld.lv.nCellBlocks + ld.lv.nFaceBlocks + ld.lv.nLowBlocks;
   double* partial = (double*)ld.partial.p;
   if (fa.prec == 8)
-    dev::dotReduceKernel<double><<<nb, dev::kBlock, 0, stream>>>(ld.lv, (const double*)data(a, L),
+    launchNext(stream, dev::dotReduceKernel<double>, nb, dev::kBlock, 0, ld.lv, (const double*)data(a, L),
                                                                  (const double*)data(b, L), mask, partial, ld.arrived, dOut);
   else
-    dev::dotReduceKernel<float><<<nb, dev::kBlock, 0, stream>>>(ld.lv, (const float*)data(a, L), (const float*)data(b, L),
+    launchNext(stream, dev::dotReduceKernel<float>, nb, dev::kBlock, 0, ld.lv, (const float*)data(a, L), (const float*)data(b, L),
                                                                 mask, partial, ld.arrived, dOut);
   ++launches;
   cudaCheck(cudaGetLastError(), "dot");
@@ -1292,8 +1291,7 @@ static std::vector<double> p2FaceStencils(const std::vector<double>& K, int nCel
 template <class T, int MODE>
 void Storage::p2AddOwners(const P2Additive& ad, T* dst, const T* rhs, unsigned mask) {
   if (!ad.n) return;
-  dev::p2AddKernel<T, MODE><<<(ad.n + dev::kBlock - 1) / dev::kBlock, dev::kBlock, 0, stream>>>(
-      (const int64_t*)ad.owner.p, (const int*)ad.ptr.p, (const int64_t*)ad.copies.p, (const unsigned char*)ad.type.p,
+  launchNext(stream, dev::p2AddKernel<T, MODE>, (ad.n + dev::kBlock - 1) / dev::kBlock, dev::kBlock, 0, (const int64_t*)ad.owner.p, (const int*)ad.ptr.p, (const int64_t*)ad.copies.p, (const unsigned char*)ad.type.p,
       ad.n, dst, rhs, mask);
   ++launches;
 }
@@ -1307,8 +1305,7 @@ void Storage::p2Sweep(P2Operator& o, int L, T* dst, const T* src, const T* rhs, 
   P2Additive& ad = p2Additive(Lf);
   const T* W = (const T*)(sizeof(T) == 8 ? o.sd[L - o.minL]->p : o.sf[L - o.minL]->p);
   const T* FW = (const T*)(sizeof(T) == 8 ? o.fd[L - o.minL]->p : o.ff[L - o.minL]->p);
-  dev::p2ApplyKernel<T, MODE><<<ld.lv.nCells * ad.nItems, dev::kBlock, dev::p2TileSmem<T>(), stream>>>(
-      ld.lv, (const dev::P2Item*)ad.items.p, W, FW, dst, src, rhs, mask);
+  launchNext(stream, dev::p2ApplyKernel<T, MODE>, ld.lv.nCells * ad.nItems, dev::kBlock, dev::p2TileSmem<T>(), ld.lv, (const dev::P2Item*)ad.items.p, W, FW, dst, src, rhs, mask);
   ++launches;
   cudaCheck(cudaGetLastError(), "P2 kernels");
 }
@@ -1400,14 +1397,12 @@ void Storage::p2SorT(P2Operator& o, int opId, int x, int b, int L, unsigned mask
     const int nOwn = ad.sorOwnerBegin[c + 1] - ad.sorOwnerBegin[c], ownBlocks = blocks(nOwn);
     const int inner = ld.lv.nCells * chunks;
     if (listBlocks + inner > 0) {
-      dev::p2SorGatherKernel<T><<<listBlocks + inner, dev::kBlock, 0, stream>>>(
-          ld.lv, W, FW, (const dev::P2ClosureNode*)ad.closureList.p + ad.closureBegin[c], nList, listBlocks,
+      launchNext(stream, dev::p2SorGatherKernel<T>, listBlocks + inner, dev::kBlock, 0, ld.lv, W, FW, (const dev::P2ClosureNode*)ad.closureList.p + ad.closureBegin[c], nList, listBlocks,
           (const unsigned*)ad.sorInner.p, cells, c, std::max(chunks, 1), xd, bd, axd, mask, omega);
       ++launches;
     }
     if (ownBlocks + inner > 0) {
-      dev::p2SorUpdateKernel<T><<<ownBlocks + inner, dev::kBlock, 0, stream>>>(
-          ld.lv, (const dev::P2Owner*)ad.sorOwners.p + ad.sorOwnerBegin[c], nOwn, ownBlocks,
+      launchNext(stream, dev::p2SorUpdateKernel<T>, ownBlocks + inner, dev::kBlock, 0, ld.lv, (const dev::P2Owner*)ad.sorOwners.p + ad.sorOwnerBegin[c], nOwn, ownBlocks,
           (const unsigned*)ad.sorCopies.p, (const unsigned*)ad.sorInner.p, cells, c, std::max(chunks, 1), xd, bd, axd,
           (const T*)data(dg, Lf), mask, omega);
       ++launches;
@@ -1568,17 +1563,17 @@ void Storage::p2Prolongate(int id, int Lc, unsigned mask, bool add) {
   const dev::P2TransferDev tr{(const unsigned char*)p2tr.nCand.p, (const unsigned char*)p2tr.cand.p};
   const int nb = lf.lv.nCells * (lf.lv.N + 1), na = (ad.n + dev::kBlock - 1) / dev::kBlock;
   if (f.prec == 8) {
-    dev::p2ProlongKernel<double><<<nb, dev::kBlock, 0, stream>>>(lc.lv, lf.lv, p2TablesOnce(), tr, (const double*)p2tr.wd.p,
+    launchNext(stream, dev::p2ProlongKernel<double>, nb, dev::kBlock, 0, lc.lv, lf.lv, p2TablesOnce(), tr, (const double*)p2tr.wd.p,
                                                                (const double*)data(id, Lcf), (double*)data(out, Lff));
     if (ad.n)
-      dev::p2PickKernel<double><<<na, dev::kBlock, 0, stream>>>((const int64_t*)ad.owner.p, (const int*)ad.ptr.p,
+      launchNext(stream, dev::p2PickKernel<double>, na, dev::kBlock, 0, (const int64_t*)ad.owner.p, (const int*)ad.ptr.p,
                                                               (const int64_t*)ad.copies.p, (const unsigned char*)ad.type.p,
                                                               ad.n, (double*)data(out, Lff), add ? HG_ALL : mask);
   } else {
-    dev::p2ProlongKernel<float><<<nb, dev::kBlock, 0, stream>>>(lc.lv, lf.lv, p2TablesOnce(), tr, (const float*)p2tr.wf.p,
+    launchNext(stream, dev::p2ProlongKernel<float>, nb, dev::kBlock, 0, lc.lv, lf.lv, p2TablesOnce(), tr, (const float*)p2tr.wf.p,
                                                               (const float*)data(id, Lcf), (float*)data(out, Lff));
     if (ad.n)
-      dev::p2PickKernel<float><<<na, dev::kBlock, 0, stream>>>((const int64_t*)ad.owner.p, (const int*)ad.ptr.p,
+      launchNext(stream, dev::p2PickKernel<float>, na, dev::kBlock, 0, (const int64_t*)ad.owner.p, (const int*)ad.ptr.p,
                                                              (const int64_t*)ad.copies.p, (const unsigned char*)ad.type.p,
                                                              ad.n, (float*)data(out, Lff), add ? HG_ALL : mask);
   }
@@ -1606,22 +1601,18 @@ void Storage::p2Restrict(int id, int Lf, unsigned mask) {
   const int bpc = (gt.nCoarse + dev::kBlock - 1) / dev::kBlock;
   const int nb = lf.lv.nCells * bpc, na = (adc.n + dev::kBlock - 1) / dev::kBlock;
   if (f.prec == 8) {
-    dev::p2RestrictGatherKernel<double><<<nb, dev::kBlock, 0, stream>>>(
-        lc.lv, lf.lv, (const int*)gt.ptr.p, (const int*)gt.idx.p, (const double*)gt.wd.p, gt.nCoarse, bpc,
+    launchNext(stream, dev::p2RestrictGatherKernel<double>, nb, dev::kBlock, 0, lc.lv, lf.lv, (const int*)gt.ptr.p, (const int*)gt.idx.p, (const double*)gt.wd.p, gt.nCoarse, bpc,
         (const double*)data(id, Lff),
         (const unsigned char*)adf.mult.p, (double*)data(id, Lcf));
     if (adc.n)
-      dev::p2AddKernel<double, dev::MODE_REPLACE><<<na, dev::kBlock, 0, stream>>>(
-          (const int64_t*)adc.owner.p, (const int*)adc.ptr.p, (const int64_t*)adc.copies.p,
+      launchNext(stream, dev::p2AddKernel<double, dev::MODE_REPLACE>, na, dev::kBlock, 0, (const int64_t*)adc.owner.p, (const int*)adc.ptr.p, (const int64_t*)adc.copies.p,
           (const unsigned char*)adc.type.p, adc.n, (double*)data(id, Lcf), nullptr, mask);
   } else {
-    dev::p2RestrictGatherKernel<float><<<nb, dev::kBlock, 0, stream>>>(
-        lc.lv, lf.lv, (const int*)gt.ptr.p, (const int*)gt.idx.p, (const float*)gt.wf.p, gt.nCoarse, bpc,
+    launchNext(stream, dev::p2RestrictGatherKernel<float>, nb, dev::kBlock, 0, lc.lv, lf.lv, (const int*)gt.ptr.p, (const int*)gt.idx.p, (const float*)gt.wf.p, gt.nCoarse, bpc,
         (const float*)data(id, Lff),
         (const unsigned char*)adf.mult.p, (float*)data(id, Lcf));
     if (adc.n)
-      dev::p2AddKernel<float, dev::MODE_REPLACE><<<na, dev::kBlock, 0, stream>>>(
-          (const int64_t*)adc.owner.p, (const int*)adc.ptr.p, (const int64_t*)adc.copies.p,
+      launchNext(stream, dev::p2AddKernel<float, dev::MODE_REPLACE>, na, dev::kBlock, 0, (const int64_t*)adc.owner.p, (const int*)adc.ptr.p, (const int64_t*)adc.copies.p,
           (const unsigned char*)adc.type.p, adc.n, (float*)data(id, Lcf), nullptr, mask);
   }
   launches += adc.n ? 2 : 1;
@@ -1736,8 +1727,7 @@ static void launchDivT(Storage& st, P2Operator& o, int p, const int v[3], int L,
   const T* WC = (const T*)(sizeof(T) == 8 ? o.wdivtcd[L - o.minL]->p : o.wdivtcf[L - o.minL]->p);
   const int nList = adv.closureBegin[11], listBlocks = (nList + dev::kBlock - 1) / dev::kBlock;
   const int inner = lvv.lv.N >= 4 ? lvv.lv.nCells * (lvv.lv.N - 3) : 0;
-  dev::p2DivTKernel<T, ADD><<<listBlocks + inner, dev::kBlock, 0, st.stream>>>(
-      lvv.lv, lvp.lv, WT, WC, (const dev::P2ClosureNode*)adv.closureList.p, nList, listBlocks, (T*)st.data(v[0], Lv),
+  launchNext(st.stream, dev::p2DivTKernel<T, ADD>, listBlocks + inner, dev::kBlock, 0, lvv.lv, lvp.lv, WT, WC, (const dev::P2ClosureNode*)adv.closureList.p, nList, listBlocks, (T*)st.data(v[0], Lv),
       (T*)st.data(v[1], Lv), (T*)st.data(v[2], Lv), (const T*)st.data(p, Lp), maskV);
   ++st.launches;
 }
@@ -1754,8 +1744,7 @@ static void launchDiv(Storage& st, P2Operator& o, const int u[3], int q, int L, 
   const T* WC = (const T*)(sizeof(T) == 8 ? o.wdivcd[L - o.minL]->p : o.wdivcf[L - o.minL]->p);
   const int nList = adp.closureBegin[11], listBlocks = (nList + dev::kBlock - 1) / dev::kBlock;
   const int inner = lvp.lv.N >= 4 ? lvp.lv.nCells * (lvp.lv.N - 3) : 0;
-  dev::p2DivKernel<T><<<listBlocks + inner, dev::kBlock, 0, st.stream>>>(
-      lvp.lv, lvv.lv, WD, WC, (const dev::P2ClosureNode*)adp.closureList.p, nList, listBlocks, (T*)st.data(q, Lp),
+  launchNext(st.stream, dev::p2DivKernel<T>, listBlocks + inner, dev::kBlock, 0, lvp.lv, lvv.lv, WD, WC, (const dev::P2ClosureNode*)adp.closureList.p, nList, listBlocks, (T*)st.data(q, Lp),
       (const T*)st.data(u[0], Lv), (const T*)st.data(u[1], Lv), (const T*)st.data(u[2], Lv), maskP);
   ++st.launches;
   st.p2AddOwners<T, dev::MODE_REPLACE>(adp, (T*)st.data(q, Lp), nullptr, maskP);
@@ -1953,6 +1942,9 @@ void Storage::reassembleOperator(int id, bool onDevice) {
     ++launches;
   }
   cudaCheck(cudaGetLastError(), "re-assembly");
+  // kernels set up ahead of their predecessor's end may read stencil weights before they wait for it;
+  // none is set up ahead of the end of a memset
+  cudaCheck(cudaMemsetAsync((double*)scalars.p + 63, 0, sizeof(double), stream), "re-assembly");
   o.hostStale = true;
 }
 
@@ -2000,8 +1992,7 @@ void Storage::stencilOp(Operator& o, int L, T* dst, const T* src, const T* rhs, 
   const int nCell = kinds & (1 << KC) ? ld.nTiles : 0, nFace = kinds & (1 << KF) ? ld.lv.nFaceBands : 0;
   const int nLow = (edges ? ld.lv.nLowEdgeBlocks : 0) + (verts ? nVertBlocks : 0);
   if (nCell + nFace + nLow == 0) return;
-  dev::levelStencilKernel<T, MODE><<<nLow + nFace + nCell, dev::kLevelThreads, 0, stream>>>(
-      ld.lv, st, ld.tiles, nLow, edges ? 0 : ld.lv.nLowEdgeBlocks, nFace, dst, src, rhs, mask);
+  launchNext(stream, dev::levelStencilKernel<T, MODE>, nLow + nFace + nCell, dev::kLevelThreads, 0, ld.lv, st, ld.tiles, nLow, edges ? 0 : ld.lv.nLowEdgeBlocks, nFace, dst, src, rhs, mask);
   ++launches;
   cudaCheck(cudaGetLastError(), "stencil kernel");
 }
@@ -2078,8 +2069,7 @@ void Storage::sorT(Operator& o, int dstId, int L, T* u, const T* rhs, unsigned m
         const int c = rev ? 3 - k : k, n = ld.nSplitPoints[c];
         if (n == 0) continue;
         const int bpc = (n + dev::kBlock - 1) / dev::kBlock;
-        dev::cellSorSplitKernel<T><<<(unsigned)(bpc * lv.nCells), dev::kBlock, 0, stream>>>(
-            lv, st.cellW, cellU, cellF, mask, ld.splitRows[c], ld.splitPoints[c], n, bpc, omega);
+        launchNext(stream, dev::cellSorSplitKernel<T>, (unsigned)(bpc * lv.nCells), dev::kBlock, 0, lv, st.cellW, cellU, cellF, mask, ld.splitRows[c], ld.splitPoints[c], n, bpc, omega);
         ++launches;
       }
       return;
@@ -2098,8 +2088,7 @@ void Storage::sorT(Operator& o, int dstId, int L, T* u, const T* rhs, unsigned m
       }
       tb.comm = ld.comm;
       tb.range = refresh ? ld.cellRange : nullptr;
-      dev::cellSorResidentKernel<T><<<lv.nCells, dev::residentThreads(lv.N), dev::residentSmem<T>(lv.N), stream>>>(
-          lv, st.cellW, u, rhs, mask, tb, omega, rev ? 1 : 0);
+      launchNext(stream, dev::cellSorResidentKernel<T>, lv.nCells, dev::residentThreads(lv.N), dev::residentSmem<T>(lv.N), lv, st.cellW, u, rhs, mask, tb, omega, rev ? 1 : 0);
       ++launches;
       return;
     }
@@ -2153,14 +2142,13 @@ void Storage::sorT(Operator& o, int dstId, int L, T* u, const T* rhs, unsigned m
     auto lowPhase = [&](bool edgesNotVerts, bool gather, bool rev) {
       const int first = edgesNotVerts ? 0 : lv.nEdges, n = edgesNotVerts ? lv.nEdges : lv.nLow - lv.nEdges;
       if (n == 0 || !(kinds & (1 << (edgesNotVerts ? KE : KV)))) return;
-      dev::lowSorPhaseKernel<T><<<n, dev::kBlock, 0, stream>>>(lv, st, u, rhs, mask, omega, first, rev ? 1 : 0, table,
+      launchNext(stream, dev::lowSorPhaseKernel<T>, n, dev::kBlock, 0, lv, st, u, rhs, mask, omega, first, rev ? 1 : 0, table,
                                                              gather && refresh ? ld.lowRange : nullptr, cellsBuf, cellEnd);
       ++launches;
     };
     auto facePhase = [&](bool gather, bool rev) {
       if (lv.nFaceBlocks == 0 || !(kinds & (1 << KF))) return;
-      dev::faceSorPhaseKernel<T><<<lv.nFaces, dev::kFacePhaseThreads, 0, stream>>>(
-          lv, st, u, rhs, mask, omega, rev ? 1 : 0, table, gather && refresh ? ld.faceRange : nullptr, cellsBuf, cellEnd);
+      launchNext(stream, dev::faceSorPhaseKernel<T>, lv.nFaces, dev::kFacePhaseThreads, 0, lv, st, u, rhs, mask, omega, rev ? 1 : 0, table, gather && refresh ? ld.faceRange : nullptr, cellsBuf, cellEnd);
       ++launches;
     };
     if (!backwards) {
@@ -2257,14 +2245,14 @@ void Storage::smoothSorSweeps(int opId, int dst, int rhs, double omega, int L, u
     buildSplit(L);
     T* cu = (T*)spareBuf(spare, L, (int)sizeof(T)).p;
     T* cf = (T*)spareBuf(splitRhs, L, (int)sizeof(T)).p;
-    dev::cellSplitKernel<T, true><<<nb, dev::kBlock, 0, stream>>>(ld.lv, cu, u);
+    launchNext(stream, dev::cellSplitKernel<T, true>, nb, dev::kBlock, 0, ld.lv, cu, u);
     ++launches;
     if (!rhsReady) {
-      dev::cellSplitKernel<T, true><<<nb, dev::kBlock, 0, stream>>>(ld.lv, cf, b);
+      launchNext(stream, dev::cellSplitKernel<T, true>, nb, dev::kBlock, 0, ld.lv, cf, b);
       ++launches;
     }
     for (int i = 0; i < sweeps; ++i) sorT<T>(o, dst, L, u, b, mask, (T)omega, backwards, 15, true, cu, cf);
-    dev::cellSplitKernel<T, false><<<nb, dev::kBlock, 0, stream>>>(ld.lv, u, cu);
+    launchNext(stream, dev::cellSplitKernel<T, false>, nb, dev::kBlock, 0, ld.lv, u, cu);
     ++launches;
     cudaCheck(cudaGetLastError(), "sor (colour-split)");
   };
@@ -2291,7 +2279,7 @@ void Storage::restrictT(int id, int Lf, unsigned mask, int coarseDst) {
   communicate(id, Lf, kAllGroups);
   const int nb = lc.lv.nLowBlocks + lc.lv.nFaceBands + lc.lv.nCellBlocks;
   if (nb == 0) return;
-  dev::levelRestrictKernel<T><<<nb, dev::kBlock, 0, stream>>>(lc.lv, lf.lv, stf, coarse, fine, mask);
+  launchNext(stream, dev::levelRestrictKernel<T>, nb, dev::kBlock, 0, lc.lv, lf.lv, stf, coarse, fine, mask);
   ++launches;
   cudaCheck(cudaGetLastError(), "restrict");
 }
@@ -2318,9 +2306,9 @@ void Storage::prolongT(int id, int Lc, unsigned mask, bool add) {
   const int nb = lf.lv.nLowBlocks + lf.lv.nFaceBands + lf.lv.nCellBlocks;
   if (nb == 0) return;
   if (add)
-    dev::levelProlongKernel<T, true><<<nb, dev::kBlock, 0, stream>>>(lf.lv, lc.lv, fine, coarse, mask);
+    launchNext(stream, dev::levelProlongKernel<T, true>, nb, dev::kBlock, 0, lf.lv, lc.lv, fine, coarse, mask);
   else
-    dev::levelProlongKernel<T, false><<<nb, dev::kBlock, 0, stream>>>(lf.lv, lc.lv, fine, coarse, mask);
+    launchNext(stream, dev::levelProlongKernel<T, false>, nb, dev::kBlock, 0, lf.lv, lc.lv, fine, coarse, mask);
   ++launches;
   cudaCheck(cudaGetLastError(), "prolongate");
 }
