@@ -873,6 +873,29 @@ __device__ __forceinline__ int loadFaceEntries(FaceShared<T>& sh, const StencilD
   return ne;
 }
 
+// The SOR update of a face row's point: off holds the entries' slots of the row (the row's own beyond
+// the ne entries), entry 0 is the diagonal (dinv = omega / a_ii). The sum is taken in four parts. The
+// loads are issued ahead of it, all 15 in FP32, five at a time in FP64, where 15 take the registers
+// (phase on level 7, 48 cells: 44 us with 15, 34 with 5; FP32 cycle on 27 cubes 11.2 / 11.5 ms).
+template <class T>
+__device__ __forceinline__ T faceSorPoint(const FaceEnt<T>* ent, int ne, const int* off, const T* uf, const T* f, int r0,
+                                          int x, T om1, T dinv) {
+  constexpr int kLoads = sizeof(T) == 4 ? 15 : 5;
+  T s[4] = {f[r0 + x], T(0), T(0), T(0)};
+  const T old = uf[r0 + x];
+#pragma unroll
+  for (int k0 = 1; k0 < 16; k0 += kLoads) {
+    if (k0 >= ne) break;
+    T v[kLoads];
+#pragma unroll
+    for (int k = 0; k < kLoads; ++k) v[k] = uf[off[k0 + k] + x];
+#pragma unroll
+    for (int k = 0; k < kLoads; ++k)
+      if (k0 + k < ne) s[k & 3] -= ent[k0 + k].w * v[k];
+  }
+  return om1 * old + ((s[0] + s[1]) + (s[2] + s[3])) * dinv;
+}
+
 // Face SOR, colour = (x + 2y) mod 3; entry 0 is the diagonal.
 template <class T>
 __global__ void __launch_bounds__(kBlock) faceSorKernel(LevelDev lv, StencilDev<T> st, T* u, const T* __restrict__ rhs,
@@ -885,18 +908,15 @@ __global__ void __launch_bounds__(kBlock) faceSorKernel(LevelDev lv, StencilDev<
   const int64_t base = lv.faceOff[b.face];
   T* uf = u + base;
   const T* __restrict__ f = rhs + base;
-  const T om = omega, om1 = T(1) - omega;
+  const T om1 = T(1) - omega, dinv = omega / sh.ent[0].w;
   const int yEnd = min(b.start + kFaceRows, w - 2);
   for (int y = b.start + warp; y < yEnd; y += kBlock / 32) {
-    if (lane < ne) sh.off[warp][lane] = faceSlot(w, sh.ent[lane].layer, sh.ent[lane].dx, y + sh.ent[lane].dy);
+    if (lane < 16)
+      sh.off[warp][lane] = lane < ne ? faceSlot(w, sh.ent[lane].layer, sh.ent[lane].dx, y + sh.ent[lane].dy) : rowStart(w, y);
     __syncwarp();
     const int len = w - 2 - y, r0 = rowStart(w, y);
     const int x0 = 1 + (((colour - 2 * y - 1) % 3) + 3) % 3;
-    for (int x = x0 + 3 * lane; x <= len; x += 96) {
-      T s = f[r0 + x];
-      for (int k = 1; k < ne; ++k) s -= sh.ent[k].w * uf[sh.off[warp][k] + x];
-      uf[r0 + x] = om1 * uf[r0 + x] + (s * om) / sh.ent[0].w;
-    }
+    for (int x = x0 + 3 * lane; x <= len; x += 96) uf[r0 + x] = faceSorPoint(sh.ent, ne, sh.off[warp], uf, f, r0, x, om1, dinv);
     __syncwarp();
   }
 }
@@ -924,76 +944,167 @@ __device__ __forceinline__ void gatherRange(T* buf, T* cells, const uint2* __res
   }
 }
 
-// Edges (both colours x mod 2) or vertices: block b is primitive firstPrim + b.
+// SOR updates of the points x0, x0 + step, ... < xEnd of an edge or vertex by the threads of a block:
+// G lanes share a point's off-diagonal entries. A phase over a few dozen points is a chain of
+// dependent reads, so each lane holds its entries' weights and offsets in registers (static, read
+// before anything else), and one round of loads and log2 G shuffles is left per point (edge phase of
+// 27 cubes, levels 3 to 5: 8.8 us with a thread per point, 6.6 with 8 lanes).
+template <class T, int G>
+struct LowSorLanes {
+  static constexpr int kHeld = 4;  // entries a lane holds; longer rows read the rest per point
+  int e0, e1, lane;
+  unsigned group;
+  T dinv, w[kHeld];
+  int rel[kHeld];
+  __device__ __forceinline__ LowSorLanes(const StencilDev<T>& st, int begin, int end, T omega)
+      : e0(begin), e1(end), lane(threadIdx.x % G) {
+    group = G == 32 ? 0xffffffffu : ((1u << (G & 31)) - 1) << ((threadIdx.x & 31) / G * G);
+    dinv = e0 < e1 ? omega / st.lowEntW[e0] : T(0);
+#pragma unroll
+    for (int j = 0; j < kHeld; ++j) {
+      const int k = e0 + 1 + lane + G * j;
+      w[j] = k < e1 ? st.lowEntW[k] : T(0);
+      rel[j] = k < e1 ? st.lowEntRel[k] : 0;
+    }
+  }
+  __device__ __forceinline__ void update(const StencilDev<T>& st, T* u, const T* rhs, int64_t o, int x0, int xEnd, int step,
+                                         T om1) const {
+    for (int x = x0 + step * ((int)threadIdx.x / G); x < xEnd; x += step * (kBlock / G)) {
+      const int64_t c = o + x;
+      T v[kHeld], s = T(0);
+#pragma unroll
+      for (int j = 0; j < kHeld; ++j) v[j] = u[c + rel[j]];
+      const T f = rhs[c], old = u[c];
+#pragma unroll
+      for (int j = 0; j < kHeld; ++j)
+        if (e0 + 1 + lane + G * j < e1) s += w[j] * v[j];
+      for (int k = e0 + 1 + lane + G * kHeld; k < e1; k += G) s += st.lowEntW[k] * u[c + st.lowEntRel[k]];
+#pragma unroll
+      for (int d = G / 2; d; d /= 2) s += __shfl_xor_sync(group, s, d);
+      if (lane == 0) u[c] = om1 * old + (f - s) * dinv;
+    }
+  }
+};
+constexpr int kEdgeLanes = 8, kVertexLanes = 32;
+
+// Edges (both colours x mod 2) or vertices of one block: primitive p refreshes its entries of range
+// (nullptr: none), then updates its DoFs.
+template <class T, int G>
+__device__ __forceinline__ void lowSorPrimitive(const LevelDev& lv, const StencilDev<T>& st, T* u, const T* rhs, unsigned mask,
+                                                T omega, int p, int backwards, const uint2* __restrict__ table,
+                                                const int2* __restrict__ range, T* cells, int64_t cellEnd) {
+  const int first = lv.lowFirst[p], count = lv.lowCount[p];
+  const int64_t o = lv.lowOff[p];
+  const bool on = (lv.lowType[p] & mask) && count > 0;
+  const int2 r = range ? range[p] : make_int2(0, 0);
+  const LowSorLanes<T, G> row(st, st.lowEntOff[p], on ? st.lowEntOff[p + 1] : st.lowEntOff[p], omega);
+  waitForPredecessor(u, rhs);
+  if (range) {
+    gatherRange(u, cells, table, r.x, r.y, cellEnd);
+    __syncthreads();
+  }
+  if (!on) return;
+  const int passes = p < lv.nEdges ? 2 : 1;
+  for (int pass = 0; pass < passes; ++pass) {
+    const int colour = backwards ? 1 - pass : pass;
+    row.update(st, u, rhs, o, passes == 2 ? first + ((first ^ colour) & 1) : first, first + count, passes, T(1) - omega);
+    __syncthreads();
+  }
+}
+
+// Block b is primitive firstPrim + b.
 template <class T>
 __global__ void __launch_bounds__(kBlock) lowSorPhaseKernel(LevelDev lv, StencilDev<T> st, T* u, const T* __restrict__ rhs,
                                                             unsigned mask, T omega, int firstPrim, int backwards,
                                                             const uint2* __restrict__ table, const int2* __restrict__ range,
                                                             T* cells, int64_t cellEnd) {
   const int p = firstPrim + blockIdx.x;
-  const int first = lv.lowFirst[p], count = lv.lowCount[p];
-  const int64_t o = lv.lowOff[p];
-  const int e0 = st.lowEntOff[p], e1 = st.lowEntOff[p + 1];
-  const bool on = lv.lowType[p] & mask;
-  waitForPredecessor(u, rhs);
-  if (range) {
-    gatherRange(u, cells, table, range[p].x, range[p].y, cellEnd);
-    __syncthreads();
-  }
-  if (!on) return;
-  const int passes = p < lv.nEdges ? 2 : 1;
-  const T om1 = T(1) - omega;
-  for (int pass = 0; pass < passes; ++pass) {
-    const int colour = passes == 2 ? (backwards ? 1 - pass : pass) : -1;
-    for (int x = first + threadIdx.x; x < first + count; x += kBlock) {
-      if (colour >= 0 && (x & 1) != colour) continue;
-      const int64_t c = o + x;
-      T s = rhs[c];
-      for (int k = e0 + 1; k < e1; ++k) s -= st.lowEntW[k] * u[c + st.lowEntRel[k]];
-      u[c] = om1 * u[c] + (s * omega) / st.lowEntW[e0];
-    }
-    __syncthreads();
-  }
+  if (p < lv.nEdges)
+    lowSorPrimitive<T, kEdgeLanes>(lv, st, u, rhs, mask, omega, p, backwards, table, range, cells, cellEnd);
+  else
+    lowSorPrimitive<T, kVertexLanes>(lv, st, u, rhs, mask, omega, p, backwards, table, range, cells, cellEnd);
 }
 
-// Faces, the three colours (x + 2y) mod 3; block b is face b, kFacePhaseThreads threads (the
-// warps take the rows).
-constexpr int kFacePhaseThreads = 1024;
+// The start of a forward sweep in one launch instead of a refresh, the vertices and a refresh. The
+// first blocks take a vertex each (its ghosts, then its update); the others refresh the copies that
+// later phases read and no vertex update changes: table entries [g0, g1), the edge copies owned by
+// edges, faces and cells and the face ghost layers (a macro-vertex owns no ghost of a face from level
+// 1 on). 27 cubes, level 5: 5.7 us instead of 5.3 + 5.4 + 3.5.
 template <class T>
+__global__ void __launch_bounds__(kBlock) vertexSorPhaseKernel(LevelDev lv, StencilDev<T> st, T* u,
+                                                               const T* __restrict__ rhs, unsigned mask, T omega, int nVert,
+                                                               const uint2* __restrict__ table,
+                                                               const int2* __restrict__ range, int64_t g0, int64_t g1,
+                                                               T* cells, int64_t cellEnd) {
+  if ((int)blockIdx.x < nVert) {
+    lowSorPrimitive<T, kVertexLanes>(lv, st, u, rhs, mask, omega, lv.nEdges + (int)blockIdx.x, 0, table, range, cells, cellEnd);
+    return;
+  }
+  constexpr int kU = 4;
+  const int64_t first = g0 + (int64_t)(blockIdx.x - nVert) * (kBlock * kU) + threadIdx.x;
+  uint2 t[kU];
+  T v[kU];
+#pragma unroll
+  for (int k = 0; k < kU; ++k)
+    if (first + k * kBlock < g1) t[k] = __ldg(table + first + k * kBlock);
+  waitForPredecessor(u);
+#pragma unroll
+  for (int k = 0; k < kU; ++k)
+    if (first + k * kBlock < g1) v[k] = cells && t[k].y < cellEnd ? cells[t[k].y] : u[t[k].y];
+#pragma unroll
+  for (int k = 0; k < kU; ++k)
+    if (first + k * kBlock < g1) {
+      if (cells && t[k].x < cellEnd) cells[t[k].x] = v[k];
+      else u[t[k].x] = v[k];
+    }
+}
+
+// Faces, the three colours (x + 2y) mod 3; block b is face b. A warp takes ROWS rows at a time, 32 / ROWS
+// lanes each. A row has at most N / 3 points of a colour, which leaves two thirds of 32 lanes idle at
+// N = 32: there four rows. On larger faces FP32 still gains from them (V(3,3) on level 7, 48 cells:
+// 3.76 ms with four rows, 3.88 with one), FP64 loses (sweep on level 7 884 us with one, 898 with four).
+// The phase is bound by latency: a block has no more threads than the face has rows for, so that small
+// faces share an SM (27 cubes, level 5, 378 faces: 18 us with 1024 threads, 10 with 256).
+constexpr int kFacePhaseThreads = 1024;
+inline int facePhaseThreads(int N) { return N <= 32 ? 256 : N <= 64 ? 512 : kFacePhaseThreads; }
+template <class T>
+int facePhaseRows(int N) { return sizeof(T) == 4 || N <= 32 ? 4 : 1; }
+template <class T, int ROWS>
 __global__ void __launch_bounds__(kFacePhaseThreads) faceSorPhaseKernel(LevelDev lv, StencilDev<T> st, T* u,
                                                                         const T* __restrict__ rhs, unsigned mask, T omega,
                                                                         int backwards, const uint2* __restrict__ table,
                                                                         const int2* __restrict__ range, T* cells,
                                                                         int64_t cellEnd) {
-  constexpr int kWarps = kFacePhaseThreads / 32;
+  constexpr int kRows = ROWS, kLanes = 32 / kRows;
+  const int warps = (int)blockDim.x / 32;
   const int face = blockIdx.x;
   __shared__ FaceEnt<T> ent[16];
-  __shared__ int off[kWarps][16];
+  __shared__ int off[kFacePhaseThreads / 32][kRows][16];
   const int ne = st.faceEntCount[face];
   const bool on = lv.faceType[face] & mask;
-  if (threadIdx.x < ne) ent[threadIdx.x] = st.faceEnt[16 * face + threadIdx.x];
+  if (threadIdx.x < 16) ent[threadIdx.x] = (int)threadIdx.x < ne ? st.faceEnt[16 * face + threadIdx.x] : FaceEnt<T>{T(0), 0, 0, 0};
+  const int2 r = range ? range[face] : make_int2(0, 0);
   waitForPredecessor(u, rhs);
-  if (range) gatherRange(u, cells, table, range[face].x, range[face].y, cellEnd);
+  if (range) gatherRange(u, cells, table, r.x, r.y, cellEnd);
   __syncthreads();
   if (!on) return;
-  const int w = lv.w, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int w = lv.w, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, row = lane / kLanes, sub = lane % kLanes;
   const int64_t base = lv.faceOff[face];
   T* uf = u + base;
-  const T* __restrict__ f = rhs + base;
-  const T om = omega, om1 = T(1) - omega;
+  const T* f = rhs + base;
+  const T om1 = T(1) - omega, dinv = omega / ent[0].w;
   for (int pass = 0; pass < 3; ++pass) {
     const int colour = backwards ? 2 - pass : pass;
-    for (int y = 1 + warp; y < w - 2; y += kWarps) {
-      if (lane < ne) off[warp][lane] = faceSlot(w, ent[lane].layer, ent[lane].dx, y + ent[lane].dy);
+    for (int y0 = 1 + warp * kRows; y0 < w - 2; y0 += warps * kRows) {
       __syncwarp();
-      const int len = w - 2 - y, r0 = rowStart(w, y);
-      const int x0 = 1 + (((colour - 2 * y - 1) % 3) + 3) % 3;
-      for (int x = x0 + 3 * lane; x <= len; x += 96) {
-        T s = f[r0 + x];
-        for (int k = 1; k < ne; ++k) s -= ent[k].w * uf[off[warp][k] + x];
-        uf[r0 + x] = om1 * uf[r0 + x] + (s * om) / ent[0].w;
+      for (int i = lane; i < kRows * 16; i += 32) {
+        const int k = i & 15, y = y0 + (i >> 4);
+        off[warp][i >> 4][k] = k < ne ? faceSlot(w, ent[k].layer, ent[k].dx, y + ent[k].dy) : rowStart(w, y);
       }
       __syncwarp();
+      const int y = y0 + row, len = w - 2 - y, r0 = rowStart(w, y);
+      const int x0 = 1 + (((colour - 2 * y - 1) % 3) + 3) % 3;
+      for (int x = x0 + 3 * sub; x <= len; x += 3 * kLanes) uf[r0 + x] = faceSorPoint(ent, ne, off[warp][row], uf, f, r0, x, om1, dinv);
     }
     __syncthreads();
   }
@@ -1464,14 +1575,13 @@ __global__ void __launch_bounds__(kBlock) lowSorKernel(LevelDev lv, StencilDev<T
                                                        unsigned mask, int colour, T omega, int blockBegin) {
   const LowBlock b = lv.lowBlocks[blockBegin + blockIdx.x];
   if (!(lv.lowType[b.prim] & mask)) return;
-  const int x = b.start + threadIdx.x;
-  if (x >= lv.lowFirst[b.prim] + lv.lowCount[b.prim]) return;
-  if (colour >= 0 && (x & 1) != colour) return;
-  const int64_t c = lv.lowOff[b.prim] + x;
-  const int e0 = st.lowEntOff[b.prim];
-  T s = rhs[c];
-  for (int k = e0 + 1; k < st.lowEntOff[b.prim + 1]; ++k) s -= st.lowEntW[k] * u[c + st.lowEntRel[k]];
-  u[c] = (T(1) - omega) * u[c] + (s * omega) / st.lowEntW[e0];
+  const int end = min(b.start + kBlock, lv.lowFirst[b.prim] + lv.lowCount[b.prim]);
+  const int64_t o = lv.lowOff[b.prim];
+  const int e0 = st.lowEntOff[b.prim], e1 = st.lowEntOff[b.prim + 1];
+  if (colour < 0)
+    LowSorLanes<T, kVertexLanes>(st, e0, e1, omega).update(st, u, rhs, o, b.start, end, 1, T(1) - omega);
+  else
+    LowSorLanes<T, kEdgeLanes>(st, e0, e1, omega).update(st, u, rhs, o, b.start + ((b.start ^ colour) & 1), end, 2, T(1) - omega);
 }
 
 // The transfers of a level, one launch each: edge and vertex blocks, face bands, then one block per

@@ -8,6 +8,7 @@
 #include <cstring>
 #include <map>
 #include <memory>
+#include <numeric>
 #include <stdexcept>
 #include <string>
 #include <type_traits>
@@ -136,6 +137,19 @@ Storage::~Storage() {
   if (ownStream) cudaStreamDestroy(ownStream);
 }
 
+static int64_t firstVertexSlot(const LevelLayout& lay) { return lay.off[KV].empty() ? lay.total : lay.off[KV][0]; }
+
+// Order of a halo group's entries in the level's table: the edge copies owned by vertices come
+// before the other edge copies, everything else as generated.
+static std::vector<size_t> commOrder(const LevelLayout& lay, int g) {
+  std::vector<size_t> order(lay.commDst[g].size());
+  std::iota(order.begin(), order.end(), size_t(0));
+  if (g == G_EDGE)
+    std::stable_partition(order.begin(), order.end(),
+                          [&](size_t i) { return lay.commSrc[g][i] >= firstVertexSlot(lay); });
+  return order;
+}
+
 void Storage::buildLevel(int L) {
   const Topology& topo = disc.topo();
   const LevelLayout& lay = disc.level(L);
@@ -203,10 +217,14 @@ void Storage::buildLevel(int L) {
   std::vector<uint2> comm;
   for (int g : kCommOrder) {
     ld.commBegin[g] = (int64_t)comm.size();
-    for (size_t i = 0; i < lay.commDst[g].size(); ++i)
+    for (size_t i : commOrder(lay, g))
       comm.push_back(make_uint2((unsigned)lay.commDst[g][i], (unsigned)lay.commSrc[g][i]));
     ld.commCount[g] = (int64_t)comm.size() - ld.commBegin[g];
   }
+  ld.commEdgeOther = ld.commBegin[G_EDGE];
+  while (ld.commEdgeOther < ld.commBegin[G_EDGE] + ld.commCount[G_EDGE] &&
+         (int64_t)comm[(size_t)ld.commEdgeOther].y >= firstVertexSlot(lay))
+    ++ld.commEdgeOther;
   argCheck(comm.size() < (size_t(1) << 31), "halo table exceeds 32-bit ranges");
   // Each primitive's entries of a group are contiguous (the tables are generated primitive by
   // primitive): the range of every primitive's destination array, found from its offsets.
@@ -214,7 +232,9 @@ void Storage::buildLevel(int L) {
     std::vector<int2> r((size_t)nPrim, make_int2(0, 0));
     std::vector<char> seen((size_t)nPrim, 0);
     int last = -1;
-    for (int64_t i = ld.commBegin[g]; i < ld.commBegin[g] + ld.commCount[g]; ++i) {
+    // of the edge copies only those owned by vertices (the phases refresh the others before)
+    const int64_t end = g == G_EDGE ? ld.commEdgeOther : ld.commBegin[g] + ld.commCount[g];
+    for (int64_t i = ld.commBegin[g]; i < end; ++i) {
       const int64_t d = comm[(size_t)i].x;
       const auto& offs = lay.off[kind];
       const int p = int(std::upper_bound(offs.begin(), offs.end(), d) - offs.begin()) - 1;
@@ -536,8 +556,7 @@ void Storage::buildSplit(int L) {
   };
   std::vector<uint2> comm;  // the same entries in the same order as the level's table
   for (int g : kCommOrder)
-    for (size_t i = 0; i < lay.commDst[g].size(); ++i)
-      comm.push_back(make_uint2(map(lay.commDst[g][i]), map(lay.commSrc[g][i])));
+    for (size_t i : commOrder(lay, g)) comm.push_back(make_uint2(map(lay.commDst[g][i]), map(lay.commSrc[g][i])));
   const uint2* commSplit = comm.empty() ? ld.comm : (const uint2*)upload(ld.keep, comm, stream);
   // rows and points per colour
   for (int col = 0; col < 4; ++col) {
@@ -2148,14 +2167,30 @@ void Storage::sorT(Operator& o, int dstId, int L, T* u, const T* rhs, unsigned m
     };
     auto facePhase = [&](bool gather, bool rev) {
       if (lv.nFaceBlocks == 0 || !(kinds & (1 << KF))) return;
-      launchNext(stream, dev::faceSorPhaseKernel<T>, lv.nFaces, dev::kFacePhaseThreads, 0, lv, st, u, rhs, mask, omega, rev ? 1 : 0, table, gather && refresh ? ld.faceRange : nullptr, cellsBuf, cellEnd);
+      launchNext(stream, dev::facePhaseRows<T>(lv.N) == 4 ? dev::faceSorPhaseKernel<T, 4> : dev::faceSorPhaseKernel<T, 1>, lv.nFaces, dev::facePhaseThreads(lv.N), 0, lv, st, u, rhs, mask, omega, rev ? 1 : 0, table, gather && refresh ? ld.faceRange : nullptr, cellsBuf, cellEnd);
+      ++launches;
+    };
+    // vertices, beside the refresh of the edge copies they do not own and of the face ghost layers
+    auto vertexPhase = [&]() {
+      const int nVert = lv.nLow - lv.nEdges;
+      static_assert(kCommOrder[0] == G_EDGE && kCommOrder[1] == G_FACE_GHOST, "one run of the table");
+      const int64_t g0 = ld.commEdgeOther, g1 = ld.commBegin[G_FACE_GHOST] + ld.commCount[G_FACE_GHOST];
+      const int64_t blocks = (g1 - g0 + 4 * dev::kBlock - 1) / (4 * dev::kBlock);
+      if (nVert + blocks == 0) return;
+      launchNext(stream, dev::vertexSorPhaseKernel<T>, (unsigned)(nVert + blocks), dev::kBlock, 0, lv, st, u, rhs, mask,
+                 omega, nVert, table, ld.lowRange, g0, g1, cellsBuf, cellEnd);
       ++launches;
     };
     if (!backwards) {
-      comm((1 << G_VERT) | (1 << G_FACE_GHOST));
-      lowPhase(false, false, false);  // vertices
-      comm(1 << G_EDGE);              // Vertex -> Edge
-      lowPhase(true, false, false);   // edges
+      if (refresh && kinds == 15 && lv.N >= 2) {
+        vertexPhase();
+        lowPhase(true, true, false);  // Vertex -> Edge, edges
+      } else {
+        comm((1 << G_VERT) | (1 << G_FACE_GHOST));
+        lowPhase(false, false, false);  // vertices
+        comm(1 << G_EDGE);              // Vertex -> Edge
+        lowPhase(true, false, false);   // edges
+      }
       facePhase(true, false);         // Edge -> Face, faces
       if (!resident) comm(1 << G_CELL);  // Face -> Cell
       cellPhase(false);

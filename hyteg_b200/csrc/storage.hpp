@@ -28,9 +28,9 @@ struct DevBuf {
 };
 
 // Order of the halo groups in a level's table: every group set one SOR phase refreshes at once
-// (vertex ghosts with face ghost layers, cell closures with face boundary rows, all five) is one
-// contiguous run, so a refresh is one launch.
-constexpr int kCommOrder[G_COUNT] = {G_EDGE, G_VERT, G_FACE_GHOST, G_CELL, G_FACE_BOUNDARY};
+// (edge copies with face ghost layers, vertex ghosts with face ghost layers, cell closures with face
+// boundary rows, all five) is one contiguous run, so a refresh is one launch.
+constexpr int kCommOrder[G_COUNT] = {G_EDGE, G_FACE_GHOST, G_VERT, G_CELL, G_FACE_BOUNDARY};
 
 void cudaCheck(cudaError_t e, const char* what);
 
@@ -59,6 +59,7 @@ struct LevelData {
   dev::LevelDev lv{};
   uint2* comm = nullptr;
   int64_t commBegin[G_COUNT] = {0, 0, 0, 0, 0}, commCount[G_COUNT] = {0, 0, 0, 0, 0};
+  int64_t commEdgeOther = 0;  // the edge copies owned by vertices end here, the others follow
   dev::Chunk* chunks = nullptr;
   int nChunks = 0;
   int nCellChunks = 0;  // the chunks of the cell arrays come first
@@ -75,8 +76,8 @@ struct LevelData {
   dev::WaveTile* waveTiles[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};
   int nWaveTiles[2][2] = {{0, 0}, {0, 0}};
   int64_t nonCellBegin = 0;  // first slot after the cell arrays (faces, edges, vertices follow)
-  // per primitive, its entries (begin, end) in comm of the group the SOR refreshes before its
-  // phase: low primitives (edges: G_EDGE, vertices: G_VERT), faces (G_FACE_BOUNDARY)
+  // per primitive, its entries (begin, end) in comm that its SOR phase refreshes: edges (their copies
+  // owned by vertices), vertices (G_VERT), faces (G_FACE_BOUNDARY)
   const int2* lowRange = nullptr;
   const int2* faceRange = nullptr;
   // SOR schedule 3 (built on first use): the halo table with every cell slot at its colour-split

@@ -199,3 +199,30 @@ def test_fused_phases_equal_per_colour_launches(cube6, L, backwards, dtype, sche
     finally:
         st.set_sor_fused_phases(True)
     assert np.array_equal(out[0], out[1])
+
+
+@pytest.mark.parametrize("L", [1, 2, 4, 5])
+@pytest.mark.parametrize("backwards", [False, True])
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+def test_small_fused_phases_equal_per_colour_launches(cube6, L, backwards, dtype):
+    """Edges from one point over fewer points than the block's lane groups up to four passes of it,
+    faces of fewer rows than a warp takes at once up to one row group per warp. Level 1 has no cell
+    and face points, and only the fused face phase refreshes the copies on its faces: there the
+    unknowns themselves are compared."""
+    st, mesh = cube6
+    if L > 1:
+        test_fused_phases_equal_per_colour_launches(cube6, L, backwards, dtype, 0)
+        return
+    n = st.level_size(L)
+    rng = np.random.default_rng(70 + backwards)
+    x0 = rng.uniform(-1, 1, n).astype(dtype)
+    b0 = rng.uniform(-1, 1, n).astype(dtype)
+    out = []
+    try:
+        for fused in (True, False):
+            st.set_sor_fused_phases(fused)
+            out.append(run_sor(st, L, x0, b0, dtype, 0, 2, backwards))
+    finally:
+        st.set_sor_fused_phases(True)
+    owned = mesh.slot_info(L)[1] == 1
+    assert np.array_equal(out[0][owned], out[1][owned])
