@@ -34,12 +34,15 @@ __device__ __forceinline__ const T* compactStencil(const StencilDev<T>& st, int 
   return st.lowEntW + st.lowEntOff[prim + (kind == 2 ? sh.z : sh.w)];
 }
 
-// A row and its first 16 entries, read independently of the row's values: the entries of 32
-// consecutive rows are coalesced (read row by row, 56 bytes apart, they cost 14 L1 wavefronts per
-// load), and a thread holds its next row while it waits for the current one. With x in shared
-// memory the V(3,3) cycle of one sub-cube (levels 0-4, FP64, one block) takes 305 us instead of 369.
+// A row and its first 16 entries, read independently of the row's values. Where one block owns the
+// group and they fit, a level's rows are copied to shared memory (packed, 40 bytes each) before its
+// sweeps: a phase of a few hundred rows is a chain of dependent reads, and each from L2 costs some
+// hundred cycles, ten times per sweep. V(3,3) cycle of one sub-cube (levels 0-4, FP64, one block):
+// 287 us, 299 from the lists in L2. Elsewhere rows are read from the transposed lists (ell), whose
+// entries are coalesced over 32 consecutive rows (read row by row, 56 bytes apart, they cost 14 L1
+// wavefronts per load: 369 us).
 struct CompactItem {
-  CompactRow row;
+  CompactRow row;  // e0, e1: 0, the number of entries, for a packed row
   int4 c[4];
 };
 __device__ __forceinline__ void compactFetch(CompactItem& it, const CompactRow* __restrict__ rows,
@@ -49,16 +52,30 @@ __device__ __forceinline__ void compactFetch(CompactItem& it, const CompactRow* 
 #pragma unroll
   for (int k = 0; k < 4; ++k) it.c[k] = __ldg(ell + (int64_t)k * pitch + r);
 }
+__device__ __forceinline__ int2 compactPair(int v) {  // two packed entries
+  return make_int2((v & 0x7fff) | ((v & 0x8000) << 16), ((v >> 16) & 0x7fff) | (v & int(0x80000000u)));
+}
+__device__ __forceinline__ void compactUnpack(CompactItem& it, const int4* rows, int pitch, int r) {
+  const int2 m = reinterpret_cast<const int2*>(rows + 2 * pitch)[r];
+  it.row = {m.x & 0xffff, m.y, 0, m.x >> 16};
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    const int4 v = rows[q * pitch + r];
+    const int2 a = compactPair(v.x), b = compactPair(v.y), c = compactPair(v.z), d = compactPair(v.w);
+    it.c[2 * q] = make_int4(a.x, a.y, b.x, b.y);
+    it.c[2 * q + 1] = make_int4(c.x, c.y, d.x, d.y);
+  }
+}
 __device__ __forceinline__ int compactEntry(const CompactItem& it, int j) {
   const int4 q = it.c[j >> 2];
   return (j & 3) == 0 ? q.x : (j & 3) == 1 ? q.y : (j & 3) == 2 ? q.z : q.w;
 }
 
 // sum_k w_k v_k over a row's off-diagonal entries (values from snap where bit 31 of the entry is
-// set, SNAP, else from x), in four partial sums; entries beyond 16 from cols.
+// set, SNAP, else from x), in four partial sums; entries beyond 16 from the row's list in cols.
 template <class T, bool SNAP>
-__device__ __forceinline__ T compactRowSum(const CompactItem& it, const T* w, int stride, const int* __restrict__ cols,
-                                           const T* x, const T* snap) {
+__device__ __forceinline__ T compactRowSum(const CompactItem& it, const T* w, int stride, const CompactRow* __restrict__ rows,
+                                           int r, const int* __restrict__ cols, const T* x, const T* snap) {
   const int n = it.row.e1 - it.row.e0;
   T v[16], s[4] = {T(0), T(0), T(0), T(0)};
 #pragma unroll
@@ -69,9 +86,12 @@ __device__ __forceinline__ T compactRowSum(const CompactItem& it, const T* w, in
 #pragma unroll
   for (int j = 0; j < 16; ++j)
     if (j < n) s[j & 3] += w[(1 + j) * stride] * v[j];
-  for (int j = 16; j < n; ++j) {
-    const int c = __ldg(cols + it.row.e0 + j);
-    s[j & 3] += w[(1 + j) * stride] * ((SNAP && c < 0) ? snap[c & 0x7fffffff] : x[c & 0x7fffffff]);
+  if (n > 16) {
+    const int e0 = rows[r].e0;
+    for (int j = 16; j < n; ++j) {
+      const int c = __ldg(cols + e0 + j);
+      s[0] += w[(1 + j) * stride] * ((SNAP && c < 0) ? snap[c & 0x7fffffff] : x[c & 0x7fffffff]);
+    }
   }
   return (s[0] + s[1]) + (s[2] + s[3]);
 }
@@ -122,45 +142,72 @@ __global__ void __launch_bounds__(kCompactThreads, 1) compactCycleKernel(const _
   }
   sync();
 
-  CompactItem next;  // the thread's next row
-  auto fetch = [&](const CompactLevel<T>& L, int r, int r1) {
-    if (r < r1) compactFetch(next, L.rows, L.ell, L.pitch, r);
+  int4* sRows = reinterpret_cast<int4*>(compactSmem + max(cd.smemRows, 0));
+  const bool packed = inSmem && cd.smemRows >= 0;
+  auto keepRows = [&](const CompactLevel<T>& L) {  // the level's rows into shared memory
+    if (!packed) return;
+    for (int i = t0; i < L.pitch * 5 / 2; i += nt) sRows[i] = __ldg(L.pk + i);
+    sync();
   };
-  // x_i <- (1 - omega) x_i + omega (b_i - sum_j a_ij x_j) / a_ii on rows [r0, r1), the
-  // lowSorPhaseKernel update; the first row is already in next.
-  auto sorRows = [&](const CompactLevel<T>& L, int r0, int r1, T* x, const T* b, const T* saved) {
-    for (int r = r0 + t0; r < r1; r += nt) {
-      const CompactItem it = next;
-      fetch(L, r + nt, r1);
+  auto getRow = [&](const CompactLevel<T>& L, int r) {
+    CompactItem it;
+    if (packed) compactUnpack(it, sRows, L.pitch, r);
+    else compactFetch(it, L.rows, L.ell, L.pitch, r);
+    return it;
+  };
+  auto dOf = [&](const CompactLevel<T>& L) { return inSmem ? sm + L.sd : sc + L.d; };
+  // omega / a_ii of every primitive: a division per row and phase otherwise
+  for (int k = 1; k <= K; ++k) {
+    const CompactLevel<T>& L = cd.lv[k];
+    T* dv = dOf(L);
+    const int n = L.nPrim[0] + L.nPrim[1] + L.nPrim[2];
+    for (int i = t0; i < n; i += nt) {
+      const int low = i - L.nPrim[0] - L.nPrim[1];
+      const int wsel = i < L.nPrim[0] ? i << 2
+                       : low < 0      ? ((i - L.nPrim[0]) << 2) | 1
+                       : low < cd.nEdges ? (low << 2) | 2
+                                         : ((low + cd.vertexShift) << 2) | 3;
       int stride;
-      const T bi = b[it.row.idx];
-      const T* w = compactStencil(L.st, it.row.wsel, sh, stride);
-      const T s = bi - compactRowSum<T, true>(it, w, stride, L.cols, x, saved);
-      x[it.row.idx] = om1 * x[it.row.idx] + (s * omega) / w[0];
+      const T* w = compactStencil(L.st, wsel, sh, stride);
+      // a primitive without DoFs on the level has no entries
+      const int q = (wsel >> 2) + ((wsel & 3) == 2 ? sh.z : sh.w);
+      dv[i] = low >= 0 && L.st.lowEntOff[q] == L.st.lowEntOff[q + 1] ? T(0) : omega / *w;
     }
-  };
+  }
+  sync();
+  // x_i <- (1 - omega) x_i + omega (b_i - sum_j a_ij x_j) / a_ii, the lowSorPhaseKernel update.
   // Sweeps. The vertex rows update while the edge and face values are saved: they write only
   // vertex values, and they read edge and face values from x, which this sweep has not changed
-  // yet; only edge and face rows read the saved values. Then one barrier per colour group; a
-  // group's first rows are read before the barrier ahead of it.
+  // yet; only edge and face rows read the saved values. Then one barrier per colour group.
   auto sweeps = [&](const CompactLevel<T>& L, int count) {
     T* x = xOf(L);
     T* saved = snap - (inSmem ? L.snapBegin : 0);
     const T* b = sc + L.b;
-    fetch(L, t0, L.nVertexRows);
+    const T* dv = dOf(L);
+    auto rows = [&](int r0, int r1) {
+      for (int r = r0 + t0; r < r1; r += nt) {
+        const CompactItem it = getRow(L, r);
+        const int kind = it.row.wsel & 3, prim = it.row.wsel >> 2;
+        const T bi = b[it.row.idx];
+        const T dinv = dv[kind == 0   ? prim
+                          : kind == 1 ? L.nPrim[0] + prim
+                                      : L.nPrim[0] + L.nPrim[1] + prim - (kind == 3 ? cd.vertexShift : 0)];
+        int stride;
+        const T* w = compactStencil(L.st, it.row.wsel, sh, stride);
+        const T s = bi - compactRowSum<T, true>(it, w, stride, L.rows, r, L.cols, x, saved);
+        x[it.row.idx] = om1 * x[it.row.idx] + s * dinv;
+      }
+    };
     for (int it = 0; it < count; ++it) {
       for (int i = L.snapBegin + t0; i < L.snapEnd; i += nt) saved[i] = x[i];
-      sorRows(L, 0, L.nVertexRows, x, b, saved);
-      int r0 = L.nVertexRows;
-      for (int gi = 0; gi < L.nGroups; ++gi) {
-        const int r1 = L.groupEnd[gi];
-        fetch(L, r0 + t0, r1);
-        sync();
-        sorRows(L, r0, r1, x, b, saved);
-        r0 = r1;
-      }
-      fetch(L, t0, L.nVertexRows);
+      rows(0, L.nVertexRows);
       sync();
+      int r0 = L.nVertexRows;
+      for (int g = 0; g < L.nGroups; ++g) {
+        rows(r0, L.groupEnd[g]);
+        r0 = L.groupEnd[g];
+        sync();
+      }
     }
   };
 
@@ -168,23 +215,23 @@ __global__ void __launch_bounds__(kCompactThreads, 1) compactCycleKernel(const _
   for (int k = K; k > 0; --k) {
     const CompactLevel<T>& F = cd.lv[k];
     const CompactLevel<T>& C = cd.lv[k - 1];
+    keepRows(F);
     sweeps(F, pre);
     T* xf = xOf(F);
     const T* bf = sc + F.b;
     T* rf = sc + F.r;
-    fetch(F, t0, F.nRows);
     for (int r = t0; r < F.nRows; r += nt) {  // every value current
-      const CompactItem it = next;
-      fetch(F, r + nt, F.nRows);
+      const CompactItem it = getRow(F, r);
       int stride;
       const T* w = compactStencil(F.st, it.row.wsel, sh, stride);
       const int i = it.row.idx;
-      rf[i] = bf[i] - (w[0] * xf[i] + compactRowSum<T, false>(it, w, stride, F.cols, xf, xf));
+      rf[i] = bf[i] - (w[0] * xf[i] + compactRowSum<T, false>(it, w, stride, F.rows, r, F.cols, xf, xf));
     }
     sync();
     T* xc = xOf(C);
     T* bc = sc + C.b;
     for (int r = t0; r < C.nRows; r += nt) {
+      CompactItem next;
       compactFetch(next, C.rows, C.rEll, C.pitch, r);
       const int e0 = C.rPtr[r], n = C.rPtr[r + 1] - e0;
       T v[16], s = T(0);
@@ -297,6 +344,7 @@ __global__ void __launch_bounds__(kCompactThreads, 1) compactCycleKernel(const _
       xf[F.rows[r].idx] += v;
     }
     sync();
+    keepRows(F);
     sweeps(F, post);
   }
 
@@ -312,7 +360,7 @@ __global__ void __launch_bounds__(kCompactThreads, 1) compactCycleKernel(const _
 
 namespace {
 
-constexpr size_t kCompactSmem = 200 << 10;  // shared memory the vectors may take
+constexpr size_t kCompactSmem = 224 << 10;  // shared memory the vectors and rows may take
 
 int batchKind(int kind) { return kind == KC ? 0 : kind == KF ? 1 : kind == KE ? 2 : 3; }
 
@@ -563,11 +611,12 @@ const V* put(CompactCycle& cc, const std::vector<V>& h, cudaStream_t st) {
 template <class T>
 void fillDev(CompactCycle& cc, dev::CompactCycleDev<T>& d, Storage& s, const Operator& o,
              const std::vector<LevelBuild>& lbs, const std::vector<int64_t>& gather, const std::vector<int64_t>& scSlot,
-             const std::vector<int>& scIdx, const std::vector<int>& scOff) {
+             const std::vector<int>& scIdx, const std::vector<int>& scOff, const int (&nPrim)[3]) {
   d = dev::CompactCycleDev<T>{};
   d.nLevels = (int)lbs.size();
   int64_t off = 0, maxN = 0, smem = 0;  // shared memory in elements
   int maxSnap = 0;
+  size_t maxPk = 0;
   auto vec = [&](int64_t n) {
     const int64_t at = off;
     off += (n + 31) / 32 * 32;
@@ -600,9 +649,30 @@ void fillDev(CompactCycle& cc, dev::CompactCycleDev<T>& d, Storage& s, const Ope
       }
     L.ell = put(cc, ell, s.stream);
     L.rEll = put(cc, rEll, s.stream);
+    if (L.n <= 32768) {
+      std::vector<int4> pk((size_t)L.pitch * 5 / 2, make_int4(0, 0, 0, 0));
+      for (size_t r = 0; r < lb.rows.size(); ++r) {
+        const dev::CompactRow& row = lb.rows[r];
+        auto* c16 = reinterpret_cast<uint16_t*>(pk.data());
+        for (int j = 0; j < 16 && row.e0 + j < row.e1; ++j) {
+          const int c = lb.cols[(size_t)(row.e0 + j)];
+          c16[((size_t)(j >> 3) * L.pitch + r) * 8 + (j & 7)] = (uint16_t)((c & 0x7fff) | (c < 0 ? 0x8000 : 0));
+        }
+        auto* meta = reinterpret_cast<int2*>(pk.data() + 2 * (size_t)L.pitch);
+        meta[r] = make_int2(row.idx | ((row.e1 - row.e0) << 16), row.wsel);
+      }
+      L.pk = put(cc, pk, s.stream);
+      maxPk = std::max(maxPk, pk.size() * sizeof(int4));
+    } else {
+      maxPk = SIZE_MAX / 2;  // the rows of this level do not pack
+    }
     L.sx = (int)smem;
     smem += (L.n + 1) / 2 * 2;
     maxSnap = std::max(maxSnap, L.snapEnd - L.snapBegin);
+    for (int q = 0; q < 3; ++q) L.nPrim[q] = nPrim[q];
+    L.sd = (int)smem;
+    smem += (nPrim[0] + nPrim[1] + nPrim[2] + 1) / 2 * 2;
+    L.d = vec(nPrim[0] + nPrim[1] + nPrim[2]);
     const int oi = lb.L - o.minL;
     if constexpr (sizeof(T) == 8)
       L.st = o.d[(size_t)oi];
@@ -616,6 +686,12 @@ void fillDev(CompactCycle& cc, dev::CompactCycleDev<T>& d, Storage& s, const Ope
   d.snap = vec(maxN);
   cc.smem = (size_t)(smem + maxSnap) * sizeof(T);
   d.smemSnap = (int)smem;
+  d.smemRows = -1;
+  const size_t rowsAt = (cc.smem + 15) / 16 * 16;
+  if (cc.cluster == 1 && rowsAt + maxPk <= kCompactSmem) {
+    d.smemRows = (int)rowsAt;
+    cc.smem = rowsAt + maxPk;
+  }
   if (cc.cluster > 1 || cc.smem > kCompactSmem) {
     d.smemSnap = -1;
     cc.smem = 0;
@@ -784,13 +860,16 @@ std::unique_ptr<CompactCycle> buildCompactCycle(Storage& s, int op, int minL, in
   for (int64_t sl : gather) argCheck(sl >= 0 && sl < lay.total, "compact cycle: gather");
   for (int64_t sl : scSlot) argCheck(sl >= 0 && sl < lay.total, "compact cycle: scatter");
   for (int j : scIdx) argCheck(j >= 0 && j < (int)tb.dofs.size(), "compact cycle: scatter");
-  if (prec == 8) {
-    fillDev<double>(*cc, cc->d64, s, o, lbs, gather, scSlot, scIdx, scOff);
-    for (int q = 0; q < 4; ++q) cc->d64.primsPerGroup[q] = perGroup[q];
-  } else {
-    fillDev<float>(*cc, cc->d32, s, o, lbs, gather, scSlot, scIdx, scOff);
-    for (int q = 0; q < 4; ++q) cc->d32.primsPerGroup[q] = perGroup[q];
-  }
+  const int perKind[3] = {(int)topo.cells.size() / groups, (int)topo.faces.size() / groups,
+                        ((int)topo.edges.size() + (int)topo.verts.size()) / groups};
+  auto fill = [&](auto& d) {
+    fillDev(*cc, d, s, o, lbs, gather, scSlot, scIdx, scOff, perKind);
+    for (int q = 0; q < 4; ++q) d.primsPerGroup[q] = perGroup[q];
+    d.nEdges = nEdges / groups;
+    d.vertexShift = nEdges - nEdges / groups;
+  };
+  if (prec == 8) fill(cc->d64);
+  else fill(cc->d32);
   cudaCheck(cudaStreamSynchronize(s.stream), "compact lists");
   return cc;
 }

@@ -50,12 +50,18 @@ struct CompactLevel {
   const int4* ell;   // the first 16 entries of row r: ell[q * pitch + r], q = 0 .. 3 (the same values)
   const int4* rEll;  // the first 16 of the restriction into row r, same layout; rPtr holds the counts
   int pitch;
+  // rows in 40 bytes for shared memory (levels of at most 32768 unknowns): the first 16 entries as
+  // 16-bit values (bit 15: as of the sweep's start), pk[q * pitch + r], q = 0, 1, then per row
+  // (unknown | entries << 16, wsel)
+  const int4* pk;
   const int2* pro;   // [nRows] coarse unknowns of the prolongation into this row (y < 0: coincident)
   const int* rPtr;   // [nRows + 1] restriction into this level's rows from the level above
   const int* rIdx;   // fine unknown index; bit 31: weight 1/2 (else 1)
   StencilDev<T> st;
   int64_t x, b, r;   // offsets of the level's vectors in a group's scratch
-  int sx;            // offset of x in shared memory (CompactCycleDev::smemSnap >= 0)
+  int sx, sd;        // offsets of x and of omega / a_ii in shared memory (CompactCycleDev::smemSnap >= 0)
+  int64_t d;         // offset of omega / a_ii (cells, faces, edges and vertices of a group) in its scratch
+  int nPrim[3];      // cells, faces, edges and vertices of a group
 };
 
 template <class T>
@@ -65,6 +71,7 @@ struct CompactCycleDev {
   int64_t groupStride;  // scratch elements per group
   int64_t snap;         // offset of the snapshot vector in a group's scratch
   int smemSnap;         // x of every level in shared memory, then from here the snapshot (-1: in scratch)
+  int smemRows;         // byte offset of the current level's packed rows in shared memory (-1: not kept there)
   int64_t cgStride;     // FP64 coarse-CG scratch per group (five vectors)
   const int64_t* gather;       // [groups][n(top)] owner slot of each top-level unknown
   const int64_t* scatterSlot;  // per group, every slot of the top level holding a DoF ...
@@ -72,6 +79,7 @@ struct CompactCycleDev {
   const int* scatterOff;       // [groups + 1]
   StencilDev<double> cgSt;     // FP64 stencils of the coarsest level
   int primsPerGroup[4];        // cells, faces, edges, vertices per group (0 for one group)
+  int nEdges, vertexShift;     // edges of a group; (wsel's number of its vertex v) - (nEdges + v)
 };
 
 }  // namespace dev
