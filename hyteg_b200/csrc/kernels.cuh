@@ -1,14 +1,11 @@
 // Device kernels of the B200 matrix-free P1 multigrid path (sm_100a).
 //
-// All kernels are bandwidth-bound stencil sweeps over the reference's per-primitive array
-// layout (see discretization.hpp). Work is distributed by host-built block tables:
-//   cell blocks  : (cell, z, first plane offset)   one 256-thread block per slice of a z-plane
-//   face blocks  : (face, first triangle offset)
-//   low  blocks  : (edge-or-vertex, first x)
-// Threads decode their (x, y) inside a triangular plane with one rounded square root, so a
-// block reads contiguous x-rows (coalesced) and the neighbouring rows of the planes z-1 and
-// z+1 are served from L1/L2. Primitive boundary types are tested in-kernel against the
-// DoFType mask, so one launch covers every primitive of a kind.
+// Stencil sweeps over the reference's per-primitive array layout (see discretization.hpp). On large
+// levels they are bound by the latency of their loads and by issue, on small ones by the latency of
+// the launches. Work is distributed by host-built tables (strips and tiles of macro-cells, chunks of
+// rows, blocks of edges and vertices), and the primitives of all kinds share a launch where none
+// reads what another writes. Primitive boundary types are tested in-kernel against the DoFType
+// mask, so one launch covers every primitive of a kind.
 #pragma once
 
 #include <cstdint>
