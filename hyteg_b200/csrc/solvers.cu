@@ -47,7 +47,8 @@ int cgSolve(Storage& s, int op, int x, int b, int L, int maxIter, double tol, in
     s.cgUpdate(L, flag, false, now, pap, x, r, p, ap);
     const double sq = residual(next);
     if (finalRes) *finalRes = sq;
-    if (sq < tol) break;
+    // nothing is launched behind the last norm: the host has waited for all of the solve's work
+    if (sq < tol || it == maxIter) break;
     s.cgUpdate(L, flag, true, next, now, -1, r, p, -1);
   }
   return it;

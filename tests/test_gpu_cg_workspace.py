@@ -1,0 +1,61 @@
+"""The work vectors that a storage keeps between CG solves: a solve gives the same bits whatever was
+solved before it and on whichever stream, and nothing of it runs after the call."""
+import numpy as np
+import pytest
+
+import hyteg_b200 as hg
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def gpu():
+    if hg.device_count() == 0:
+        pytest.skip("no CUDA device")
+
+
+def storage(level, cubes=1):
+    return hg.PrimitiveStorage.cuboid((0, 0, 0), (1, 1, 1), cubes, cubes, cubes, level)
+
+
+def solve(st, L, seed, iterations, dtype=np.float64, operator=hg.P1ConstantLaplaceOperator, spoil=False):
+    A = operator(st, L, L)
+    x, b = hg.P1Function("x", st, L, L, dtype=dtype), hg.P1Function("b", st, L, L, dtype=dtype)
+    b.fill_random(seed, L)
+    if spoil:
+        b.interpolate(float("nan"), L, hg.Inner)
+    hg.CGSolver(st, L, L, maxIter=iterations).solve(A, x, b, L)
+    return x.to_numpy(L)
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("L", [1, 3])
+def test_solve_does_not_depend_on_earlier_ones(gpu, L, dtype):
+    fresh = solve(storage(L), L, 5, 4, dtype)
+    st = storage(L)
+    solve(st, L, 6, 3, dtype, hg.P1ConstantMassOperator)
+    solve(st, L, 7, 3, dtype, spoil=True)
+    assert np.isfinite(fresh).all()
+    assert np.array_equal(fresh, solve(st, L, 5, 4, dtype))
+
+
+def test_stream_change_between_solves(gpu):
+    import torch
+    L = 6
+    one = storage(L, 2)
+    ref = [solve(one, L, 10 + k, 3) for k in range(4)]
+    st = storage(L, 2)
+    A = hg.P1ConstantLaplaceOperator(st, L, L)
+    xs = [hg.P1Function("x", st, L, L) for _ in ref]
+    bs = [hg.P1Function("b", st, L, L) for _ in ref]
+    for k, b in enumerate(bs):
+        b.fill_random(10 + k, L)
+    st.synchronize()
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    cg = hg.CGSolver(st, L, L, maxIter=3)
+    for k in range(len(ref)):
+        st.set_stream(streams[k % 2].cuda_stream)
+        cg.solve(A, xs[k], bs[k], L)
+    assert all(s.query() for s in streams)  # the calls have returned, so their work is done
+    for x, r in zip(xs, ref):
+        assert np.array_equal(x.to_numpy(L), r)
