@@ -322,6 +322,12 @@ class PrimitiveStorage:
     def synchronize(self):
         call("hg_storage_synchronize", self._h)
 
+    def release_workspace(self):
+        """Gives the device buffers kept for the next call (CG work vectors) back; returns the bytes."""
+        n = ctypes.c_ulonglong()
+        call("hg_storage_release_workspace", self._h, ctypes.byref(n))
+        return n.value
+
     def set_l2_budget(self, nbytes):
         call("hg_storage_set_l2_budget", self._h, int(nbytes))
 

@@ -179,6 +179,13 @@ int hg_storage_synchronize(hg_storage* h) {
   HG_CATCH
 }
 
+int hg_storage_release_workspace(hg_storage* h, unsigned long long* bytes) {
+  HG_TRY
+  const size_t n = S(h).kept->release();
+  if (bytes) *bytes = n;
+  HG_CATCH
+}
+
 int hg_storage_set_l2_budget(hg_storage* h, int64_t bytes) {
   HG_TRY
   S(h).setL2Budget(bytes);
@@ -525,9 +532,18 @@ int hg_cg_solve(hg_storage* h, int op, int x, int b, int level, int max_iter, do
                 double* final_residual) {
   HG_TRY
   hg::Storage& s = S(h);
-  const std::array<int, 3> w = s.cgWork(level, s.fn(x).prec);
+  const int prec = s.fn(x).prec;
+  int w[3] = {-1, -1, -1}, it = 0;
   double res = 0;
-  const int it = hg::cgSolve(s, op, x, b, level, max_iter, tol, w[0], w[1], w[2], &res);
+  try {
+    for (int& id : w) id = s.borrowFunction(level, prec);
+    it = hg::cgSolve(s, op, x, b, level, max_iter, tol, w[0], w[1], w[2], &res);
+  } catch (...) {
+    for (int id : w) s.returnFunction(id, false);
+    throw;
+  }
+  // a solve of no iterations does not wait for the vectors' zeroing: those are freed, which does
+  for (int id : w) s.returnFunction(id, max_iter != 0);
   if (iterations) *iterations = it;
   if (final_residual) *final_residual = res;
   HG_CATCH

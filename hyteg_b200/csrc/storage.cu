@@ -2,12 +2,12 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <array>
 #include <cmath>
 #include <cstdint>
 #include <cstring>
 #include <map>
 #include <memory>
+#include <mutex>
 #include <numeric>
 #include <stdexcept>
 #include <string>
@@ -49,8 +49,65 @@ void* DevBuf::alloc(size_t n) {
   if (p) cudaFree(p);
   p = nullptr;
   bytes = n;
-  if (n) cudaCheck(cudaMalloc(&p, n), "cudaMalloc");
+  if (!n) return p;
+  cudaError_t e = cudaMalloc(&p, n);
+  if (e == cudaErrorMemoryAllocation) {  // kept buffers go first
+    (void)cudaGetLastError();
+    int device = 0;
+    cudaCheck(cudaGetDevice(&device), "cudaGetDevice");
+    if (KeptBuffers::releaseAll(device)) e = cudaMalloc(&p, n);
+  }
+  cudaCheck(e, "cudaMalloc");
   return p;
+}
+
+// Every pool of the process; the mutex guards the list and the pools, which other storages' threads release.
+static std::mutex keptMutex;
+static std::vector<KeptBuffers*>& keptPools() {
+  static auto* pools = new std::vector<KeptBuffers*>();
+  return *pools;
+}
+
+KeptBuffers::KeptBuffers(int dev) : device(dev) {
+  std::lock_guard<std::mutex> lock(keptMutex);
+  keptPools().push_back(this);
+}
+KeptBuffers::~KeptBuffers() {
+  std::lock_guard<std::mutex> lock(keptMutex);
+  auto& pools = keptPools();
+  pools.erase(std::find(pools.begin(), pools.end(), this));
+  drop();
+}
+std::unique_ptr<DevBuf> KeptBuffers::take(int key) {
+  std::lock_guard<std::mutex> lock(keptMutex);
+  std::unique_ptr<DevBuf> b;
+  for (size_t i = 0; i < free.size() && !b; ++i)
+    if (free[i].first == key) {
+      b = std::move(free[i].second);
+      free.erase(free.begin() + (std::ptrdiff_t)i);
+    }
+  return b;
+}
+void KeptBuffers::give(int key, std::unique_ptr<DevBuf> buf) {
+  std::lock_guard<std::mutex> lock(keptMutex);
+  free.emplace_back(key, std::move(buf));
+}
+size_t KeptBuffers::drop() {
+  size_t n = 0;
+  for (auto& b : free) n += b.second->bytes;
+  free.clear();
+  return n;
+}
+size_t KeptBuffers::release() {
+  std::lock_guard<std::mutex> lock(keptMutex);
+  return drop();
+}
+size_t KeptBuffers::releaseAll(int device) {
+  std::lock_guard<std::mutex> lock(keptMutex);
+  size_t n = 0;
+  for (KeptBuffers* p : keptPools())
+    if (p->device == device) n += p->drop();
+  return n;
 }
 
 template <class V>
@@ -78,6 +135,7 @@ static void allowSmem(F kernel, size_t bytes) {
 
 Storage::Storage(const Topology& topo, int maxLevel) : disc(topo, maxLevel) {
   cudaCheck(cudaGetDevice(&device), "cudaGetDevice");
+  kept.reset(new KeptBuffers(device));
   cudaCheck(cudaStreamCreateWithFlags(&ownStream, cudaStreamNonBlocking), "cudaStreamCreate");
   cudaCheck(cudaFuncSetAttribute(dev::cellSorWaveKernel<double, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)dev::waveSmemBytes<double, 0>(dev::kWaveMaxN)),
@@ -357,23 +415,28 @@ void Storage::setL2Budget(int64_t bytes) {
 // ------------------------------------------------------------------------------------------
 // functions
 // ------------------------------------------------------------------------------------------
-const std::array<int, 3>& Storage::cgWork(int L, int prec) {
-  auto it = cgWorks.find({L, prec});
-  if (it != cgWorks.end()) return it->second;
-  std::array<int, 3> w{-1, -1, -1};
-  try {
-    for (int& id : w) id = createFunction(L, L, prec);
-  } catch (...) {
-    for (int id : w) fns.erase(id);
-    throw;
-  }
-  return cgWorks[{L, prec}] = w;
+static int keptKey(int L, int prec) { return 2 * L + (prec == 4 ? 1 : 0); }
+
+int Storage::borrowFunction(int L, int prec) {
+  argCheck(L >= 0 && L <= maxLevel(), "invalid level range");
+  argCheck(prec == 8 || prec == 4, "precision must be 8 or 4");
+  std::unique_ptr<DevBuf> buf = kept->take(keptKey(L, prec));
+  if (!buf) return createFunction(L, L, prec);
+  std::unique_ptr<Function> f(new Function());
+  f->minL = f->maxL = L;
+  f->prec = prec;
+  f->levels.push_back(std::move(buf));
+  const int id = nextId++;
+  fns[id] = std::move(f);
+  return id;
 }
 
-void Storage::releaseCgWork() {
-  for (auto& w : cgWorks)
-    for (int id : w.second) fns.erase(id);
-  cgWorks.clear();
+void Storage::returnFunction(int id, bool give) {
+  auto it = fns.find(id);
+  if (it == fns.end()) return;
+  Function& f = *it->second;
+  if (give) kept->give(keptKey(f.minL, f.prec), std::move(f.levels[0]));
+  fns.erase(it);
 }
 
 void Storage::cgUpdate(int L, unsigned mask, bool direction, const double* num, const double* den, int x, int r, int p,
@@ -416,13 +479,7 @@ int Storage::createFunction(int minL, int maxL, int prec) {
   for (int L = minL; L <= maxL; ++L) {
     f->levels.emplace_back(new DevBuf());
     const size_t bytes = (size_t)levels[L].lay->total * prec;
-    try {
-      f->levels.back()->alloc(bytes);
-    } catch (const Error& e) {  // kept workspace goes first
-      if (e.code != HG_ERR_OOM || cgWorks.empty()) throw;
-      releaseCgWork();
-      f->levels.back()->alloc(bytes);
-    }
+    f->levels.back()->alloc(bytes);
     cudaCheck(cudaMemsetAsync(f->levels.back()->p, 0, bytes, stream), "memset");
   }
   const int id = nextId++;

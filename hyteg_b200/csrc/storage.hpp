@@ -3,7 +3,6 @@
 
 #include <cuda_runtime.h>
 
-#include <array>
 #include <deque>
 #include <map>
 #include <memory>
@@ -25,6 +24,27 @@ struct DevBuf {
   DevBuf& operator=(const DevBuf&) = delete;
   ~DevBuf();
   void* alloc(size_t n);
+};
+
+// Device buffers of finished calls, kept under a key for later calls. take() hands a buffer to one call
+// (nullptr: none is kept), give() returns it; only buffers that no call holds are ever released: by
+// release(), by the destructor, and by any DevBuf::alloc of the process that runs out of memory on
+// their device. Give a buffer back only once the device has finished the work on it.
+class KeptBuffers {
+ public:
+  explicit KeptBuffers(int device);
+  ~KeptBuffers();
+  KeptBuffers(const KeptBuffers&) = delete;
+  KeptBuffers& operator=(const KeptBuffers&) = delete;
+  std::unique_ptr<DevBuf> take(int key);
+  void give(int key, std::unique_ptr<DevBuf> buf);
+  size_t release();                         // bytes released
+  static size_t releaseAll(int device);     // those of every pool on the device
+
+ private:
+  size_t drop();
+  const int device;
+  std::vector<std::pair<int, std::unique_ptr<DevBuf>>> free;
 };
 
 // Order of the halo groups in a level's table: every group set one SOR phase refreshes at once
@@ -254,11 +274,13 @@ struct Storage {
   // dst = a / b elementwise on the flagged primitives' slots (FP64)
   void divideBy(int dst, int a, int b, int L, unsigned mask);
   void dotAsync(int a, int b, int L, unsigned mask, double* dOut);
-  // Work vectors (p, ap, r) of CG solves on one level, kept from solve to solve with the storage and
-  // given up when a function cannot be allocated otherwise.
-  std::map<std::pair<int, int>, std::array<int, 3>> cgWorks;  // (level, precision)
-  const std::array<int, 3>& cgWork(int L, int prec);
-  void releaseCgWork();
+  // Buffers of the CG work vectors between solves.
+  std::unique_ptr<KeptBuffers> kept;
+  // A work vector of a CG solve, its buffer from `kept`, and its end: the buffer goes back (give) or
+  // is freed. A solve writes the DoFs it solves for before it reads them and refreshes the copies
+  // that it reads; what it never writes is zero, as in a new function.
+  int borrowFunction(int L, int prec);
+  void returnFunction(int id, bool give);
   // x += alpha p, r -= alpha ap with alpha = num / den, or (direction) p = r + beta p with beta = num / den
   void cgUpdate(int L, unsigned mask, bool direction, const double* num, const double* den, int x, int r, int p, int ap);
   // Batched solves on a storage of `copies` disjoint copies of one macro-mesh (meshCuboidCopies):

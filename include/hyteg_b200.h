@@ -104,6 +104,10 @@ int hg_storage_counts(const hg_storage* s, int counts[4]);
 /* Use this CUDA stream (cudaStream_t) for all subsequent work; NULL = the storage's own stream. */
 int hg_storage_set_stream(hg_storage* s, void* stream);
 int hg_storage_synchronize(hg_storage* s);
+/* Device buffers that the storage keeps for its next call (three vectors per level and precision after
+ * hg_cg_solve) go back to the device: for callers with another allocator on it. The library's own
+ * allocations release them when the device is out of memory. bytes (nullable): the bytes released. */
+int hg_storage_release_workspace(hg_storage* s, unsigned long long* bytes);
 /* Bytes of L2 that one group of macro-cells may occupy during the cell phase of an SOR sweep
  * (the four colour passes of a group run back to back); default: all macro-cells form one group. */
 int hg_storage_set_l2_budget(hg_storage* s, int64_t bytes);

@@ -1,5 +1,6 @@
 """The work vectors that a storage keeps between CG solves: a solve gives the same bits whatever was
-solved before it and on whichever stream, and nothing of it runs after the call."""
+solved before it and on whichever stream, nothing of it runs after the call, and the buffers go back
+on request and when the device runs out of memory."""
 import numpy as np
 import pytest
 
@@ -59,3 +60,46 @@ def test_stream_change_between_solves(gpu):
     assert all(s.query() for s in streams)  # the calls have returned, so their work is done
     for x, r in zip(xs, ref):
         assert np.array_equal(x.to_numpy(L), r)
+
+
+def test_no_iterations(gpu):
+    L = 2
+    st = storage(L)
+    assert not solve(st, L, 3, 0).any()
+    assert st.release_workspace() == 0
+
+
+def test_release(gpu):
+    L = 3
+    st = storage(L)
+    first = solve(st, L, 5, 4)
+    assert st.release_workspace() == 3 * 8 * st.level_size(L)
+    assert st.release_workspace() == 0
+    assert np.array_equal(first, solve(st, L, 5, 4))
+
+
+def test_given_back_when_memory_runs_out(gpu):
+    # two storages keep three vectors each; the memory left then holds none, so that a function of
+    # a third storage and its second SOR buffer need what was kept
+    import torch
+    L = 7
+    keepers = [storage(L, 2), storage(L, 2)]
+    st = storage(L, 2)
+    vector = 8 * st.level_size(L)
+    A = hg.P1ConstantLaplaceOperator(st, L, L)
+    x, b = hg.P1Function("x", st, L, L), hg.P1Function("b", st, L, L)
+    b.fill_random(4, L)
+    for k in keepers:
+        solve(k, L, 5, 2)
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    filler = torch.empty(torch.cuda.mem_get_info()[0] - vector // 2, dtype=torch.uint8, device="cuda")
+    try:
+        y = hg.P1Function("y", st, L, L)
+        assert [k.release_workspace() for k in keepers] == [0, 0]
+        assert not y.to_numpy(L).any()
+        A.smooth_sor(x, b, 1.0, L, hg.Inner)  # its second buffer
+        st.synchronize()
+    finally:
+        del filler
+        torch.cuda.empty_cache()
