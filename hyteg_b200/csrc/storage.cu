@@ -314,7 +314,10 @@ void Storage::buildLevel(int L) {
     std::vector<int2> fr = ranges(G_FACE_BOUNDARY, KF, lv.nFaces);
     if (!low.empty()) ld.lowRange = (const int2*)upload(ld.keep, low, stream);
     if (!fr.empty()) ld.faceRange = (const int2*)upload(ld.keep, fr, stream);
-    if (dev::residentLevel((int)N)) ld.cellRange = (const int2*)upload(ld.keep, ranges(G_CELL, KC, lv.nCells), stream);
+    if (dev::residentLevel((int)N)) {
+      ld.cellRange = (const int2*)upload(ld.keep, ranges(G_CELL, KC, lv.nCells), stream);
+      buildSplitRows(L);
+    }
   }
 
   auto& keep = ld.keep;
@@ -575,28 +578,73 @@ void splitTables(int64_t w, int col, std::vector<dev::SplitRow>& rows, std::vect
   }
 }
 
-// Schedule-3 tables of level L: the halo table with every slot of a cell array replaced by its
-// position in the colour-split order (a permutation inside each row of the cell's array), and
-// per colour the interior rows (their 15 slots at j = 0) and points (row << 10 | j) that
-// cellSorSplitKernel walks; the same for every macro-cell of the level.
+// Position of every point of a closed macro-cell with w points per edge in the colour-split order (a
+// permutation inside each row).
+static std::vector<int> splitPermutation(int64_t w) {
+  auto tet = [](int64_t a) { return a * (a + 1) * (a + 2) / 6; };
+  std::vector<int> perm((size_t)tet(w));
+  int64_t r0 = 0;
+  for (int64_t z = 0; z < w; ++z)
+    for (int64_t y = 0; y < w - z; ++y) {
+      const int m = (int)(w - z - y);
+      for (int x = 0; x < m; ++x) perm[(size_t)(r0 + x)] = (int)(r0 + dev::splitSub(m, x & 3) + (x >> 2));
+      r0 += m;
+    }
+  return perm;
+}
+
+// Per colour the interior rows (their 15 slots at j = 0) and points (row << 10 | j) that
+// cellSorSplitKernel and cellSorResidentKernel walk, the same for every macro-cell of the level, and for
+// the latter the permutation: one buffer, from the lattice size alone. Resident levels have it from the
+// storage's creation, so that no sweep allocates or waits for it.
+void Storage::buildSplitRows(int L) {
+  LevelData& ld = levels[L];
+  if (ld.splitBuf) return;
+  const int64_t w = ld.lay->w;
+  std::vector<dev::SplitRow> rows[4];
+  std::vector<unsigned> points[4];
+  std::vector<uint16_t> perm16;
+  size_t nRows = 0, nPoints = 0;
+  for (int col = 0; col < 4; ++col) {
+    splitTables(w, col, rows[col], points[col]);
+    nRows += rows[col].size();
+    nPoints += points[col].size();
+  }
+  if (dev::residentLevel((int)w - 1)) {
+    const std::vector<int> perm = splitPermutation(w);
+    perm16.assign(perm.begin(), perm.end());
+  }
+  const size_t pointsAt = nRows * sizeof(dev::SplitRow), permAt = pointsAt + nPoints * sizeof(unsigned);
+  std::vector<unsigned char> host(std::max<size_t>(permAt + perm16.size() * sizeof(uint16_t), 16));
+  std::unique_ptr<DevBuf> buf(new DevBuf());
+  unsigned char* d = (unsigned char*)buf->alloc(host.size());
+  size_t r = 0, p = pointsAt;
+  for (int col = 0; col < 4; ++col) {
+    if (!rows[col].empty()) std::memcpy(&host[r], rows[col].data(), rows[col].size() * sizeof(dev::SplitRow));
+    if (!points[col].empty()) std::memcpy(&host[p], points[col].data(), points[col].size() * sizeof(unsigned));
+    ld.splitRows[col] = (const dev::SplitRow*)(d + r);
+    ld.splitPoints[col] = (const unsigned*)(d + p);
+    ld.nSplitPoints[col] = (int)points[col].size();
+    r += rows[col].size() * sizeof(dev::SplitRow);
+    p += points[col].size() * sizeof(unsigned);
+  }
+  if (!perm16.empty()) {
+    std::memcpy(&host[permAt], perm16.data(), perm16.size() * sizeof(uint16_t));
+    ld.splitPerm = (const uint16_t*)(d + permAt);
+  }
+  cudaCheck(cudaMemcpyAsync(d, host.data(), host.size(), cudaMemcpyHostToDevice, stream), "colour-split rows");
+  cudaCheck(cudaStreamSynchronize(stream), "colour-split rows");  // the host copy goes out of scope
+  ld.splitBuf = std::move(buf);
+}
+
+// Schedule-3 tables of level L: the rows, and the halo table with every slot of a cell array replaced by
+// its position in the colour-split order.
 void Storage::buildSplit(int L) {
   LevelData& ld = levels[L];
   if (ld.commSplit) return;
   const LevelLayout& lay = *ld.lay;
-  const int64_t w = lay.w, N = w - 1;
-  argCheck(N <= 4096, "colour-split SOR: level too large");
-  auto tet = [](int64_t a) { return a * (a + 1) * (a + 2) / 6; };
-  auto rowStart = [&](int64_t z, int64_t y) {
-    const int64_t W = w - z;
-    return tet(w) - tet(W) + y * (W + 1) - y * (y + 1) / 2;
-  };
-  std::vector<int> perm((size_t)tet(w));
-  for (int64_t z = 0; z < w; ++z)
-    for (int64_t y = 0; y < w - z; ++y) {
-      const int64_t r0 = rowStart(z, y);
-      const int m = (int)(w - z - y);
-      for (int x = 0; x < m; ++x) perm[(size_t)(r0 + x)] = (int)(r0 + dev::splitSub(m, x & 3) + (x >> 2));
-    }
+  argCheck(lay.w - 1 <= 4096, "colour-split SOR: level too large");
+  const std::vector<int> perm = splitPermutation(lay.w);
   std::vector<std::pair<int64_t, int64_t>> cells;  // (offset, size), ascending
   for (size_t c = 0; c < lay.off[KC].size(); ++c) cells.push_back({lay.off[KC][c], lay.size[KC][c]});
   std::sort(cells.begin(), cells.end());
@@ -615,19 +663,7 @@ void Storage::buildSplit(int L) {
   for (int g : kCommOrder)
     for (size_t i : commOrder(lay, g)) comm.push_back(make_uint2(map(lay.commDst[g][i]), map(lay.commSrc[g][i])));
   const uint2* commSplit = comm.empty() ? ld.comm : (const uint2*)upload(ld.keep, comm, stream);
-  // rows and points per colour
-  for (int col = 0; col < 4; ++col) {
-    std::vector<dev::SplitRow> rows;
-    std::vector<unsigned> points;
-    splitTables(w, col, rows, points);
-    ld.splitRows[col] = (const dev::SplitRow*)upload(ld.keep, rows, stream);
-    ld.splitPoints[col] = (const unsigned*)upload(ld.keep, points, stream);
-    ld.nSplitPoints[col] = (int)points.size();
-  }
-  if (dev::residentLevel((int)N)) {
-    const std::vector<uint16_t> perm16(perm.begin(), perm.end());
-    ld.splitPerm = (const uint16_t*)upload(ld.keep, perm16, stream);
-  }
+  buildSplitRows(L);
   cudaCheck(cudaStreamSynchronize(stream), "colour-split tables");  // the host vectors go out of scope
   ld.commSplit = commSplit;
 }
@@ -2154,7 +2190,6 @@ void Storage::sorT(Operator& o, int dstId, int L, T* u, const T* rhs, unsigned m
     // Schedule 0 keeps a small macro-cell resident in shared memory (in place, closure refresh
     // folded in) and sweeps larger ones in the wavefront pass.
     if (schedule == 0 && dev::residentLevel(lv.N)) {
-      buildSplit(L);
       dev::ResidentTables tb{};
       tb.perm = ld.splitPerm;
       for (int k = 0; k < 4; ++k) {

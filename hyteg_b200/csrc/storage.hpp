@@ -106,6 +106,7 @@ struct LevelData {
   const dev::SplitRow* splitRows[4] = {nullptr, nullptr, nullptr, nullptr};
   const unsigned* splitPoints[4] = {nullptr, nullptr, nullptr, nullptr};
   int nSplitPoints[4] = {0, 0, 0, 0};
+  std::unique_ptr<DevBuf> splitBuf;  // splitRows, splitPoints and splitPerm
   // resident cell phase (dev::residentLevel): positions in the colour-split order, and per cell its
   // entries (begin, end) in comm of the cell-closure group
   const uint16_t* splitPerm = nullptr;
@@ -260,7 +261,8 @@ struct Storage {
   void downloadOwned(int id, int L, void* host, int64_t n, cudaStream_t copyStream);
   std::map<std::pair<int, int>, std::unique_ptr<DevBuf>> splitRhs;  // (level, precision) -> split rhs copy
   DevBuf& spareBuf(std::map<std::pair<int, int>, std::unique_ptr<DevBuf>>& pool, int L, int prec);
-  void buildSplit(int L);  // the schedule-3 tables of level L (no-op once built)
+  void buildSplitRows(int L);  // the rows and points of the colour-split order (no-op once built)
+  void buildSplit(int L);      // the schedule-3 tables of level L (no-op once built)
   dev::Geometry geom{};              // macro-vertex coordinates and primitive vertex lists (device)
   std::vector<std::unique_ptr<DevBuf>> geomKeep;
 

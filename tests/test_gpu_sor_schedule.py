@@ -71,6 +71,33 @@ def test_resident_cells_equal_colour_passes(cube6, L, backwards, dtype, tol):
     test_single_pass_equals_colour_passes(cube6, L, backwards, dtype, tol, 0)
 
 
+@pytest.mark.parametrize("backwards", [False, True])
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+def test_first_resident_sweep_allocates_nothing(cube6, backwards, dtype):
+    """The tables of the resident cell phase come with the storage: the very first sweep on it neither
+    allocates nor waits, so it can be captured, and the replay gives the bits of an eager sweep."""
+    import torch
+    L, omega = 3, 1.3
+    rng = np.random.default_rng(9)
+    n = cube6[0].level_size(L)
+    x0, b0 = rng.uniform(-1, 1, n).astype(dtype), rng.uniform(-1, 1, n).astype(dtype)
+    eager = run_sor(cube6[0], L, x0, b0, dtype, 0, 1, backwards, omega)
+    st = hg.PrimitiveStorage.cuboid((0, 0, 0), (1, 1, 1), 2, 2, 2, L)
+    stream = torch.cuda.Stream()
+    st.set_stream(stream.cuda_stream)
+    A = hg.P1ConstantLaplaceOperator(st, L, L)
+    x, b = hg.P1Function("x", st, L, L, dtype=dtype), hg.P1Function("b", st, L, L, dtype=dtype)
+    x.from_numpy(L, x0)
+    b.from_numpy(L, b0)
+    stream.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream, capture_error_mode="thread_local"):
+        (A.smooth_sor_backwards if backwards else A.smooth_sor)(x, b, omega, L, hg.Inner)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert np.array_equal(x.to_numpy(L).astype(np.float64), eager)
+
+
 @pytest.mark.parametrize("schedule", [0, 3])
 def test_single_pass_matches_oracle_level5(schedule):
     if hg.device_count() == 0:
