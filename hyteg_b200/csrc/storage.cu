@@ -8,7 +8,6 @@
 #include <map>
 #include <memory>
 #include <mutex>
-#include <numeric>
 #include <stdexcept>
 #include <string>
 #include <type_traits>
@@ -149,10 +148,6 @@ Storage::Storage(const Topology& topo, int maxLevel) : disc(topo, maxLevel) {
   cudaCheck(cudaFuncSetAttribute(dev::cellSorWaveKernel<float, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)dev::waveSmemBytes<float, 1>(dev::kWaveMaxN)),
             "wave kernel shared memory");
-  allowSmem(dev::p2ApplyKernel<double, dev::MODE_REPLACE>, dev::p2TileSmem<double>());
-  allowSmem(dev::p2ApplyKernel<double, dev::MODE_RESIDUAL>, dev::p2TileSmem<double>());
-  allowSmem(dev::p2ApplyKernel<float, dev::MODE_REPLACE>, dev::p2TileSmem<float>());
-  allowSmem(dev::p2ApplyKernel<float, dev::MODE_RESIDUAL>, dev::p2TileSmem<float>());
   allowSmem(dev::cellSorResidentKernel<double>, dev::residentSmem<double>(dev::kResidentMaxN));
   allowSmem(dev::cellSorResidentKernel<float>, dev::residentSmem<float>(dev::kResidentMaxN));
   stream = ownStream;
@@ -197,15 +192,19 @@ Storage::~Storage() {
 
 static int64_t firstVertexSlot(const LevelLayout& lay) { return lay.off[KV].empty() ? lay.total : lay.off[KV][0]; }
 
-// Order of a halo group's entries in the level's table: the edge copies owned by vertices come
-// before the other edge copies, everything else as generated.
-static std::vector<size_t> commOrder(const LevelLayout& lay, int g) {
-  std::vector<size_t> order(lay.commDst[g].size());
-  std::iota(order.begin(), order.end(), size_t(0));
-  if (g == G_EDGE)
-    std::stable_partition(order.begin(), order.end(),
-                          [&](size_t i) { return lay.commSrc[g][i] >= firstVertexSlot(lay); });
-  return order;
+// Calls f(destination, source) on the halo entries in the order of the level's table: group by group as
+// generated, but the edge copies owned by vertices before the other edge copies.
+template <class F>
+static void forComm(const LevelLayout& lay, int g, F f) {
+  const auto &d = lay.commDst[g], &s = lay.commSrc[g];
+  if (g != G_EDGE) {
+    for (size_t i = 0; i < d.size(); ++i) f(d[i], s[i]);
+    return;
+  }
+  const int64_t first = firstVertexSlot(lay);
+  for (const bool vertex : {true, false})
+    for (size_t i = 0; i < d.size(); ++i)
+      if ((s[i] >= first) == vertex) f(d[i], s[i]);
 }
 
 void Storage::buildLevel(int L) {
@@ -273,10 +272,12 @@ void Storage::buildLevel(int L) {
 
   // halo table in the five destination groups
   std::vector<uint2> comm;
+  size_t nComm = 0;
+  for (int g : kCommOrder) nComm += lay.commDst[g].size();
+  comm.reserve(nComm);
   for (int g : kCommOrder) {
     ld.commBegin[g] = (int64_t)comm.size();
-    for (size_t i : commOrder(lay, g))
-      comm.push_back(make_uint2((unsigned)lay.commDst[g][i], (unsigned)lay.commSrc[g][i]));
+    forComm(lay, g, [&](int64_t d, int64_t s) { comm.push_back(make_uint2((unsigned)d, (unsigned)s)); });
     ld.commCount[g] = (int64_t)comm.size() - ld.commBegin[g];
   }
   ld.commEdgeOther = ld.commBegin[G_EDGE];
@@ -284,22 +285,20 @@ void Storage::buildLevel(int L) {
          (int64_t)comm[(size_t)ld.commEdgeOther].y >= firstVertexSlot(lay))
     ++ld.commEdgeOther;
   argCheck(comm.size() < (size_t(1) << 31), "halo table exceeds 32-bit ranges");
-  // Each primitive's entries of a group are contiguous (the tables are generated primitive by
-  // primitive): the range of every primitive's destination array, found from its offsets.
+  // Each primitive's entries of a group are contiguous and the primitives follow one another (the
+  // tables are generated primitive by primitive, and so are the arrays): the range of every
+  // primitive's destination array in one walk over both.
   auto ranges = [&](int g, int kind, int nPrim) {
     std::vector<int2> r((size_t)nPrim, make_int2(0, 0));
-    std::vector<char> seen((size_t)nPrim, 0);
-    int last = -1;
+    const auto &offs = lay.off[kind], &size = lay.size[kind];
+    int p = 0, last = -1;
     // of the edge copies only those owned by vertices (the phases refresh the others before)
     const int64_t end = g == G_EDGE ? ld.commEdgeOther : ld.commBegin[g] + ld.commCount[g];
     for (int64_t i = ld.commBegin[g]; i < end; ++i) {
       const int64_t d = comm[(size_t)i].x;
-      const auto& offs = lay.off[kind];
-      const int p = int(std::upper_bound(offs.begin(), offs.end(), d) - offs.begin()) - 1;
-      argCheck(p >= 0 && p < nPrim && d < offs[(size_t)p] + lay.size[kind][(size_t)p], "halo entry outside its group's kind");
+      while (p < nPrim && d >= offs[(size_t)p] + size[(size_t)p]) ++p;
+      argCheck(p < nPrim && d >= offs[(size_t)p], "halo entry outside its group's kind, or out of order");
       if (p != last) {
-        argCheck(!seen[(size_t)p], "halo entries of a primitive are not contiguous");
-        seen[(size_t)p] = 1;
         r[(size_t)p].x = (int)i;
         last = p;
       }
@@ -315,7 +314,17 @@ void Storage::buildLevel(int L) {
     if (!low.empty()) ld.lowRange = (const int2*)upload(ld.keep, low, stream);
     if (!fr.empty()) ld.faceRange = (const int2*)upload(ld.keep, fr, stream);
     if (dev::residentLevel((int)N)) {
-      ld.cellRange = (const int2*)upload(ld.keep, ranges(G_CELL, KC, lv.nCells), stream);
+      // every cell has the same closure
+      const int per = lv.nCells ? (int)(ld.commCount[G_CELL] / lv.nCells) : 0;
+      std::vector<int2> cells;
+      for (int c = 0; c < lv.nCells; ++c) {
+        const int first = (int)ld.commBegin[G_CELL] + c * per;
+        cells.push_back(make_int2(first, first + per));
+        for (const int i : {first, first + per - 1})
+          argCheck(comm[(size_t)i].x >= lay.off[KC][c] && comm[(size_t)i].x < lay.off[KC][c] + lay.size[KC][c],
+                   "closure entry outside its cell");
+      }
+      ld.cellRange = (const int2*)upload(ld.keep, cells, stream);
       buildSplitRows(L);
     }
   }
@@ -660,8 +669,7 @@ void Storage::buildSplit(int L) {
     return (unsigned)slot;
   };
   std::vector<uint2> comm;  // the same entries in the same order as the level's table
-  for (int g : kCommOrder)
-    for (size_t i : commOrder(lay, g)) comm.push_back(make_uint2(map(lay.commDst[g][i]), map(lay.commSrc[g][i])));
+  for (int g : kCommOrder) forComm(lay, g, [&](int64_t d, int64_t s) { comm.push_back(make_uint2(map(d), map(s))); });
   const uint2* commSplit = comm.empty() ? ld.comm : (const uint2*)upload(ld.keep, comm, stream);
   buildSplitRows(L);
   cudaCheck(cudaStreamSynchronize(stream), "colour-split tables");  // the host vectors go out of scope
@@ -1081,6 +1089,11 @@ int Storage::createP2Operator(int form, int minL, int maxL) {
   argCheck(form == FORM_LAPLACE, "P2 operators: only the Laplace form is available");
   argCheck(minL >= 0 && maxL + 1 <= maxLevel() && minL <= maxL,
            "P2 level range needs the storage's levels up to max_level + 1");
+  // here, not with the storage: this loads the kernels, which P1 programs never run
+  allowSmem(dev::p2ApplyKernel<double, dev::MODE_REPLACE>, dev::p2TileSmem<double>());
+  allowSmem(dev::p2ApplyKernel<double, dev::MODE_RESIDUAL>, dev::p2TileSmem<double>());
+  allowSmem(dev::p2ApplyKernel<float, dev::MODE_REPLACE>, dev::p2TileSmem<float>());
+  allowSmem(dev::p2ApplyKernel<float, dev::MODE_RESIDUAL>, dev::p2TileSmem<float>());
   std::unique_ptr<P2Operator> o(new P2Operator());
   o->form = form;
   o->minL = minL;
