@@ -420,7 +420,7 @@ struct GroupSel {
 struct LevelBuild {
   int L = 0;
   std::vector<Dof> dofs;          // unknowns in SOR order
-  std::vector<int> unknownOf;     // absolute owner slot -> unknown (group 0), -1 elsewhere
+  std::vector<int> unknownOf;     // slot -> unknown that it holds, itself or as a copy (group 0), -1 elsewhere
   std::vector<int> rowOf;         // unknown -> row, -1
   std::vector<dev::CompactRow> rows, cgRows;
   std::vector<int> cols;
@@ -472,6 +472,11 @@ LevelBuild buildLevel(Storage& s, const LevelStencils& hs, int L, const GroupSel
   const int n = (int)dofs.size();
   lb.unknownOf.assign((size_t)lay.total, -1);
   for (int i = 0; i < n; ++i) lb.unknownOf[(size_t)dofs[(size_t)i].slot] = i;
+  // every copy by the level's halo entries: finding the owner of each entry of each row anew (by its
+  // barycentric weights) took 7 of the 11 ms of the build at levels 0-4 of one sub-cube
+  for (int g = 0; g < G_COUNT; ++g)
+    for (size_t e = 0; e < lay.commDst[g].size(); ++e)
+      lb.unknownOf[(size_t)lay.commDst[g][e]] = lb.unknownOf[(size_t)lay.commSrc[g][e]];
   lb.snapBegin = lb.snapEnd = n;
   for (int i = n - 1; i >= 0; --i) {
     if (dofs[(size_t)i].kind >= KE) lb.snapBegin = i;
@@ -486,8 +491,8 @@ LevelBuild buildLevel(Storage& s, const LevelStencils& hs, int L, const GroupSel
     if (!(d.type & (mask | (coarsest ? cgMask : 0u)))) continue;
     e0[(size_t)i] = (int)lb.cols.size();
     auto add = [&](int kind, int prim, int64_t local) {
-      const Slot o = D.owner(L, D.slotBary(L, kind, prim, local));
-      const int j = lb.unknownOf[(size_t)(lay.off[o.kind][(size_t)o.prim] + o.local)];
+      argCheck(local >= 0 && local < lay.size[kind][(size_t)prim], "compact cycle: a stencil entry outside its primitive");
+      const int j = lb.unknownOf[(size_t)(lay.off[kind][(size_t)prim] + local)];
       argCheck(j >= 0, "compact cycle: a stencil entry outside the group");
       if (coarsest) {  // the coarsest level is solved by CG only: no smoother reads
         lb.cols.push_back(j);
@@ -555,8 +560,7 @@ void buildTransfers(Storage& s, LevelBuild& f, LevelBuild& c, const GroupSel& se
   const LevelLayout& lc = *s.levels[(size_t)c.L].lay;
   const int64_t Nf = int64_t(1) << f.L, wf = Nf + 1, wc = Nf / 2 + 1;
   auto unknown = [&](const LevelBuild& lb, const LevelLayout& lay, int cell, int64_t w, int64_t x, int64_t y, int64_t z) {
-    const Slot o = D.owner(lb.L, D.slotBary(lb.L, KC, cell, cellIdx(w, x, y, z)));
-    const int j = lb.unknownOf[(size_t)(lay.off[o.kind][(size_t)o.prim] + o.local)];
+    const int j = lb.unknownOf[(size_t)(lay.off[KC][(size_t)cell] + cellIdx(w, x, y, z))];
     argCheck(j >= 0, "compact cycle: a transfer entry outside the group");
     return j;
   };
@@ -795,8 +799,7 @@ std::unique_ptr<CompactCycle> buildCompactCycle(Storage& s, int op, int minL, in
     for (size_t p = 0; p < nPrim[kind]; ++p) {
       if (!ts.inGroup0(kind, lay.off[kind][p])) continue;
       for (int64_t local = 0; local < lay.size[kind][p]; ++local) {
-        const Slot o2 = s.disc.owner(top, s.disc.slotBary(top, kind, (int)p, local));
-        const int j = tb.unknownOf[(size_t)(lay.off[o2.kind][(size_t)o2.prim] + o2.local)];
+        const int j = tb.unknownOf[(size_t)(lay.off[kind][p] + local)];
         argCheck(j >= 0, "compact cycle: a copy slot outside the group");
         slots0.push_back({lay.off[kind][p] + local, kind});
         idx0.push_back(j);

@@ -399,6 +399,10 @@ struct Error : std::runtime_error {
 };
 void cudaCheck(cudaError_t e, const char* what);
 void argCheck(bool ok, const std::string& msg);
+// no string is made for a check that holds: table builders check every entry
+inline void argCheck(bool ok, const char* msg) {
+  if (!ok) argCheck(false, std::string(msg));
+}
 extern thread_local std::string g_lastError;
 
 }  // namespace hg
