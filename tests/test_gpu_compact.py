@@ -171,3 +171,26 @@ def test_compact_cycle_above_level_zero(env, minL):
     oref, _ = orc.gmg(L, minL, np.zeros(n), bg, 3, 3, 3, 1.0, multicolour=True, cg_iter=2000, cg_tol=1e-16)
     assert relerr(out[True], oref, inner) < 1e-12
     assert relerr(out[False], oref, inner) < 1e-12
+
+
+@pytest.mark.parametrize("dtype,tol", [(np.float64, 1e-12), (np.float32, 2e-5)])
+def test_vectors_in_shared_memory_and_rows_not(dtype, tol):
+    """Two sub-cubes up to level 4, one block: the vectors (9537 unknowns on the top level) fit into the
+    block's shared memory, their packed rows (6975 of 40 bytes) do not and are read from the lists."""
+    if hg.device_count() == 0:
+        pytest.skip("no CUDA device")
+    L = 4
+    st = hg.PrimitiveStorage.cuboid((0, 0, 0), (1, 1, 2), 1, 1, 2, L)
+    A = hg.P1ConstantLaplaceOperator(st, 0, L)
+    out = {}
+    for kind, compact in ((dtype, 10000), (np.float64, 0)):
+        x, b = hg.P1Function("x", st, 0, L, dtype=kind), hg.P1Function("b", st, 0, L, dtype=kind)
+        b.fill_random(17, L, hg.Inner)
+        gmg = solver(st, L, kind)
+        gmg.set_compact(A, compact, 1)
+        assert gmg.compact_top(A) == (4 if compact else -1)
+        for _ in range(3):
+            gmg.solve(A, x, b, L)
+        x.communicate(L)
+        out[compact] = x.to_numpy(L).astype(np.float64)
+    assert relerr(out[10000], out[0], np.ones(st.level_size(L), dtype=bool)) < tol
