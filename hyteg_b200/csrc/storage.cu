@@ -1363,53 +1363,70 @@ static const dev::P2Tables& p2TablesOnce() {
   return tb;
 }
 
+// Index of offset (dx, dy, dz) in one of the lists of p2_stencil.h.
+static short offsetIndex(const signed char (*list)[3], int len, int dx, int dy, int dz) {
+  for (int e = 0; e < len; ++e)
+    if (list[e][0] == dx && list[e][1] == dy && list[e][2] == dz) return (short)e;
+  throw Error(HG_ERR_INTERNAL, "P2 stencil offset table does not match the micro-cells");
+}
+// That of local node m of micro-cell type t seen from its local node j.
+static short nodeIndex(const signed char (*list)[3], int len, int t, int j, int m) {
+  const dev::P2Tables& tb = p2TablesOnce();
+  return offsetIndex(list, len, tb.off[t][m][0] - tb.off[t][j][0], tb.off[t][m][1] - tb.off[t][j][1],
+                     tb.off[t][m][2] - tb.off[t][j][2]);
+}
+
+// One product of a stencil: weight `to` of a cell takes element entry `from` of that cell. The lists
+// depend on neither the cell nor the level; finding the offsets anew for each took most of an
+// operator's set-up.
+struct StencilTerm {
+  short to, from;
+};
+static std::vector<double> stencilWeights(const std::vector<StencilTerm>& terms, int weights, const std::vector<double>& K,
+                                          int entries, int nCells) {
+  std::vector<double> S((size_t)nCells * (size_t)weights, 0.0);
+  for (int c = 0; c < nCells; ++c) {
+    double* s = S.data() + (size_t)c * (size_t)weights;
+    const double* k = K.data() + (size_t)c * (size_t)entries;
+    for (const StencilTerm& q : terms) s[q.to] += k[q.from];
+  }
+  return S;
+}
+
 // Interior stencil weights of every cell: for each parity class, the sum over the class's
 // candidate micro-cells (type t, local node j) of row j of their element matrices, scattered
 // to the lattice offsets of the ten nodes in the order of p2s::kOff.
 static std::vector<double> p2Stencils(const std::vector<double>& K, int nCells) {
-  const dev::P2Tables& tb = p2TablesOnce();
-  std::vector<double> S((size_t)nCells * p2s::kTotal, 0.0);
-  for (int c = 0; c < nCells; ++c)
-    for (int pc = 0; pc < 8; ++pc) {
-      double* sc = S.data() + (size_t)c * p2s::kTotal + p2s::kFirst[pc];
+  static const std::vector<StencilTerm> terms = [] {
+    const dev::P2Tables& tb = p2TablesOnce();
+    std::vector<StencilTerm> v;
+    for (int pc = 0; pc < 8; ++pc)
       for (int k = 0; k < tb.nCand[pc]; ++k) {
         const int t = tb.cand[pc][k][0], j = tb.cand[pc][k][1];
-        for (int m = 0; m < 10; ++m) {
-          int e = 0;
-          while (e < p2s::kLen[pc] && !(p2s::kOff[pc][e][0] == tb.off[t][m][0] - tb.off[t][j][0] &&
-                                        p2s::kOff[pc][e][1] == tb.off[t][m][1] - tb.off[t][j][1] &&
-                                        p2s::kOff[pc][e][2] == tb.off[t][m][2] - tb.off[t][j][2]))
-            ++e;
-          if (e == p2s::kLen[pc]) throw Error(HG_ERR_INTERNAL, "P2 stencil offset table does not match the micro-cells");
-          sc[e] += K[(size_t)c * 600 + t * 100 + j * 10 + m];
-        }
+        for (int m = 0; m < 10; ++m)
+          v.push_back({(short)(p2s::kFirst[pc] + nodeIndex(p2s::kOff[pc], p2s::kLen[pc], t, j, m)),
+                       (short)(t * 100 + j * 10 + m)});
       }
-    }
-  return S;
+    return v;
+  }();
+  return stencilWeights(terms, p2s::kTotal, K, 600, nCells);
 }
 
-// Face-interior stencil weights of every cell: per (face, class) entry k, the sum over its
-// micro-cells p2s::kFaceCand[k] of their element rows, scattered to the offsets p2s::kFaceOff[k].
+// Closure stencil weights of every cell: per entry k (face and class, edge and parity, vertex), the sum
+// over its micro-cells p2s::kFaceCand[k] of their element rows, scattered to the offsets p2s::kFaceOff[k].
 static std::vector<double> p2FaceStencils(const std::vector<double>& K, int nCells) {
-  const dev::P2Tables& tb = p2TablesOnce();
-  std::vector<double> S((size_t)nCells * p2s::kFaceTotal, 0.0);
-  for (int c = 0; c < nCells; ++c)
-    for (int k = 0; k < p2s::kFaceStencils; ++k) {
-      double* sc = S.data() + (size_t)c * p2s::kFaceTotal + p2s::kFaceFirst[k];
+  static const std::vector<StencilTerm> terms = [] {
+    std::vector<StencilTerm> v;
+    for (int k = 0; k < p2s::kFaceStencils; ++k)
       for (int q = 0; q < p2s::kFaceNCand[k]; ++q) {
         const int t = p2s::kFaceCand[k][q][0], j = p2s::kFaceCand[k][q][1];
-        for (int m = 0; m < 10; ++m) {
-          int e = 0;
-          while (e < p2s::kFaceLen[k] && !(p2s::kFaceOff[k][e][0] == tb.off[t][m][0] - tb.off[t][j][0] &&
-                                           p2s::kFaceOff[k][e][1] == tb.off[t][m][1] - tb.off[t][j][1] &&
-                                           p2s::kFaceOff[k][e][2] == tb.off[t][m][2] - tb.off[t][j][2]))
-            ++e;
-          if (e == p2s::kFaceLen[k]) throw Error(HG_ERR_INTERNAL, "P2 face stencil table does not match the micro-cells");
-          sc[e] += K[(size_t)c * 600 + t * 100 + j * 10 + m];
-        }
+        for (int m = 0; m < 10; ++m)
+          v.push_back({(short)(p2s::kFaceFirst[k] + nodeIndex(p2s::kFaceOff[k], p2s::kFaceLen[k], t, j, m)),
+                       (short)(t * 100 + j * 10 + m)});
       }
-    }
-  return S;
+    return v;
+  }();
+  return stencilWeights(terms, p2s::kFaceTotal, K, 600, nCells);
 }
 
 // Sums of the cells' shares into the owners: dst = sum, or rhs - sum for a residual.
@@ -1754,63 +1771,49 @@ struct DivStencils {
 };
 
 static DivStencils p2DivStencils(const std::vector<double>& D, int nCells) {
-  const dev::P2Tables& tb = p2TablesOnce();
-  DivStencils S;
-  S.div.assign((size_t)nCells * 195, 0.0);
-  S.divT.assign((size_t)nCells * 195, 0.0);
-  S.divClosure.assign((size_t)nCells * 3 * p2s::kFaceTotal, 0.0);
-  S.divTClosure.assign((size_t)nCells * 3 * p2s::kDivTFaceTotal, 0.0);
-  auto find = [](const signed char (*tab)[3], int len, int dx, int dy, int dz) {
-    for (int e = 0; e < len; ++e)
-      if (tab[e][0] == dx && tab[e][1] == dy && tab[e][2] == dz) return e;
-    throw Error(HG_ERR_INTERNAL, "Taylor-Hood stencil table does not match the micro-cells");
+  struct Terms {
+    std::vector<StencilTerm> div, divT, divClosure, divTClosure;
   };
-  auto velocity = [&](const signed char (*tab)[3], int len, int t, int i, int j) {
-    return find(tab, len, tb.off[t][j][0] - tb.off[t][i][0], tb.off[t][j][1] - tb.off[t][i][1],
-                tb.off[t][j][2] - tb.off[t][i][2]);
-  };
-  auto pressure = [&](const signed char (*tab)[3], int len, int pc, int t, int i, int j) {
-    return find(tab, len, (tb.off[t][i][0] - tb.off[t][j][0] + (pc & 1)) / 2,
-                (tb.off[t][i][1] - tb.off[t][j][1] + ((pc >> 1) & 1)) / 2,
-                (tb.off[t][i][2] - tb.off[t][j][2] + ((pc >> 2) & 1)) / 2);
-  };
-  for (int c = 0; c < nCells; ++c) {
-    const double* Dc = D.data() + (size_t)c * 720;
+  static const Terms terms = [] {
+    const dev::P2Tables& tb = p2TablesOnce();
+    Terms s;
+    auto pressure = [&](const signed char (*list)[3], int len, int pc, int t, int i, int j) {
+      return offsetIndex(list, len, (tb.off[t][i][0] - tb.off[t][j][0] + (pc & 1)) / 2,
+                         (tb.off[t][i][1] - tb.off[t][j][1] + ((pc >> 1) & 1)) / 2,
+                         (tb.off[t][i][2] - tb.off[t][j][2] + ((pc >> 2) & 1)) / 2);
+    };
+    auto add = [](std::vector<StencilTerm>& v, int stride, int to, int t, int i, int j) {  // the three components
+      for (int k = 0; k < 3; ++k) v.push_back({(short)(k * stride + to), (short)(t * 120 + k * 40 + i * 10 + j)});
+    };
     for (int t = 0; t < 6; ++t)
       for (int i = 0; i < 4; ++i)
-        for (int j = 0; j < 10; ++j) {
-          const int e = velocity(p2s::kOff[0], p2s::kLen[0], t, i, j);
-          for (int k = 0; k < 3; ++k) S.div[(size_t)c * 195 + k * 65 + e] += Dc[t * 120 + k * 40 + i * 10 + j];
-        }
+        for (int j = 0; j < 10; ++j) add(s.div, 65, nodeIndex(p2s::kOff[0], p2s::kLen[0], t, i, j), t, i, j);
     for (int pc = 0; pc < 8; ++pc)
       for (int q = 0; q < tb.nCand[pc]; ++q) {
         const int t = tb.cand[pc][q][0], j = tb.cand[pc][q][1];
-        for (int i = 0; i < 4; ++i) {
-          const int e = pressure(p2s::kDivTOff[pc], p2s::kDivTLen[pc], pc, t, i, j);
-          for (int k = 0; k < 3; ++k)
-            S.divT[(size_t)c * 195 + k * 65 + p2s::kDivTFirst[pc] + e] += Dc[t * 120 + k * 40 + i * 10 + j];
-        }
+        for (int i = 0; i < 4; ++i)
+          add(s.divT, 65, p2s::kDivTFirst[pc] + pressure(p2s::kDivTOff[pc], p2s::kDivTLen[pc], pc, t, i, j), t, i, j);
       }
     for (int n = 0; n < p2s::kFaceStencils; ++n) {
       const int pc = p2s::kFaceClass[n];
       for (int q = 0; q < p2s::kFaceNCand[n]; ++q) {
         const int t = p2s::kFaceCand[n][q][0], j = p2s::kFaceCand[n][q][1];
-        for (int i = 0; i < 4; ++i) {
-          const int e = pressure(p2s::kDivTFaceOff[n], p2s::kDivTFaceLen[n], pc, t, i, j);
-          for (int k = 0; k < 3; ++k)
-            S.divTClosure[((size_t)c * 3 + k) * p2s::kDivTFaceTotal + p2s::kDivTFaceFirst[n] + e] +=
-                Dc[t * 120 + k * 40 + i * 10 + j];
-        }
+        for (int i = 0; i < 4; ++i)
+          add(s.divTClosure, p2s::kDivTFaceTotal,
+              p2s::kDivTFaceFirst[n] + pressure(p2s::kDivTFaceOff[n], p2s::kDivTFaceLen[n], pc, t, i, j), t, i, j);
         if (pc != 0) continue;
-        for (int m = 0; m < 10; ++m) {  // local node j of a vertex-class entry is pressure vertex j
-          const int e = velocity(p2s::kFaceOff[n], p2s::kFaceLen[n], t, j, m);
-          for (int k = 0; k < 3; ++k)
-            S.divClosure[((size_t)c * 3 + k) * p2s::kFaceTotal + p2s::kFaceFirst[n] + e] +=
-                Dc[t * 120 + k * 40 + j * 10 + m];
-        }
+        for (int m = 0; m < 10; ++m)  // local node j of a vertex-class entry is pressure vertex j
+          add(s.divClosure, p2s::kFaceTotal, p2s::kFaceFirst[n] + nodeIndex(p2s::kFaceOff[n], p2s::kFaceLen[n], t, j, m), t,
+              j, m);
       }
     }
-  }
+    return s;
+  }();
+  DivStencils S;
+  S.div = stencilWeights(terms.div, 195, D, 720, nCells);
+  S.divT = stencilWeights(terms.divT, 195, D, 720, nCells);
+  S.divClosure = stencilWeights(terms.divClosure, 3 * p2s::kFaceTotal, D, 720, nCells);
+  S.divTClosure = stencilWeights(terms.divTClosure, 3 * p2s::kDivTFaceTotal, D, 720, nCells);
   return S;
 }
 
