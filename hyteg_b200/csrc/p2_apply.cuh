@@ -35,15 +35,24 @@ constexpr int kP2FaceTile = 32;               // face nodes per piece edge
 constexpr int kP2RowTab = kP2Region * kP2Region;
 
 // Interior blocks. Node i of a block sits at origin + 1 + (bits of i), so its parity class is
-// 7 - i (the block's origin is even). Entries in the order of the lattice positions (z, y, x).
+// 7 - i (the block's origin is even). Entries by lattice position.
 struct P2BlockEntry {
   signed char x, y, z;  // lattice position relative to the block's origin, 0 .. 4
   unsigned char node;
-  unsigned char acc;    // the vertex class (65 products) is summed in four parts, the others in one
+  unsigned char acc;    // the accumulator of the product
   bool first;           // first entry of its position
   short weight;         // index into the cell's weights p2s::kTotal
 };
-constexpr int kP2Accs = 11;
+// The vertex class (65 products) is summed in four parts (7 .. 10), the edge classes of 27 products
+// (nodes 1, 3, 4, 6) in two halves, those of 19 in one: more accumulators spill in FP64 (two halves
+// everywhere: 335 us instead of 321 for the apply below). The positions of the nodes themselves come
+// last, so that the diagonal, the largest product, is added late and the partial sums before it round
+// less. Error against 64 bits, 48 cells, P2 level 5: FP64 6.2e-17, FP32 1.74e-8; with one chain per
+// edge class in the order of the positions 6.9e-17 and 2.34e-8, with four parts for every row 6.3e-17
+// and 1.80e-8.
+constexpr int kP2Accs = 15;
+__host__ __device__ constexpr bool p2Halves(int node) { return node == 1 || node == 3 || node == 4 || node == 6; }
+__host__ __device__ constexpr int p2Second(int node) { return node == 1 ? 11 : node == 3 ? 12 : node == 4 ? 13 : 14; }
 
 struct P2BlockTable {
   P2BlockEntry e[p2s::kTotal];
@@ -51,30 +60,48 @@ struct P2BlockTable {
 
 constexpr P2BlockTable makeP2BlockTable() {
   P2BlockTable t{};
-  int n = 0;
-  for (int z = 0; z <= 4; ++z)
-    for (int y = 0; y <= 4; ++y)
-      for (int x = 0; x <= 4; ++x) {
-        bool first = true;
-        for (int i = 0; i < 8; ++i) {
-          const int pc = 7 - i, nx = 1 + (i & 1), ny = 1 + ((i >> 1) & 1), nz = 1 + (i >> 2);
-          for (int k = 0; k < p2s::kLen[pc]; ++k)
-            if (nx + p2s::kOff[pc][k][0] == x && ny + p2s::kOff[pc][k][1] == y && nz + p2s::kOff[pc][k][2] == z) {
-              P2BlockEntry& q = t.e[n++];
-              q.x = (signed char)x;
-              q.y = (signed char)y;
-              q.z = (signed char)z;
-              q.node = (unsigned char)i;
-              q.acc = (unsigned char)(pc == 0 ? 7 + (k & 3) : i);
-              q.first = first;
-              q.weight = (short)(p2s::kFirst[pc] + k);
-              first = false;
-            }
+  int n = 0, done[8] = {};
+  for (const bool own : {false, true})
+    for (int z = 0; z <= 4; ++z)
+      for (int y = 0; y <= 4; ++y)
+        for (int x = 0; x <= 4; ++x) {
+          if (((x == 1 || x == 2) && (y == 1 || y == 2) && (z == 1 || z == 2)) != own) continue;
+          bool first = true;
+          for (int i = 0; i < 8; ++i) {
+            const int pc = 7 - i, nx = 1 + (i & 1), ny = 1 + ((i >> 1) & 1), nz = 1 + (i >> 2);
+            for (int k = 0; k < p2s::kLen[pc]; ++k)
+              if (nx + p2s::kOff[pc][k][0] == x && ny + p2s::kOff[pc][k][1] == y && nz + p2s::kOff[pc][k][2] == z) {
+                P2BlockEntry& q = t.e[n++];
+                q.x = (signed char)x;
+                q.y = (signed char)y;
+                q.z = (signed char)z;
+                q.node = (unsigned char)i;
+                const bool second = p2Halves(i) && 2 * done[i]++ >= p2s::kLen[pc];
+                q.acc = (unsigned char)(pc == 0 ? 7 + (k & 3) : second ? p2Second(i) : i);
+                q.first = first;
+                q.weight = (short)(p2s::kFirst[pc] + k);
+                first = false;
+              }
+          }
         }
-      }
   return t;
 }
 constexpr P2BlockTable kP2Block = makeP2BlockTable();
+// No accumulator takes more than 19 products, and every diagonal is among the products of the last eight
+// positions.
+constexpr bool p2SumsAreShort() {
+  int taken[8][kP2Accs] = {}, left = 8;
+  for (int e = p2s::kTotal - 1; e >= 0; --e) {
+    const P2BlockEntry& q = kP2Block.e[e];
+    const int i = q.node;
+    if (++taken[i][q.acc] > 19) return false;
+    const bool diagonal = q.x == 1 + (i & 1) && q.y == 1 + ((i >> 1) & 1) && q.z == 1 + (i >> 2);
+    if (diagonal && left <= 0) return false;
+    if (q.first) --left;
+  }
+  return true;
+}
+static_assert(p2SumsAreShort(), "P2 rows: summation order");
 static __constant__ P2BlockTable kP2BlockDev = makeP2BlockTable();
 
 // Face blocks: node i of face f at (s, t) = block origin + (bits of i); faces Z = 0: (X, Y),
@@ -82,6 +109,7 @@ static __constant__ P2BlockTable kP2BlockDev = makeP2BlockTable();
 struct P2FaceEntry {
   signed char x, y, z;
   unsigned char node;
+  unsigned char part;  // the products of a row are summed in two halves
   bool first;
   short weight;  // index into the cell's face weights p2s::kFaceTotal
 };
@@ -98,38 +126,44 @@ __host__ __device__ constexpr int p2FaceNode(int f, int i, int axis) {  // offse
   return axis == 0 ? -a - b : axis == 1 ? a : b;
 }
 
-constexpr P2FaceTable makeP2FaceTable() {
+constexpr P2FaceTable makeP2FaceTable() {  // the positions of the nodes themselves last, as above
   P2FaceTable t{};
   for (int f = 0; f < 4; ++f) {
-    int n = 0;
-    // node 0 has odd (s, t): its class, and that of the others, as in p2FaceEntry
-    for (int z = -2; z <= 3; ++z)
-      for (int y = -2; y <= 3; ++y)
-        for (int x = -4; x <= 3; ++x) {
-          bool first = true;
-          for (int i = 0; i < 4; ++i) {
-            const int s = 1 + (i & 1), u = 1 + (i >> 1);  // parities of (s, t)
-            int pc = 0;
-            if (f == 0) pc = (s & 1) | ((u & 1) << 1);
-            if (f == 1) pc = (s & 1) | ((u & 1) << 2);
-            if (f == 2) pc = ((s & 1) << 1) | ((u & 1) << 2);
-            if (f == 3) pc = ((s + u) & 1) | ((s & 1) << 1) | ((u & 1) << 2);
-            int k = 4 * f;
-            while (p2s::kFaceClass[k] != pc) ++k;
-            for (int e = 0; e < p2s::kFaceLen[k]; ++e)
-              if (p2FaceNode(f, i, 0) + p2s::kFaceOff[k][e][0] == x && p2FaceNode(f, i, 1) + p2s::kFaceOff[k][e][1] == y &&
-                  p2FaceNode(f, i, 2) + p2s::kFaceOff[k][e][2] == z) {
+    int n = 0, done[4] = {};
+    // node 0 has odd (s, t): its class, and that of the others, as in p2ClosureEntry
+    for (const bool own : {false, true})
+      for (int z = -2; z <= 3; ++z)
+        for (int y = -2; y <= 3; ++y)
+          for (int x = -4; x <= 3; ++x) {
+            bool node = false, first = true;
+            for (int i = 0; i < 4; ++i)
+              node = node || (p2FaceNode(f, i, 0) == x && p2FaceNode(f, i, 1) == y && p2FaceNode(f, i, 2) == z);
+            if (node != own) continue;
+            for (int i = 0; i < 4; ++i) {
+              const int s = 1 + (i & 1), u = 1 + (i >> 1);  // parities of (s, t)
+              int pc = 0;
+              if (f == 0) pc = (s & 1) | ((u & 1) << 1);
+              if (f == 1) pc = (s & 1) | ((u & 1) << 2);
+              if (f == 2) pc = ((s & 1) << 1) | ((u & 1) << 2);
+              if (f == 3) pc = ((s + u) & 1) | ((s & 1) << 1) | ((u & 1) << 2);
+              int k = 4 * f;
+              while (p2s::kFaceClass[k] != pc) ++k;
+              for (int e = 0; e < p2s::kFaceLen[k]; ++e) {
+                const auto& o = p2s::kFaceOff[k][e];
+                if (p2FaceNode(f, i, 0) + o[0] != x || p2FaceNode(f, i, 1) + o[1] != y || p2FaceNode(f, i, 2) + o[2] != z)
+                  continue;
                 P2FaceEntry& q = t.e[f][n++];
                 q.x = (signed char)x;
                 q.y = (signed char)y;
                 q.z = (signed char)z;
                 q.node = (unsigned char)i;
+                q.part = (unsigned char)(2 * done[i]++ / p2s::kFaceLen[k]);
                 q.first = first;
                 q.weight = (short)(p2s::kFaceFirst[k] + e);
                 first = false;
               }
+            }
           }
-        }
   }
   return t;
 }
@@ -180,7 +214,7 @@ __device__ __forceinline__ int p2Row(int w, int Y, int Z) { return int(tetSize(w
 
 template <class T, int F, int E>
 __device__ __forceinline__ void p2FaceBlockEntry(const T* __restrict__ u, const T* __restrict__ fw, int w, int last, int X,
-                                                 int Y, int Z, const int (&pbz)[6], T& v, T (&acc)[4]) {
+                                                 int Y, int Z, const int (&pbz)[6], T& v, T (&acc)[4][2]) {
   constexpr P2FaceEntry q = kP2Face.e[F][E];
   if constexpr (q.first) {
     // a partly empty block at the face's far side also walks over positions outside the cell: the
@@ -188,7 +222,7 @@ __device__ __forceinline__ void p2FaceBlockEntry(const T* __restrict__ u, const 
     const int i = pbz[q.z + 2] + rowStart(w - Z - q.z, Y + q.y) + X + q.x;
     v = __ldg(u + min(unsigned(i), unsigned(last)));
   }
-  acc[q.node] += __ldg(fw + q.weight) * v;
+  acc[q.node][q.part] += __ldg(fw + q.weight) * v;
 }
 
 template <class T, int F, int... E>
@@ -202,12 +236,13 @@ __device__ __forceinline__ void p2FaceBlock(std::integer_sequence<int, E...>, co
     pbz[k] = z >= 0 && z <= M ? int(tetSize(w) - tetSize(w - z)) : 0;
   }
   const int last = int(tetSize(w)) - 1;
-  T acc[4] = {T(0), T(0), T(0), T(0)}, v = T(0);
+  T acc[4][2] = {}, v = T(0);
   (p2FaceBlockEntry<T, F, E>(u, fw, w, last, X, Y, Z, pbz, v, acc), ...);
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const int a = i & 1, b = i >> 1;
-    if (s + a + t + b <= M - 1) d[p2Row(w, Y + p2FaceNode(F, i, 1), Z + p2FaceNode(F, i, 2)) + X + p2FaceNode(F, i, 0)] = acc[i];
+    if (s + a + t + b <= M - 1)
+      d[p2Row(w, Y + p2FaceNode(F, i, 1), Z + p2FaceNode(F, i, 2)) + X + p2FaceNode(F, i, 0)] = acc[i][0] + acc[i][1];
   }
 }
 
@@ -296,7 +331,9 @@ __global__ void __launch_bounds__(kBlock, 2) p2ApplyKernel(LevelDev lv, const P2
         for (int a = 0; a < 2; ++a)
           if (X + a + y + z <= M - 1) {
             const int i = a + 2 * k;
-            const T s = i < 7 ? acc[b][i] : (acc[b][7] + acc[b][8]) + (acc[b][9] + acc[b][10]);
+            const T s = i == 7        ? (acc[b][7] + acc[b][8]) + (acc[b][9] + acc[b][10])
+                        : p2Halves(i) ? acc[b][i] + acc[b][p2Second(i)]
+                                      : acc[b][i];
             d[g + a] = MODE == MODE_RESIDUAL ? rhs[base + g + a] - s : s;
           }
       }
