@@ -1,8 +1,7 @@
 """P2 Laplace apply and residual on the device against the oracle's globally assembled P2
 matrix (48-tet cube, P2 levels 0-4 = vertex lattices 1-5; 3x3x3 cube for coarse levels with
 inner DoFs on every primitive kind). From lattice 8 per macro-cell on, every parity class has
-interior nodes, which take the constant-stencil kernels; the closure nodes take the element
-gather.
+interior nodes; these and the closure nodes are rows of constant stencils.
 
 Tolerances: 1e-13 relative in FP64 and 2e-5 in FP32 (max-norm over inner DoFs); Dirichlet DoFs
 are not written."""
