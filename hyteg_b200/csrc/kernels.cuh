@@ -20,9 +20,13 @@ namespace dev {
 constexpr int kBlock = 256;
 
 // Start of a kernel that is launched while its predecessor on the stream may still run (launchNext):
-// lets its own successor be set up, then waits until every predecessor has finished and its writes
-// are visible. The pointers are those to data that earlier kernels write; passing them through here
-// keeps the compiler from moving loads of read-only data in front of the wait.
+// waits until every predecessor has finished and its writes are visible, then lets its own successor be
+// set up. Behind the wait at most one kernel of a stream is set up ahead; with the trigger first a third
+// and a fourth could be, and their blocks held SMs that other streams' kernels could have used. Eight
+// workers serving 1000 solves, each on its stream: 0.176 GDoF/s with the trigger first, 0.213 behind
+// the wait; alone, V(3,3) at P2 level 5 on 48 cells takes 3.76 and 3.63 ms, the mixed-precision solve on
+// 27 cubes 10.41 and 10.16. The pointers are those to data that earlier kernels write; passing them
+// through here keeps the compiler from moving loads of read-only data in front of the wait.
 template <class P>
 __device__ __forceinline__ void heldBack(P& p) {
   asm volatile("" : "+l"(p)::"memory");
@@ -30,8 +34,8 @@ __device__ __forceinline__ void heldBack(P& p) {
 }
 template <class... P>
 __device__ __forceinline__ void waitForPredecessor(P&... p) {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   (heldBack(p), ...);
 }
 
