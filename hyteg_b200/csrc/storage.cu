@@ -1972,6 +1972,31 @@ void Storage::stokesApply(int opId, const int u[3], int p, const int v[3], int q
   for (int k = 0; k < 3; ++k) argCheck(fn(u[k]).prec == prec && fn(v[k]).prec == prec, "Stokes: precision mismatch");
   argCheck(fn(q).prec == prec, "Stokes: precision mismatch");
   for (int k = 0; k < 3; ++k) argCheck(u[k] != v[k], "P2 apply: distinct functions required");
+  // One launch per block needs the velocity block's shares in the closure slots of v until they are
+  // summed: a function that is v of one component and u or v of another takes the blocks one by one, each
+  // complete before the next reads or writes it.
+  bool shared = false;
+  for (int j = 0; j < 3; ++j)
+    for (int k = 0; k < 3; ++k) shared = shared || (j != k && (u[j] == v[k] || v[j] == v[k]));
+  if (shared) {
+    for (int k = 0; k < 3; ++k) p2Apply(opId, u[k], v[k], -1, L, maskV, 0);
+    int t[3] = {-1, -1, -1};
+    try {
+      for (int& id : t) id = createFunction(L + 1, L + 1, prec);
+      stokesDivT(opId, p, t, L, maskV);
+      const double one = 1.0;
+      for (int k = 0; k < 3; ++k) {
+        lincomb(v[k], L + 1, maskV, 1, &one, &t[k], true, 0.0);
+        communicate(v[k], L + 1, kAllGroups);
+      }
+    } catch (...) {
+      for (int id : t) fns.erase(id);
+      throw;
+    }
+    for (int id : t) fns.erase(id);
+    stokesDiv(opId, u, q, L, maskP);
+    return;
+  }
   if (prec == 8)
     stokesApplyT<double>(o, u, p, v, q, L, maskV, maskP);
   else

@@ -62,6 +62,41 @@ def test_stokes_apply(env, L):
     assert rel(gq, qr, np.ones(np_, dtype=bool)) < 1e-13
 
 
+@pytest.mark.parametrize("order", [(1, 2, 0), (2, 0, 1)])
+def test_stokes_apply_with_shared_components(env, order):
+    """Outputs that are inputs of other components: the velocity block component by component, then the
+    gradient added, then the divergence of what the inputs hold by then."""
+    st, orc, maps = env
+    L = LMAX
+    S, A = hg.P2P1TaylorHoodStokesOperator(st, 0, LMAX), hg.P2ConstantLaplaceOperator(st, 0, LMAX)
+
+    def inputs():
+        u, p = funcs(st)
+        for k in range(3):
+            u[k].fill_random(80 + k, L)
+            u[k].communicate(L)
+        p.fill_random(90, L)
+        return u, p
+
+    u, p = inputs()
+    q = hg.P1Function("q", st, 0, LMAX)
+    S.apply(u, p, [u[k] for k in order], q, L)
+    w, p = inputs()
+    zero, none = funcs(st)
+    grad, div = funcs(st)
+    for k in range(3):
+        A.apply(w[k], w[order[k]], L, hg.Inner | hg.NeumannBoundary)
+    S.apply(zero, p, grad, div, L)  # the gradient alone
+    for k in range(3):
+        w[order[k]].v.add([1.0], [grad[k].v], L + 1, hg.Inner | hg.NeumannBoundary)
+        w[order[k]].communicate(L)
+    S.apply(w, none, grad, div, L)  # the divergence alone
+    owned = maps[L + 1][1] >= 0
+    for k in range(3):
+        assert rel(u[k].to_numpy(L), w[k].to_numpy(L), owned) < 1e-13
+    assert rel(q.to_numpy(L), div.to_numpy(L), maps[L][1] >= 0) < 1e-13
+
+
 def dense_lid_solution(orc, L):
     nv, np_ = orc.n(L + 1), orc.n(L)
     xyz = orc.nodes(L + 1)[0]
