@@ -365,7 +365,7 @@ constexpr size_t kCompactSmem = 224 << 10;  // shared memory the vectors and row
 int batchKind(int kind) { return kind == KC ? 0 : kind == KF ? 1 : kind == KE ? 2 : 3; }
 
 // Directions of the coarse micro-edge a fine point bisects, by the parity code x | y << 1 | z << 2
-// of its cell-local coordinates (the convention of cellProlongKernel).
+// of its cell-local coordinates (the convention of the level prolongation).
 const int kBisectDir[8][3] = {{0, 0, 0}, {1, 0, 0}, {0, 1, 0}, {-1, 1, 0}, {0, 0, 1}, {-1, 0, 1}, {0, -1, 1}, {-1, 1, -1}};
 
 struct Dof {

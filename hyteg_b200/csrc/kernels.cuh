@@ -768,11 +768,6 @@ __device__ __forceinline__ void cellStrip(const LevelDev& lv, const StripItem it
   }
 }
 
-__device__ __forceinline__ int cellIndexDev(int w, int x, int y, int z) {
-  const int W = w - z;
-  return int(tetSize(w) - tetSize(W)) + rowStart(W, y) + x;
-}
-
 // Full-weighting restriction at coarse cell-interior points: coarse = fine[2p] + 1/2 sum fine[2p+d]
 // (restrict_3D_macrocell_P1_pull_additive.cpp; on interior points every weight is 1 or 1/2). Plane z
 // of macro-cell c.
@@ -1051,8 +1046,8 @@ __global__ void __launch_bounds__(kBlock) vertexSorPhaseKernel(LevelDev lv, Sten
 // lanes each. A row has at most N / 3 points of a colour, which leaves two thirds of 32 lanes idle at
 // N = 32: there four rows. On larger faces FP32 still gains from them (V(3,3) on level 7, 48 cells:
 // 3.76 ms with four rows, 3.88 with one), FP64 loses (sweep on level 7 884 us with one, 898 with four).
-// The phase is bound by latency: a block has no more threads than the face has rows for, so that small
-// faces share an SM (27 cubes, level 5, 378 faces: 18 us with 1024 threads, 10 with 256).
+// The phase is bound by latency: at N = 32 and 64 a block has no more threads than the face has rows for,
+// so that small faces share an SM (27 cubes, level 5, 378 faces: 18 us with 1024 threads, 10 with 256).
 constexpr int kFacePhaseThreads = 1024;
 inline int facePhaseThreads(int N) { return N <= 32 ? 256 : N <= 64 ? 512 : kFacePhaseThreads; }
 template <class T>

@@ -702,8 +702,9 @@ void P2Gmg::coarseSolve(int x, int b, int L) {
   }
   const unsigned flag = HG_INNER | HG_NEUMANN | HG_FREESLIP;
   s.p2Apply(op, x, cr, b, L, flag, 2);
-  launchNext(s.stream, dev::denseCorrectKernel, (coarseN + dev::kBlock - 1) / dev::kBlock, dev::kBlock, (size_t)coarseN * 8, (const int64_t*)coarseIdx->p, coarseN, (const double*)coarseInv->p, (const double*)s.data(cr, L + 1),
-      (double*)s.data(x, L + 1));
+  launchNext(s.stream, dev::denseCorrectKernel, (coarseN + dev::kBlock - 1) / dev::kBlock, dev::kBlock,
+             (size_t)coarseN * 8, (const int64_t*)coarseIdx->p, coarseN, (const double*)coarseInv->p,
+             (const double*)s.data(cr, L + 1), (double*)s.data(x, L + 1));
   ++s.launches;
   cudaCheck(cudaGetLastError(), "coarse solve");
   s.communicate(x, L + 1, (1 << G_COUNT) - 1);

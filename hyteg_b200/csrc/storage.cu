@@ -265,7 +265,6 @@ void Storage::buildLevel(int L) {
     for (int64_t s = 0; s < size; s += 8192) chunks.push_back({off + s, (int)std::min<int64_t>(8192, size - s), type});
   };
   for (int c = 0; c < lv.nCells; ++c) addChunks(lay.off[KC][c], lay.size[KC][c], cellType[c]);
-  ld.nCellChunks = (int)chunks.size();
   for (int f = 0; f < lv.nFaces; ++f) addChunks(lay.off[KF][f], lay.size[KF][f], faceType[f]);
   for (int e = 0; e < lv.nEdges; ++e) addChunks(lay.off[KE][e], lay.size[KE][e], lowType[e]);
   for (size_t v = 0; v < topo.verts.size(); ++v) addChunks(lay.off[KV][v], lay.size[KV][v], lowType[lv.nEdges + v]);
@@ -459,11 +458,11 @@ void Storage::cgUpdate(int L, unsigned mask, bool direction, const double* num, 
     using T = decltype(zero);
     T *xd = direction ? nullptr : (T*)data(x, L), *ad = direction ? nullptr : (T*)data(ap, L);
     if (direction)
-      launchNext(stream, dev::cgUpdateKernel<T, true>, ld.nChunks, dev::kBlock, 0, ld.chunks, mask, num, den, xd, (T*)data(r, L),
-                                                                           (T*)data(p, L), ad);
+      launchNext(stream, dev::cgUpdateKernel<T, true>, ld.nChunks, dev::kBlock, 0, ld.chunks, mask, num, den, xd,
+                 (T*)data(r, L), (T*)data(p, L), ad);
     else
-      launchNext(stream, dev::cgUpdateKernel<T, false>, ld.nChunks, dev::kBlock, 0, ld.chunks, mask, num, den, xd, (T*)data(r, L),
-                                                                            (T*)data(p, L), ad);
+      launchNext(stream, dev::cgUpdateKernel<T, false>, ld.nChunks, dev::kBlock, 0, ld.chunks, mask, num, den, xd,
+                 (T*)data(r, L), (T*)data(p, L), ad);
   };
   if (fn(r).prec == 8) run(0.0);
   else run(0.0f);
@@ -709,8 +708,9 @@ void Storage::lincomb(int dst, int L, unsigned mask, int n, const double* a, con
   auto run = [&](auto zero) {
     using T = decltype(zero);
     auto go = [&](auto nsrc, auto addTo) {
-      launchNext(stream, dev::lincombKernel<T, decltype(nsrc)::value, decltype(addTo)::value>, ld.nChunks, dev::kBlock, 0, ld.chunks, mask, (T*)pd, (const T*)ps[0], (const T*)ps[1], (const T*)ps[2], T(sc[0]), T(sc[1]), T(sc[2]),
-          T(constant));
+      launchNext(stream, dev::lincombKernel<T, decltype(nsrc)::value, decltype(addTo)::value>, ld.nChunks,
+                 dev::kBlock, 0, ld.chunks, mask, (T*)pd, (const T*)ps[0], (const T*)ps[1], (const T*)ps[2], T(sc[0]),
+                 T(sc[1]), T(sc[2]), T(constant));
     };
     auto pick = [&](auto nsrc) {
       if (add) go(nsrc, std::true_type{});
@@ -746,13 +746,17 @@ void Storage::copyCast(int dst, int src, int L, unsigned mask, bool add) {
   if (ld.nChunks == 0) return;
   const int a = add ? 1 : 0;
   if (fd.prec == 8 && fs.prec == 8)
-    launchNext(stream, dev::castKernel<double, double>, ld.nChunks, dev::kBlock, 0, ld.chunks, mask, (double*)pd, (const double*)ps, a);
+    launchNext(stream, dev::castKernel<double, double>, ld.nChunks, dev::kBlock, 0, ld.chunks, mask, (double*)pd,
+               (const double*)ps, a);
   else if (fd.prec == 8)
-    launchNext(stream, dev::castKernel<double, float>, ld.nChunks, dev::kBlock, 0, ld.chunks, mask, (double*)pd, (const float*)ps, a);
+    launchNext(stream, dev::castKernel<double, float>, ld.nChunks, dev::kBlock, 0, ld.chunks, mask, (double*)pd,
+               (const float*)ps, a);
   else if (fs.prec == 8)
-    launchNext(stream, dev::castKernel<float, double>, ld.nChunks, dev::kBlock, 0, ld.chunks, mask, (float*)pd, (const double*)ps, a);
+    launchNext(stream, dev::castKernel<float, double>, ld.nChunks, dev::kBlock, 0, ld.chunks, mask, (float*)pd,
+               (const double*)ps, a);
   else
-    launchNext(stream, dev::castKernel<float, float>, ld.nChunks, dev::kBlock, 0, ld.chunks, mask, (float*)pd, (const float*)ps, a);
+    launchNext(stream, dev::castKernel<float, float>, ld.nChunks, dev::kBlock, 0, ld.chunks, mask, (float*)pd,
+               (const float*)ps, a);
   ++launches;
   cudaCheck(cudaGetLastError(), "copyCast");
 }
@@ -765,10 +769,10 @@ void Storage::dotAsync(int a, int b, int L, unsigned mask, double* dOut) {
   double* partial = (double*)ld.partial.p;
   if (fa.prec == 8)
     launchNext(stream, dev::dotReduceKernel<double>, nb, dev::kBlock, 0, ld.lv, (const double*)data(a, L),
-                                                                 (const double*)data(b, L), mask, partial, ld.arrived, dOut);
+               (const double*)data(b, L), mask, partial, ld.arrived, dOut);
   else
-    launchNext(stream, dev::dotReduceKernel<float>, nb, dev::kBlock, 0, ld.lv, (const float*)data(a, L), (const float*)data(b, L),
-                                                                mask, partial, ld.arrived, dOut);
+    launchNext(stream, dev::dotReduceKernel<float>, nb, dev::kBlock, 0, ld.lv, (const float*)data(a, L),
+               (const float*)data(b, L), mask, partial, ld.arrived, dOut);
   ++launches;
   cudaCheck(cudaGetLastError(), "dot");
 }
@@ -1304,8 +1308,7 @@ P2Additive& Storage::p2Additive(int Lf) {
     const std::vector<unsigned> cp32(cp.begin(), cp.end());
     put(ad.sorOwners, owners.data(), owners.size() * sizeof(dev::P2Owner));
     put(ad.sorCopies, cp32.data(), cp32.size() * sizeof(unsigned));
-    // interior nodes by class
-    argCheck(M <= 1024, "P2 smoother: lattice too large");
+    // interior nodes by class (ten bits a coordinate: the levels of a storage end at lattice 1024)
     std::vector<unsigned> inner(dev::kP2NodeHead);
     for (int pc = 0; pc < 8; ++pc) {
       inner[(size_t)pc] = (unsigned)inner.size();
@@ -1433,8 +1436,9 @@ static std::vector<double> p2FaceStencils(const std::vector<double>& K, int nCel
 template <class T, int MODE>
 void Storage::p2AddOwners(const P2Additive& ad, T* dst, const T* rhs, unsigned mask) {
   if (!ad.n) return;
-  launchNext(stream, dev::p2AddKernel<T, MODE>, (ad.n + dev::kBlock - 1) / dev::kBlock, dev::kBlock, 0, (const int64_t*)ad.owner.p, (const int*)ad.ptr.p, (const int64_t*)ad.copies.p, (const unsigned char*)ad.type.p,
-      ad.n, dst, rhs, mask);
+  launchNext(stream, dev::p2AddKernel<T, MODE>, (ad.n + dev::kBlock - 1) / dev::kBlock, dev::kBlock, 0,
+             (const int64_t*)ad.owner.p, (const int*)ad.ptr.p, (const int64_t*)ad.copies.p,
+             (const unsigned char*)ad.type.p, ad.n, dst, rhs, mask);
   ++launches;
 }
 
@@ -1447,7 +1451,8 @@ void Storage::p2Sweep(P2Operator& o, int L, T* dst, const T* src, const T* rhs, 
   P2Additive& ad = p2Additive(Lf);
   const T* W = (const T*)(sizeof(T) == 8 ? o.sd[L - o.minL]->p : o.sf[L - o.minL]->p);
   const T* FW = (const T*)(sizeof(T) == 8 ? o.fd[L - o.minL]->p : o.ff[L - o.minL]->p);
-  launchNext(stream, dev::p2ApplyKernel<T, MODE>, ld.lv.nCells * ad.nItems, dev::kBlock, dev::p2TileSmem<T>(), ld.lv, (const dev::P2Item*)ad.items.p, W, FW, dst, src, rhs, mask);
+  launchNext(stream, dev::p2ApplyKernel<T, MODE>, ld.lv.nCells * ad.nItems, dev::kBlock, dev::p2TileSmem<T>(), ld.lv,
+             (const dev::P2Item*)ad.items.p, W, FW, dst, src, rhs, mask);
   ++launches;
   cudaCheck(cudaGetLastError(), "P2 kernels");
 }
@@ -1539,14 +1544,16 @@ void Storage::p2SorT(P2Operator& o, int opId, int x, int b, int L, unsigned mask
     const int nOwn = ad.sorOwnerBegin[c + 1] - ad.sorOwnerBegin[c], ownBlocks = blocks(nOwn);
     const int inner = ld.lv.nCells * chunks;
     if (listBlocks + inner > 0) {
-      launchNext(stream, dev::p2SorGatherKernel<T>, listBlocks + inner, dev::kBlock, 0, ld.lv, W, FW, (const dev::P2ClosureNode*)ad.closureList.p + ad.closureBegin[c], nList, listBlocks,
-          (const unsigned*)ad.sorInner.p, cells, c, std::max(chunks, 1), xd, bd, axd, mask, omega);
+      launchNext(stream, dev::p2SorGatherKernel<T>, listBlocks + inner, dev::kBlock, 0, ld.lv, W, FW,
+                 (const dev::P2ClosureNode*)ad.closureList.p + ad.closureBegin[c], nList, listBlocks,
+                 (const unsigned*)ad.sorInner.p, cells, c, std::max(chunks, 1), xd, bd, axd, mask, omega);
       ++launches;
     }
     if (ownBlocks + inner > 0) {
-      launchNext(stream, dev::p2SorUpdateKernel<T>, ownBlocks + inner, dev::kBlock, 0, ld.lv, (const dev::P2Owner*)ad.sorOwners.p + ad.sorOwnerBegin[c], nOwn, ownBlocks,
-          (const unsigned*)ad.sorCopies.p, (const unsigned*)ad.sorInner.p, cells, c, std::max(chunks, 1), xd, bd, axd,
-          (const T*)data(dg, Lf), mask, omega);
+      launchNext(stream, dev::p2SorUpdateKernel<T>, ownBlocks + inner, dev::kBlock, 0, ld.lv,
+                 (const dev::P2Owner*)ad.sorOwners.p + ad.sorOwnerBegin[c], nOwn, ownBlocks,
+                 (const unsigned*)ad.sorCopies.p, (const unsigned*)ad.sorInner.p, cells, c, std::max(chunks, 1), xd,
+                 bd, axd, (const T*)data(dg, Lf), mask, omega);
       ++launches;
     }
   }
@@ -1705,19 +1712,19 @@ void Storage::p2Prolongate(int id, int Lc, unsigned mask, bool add) {
   const dev::P2TransferDev tr{(const unsigned char*)p2tr.nCand.p, (const unsigned char*)p2tr.cand.p};
   const int nb = lf.lv.nCells * (lf.lv.N + 1), na = (ad.n + dev::kBlock - 1) / dev::kBlock;
   if (f.prec == 8) {
-    launchNext(stream, dev::p2ProlongKernel<double>, nb, dev::kBlock, 0, lc.lv, lf.lv, p2TablesOnce(), tr, (const double*)p2tr.wd.p,
-                                                               (const double*)data(id, Lcf), (double*)data(out, Lff));
+    launchNext(stream, dev::p2ProlongKernel<double>, nb, dev::kBlock, 0, lc.lv, lf.lv, p2TablesOnce(), tr,
+               (const double*)p2tr.wd.p, (const double*)data(id, Lcf), (double*)data(out, Lff));
     if (ad.n)
-      launchNext(stream, dev::p2PickKernel<double>, na, dev::kBlock, 0, (const int64_t*)ad.owner.p, (const int*)ad.ptr.p,
-                                                              (const int64_t*)ad.copies.p, (const unsigned char*)ad.type.p,
-                                                              ad.n, (double*)data(out, Lff), add ? HG_ALL : mask);
+      launchNext(stream, dev::p2PickKernel<double>, na, dev::kBlock, 0, (const int64_t*)ad.owner.p,
+                 (const int*)ad.ptr.p, (const int64_t*)ad.copies.p, (const unsigned char*)ad.type.p, ad.n,
+                 (double*)data(out, Lff), add ? HG_ALL : mask);
   } else {
-    launchNext(stream, dev::p2ProlongKernel<float>, nb, dev::kBlock, 0, lc.lv, lf.lv, p2TablesOnce(), tr, (const float*)p2tr.wf.p,
-                                                              (const float*)data(id, Lcf), (float*)data(out, Lff));
+    launchNext(stream, dev::p2ProlongKernel<float>, nb, dev::kBlock, 0, lc.lv, lf.lv, p2TablesOnce(), tr,
+               (const float*)p2tr.wf.p, (const float*)data(id, Lcf), (float*)data(out, Lff));
     if (ad.n)
-      launchNext(stream, dev::p2PickKernel<float>, na, dev::kBlock, 0, (const int64_t*)ad.owner.p, (const int*)ad.ptr.p,
-                                                             (const int64_t*)ad.copies.p, (const unsigned char*)ad.type.p,
-                                                             ad.n, (float*)data(out, Lff), add ? HG_ALL : mask);
+      launchNext(stream, dev::p2PickKernel<float>, na, dev::kBlock, 0, (const int64_t*)ad.owner.p,
+                 (const int*)ad.ptr.p, (const int64_t*)ad.copies.p, (const unsigned char*)ad.type.p, ad.n,
+                 (float*)data(out, Lff), add ? HG_ALL : mask);
   }
   launches += ad.n ? 2 : 1;
   cudaCheck(cudaGetLastError(), "P2 prolongation");
@@ -1743,19 +1750,21 @@ void Storage::p2Restrict(int id, int Lf, unsigned mask) {
   const int bpc = (gt.nCoarse + dev::kBlock - 1) / dev::kBlock;
   const int nb = lf.lv.nCells * bpc, na = (adc.n + dev::kBlock - 1) / dev::kBlock;
   if (f.prec == 8) {
-    launchNext(stream, dev::p2RestrictGatherKernel<double>, nb, dev::kBlock, 0, lc.lv, lf.lv, (const int*)gt.ptr.p, (const int*)gt.idx.p, (const double*)gt.wd.p, gt.nCoarse, bpc,
-        (const double*)data(id, Lff),
-        (const unsigned char*)adf.mult.p, (double*)data(id, Lcf));
+    launchNext(stream, dev::p2RestrictGatherKernel<double>, nb, dev::kBlock, 0, lc.lv, lf.lv, (const int*)gt.ptr.p,
+               (const int*)gt.idx.p, (const double*)gt.wd.p, gt.nCoarse, bpc, (const double*)data(id, Lff),
+               (const unsigned char*)adf.mult.p, (double*)data(id, Lcf));
     if (adc.n)
-      launchNext(stream, dev::p2AddKernel<double, dev::MODE_REPLACE>, na, dev::kBlock, 0, (const int64_t*)adc.owner.p, (const int*)adc.ptr.p, (const int64_t*)adc.copies.p,
-          (const unsigned char*)adc.type.p, adc.n, (double*)data(id, Lcf), nullptr, mask);
+      launchNext(stream, dev::p2AddKernel<double, dev::MODE_REPLACE>, na, dev::kBlock, 0, (const int64_t*)adc.owner.p,
+                 (const int*)adc.ptr.p, (const int64_t*)adc.copies.p, (const unsigned char*)adc.type.p, adc.n,
+                 (double*)data(id, Lcf), nullptr, mask);
   } else {
-    launchNext(stream, dev::p2RestrictGatherKernel<float>, nb, dev::kBlock, 0, lc.lv, lf.lv, (const int*)gt.ptr.p, (const int*)gt.idx.p, (const float*)gt.wf.p, gt.nCoarse, bpc,
-        (const float*)data(id, Lff),
-        (const unsigned char*)adf.mult.p, (float*)data(id, Lcf));
+    launchNext(stream, dev::p2RestrictGatherKernel<float>, nb, dev::kBlock, 0, lc.lv, lf.lv, (const int*)gt.ptr.p,
+               (const int*)gt.idx.p, (const float*)gt.wf.p, gt.nCoarse, bpc, (const float*)data(id, Lff),
+               (const unsigned char*)adf.mult.p, (float*)data(id, Lcf));
     if (adc.n)
-      launchNext(stream, dev::p2AddKernel<float, dev::MODE_REPLACE>, na, dev::kBlock, 0, (const int64_t*)adc.owner.p, (const int*)adc.ptr.p, (const int64_t*)adc.copies.p,
-          (const unsigned char*)adc.type.p, adc.n, (float*)data(id, Lcf), nullptr, mask);
+      launchNext(stream, dev::p2AddKernel<float, dev::MODE_REPLACE>, na, dev::kBlock, 0, (const int64_t*)adc.owner.p,
+                 (const int*)adc.ptr.p, (const int64_t*)adc.copies.p, (const unsigned char*)adc.type.p, adc.n,
+                 (float*)data(id, Lcf), nullptr, mask);
   }
   launches += adc.n ? 2 : 1;
   cudaCheck(cudaGetLastError(), "P2 restriction");
@@ -1855,8 +1864,9 @@ static void launchDivT(Storage& st, P2Operator& o, int p, const int v[3], int L,
   const T* WC = (const T*)(sizeof(T) == 8 ? o.wdivtcd[L - o.minL]->p : o.wdivtcf[L - o.minL]->p);
   const int nList = adv.closureBegin[11], listBlocks = (nList + dev::kBlock - 1) / dev::kBlock;
   const int inner = lvv.lv.N >= 4 ? lvv.lv.nCells * (lvv.lv.N - 3) : 0;
-  launchNext(st.stream, dev::p2DivTKernel<T, ADD>, listBlocks + inner, dev::kBlock, 0, lvv.lv, lvp.lv, WT, WC, (const dev::P2ClosureNode*)adv.closureList.p, nList, listBlocks, (T*)st.data(v[0], Lv),
-      (T*)st.data(v[1], Lv), (T*)st.data(v[2], Lv), (const T*)st.data(p, Lp), maskV);
+  launchNext(st.stream, dev::p2DivTKernel<T, ADD>, listBlocks + inner, dev::kBlock, 0, lvv.lv, lvp.lv, WT, WC,
+             (const dev::P2ClosureNode*)adv.closureList.p, nList, listBlocks, (T*)st.data(v[0], Lv),
+             (T*)st.data(v[1], Lv), (T*)st.data(v[2], Lv), (const T*)st.data(p, Lp), maskV);
   ++st.launches;
 }
 
@@ -1872,8 +1882,9 @@ static void launchDiv(Storage& st, P2Operator& o, const int u[3], int q, int L, 
   const T* WC = (const T*)(sizeof(T) == 8 ? o.wdivcd[L - o.minL]->p : o.wdivcf[L - o.minL]->p);
   const int nList = adp.closureBegin[11], listBlocks = (nList + dev::kBlock - 1) / dev::kBlock;
   const int inner = lvp.lv.N >= 4 ? lvp.lv.nCells * (lvp.lv.N - 3) : 0;
-  launchNext(st.stream, dev::p2DivKernel<T>, listBlocks + inner, dev::kBlock, 0, lvp.lv, lvv.lv, WD, WC, (const dev::P2ClosureNode*)adp.closureList.p, nList, listBlocks, (T*)st.data(q, Lp),
-      (const T*)st.data(u[0], Lv), (const T*)st.data(u[1], Lv), (const T*)st.data(u[2], Lv), maskP);
+  launchNext(st.stream, dev::p2DivKernel<T>, listBlocks + inner, dev::kBlock, 0, lvp.lv, lvv.lv, WD, WC,
+             (const dev::P2ClosureNode*)adp.closureList.p, nList, listBlocks, (T*)st.data(q, Lp),
+             (const T*)st.data(u[0], Lv), (const T*)st.data(u[1], Lv), (const T*)st.data(u[2], Lv), maskP);
   ++st.launches;
   st.p2AddOwners<T, dev::MODE_REPLACE>(adp, (T*)st.data(q, Lp), nullptr, maskP);
   cudaCheck(cudaGetLastError(), "Stokes div");
@@ -2145,7 +2156,8 @@ void Storage::stencilOp(Operator& o, int L, T* dst, const T* src, const T* rhs, 
   const int nCell = kinds & (1 << KC) ? ld.nTiles : 0, nFace = kinds & (1 << KF) ? ld.lv.nFaceBands : 0;
   const int nLow = (edges ? ld.lv.nLowEdgeBlocks : 0) + (verts ? nVertBlocks : 0);
   if (nCell + nFace + nLow == 0) return;
-  launchNext(stream, dev::levelStencilKernel<T, MODE>, nLow + nFace + nCell, dev::kLevelThreads, 0, ld.lv, st, ld.tiles, nLow, edges ? 0 : ld.lv.nLowEdgeBlocks, nFace, dst, src, rhs, mask);
+  launchNext(stream, dev::levelStencilKernel<T, MODE>, nLow + nFace + nCell, dev::kLevelThreads, 0, ld.lv, st,
+             ld.tiles, nLow, edges ? 0 : ld.lv.nLowEdgeBlocks, nFace, dst, src, rhs, mask);
   ++launches;
   cudaCheck(cudaGetLastError(), "stencil kernel");
 }
@@ -2222,7 +2234,8 @@ void Storage::sorT(Operator& o, int dstId, int L, T* u, const T* rhs, unsigned m
         const int c = rev ? 3 - k : k, n = ld.nSplitPoints[c];
         if (n == 0) continue;
         const int bpc = (n + dev::kBlock - 1) / dev::kBlock;
-        launchNext(stream, dev::cellSorSplitKernel<T>, (unsigned)(bpc * lv.nCells), dev::kBlock, 0, lv, st.cellW, cellU, cellF, mask, ld.splitRows[c], ld.splitPoints[c], n, bpc, omega);
+        launchNext(stream, dev::cellSorSplitKernel<T>, (unsigned)(bpc * lv.nCells), dev::kBlock, 0, lv, st.cellW,
+                   cellU, cellF, mask, ld.splitRows[c], ld.splitPoints[c], n, bpc, omega);
         ++launches;
       }
       return;
@@ -2240,7 +2253,8 @@ void Storage::sorT(Operator& o, int dstId, int L, T* u, const T* rhs, unsigned m
       }
       tb.comm = ld.comm;
       tb.range = refresh ? ld.cellRange : nullptr;
-      launchNext(stream, dev::cellSorResidentKernel<T>, lv.nCells, dev::residentThreads(lv.N), dev::residentSmem<T>(lv.N), lv, st.cellW, u, rhs, mask, tb, omega, rev ? 1 : 0);
+      launchNext(stream, dev::cellSorResidentKernel<T>, lv.nCells, dev::residentThreads(lv.N),
+                 dev::residentSmem<T>(lv.N), lv, st.cellW, u, rhs, mask, tb, omega, rev ? 1 : 0);
       ++launches;
       return;
     }
@@ -2294,13 +2308,16 @@ void Storage::sorT(Operator& o, int dstId, int L, T* u, const T* rhs, unsigned m
     auto lowPhase = [&](bool edgesNotVerts, bool gather, bool rev) {
       const int first = edgesNotVerts ? 0 : lv.nEdges, n = edgesNotVerts ? lv.nEdges : lv.nLow - lv.nEdges;
       if (n == 0 || !(kinds & (1 << (edgesNotVerts ? KE : KV)))) return;
-      launchNext(stream, dev::lowSorPhaseKernel<T>, n, dev::kBlock, 0, lv, st, u, rhs, mask, omega, first, rev ? 1 : 0, table,
-                                                             gather && refresh ? ld.lowRange : nullptr, cellsBuf, cellEnd);
+      launchNext(stream, dev::lowSorPhaseKernel<T>, n, dev::kBlock, 0, lv, st, u, rhs, mask, omega, first,
+                 rev ? 1 : 0, table, gather && refresh ? ld.lowRange : nullptr, cellsBuf, cellEnd);
       ++launches;
     };
     auto facePhase = [&](bool gather, bool rev) {
       if (lv.nFaceBlocks == 0 || !(kinds & (1 << KF))) return;
-      launchNext(stream, dev::facePhaseRows<T>(lv.N) == 4 ? dev::faceSorPhaseKernel<T, 4> : dev::faceSorPhaseKernel<T, 1>, lv.nFaces, dev::facePhaseThreads(lv.N), 0, lv, st, u, rhs, mask, omega, rev ? 1 : 0, table, gather && refresh ? ld.faceRange : nullptr, cellsBuf, cellEnd);
+      launchNext(stream,
+                 dev::facePhaseRows<T>(lv.N) == 4 ? dev::faceSorPhaseKernel<T, 4> : dev::faceSorPhaseKernel<T, 1>,
+                 lv.nFaces, dev::facePhaseThreads(lv.N), 0, lv, st, u, rhs, mask, omega, rev ? 1 : 0, table,
+                 gather && refresh ? ld.faceRange : nullptr, cellsBuf, cellEnd);
       ++launches;
     };
     // vertices, beside the refresh of the edge copies they do not own and of the face ghost layers

@@ -82,7 +82,6 @@ struct LevelData {
   int64_t commEdgeOther = 0;  // the edge copies owned by vertices end here, the others follow
   dev::Chunk* chunks = nullptr;
   int nChunks = 0;
-  int nCellChunks = 0;  // the chunks of the cell arrays come first
   // register-blocked cell sweep: work items grouped by macro-cell groups small enough to stay in L2
   dev::StripItem* tiles = nullptr;
   int nTiles = 0;
