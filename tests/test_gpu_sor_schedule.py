@@ -1,8 +1,10 @@
-"""The single-pass (z-wavefront, double-buffered) multicolour SOR and the colour passes on
-colour-split copies (schedule 3) against the four in-place colour passes and against the oracle,
-at levels where a macro-cell spans several tiles (32 x 24 or 32 x 28, and the shorter 32 x 12
-tiles of schedule 2). Schedule 3 also runs inside multigrid cycles, where the copies are made once
-per smoothing step and the right-hand side's copy is kept from the pre- to the post-smoothing.
+"""The cell phases of the multicolour SOR against one another and against the oracle: the resident
+macro-cells (schedule 0 up to level 5), the single-pass z-wavefront into a second buffer (schedule 0
+from level 6 on, 32 x 24 tiles in FP64, 32 x 28 in FP32; schedule 2 on every level, 32 x 12 tiles),
+the four in-place colour passes (schedule 1) and the colour passes on colour-split copies (schedule 3),
+at levels where a macro-cell spans several tiles. Schedule 3 also runs inside multigrid cycles, where
+the copies are made once per smoothing step and the right-hand side's copy is kept from the pre- to the
+post-smoothing.
 
 Tolerances: FP64 1e-13 relative (max-norm over inner DoFs); FP32 1e-5 relative (the two
 schedules round the relaxation differently)."""
@@ -46,8 +48,8 @@ def cube6():
 @pytest.mark.parametrize("dtype,tol", [(np.float64, 1e-13), (np.float32, 1e-5)])
 @pytest.mark.parametrize("schedule", [0, 2, 3])
 def test_single_pass_equals_colour_passes(cube6, L, backwards, dtype, tol, schedule):
-    # schedule 0: 32 x 24 (FP64) / 32 x 28 (FP32) tiles; schedule 2: 32 x 12 tiles; schedule 3:
-    # colour passes on colour-split copies
+    # schedule 0: resident cells on level 5, wavefront tiles of 32 x 24 (FP64) / 32 x 28 (FP32) on 6;
+    # schedule 2: 32 x 12 tiles; schedule 3: colour passes on colour-split copies
     st, mesh = cube6
     n = st.level_size(L)
     _, owned = mesh.slot_info(L)
@@ -121,6 +123,33 @@ def test_single_pass_matches_oracle_level5(schedule):
     ref = orc.sor(L, u0, f0, 0.9, sweeps=2, multicolour=True)
     inner = ~orc.dirichlet(L)
     assert np.abs(got - ref)[inner].max() / np.abs(ref[inner]).max() < 1e-13
+
+
+@pytest.fixture(scope="module")
+def one_cube6():
+    if hg.device_count() == 0:
+        pytest.skip("no CUDA device")
+    L = 6
+    coords, tets, mesh, orc = H.cube(L, nx=1)
+    xyz, owned = mesh.slot_info(L)
+    return hg.PrimitiveStorage.cuboid((0, 0, 0), (1, 1, 1), 1, 1, 1, L), orc, H.match_slots(xyz, orc.nodes(L)[0]), owned
+
+
+@pytest.mark.parametrize("backwards", [False, True])
+@pytest.mark.parametrize("dtype,tol", [(np.float64, 1e-13), (np.float32, 1e-5)])
+@pytest.mark.parametrize("schedule", [0, 2])
+def test_wavefront_matches_oracle_level6(one_cube6, schedule, dtype, tol, backwards):
+    st, orc, node, owned = one_cube6
+    L, omega = 6, 0.9
+    n = orc.n(L)
+    rng = np.random.default_rng(56)
+    u0, f0 = (rng.uniform(-1, 1, n).astype(dtype) for _ in range(2))
+    x = run_sor(st, L, H.scatter(node, u0).astype(dtype), H.scatter(node, f0).astype(dtype), dtype, schedule, 2, backwards,
+                omega)
+    got = H.gather_owned(x, node, owned, n)
+    ref = orc.sor(L, u0, f0, omega, sweeps=2, multicolour=True, backwards=backwards)
+    inner = ~orc.dirichlet(L)
+    assert np.abs(got - ref)[inner].max() / np.abs(ref[inner]).max() < tol
 
 
 def test_buffer_exchange_and_padding(cube6):
