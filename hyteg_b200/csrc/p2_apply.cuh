@@ -14,7 +14,7 @@
 // 58 KB in FP64) leave two blocks of 256 threads per SM and waste the fewest threads at the sloped
 // face (73 % of a cell's threads update a node at lattice 128, 55 % at 64, 34 % at 32).
 // Measured, 48 cells, P2 level 6 (lattice 128, 16.6 M nodes), FP64, the whole apply with its halo
-// exchanges: 0.707 ms with one launch for rows by parity class and one for the closure, 0.331 ms so.
+// exchanges: 0.707 ms with one launch for rows by parity class and one for the closure, 0.321 ms so.
 #pragma once
 
 #include "kernels.cuh"

@@ -12,7 +12,8 @@
 // left two thirds of the lanes idle at N = 32. Bound by latency and L2 at the sizes met (P2 level 5:
 // velocity vectors of 18 MB).
 // Measured, 48 cells, P2 level 5, FP64: the block apply 0.685 ms with element gathers on the closure,
-// separate interior launches and the gradient in scratch vectors, 0.380 ms so.
+// separate interior launches and the gradient in scratch vectors, 0.380 ms so, 0.357 ms with every launch
+// set up while its predecessor runs.
 #pragma once
 
 #include "kernels.cuh"

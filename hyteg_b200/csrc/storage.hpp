@@ -56,9 +56,9 @@ void cudaCheck(cudaError_t e, const char* what);
 
 // Launches a kernel that starts with dev::waitForPredecessor: it may be set up on the device while
 // its predecessor on the stream still runs, with its list entries read before the wait, in captured
-// graphs too. Large kernels that rely on non-aliasing arguments are launched the plain way. Measured
-// before and after, FP64, 48 cells: V(3,3) at P2 level 5 3.98 / 3.75 ms, 20 MINRES iterations at P2
-// level 4 98 / 91 ms, ten CG iterations on level 6 1.39 / 1.31 ms, transfers on level 8 1.31 / 1.12 ms.
+// graphs too. The wavefront SOR and the unfused phases, which rely on non-aliasing arguments, are
+// launched the plain way. Measured without and with it, FP64, 48 cells: V(3,3) at P2 level 5 3.98 / 3.65
+// ms, 20 MINRES iterations at P2 level 4 98 / 85 to 92 ms, ten CG iterations on level 6 1.39 / 1.29 ms.
 template <class... P, class... A>
 void launchNext(cudaStream_t stream, void (*kernel)(P...), unsigned grid, unsigned block, size_t smem, A&&... args) {
   cudaLaunchConfig_t cfg = {};
