@@ -24,8 +24,9 @@ constexpr int kBlock = 256;
 // set up. Behind the wait at most one kernel of a stream is set up ahead; with the trigger first a third
 // and a fourth could be, and their blocks held SMs that other streams' kernels could have used. Eight
 // workers serving 1000 solves, each on its stream: 0.176 GDoF/s with the trigger first, 0.213 behind
-// the wait; alone, V(3,3) at P2 level 5 on 48 cells takes 3.76 and 3.63 ms, the mixed-precision solve on
-// 27 cubes 10.41 and 10.16. The pointers are those to data that earlier kernels write; passing them
+// the wait (0.176 too with the halo gathers' trigger first and all others behind); alone, V(3,3) at P2
+// level 5 on 48 cells takes 3.76 and 3.63 ms, the mixed-precision solve on 27 cubes 10.41 and 10.16, an
+// apply on level 6 37.4 and 37.6 us, on one cube 15.4 and 14.4. The pointers are those to data that earlier kernels write; passing them
 // through here keeps the compiler from moving loads of read-only data in front of the wait.
 template <class P>
 __device__ __forceinline__ void heldBack(P& p) {

@@ -103,3 +103,25 @@ def test_given_back_when_memory_runs_out(gpu):
     finally:
         del filler
         torch.cuda.empty_cache()
+
+
+def test_release_while_another_thread_solves(gpu):
+    import threading
+    L = 3
+    ref = solve(storage(L), L, 5, 4)
+    stores, out = [storage(L), storage(L)], [[], []]
+
+    def work(k):
+        for _ in range(20):
+            out[k].append(solve(stores[k], L, 5, 4))
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(2)]
+    for t in threads:
+        t.start()
+    while any(t.is_alive() for t in threads):
+        for st in stores:
+            st.release_workspace()
+    for t in threads:
+        t.join()
+    assert [len(o) for o in out] == [20, 20]
+    assert all(np.array_equal(ref, x) for o in out for x in o)
